@@ -114,3 +114,15 @@ def test_pipeline_from_pcm_equals_pipeline_from_its_own_mel(pk, cuda):
     assert eng.longest_out_frames == eng.frames_out
     want_full = eng.transcribe_batch(torch.from_numpy(mel), [201, 201])
     assert all(np.array_equal(a, b) for a, b in zip(full, want_full))
+
+
+def test_both_tile_widths_give_the_same_bits(pk, cuda):
+    """Batches of 9472 frames or more take 32 frames per CTA, smaller ones 8 (ragged last tiles in both)."""
+    counts = [190000 - 1234 * u for u in range(8)]
+    pcm = torch.randn((8, 190000), generator=torch.Generator().manual_seed(4)).to(cuda) * 0.1
+    fe = pk.frontend.MelFrontend(F.hann_window(), F.triangular_filters(), cuda)
+    together, valid = fe.compute(pcm, torch.tensor(counts, dtype=torch.int32, device=cuda))
+    assert together.shape[0] * together.shape[1] >= 32 * 2 * 148
+    for u in range(8):
+        alone, v = fe.compute(pcm[u:u + 1].contiguous(), torch.tensor(counts[u:u + 1], dtype=torch.int32, device=cuda))
+        assert int(v[0]) == int(valid[u]) and torch.equal(alone[0], together[u])
