@@ -35,3 +35,21 @@ def test_subsampling_matches_oracle(pk, cuda, frames_list, precision):
         # (src/cuda/subsampling.rs:375); ours is far inside it
         assert np.max(np.abs(got - want)) <= max_abs
         assert nrmse(got, want) <= max_nrmse
+
+
+@pytest.mark.parametrize("precision", ["fp16", "fp8"])
+@pytest.mark.parametrize("frames_list", [[2501, 97, 2], [6000] * 3])
+def test_frames_per_cta_do_not_change_a_bit(pk, cuda, frames_list, precision):
+    """The first kernel walks 1 to 8 output frames per CTA depending on the batch: an utterance in a
+    batch (5 and 8 frames per CTA here) gives the bits of the utterance alone (1 to 6)."""
+    sub = pk.subsampling.Subsampling(pk.synth.subsampling_weights(2), cuda, precision=precision)
+    cap = max(frames_list)
+    batch = torch.zeros((len(frames_list), cap, 128), dtype=torch.float32, device=cuda)
+    for i, f in enumerate(frames_list):
+        batch[i, :f] = dev(pk.synth.mel_input(60 + i, f))
+    stride = pk.pipeline.seg_stride_for(pk.subsampling.output_frames(cap))
+    together = sub.run(batch, stride, mel_frames=torch.tensor(frames_list, dtype=torch.int32, device=cuda)).clone()
+    for i, f in enumerate(frames_list):
+        alone = sub.run(batch[i:i + 1, :f].contiguous(), stride)
+        rows = pk.subsampling.output_frames(f)
+        assert torch.equal(alone[:rows], together[i * stride:i * stride + rows]) and bool(alone[:rows].any())
