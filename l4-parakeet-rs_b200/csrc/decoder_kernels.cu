@@ -119,8 +119,8 @@ __device__ __forceinline__ float cache_scale(const float* absmax, int i) {
     return m > 0.0f ? __fdividef(m, 127.0f) : 1.0f;
 }
 __device__ __forceinline__ float cache_mul(float scale) { return __fdividef(scale, 127.0f); }
-__device__ __forceinline__ __half cache_code(__half w, float scale) {
-    return __int2half_rn(quantize_i8(__fdividef(__half2float(w), scale)));
+__device__ __forceinline__ int cache_code(__half w, float scale) {
+    return quantize_i8(__fdividef(__half2float(w), scale));
 }
 __device__ __forceinline__ float ref_sigmoid(float x) { return __fdividef(1.0f, 1.0f + __expf(-x)); }
 __device__ __forceinline__ float ref_tanh(float x) { return __tanhf(x); }
@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(kDecThreads, 1) tdt_greedy_kernel(const DecPar
                 const int coded = !cache ? -1 : (r >= 4 ? l : (l == 1 ? 2 : -1));
                 for (int c = tid; c < kHidden; c += kDecThreads) {
                     __half v = unit < kHidden ? src[c] : __float2half(0.0f);
-                    if (coded >= 0) v = cache_code(v, cscale[coded]);
+                    if (coded >= 0) v = __int2half_rn(cache_code(v, cscale[coded]));
                     dst[c] = v;
                 }
             }
@@ -1106,924 +1106,7 @@ __global__ void __launch_bounds__(kXThreads, 1) tdt_exchange_kernel(const DecPar
 }
 
 
-// ---------------------------------------------------------------------------
-// Cluster decoder.
-//
-// One thread-block cluster of 16 CTAs decodes the batch.  The phases of a round hand their
-// vectors to the peers through distributed shared memory: every CTA pushes its slice into all
-// 16 CTAs with st.async, which also credits the bytes to an mbarrier of the receiving CTA, and
-// each CTA waits (bounded) on its own mbarrier only.  An exchange costs one SM-to-SM hop
-// instead of the 2-3 us of global-memory slots polled by 148 CTAs.  The price: 16 CTAs
-// cannot hold the 8 MB of fp16 weights in shared memory, so
-//   - the joint rows (needed every round) stay resident,
-//   - the recurrent LSTM weights of layer 0 sit in tensor memory (unused otherwise: the MMAs
-//     here are mma.sync), written once per call and read back per k-step pair,
-//   - the prediction projection (and a second LSTM layer) is streamed from L2 on the rounds
-//     that follow a non-blank token, from a copy in "fragment order": the 16 bytes a lane
-//     needs for two k-steps of mma.m16n8k16 are contiguous, so a warp pulls 512 contiguous
-//     bytes per load straight into registers, several loads deep,
-//   - the input half of the LSTM, W_ih . embedding[token], is a table [1025, 2560] computed
-//     once per call by one GEMM; a round gathers 4 x 40 floats of the token's row per CTA.
-// Every CTA runs the same control flow on replicated utterance state.
-constexpr int kCl = 16;                          // CTAs per cluster
-constexpr int kClUnits = kHidden / kCl;          // 40 hidden units / prediction rows per CTA
-constexpr int kClJoint = 65;                     // joint rows per CTA (16 x 65 >= 1030)
-constexpr int kClThreads = 640;
-constexpr int kClWarps = kClThreads / 32;
-constexpr int kPartFloats = 6400;                // K-split partial sums of any of the three GEMMs
-
-// A [rows x K] weight slice split over the 20 warps as KG k-groups x NG row-groups; a warp
-// walks KP pairs of k-steps (32 columns each) over up to NT row tiles of 8 (TILES in total).
-template <int KG_, int NG_, int KP_, int NT_, int TILES_>
-struct FragShape {
-    static constexpr int KG = KG_, NG = NG_, KP = KP_, NT = NT_, kTiles = TILES_;
-    static constexpr int kRows = kTiles * 8;
-    // row pitch of the partial sums: = 8 (mod 32) floats, so the 8-byte stores of a half-warp
-    // (4 utterances x 4 column pairs) fall into 16 different bank pairs
-    static constexpr int kPitch = kRows + ((8 - kRows % 32) + 32) % 32;
-    static constexpr int kCols = KG * KP * 32;
-    static constexpr int kPerCta = KG * KP * kTiles * 32;   // uint4 per CTA
-    static_assert(KG * NG == kClWarps, "one (k-group, row-group) per warp");
-    static_assert(NG * NT >= kTiles && (NG - 1) * NT < kTiles, "row groups cover the tiles");
-    static_assert(KG * 8 * kPitch <= kPartFloats, "partials fit");
-    static_assert(kCols % kHidden == 0, "K = 640, or 1280 for [input | recurrent]");
-};
-using LstmShape = FragShape<4, 5, 5, 4, 20>;   // 160 gate rows x 640 (recurrent weights)
-using PredShape = FragShape<20, 1, 1, 5, 5>;   // 40 rows x 640
-using JointShape = FragShape<10, 2, 2, 5, 9>;  // 72 rows (65 used) x 640
-using Lstm1Shape = FragShape<4, 5, 10, 4, 20>; // second LSTM layer: 160 gate rows x 1280 ([h of layer 0 | own h])
-// Measured alternatives that were not kept: four k-groups for the prediction and joint GEMMs (fewer
-// partial sums to add, but longer dependent MMA chains: 8.7 instead of 8.0 us per round), and layer 0's
-// recurrent GEMM moved into the wait for the keys (it overlaps little: the keys arrive within a few
-// hundred cycles, and the token's table row is then waited for at the top of the next round).
-
-struct ClLayout { size_t base, lstm, pred, joint, xtab, lstm1, cache, total; };
-__host__ __device__ inline ClLayout cl_layout(int utts) {
-    ClLayout l;
-    const size_t a = dec_layout(utts).total, b = xch_layout(utts).total;
-    l.base = ((a > b ? a : b) + 255) / 256 * 256;
-    size_t off = l.base;
-    l.lstm = off; off += static_cast<size_t>(kCl) * LstmShape::kPerCta * 16;
-    l.pred = off; off += static_cast<size_t>(kCl) * PredShape::kPerCta * 16;
-    l.joint = off; off += static_cast<size_t>(kCl) * JointShape::kPerCta * 16;
-    l.xtab = off; off += static_cast<size_t>(kTokenOutputs) * kGates * 4;
-    l.lstm1 = off; off += static_cast<size_t>(kCl) * Lstm1Shape::kPerCta * 16;
-    l.cache = off; off += 256;        // max |w| of the three tensors of the INT8 cache
-    l.total = off;
-    return l;
-}
-
-enum : int { CLPACK_LSTM = 0, CLPACK_PRED = 1, CLPACK_JOINT = 2, CLPACK_LSTM_IH_HH = 3 };
-
-// dst[cta][kg][kp][tile][lane] = the B fragments (b0, b1) of k-steps 2*kp and 2*kp+1 of row tile
-// `tile`: lane (g = lane / 4, t = lane % 4) holds W[row g][k0 + 2t, +1, +8, +9] per k-step.
-// With `absmax` (long-request numerics) the values stored are the INT8 codes of the tensor,
-// scale index `scale_first` for w and `scale_second` for w_second.
-template <typename Shape, int Mode>
-__global__ void tdt_pack_kernel(uint4* dst, const __half* w, const __half* w_second, const float* absmax,
-                                int scale_first, int scale_second) {
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= kCl * Shape::kPerCta) return;
-    int rest = idx;
-    const int lane = rest % 32; rest /= 32;
-    const int tile = rest % Shape::kTiles; rest /= Shape::kTiles;
-    const int kp = rest % Shape::KP; rest /= Shape::KP;
-    const int kg = rest % Shape::KG; rest /= Shape::KG;
-    const int r = rest;
-    const int g = lane / 4, t = lane % 4;
-    const int n = tile * 8 + g;
-    const int k0 = (kg * Shape::KP + kp) * 32;
-    int row = -1;
-    if (Mode == CLPACK_LSTM || Mode == CLPACK_LSTM_IH_HH) row = (n % 4) * kHidden + r * kClUnits + n / 4;   // gate-major rows
-    else if (Mode == CLPACK_PRED) row = r * kClUnits + n;
-    else if (n < kClJoint && r * kClJoint + n < kJointRows) row = r * kClJoint + n;
-    auto pair = [&](int k) -> unsigned {
-        if (row < 0) return 0u;
-        // CLPACK_LSTM_IH_HH: columns 0..639 from w (input weights), 640..1279 from w_second (recurrent)
-        const bool second = Mode == CLPACK_LSTM_IH_HH && k >= kHidden;
-        const __half* src = second ? w_second + static_cast<size_t>(row) * kHidden + (k - kHidden)
-                                   : w + static_cast<size_t>(row) * kHidden + k;
-        __half v0 = src[0], v1 = src[1];
-        if (absmax != nullptr) {
-            const float scale = cache_scale(absmax, second ? scale_second : scale_first);
-            v0 = cache_code(v0, scale);
-            v1 = cache_code(v1, scale);
-        }
-        return static_cast<unsigned>(__half_as_ushort(v0)) | (static_cast<unsigned>(__half_as_ushort(v1)) << 16);
-    };
-    dst[idx] = make_uint4(pair(k0 + 2 * t), pair(k0 + 2 * t + 8), pair(k0 + 16 + 2 * t), pair(k0 + 16 + 2 * t + 8));
-}
-
-constexpr int kEncChunks = kHidden / 8;          // 16-byte chunks of one projected encoder row
-
-// Two LSTM layers: second committed state, its receive buffer, cell state, bias, barrier.
-template <int Layers> struct CSecondLayer {};
-template <> struct CSecondLayer<2> {
-    __half ah1[16][kAct];
-    __half hx1[16][kAct];
-    float cstate1[kMaxUtt][kClUnits];
-    float lstm_bias1[kClUnits][4];
-    uint64_t hbar1;
-};
-
-// With one layer the joint rows stay resident; with two they are streamed like the other
-// weights (the second layer's state needs the room).
-template <int Layers>
-struct CSmemT {
-    uint4 wj[Layers == 1 ? JointShape::kPerCta : 1];   // this CTA's joint rows in fragment order (resident)
-    __half ax[16][kAct];                  // joint input (hi rows 0-7, lo rows 8-15)
-    __half ah[16][kAct];                  // committed hidden state, all 640 units
-    __half hx[16][kAct];                  // fresh hidden state, written by all CTAs of the cluster
-    float pred[kMaxUtt][kHidden];         // prediction vectors, written by all CTAs of the cluster
-    float part[kPartFloats];              // [k-group][utterance][row] partial sums
-    __half enc[kMaxUtt][kHidden];         // projected encoder row of each utterance's current frame
-    float xg[kMaxUtt][kClUnits * 4];      // W_ih . embedding[last token] for this CTA's gate rows
-    float cstate[kMaxUtt][kClUnits];
-    alignas(16) __half stage_h[16][kClUnits];     // this CTA's slice of h (hi / lo) on its way out
-    alignas(16) __half stage_q[kMaxUtt][kClUnits];  // long-request numerics: its INT8 codes rne(h * 127)
-    float cache_mul[3];                           // scale / 127 of w_hh[0], w_hh[1], w_ih[1]
-    uint32_t tmem_base;                           // tensor memory holding layer 0's recurrent weights
-    alignas(16) float stage_p[kMaxUtt][kClUnits]; // this CTA's slice of the prediction vector
-    float lstm_bias[kClUnits][4];
-    float pred_bias[kClUnits];
-    float joint_bias[JointShape::kRows];
-    unsigned long long keys[2][kCl][kMaxUtt];   // [round parity][source CTA][utterance], written by peers
-    float dur[2][kMaxUtt][8];                   // [round parity][utterance][duration], written by the owner
-    uint64_t hbar, pbar, kbar[2];               // exchange mbarriers (count 1 + transaction bytes)
-    int frame[kMaxUtt], symbols[kMaxUtt], count[kMaxUtt], total_frames[kMaxUtt];
-    alignas(8) unsigned char valid[kMaxUtt];
-    alignas(8) unsigned char done[kMaxUtt];      // read as one 64-bit word: entries >= utts are 1
-    alignas(8) unsigned char need[kMaxUtt];      // !done && !valid
-    int abort;
-    CSecondLayer<Layers> second;
-#ifdef PK100_DEC_PROFILE
-    long long prof[16], last_stamp;       // per-phase cycle totals of thread 0
-#endif
-};
-using CSmem = CSmemT<1>;
-static_assert(sizeof(CSmemT<2>) <= 227 * 1024 && sizeof(CSmem) <= 227 * 1024, "cluster decoder state fits one CTA's shared memory");
-
-// Remote store that credits its bytes to an mbarrier of the destination CTA.  `addr` and `bar`
-// are shared::cluster addresses of the same CTA.
-__device__ __forceinline__ void st_async_v4(uint32_t addr, uint4 v, uint32_t bar) {
-    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
-                 ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(bar) : "memory");
-}
-__device__ __forceinline__ void st_async_b64(uint32_t addr, unsigned long long v, uint32_t bar) {
-    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];"
-                 ::"r"(addr), "l"(v), "r"(bar) : "memory");
-}
-__device__ __forceinline__ void st_async_b32(uint32_t addr, unsigned v, uint32_t bar) {
-    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];"
-                 ::"r"(addr), "r"(v), "r"(bar) : "memory");
-}
-__device__ __forceinline__ void cp_async_4(void* smem_dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(smem_dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_16(void* smem_dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
-__device__ __forceinline__ float fast_sigmoid(float x) { return __fdividef(1.0f, 1.0f + __expf(-x)); }
-__device__ __forceinline__ float fast_tanh(float x) { return 2.0f * fast_sigmoid(2.0f * x) - 1.0f; }
-
-// part[kg][u][row] = A(16 x 640, hi / lo rows) . W^T for this warp's k-group and row group.
-// The weight fragments run through a register ring `Depth` k-step pairs ahead of the MMAs;
-// frag_prefetch issues the loads of the first `Stages` pairs (weights do not depend on the
-// activations, so this can be done before the activations have arrived), frag_compute the rest.
-template <typename Shape, int Depth>
-struct FragRing { uint4 buf[Depth + 1][Shape::NT]; };
-
-template <typename Shape, bool Global>
-__device__ __forceinline__ uint4 frag_fetch(const uint4* w, int warp, int lane, int kp, int j) {
-    const int kg = warp / Shape::NG, ng = warp % Shape::NG;
-    const uint4* ptr = w + static_cast<size_t>(kg * Shape::KP + kp) * Shape::kTiles * 32 + (ng * Shape::NT + j) * 32 + lane;
-    return Global ? __ldg(ptr) : *ptr;
-}
-template <typename Shape>
-__device__ __forceinline__ bool frag_live(int warp, int j) {
-    return Shape::NG * Shape::NT == Shape::kTiles || (warp % Shape::NG) * Shape::NT + j < Shape::kTiles;
-}
-
-template <typename Shape, bool Global, int Depth, int First, int Stages>
-__device__ __forceinline__ void frag_prefetch(const uint4* w, FragRing<Shape, Depth>& ring, int warp, int lane) {
-#pragma unroll
-    for (int s = First; s < First + Stages && s < Shape::KP && s < Depth; ++s)
-#pragma unroll
-        for (int j = 0; j < Shape::NT; ++j)
-            if (frag_live<Shape>(warp, j)) ring.buf[s][j] = frag_fetch<Shape, Global>(w, warp, lane, s, j);
-}
-
-// `Loaded` = prologue stages already issued by frag_prefetch.  `HiOnly`: A has 8 rows (one per
-// utterance, no low-order rows), as for the integer codes of the long-request numerics.
-template <typename Shape, bool Global, int Depth, int Loaded, bool HiOnly = false>
-__device__ __forceinline__ void frag_compute(const uint4* w, const __half* a, float* part,
-                                             FragRing<Shape, Depth>& ring, int warp, int lane) {
-    constexpr int KP = Shape::KP, NT = Shape::NT;
-    const int kg = warp / Shape::NG, ng = warp % Shape::NG;
-    const int g = lane / 4, t = lane % 4;
-    frag_prefetch<Shape, Global, Depth, Loaded, Depth - Loaded>(w, ring, warp, lane);
-    float acc[NT][4];
-#pragma unroll
-    for (int j = 0; j < NT; ++j)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) acc[j][e] = 0.0f;
-    const __half* arow = HiOnly ? a + (lane % 8) * kAct + ((lane / 8) % 2) * 8 + kg * KP * 32
-                                : a + (lane % 16) * kAct + (lane / 16) * 8 + kg * KP * 32;
-#pragma unroll
-    for (int kp = 0; kp < KP; ++kp) {
-        if (kp + Depth < KP) {
-#pragma unroll
-            for (int j = 0; j < NT; ++j)
-                if (frag_live<Shape>(warp, j))
-                    ring.buf[(kp + Depth) % (Depth + 1)][j] = frag_fetch<Shape, Global>(w, warp, lane, kp + Depth, j);
-        }
-        unsigned a0[4], a1[4];
-        if constexpr (HiOnly) {
-            unsigned lo[2], hi[2];       // rows 0-7: columns k .. k+7 and k+8 .. k+15
-            dec_ldmatrix_x2(lo, arow + kp * 32);
-            dec_ldmatrix_x2(hi, arow + kp * 32 + 16);
-            a0[0] = lo[0]; a0[1] = 0u; a0[2] = lo[1]; a0[3] = 0u;
-            a1[0] = hi[0]; a1[1] = 0u; a1[2] = hi[1]; a1[3] = 0u;
-        } else {
-            dec_ldmatrix_x4(a0, arow + kp * 32);
-            dec_ldmatrix_x4(a1, arow + kp * 32 + 16);
-        }
-#pragma unroll
-        for (int j = 0; j < NT; ++j) {
-            if (!frag_live<Shape>(warp, j)) continue;
-            const uint4 b = ring.buf[kp % (Depth + 1)][j];
-            dec_mma(acc[j], a0, b.x, b.y);
-            dec_mma(acc[j], a1, b.z, b.w);
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < NT; ++j) {
-        if (!frag_live<Shape>(warp, j)) continue;
-        float* dst = part + (kg * 8 + g) * Shape::kPitch + (ng * NT + j) * 8 + 2 * t;
-        // hi row + lo row of utterance g
-        *reinterpret_cast<float2*>(dst) = HiOnly ? make_float2(acc[j][0], acc[j][1])
-                                                 : make_float2(acc[j][0] + acc[j][2], acc[j][1] + acc[j][3]);
-    }
-}
-
-// Layer 0's recurrent weights live in TENSOR MEMORY for the whole call: the 205 KB slice of a CTA
-// (160 gate rows x 640, fragment order) does not fit beside the joint rows in shared memory, but
-// the 256 KB of TMEM are otherwise unused by this kernel (its MMAs are register-operand
-// mma.sync).  A warp can reach the 32 lanes of its quadrant (warp % 4); the five warps of a quadrant
-// take 80 columns each: lane L, columns 16 * kp + 4 * j .. + 3 = the uint4 that lane L feeds to the
-// MMAs of k-step pair kp and row tile j.  One tcgen05.ld.32x32b.x16 per k-step pair replaces four
-// 512-byte loads from L2, which bounded this GEMM at the SM's L2 port (about 70 bytes per cycle).
-constexpr uint32_t kTmemColumns = 512;
-static_assert(LstmShape::NT == 4 && LstmShape::NG * LstmShape::NT == LstmShape::kTiles, "16 columns per k-step pair");
-static_assert((kClWarps / 4) * LstmShape::KP * 16 <= kTmemColumns && kClWarps % 4 == 0, "recurrent slice fits TMEM");
-
-__device__ __forceinline__ uint32_t lstm_tmem_addr(uint32_t base, int warp) {
-    return base + (static_cast<uint32_t>((warp % 4) * 32) << 16) + static_cast<uint32_t>((warp / 4) * LstmShape::KP * 16);
-}
-
-// set-up: this warp's fragments, global (fragment-ordered copy) -> TMEM
-__device__ __forceinline__ void lstm_tmem_fill(const uint4* w, uint32_t taddr, int warp, int lane) {
-#pragma unroll
-    for (int kp = 0; kp < LstmShape::KP; ++kp) {
-        uint32_t r[16];
-#pragma unroll
-        for (int j = 0; j < LstmShape::NT; ++j) {
-            const uint4 v = frag_fetch<LstmShape, true>(w, warp, lane, kp, j);
-            r[4 * j] = v.x; r[4 * j + 1] = v.y; r[4 * j + 2] = v.z; r[4 * j + 3] = v.w;
-        }
-        tmem_st_32x16(taddr + kp * 16, r);
-    }
-    tmem_st_wait();
-}
-
-// part[kg][u][row] = A . W_hh^T with the weights read from TMEM; the load of k-step pair kp + 1 is
-// in flight while the MMAs of pair kp issue
-template <bool HiOnly>
-__device__ __forceinline__ void lstm_compute_tmem(uint32_t taddr, const __half* a, float* part, int warp, int lane) {
-    using Shape = LstmShape;
-    constexpr int KP = Shape::KP, NT = Shape::NT;
-    const int kg = warp / Shape::NG, ng = warp % Shape::NG;
-    const int g = lane / 4, t = lane % 4;
-    float acc[NT][4];
-#pragma unroll
-    for (int j = 0; j < NT; ++j)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) acc[j][e] = 0.0f;
-    const __half* arow = HiOnly ? a + (lane % 8) * kAct + ((lane / 8) % 2) * 8 + kg * KP * 32
-                                : a + (lane % 16) * kAct + (lane / 16) * 8 + kg * KP * 32;
-    uint32_t wbuf[2][16];
-    tmem_ld_32x16(taddr, wbuf[0]);
-    tmem_ld_wait();
-#pragma unroll
-    for (int kp = 0; kp < KP; ++kp) {
-        if (kp + 1 < KP) tmem_ld_32x16(taddr + (kp + 1) * 16, wbuf[(kp + 1) % 2]);
-        unsigned a0[4], a1[4];
-        if constexpr (HiOnly) {
-            unsigned lo[2], hi[2];
-            dec_ldmatrix_x2(lo, arow + kp * 32);
-            dec_ldmatrix_x2(hi, arow + kp * 32 + 16);
-            a0[0] = lo[0]; a0[1] = 0u; a0[2] = lo[1]; a0[3] = 0u;
-            a1[0] = hi[0]; a1[1] = 0u; a1[2] = hi[1]; a1[3] = 0u;
-        } else {
-            dec_ldmatrix_x4(a0, arow + kp * 32);
-            dec_ldmatrix_x4(a1, arow + kp * 32 + 16);
-        }
-#pragma unroll
-        for (int j = 0; j < NT; ++j) {
-            const uint32_t* b = &wbuf[kp % 2][4 * j];
-            dec_mma(acc[j], a0, b[0], b[1]);
-            dec_mma(acc[j], a1, b[2], b[3]);
-        }
-        if (kp + 1 < KP) tmem_ld_wait();
-    }
-#pragma unroll
-    for (int j = 0; j < NT; ++j) {
-        float* dst = part + (kg * 8 + g) * Shape::kPitch + (ng * NT + j) * 8 + 2 * t;
-        *reinterpret_cast<float2*>(dst) = HiOnly ? make_float2(acc[j][0], acc[j][1])
-                                                 : make_float2(acc[j][0] + acc[j][2], acc[j][1] + acc[j][3]);
-    }
-}
-
-#ifdef PK100_DEC_PROFILE
-#define CL_STAMP(i) do { if (tid == 0) { const long long now__ = clock64(); sm.prof[i] += now__ - sm.last_stamp; sm.last_stamp = now__; } } while (0)
-#else
-#define CL_STAMP(i) do { } while (0)
-#endif
-
-// `Cache` = long-request numerics: recurrent weights (and layer 1's input weights) arrive as INT8
-// codes in the packed copies, `xtab` is rounded to fp16, and every hidden state also travels as
-// codes: rows 0-7 of ah / ah1 hold the committed codes (the A operand of the recurrent GEMMs),
-// rows 8-15 receive the fresh codes from the cluster.
-template <int Layers, bool Cache>
-__global__ void __launch_bounds__(kClThreads, 1)
-tdt_cluster_kernel(const DecParams p, const uint4* packed_lstm, const uint4* packed_pred,
-                   const uint4* packed_joint, const float* xtab, const uint4* packed_lstm1) {
-    extern __shared__ __align__(16) uint8_t cs_raw[];
-    CSmemT<Layers>& sm = *reinterpret_cast<CSmemT<Layers>*>(cs_raw);
-#ifdef PK100_DEC_PROFILE
-    if (threadIdx.x == 0) {
-        for (int i = 0; i < 16; ++i) sm.prof[i] = 0;
-        sm.last_stamp = clock64();
-    }
-#endif
-    const int tid = threadIdx.x, lane = tid % 32, warp = tid / 32;
-    const int r = static_cast<int>(cluster_ctarank());
-    const int U = p.utts;
-    volatile int* abort_flag = &sm.abort;
-
-    // ---- set-up: resident joint slice, biases, cleared state, first encoder rows
-    const uint4* wjoint = packed_joint + static_cast<size_t>(r) * JointShape::kPerCta;
-    if constexpr (Layers == 1) {
-        // (the long-request numerics read the joint rows from the caller's matrix instead)
-        if constexpr (!Cache)
-            for (int i = tid; i < JointShape::kPerCta; i += kClThreads) sm.wj[i] = __ldg(wjoint + i);
-    } else {
-        for (int i = tid; i < 16 * kAct; i += kClThreads) {
-            (&sm.second.ah1[0][0])[i] = __float2half(0.0f);
-            (&sm.second.hx1[0][0])[i] = __float2half(0.0f);
-        }
-        for (int i = tid; i < kMaxUtt * kClUnits; i += kClThreads) (&sm.second.cstate1[0][0])[i] = 0.0f;
-        if (tid < kClUnits * 4) {
-            const int slot = tid / 4, gt = tid % 4;
-            const int row = gt * kHidden + r * kClUnits + slot;
-            sm.second.lstm_bias1[slot][gt] = p.b_ih[1][row] + p.b_hh[1][row];
-        }
-        if (tid == 0) mbar_init(&sm.second.hbar1, 1);
-    }
-    for (int i = tid; i < 16 * kAct; i += kClThreads) {
-        (&sm.ax[0][0])[i] = __float2half(0.0f);
-        (&sm.ah[0][0])[i] = __float2half(0.0f);
-        (&sm.hx[0][0])[i] = __float2half(0.0f);
-    }
-    for (int i = tid; i < kMaxUtt * kHidden; i += kClThreads) {
-        (&sm.pred[0][0])[i] = 0.0f;
-        (&sm.enc[0][0])[i] = __float2half(0.0f);
-    }
-    for (int i = tid; i < kMaxUtt * kClUnits * 4; i += kClThreads) (&sm.xg[0][0])[i] = 0.0f;   // no token yet: zero input
-    for (int i = tid; i < kMaxUtt * kClUnits; i += kClThreads) (&sm.cstate[0][0])[i] = 0.0f;
-    if (tid < kClUnits * 4) {
-        const int slot = tid / 4, gt = tid % 4;
-        const int row = gt * kHidden + r * kClUnits + slot;
-        sm.lstm_bias[slot][gt] = p.b_ih[0][row] + p.b_hh[0][row];
-    }
-    if (tid < kClUnits) sm.pred_bias[tid] = p.b_pred[r * kClUnits + tid];
-    if (tid < 3) sm.cache_mul[tid] = (Cache && (tid == 0 || Layers == 2)) ? cache_mul(cache_scale(p.cache_absmax, tid)) : 0.0f;
-    if (tid < JointShape::kRows) {
-        const int row = r * kClJoint + tid;
-        sm.joint_bias[tid] = (tid < kClJoint && row < kJointRows) ? p.b_joint[row] : 0.0f;
-    }
-    if (tid < kMaxUtt) {
-        sm.frame[tid] = 0; sm.symbols[tid] = 0; sm.count[tid] = 0; sm.valid[tid] = 0;
-        sm.total_frames[tid] = tid < U ? min(p.frames[tid], p.seg_stride) : 0;   // never past the utterance's block
-        const bool done = tid >= U || p.frames[tid] <= 0 || !in_window(p, tid);
-        sm.done[tid] = done;
-        sm.need[tid] = !done;
-    }
-    for (int i = tid; i < 2 * kCl * kMaxUtt; i += kClThreads) (&sm.keys[0][0][0])[i] = 0ull;
-    for (int i = tid; i < 2 * kMaxUtt * 8; i += kClThreads) (&sm.dur[0][0][0])[i] = 0.0f;
-    if (tid == 0) {
-        mbar_init(&sm.hbar, 1);
-        mbar_init(&sm.pbar, 1);
-        mbar_init(&sm.kbar[0], 1);
-        mbar_init(&sm.kbar[1], 1);
-        sm.abort = 0;
-        fence_barrier_init();
-    }
-    if (warp == 1) {                 // one warp owns the tensor-memory allocation (all of it; one CTA per SM)
-        tmem_alloc(&sm.tmem_base, kTmemColumns);
-        tmem_relinquish();
-    }
-    tc_fence_before_sync();
-    __syncthreads();
-    tc_fence_after_sync();
-    if (warp < U && !sm.done[warp]) {
-        const __half* src = p.enc_proj + static_cast<size_t>(warp) * p.seg_stride * kHidden;
-        for (int c = lane; c < kEncChunks; c += 32) cp_async_16(&sm.enc[warp][c * 8], src + c * 8);
-    }
-    __syncthreads();
-    cluster_sync_all();      // every CTA's shared memory and mbarriers are ready before a peer writes
-
-    const uint4* wl = packed_lstm + static_cast<size_t>(r) * LstmShape::kPerCta;
-    const uint4* wp = packed_pred + static_cast<size_t>(r) * PredShape::kPerCta;
-    // sender role of this thread: peer CTA and two of the 80 16-byte items of a slice
-    const uint32_t peer = static_cast<uint32_t>(tid / kClUnits);
-    const int item0 = tid % kClUnits;
-    uint32_t hphase = 0, pphase = 0, kphase[2] = {0, 0};
-    [[maybe_unused]] uint32_t h1phase = 0;
-    [[maybe_unused]] const uint4* wl1 = packed_lstm1 + static_cast<size_t>(r) * Lstm1Shape::kPerCta;
-    // layer 0's recurrent weights: once from the fragment-ordered copy into tensor memory
-    const uint32_t lstm_taddr = lstm_tmem_addr(sm.tmem_base, warp);
-    lstm_tmem_fill(wl, lstm_taddr, warp, lane);
-
-    // LSTM cell of one (utterance, unit) from its four gate sums; stages h for the exchange
-    auto cell_update = [&](const float (&gsum)[4], float& cstate, int u, int slot) {
-        float h;
-        if constexpr (Cache) {
-            // the reference's approximations: h is rounded to 8 bits next, and a code that flips moves a gate
-            h = ref_lstm_cell(gsum, cstate);
-            sm.stage_q[u][slot] = __int2half_rn(quantize_i8(h * 127.0f));
-            // the prediction projection of this mode reads the fp32 state (decoder.cu:672-681), so the
-            // slice travels as fp32: stage_h viewed as float[8][40], the same bytes as a hi / lo pair
-            reinterpret_cast<float*>(&sm.stage_h[0][0])[u * kClUnits + slot] = h;
-        } else {
-            const float cell = fast_sigmoid(gsum[1]) * cstate + fast_sigmoid(gsum[0]) * fast_tanh(gsum[2]);
-            cstate = cell;
-            h = fast_sigmoid(gsum[3]) * fast_tanh(cell);
-            const __half hi = __float2half_rn(h);
-            sm.stage_h[u][slot] = hi;
-            sm.stage_h[u + 8][slot] = __float2half_rn(h - __half2float(hi));
-        }
-    };
-    // this CTA's staged slice of a hidden state -> `fresh` (hi / lo rows) of every CTA, and with
-    // Cache its codes -> rows 8-15 of `committed`; all bytes are credited to `bar_local` there
-    auto send_hidden = [&](__half (*fresh)[kAct], __half (*committed)[kAct], uint64_t* bar_local) {
-        const uint32_t bar = map_to_cta(smem_u32(bar_local), peer);
-#pragma unroll
-        for (int it = 0; it < 2; ++it) {
-            const int item = item0 + it * kClUnits;
-            if constexpr (Cache) {
-                // 0..79: 8 utterances x 10 chunks of 4 floats into `fresh` viewed as float[8][640]
-                const int u = item / 10, chunk = item % 10;
-                if (u < U && sm.need[u]) {
-                    const uint4 v = *reinterpret_cast<const uint4*>(
-                        reinterpret_cast<const float*>(&sm.stage_h[0][0]) + u * kClUnits + chunk * 4);
-                    float* dst = reinterpret_cast<float*>(&fresh[0][0]) + u * kHidden + r * kClUnits + chunk * 4;
-                    st_async_v4(map_to_cta(smem_u32(dst), peer), v, bar);
-                }
-            } else {
-                // 0..79: 16 rows x 5 chunks of 8 units
-                const int row = item / 5, chunk = item % 5;
-                const int u = row % 8;
-                if (u < U && sm.need[u]) {
-                    const uint4 v = *reinterpret_cast<const uint4*>(&sm.stage_h[row][chunk * 8]);
-                    st_async_v4(map_to_cta(smem_u32(&fresh[row][r * kClUnits + chunk * 8]), peer), v, bar);
-                }
-            }
-        }
-        if constexpr (Cache) {
-            const int u = item0 / 5, chunk = item0 % 5;
-            if (u < U && sm.need[u]) {
-                const uint4 v = *reinterpret_cast<const uint4*>(&sm.stage_q[u][chunk * 8]);
-                st_async_v4(map_to_cta(smem_u32(&committed[8 + u][r * kClUnits + chunk * 8]), peer), v, bar);
-            }
-        }
-    };
-    // bytes one stepping utterance contributes to a hidden-state exchange
-    constexpr uint32_t kHiddenTx = 2 * kHidden * 2 + (Cache ? kHidden * 2 : 0);
-    // the threads from `first` on make the fresh state the committed one
-    auto commit_hidden = [&](const __half (*fresh)[kAct], __half (*committed)[kAct], int first) {
-        constexpr int kRows = Cache ? 8 : 16;
-        for (int i = tid - first; i < kRows * kEncChunks; i += kClThreads - first) {
-            const int row = i / kEncChunks, c = i % kEncChunks;
-            const int u = row % 8;
-            if (u < U && sm.need[u]) {
-                const __half* src = Cache ? &committed[8 + row][c * 8] : &fresh[row][c * 8];
-                *reinterpret_cast<uint4*>(&committed[row][c * 8]) = *reinterpret_cast<const uint4*>(src);
-            }
-        }
-    };
-
-    unsigned round = 0;
-    while (true) {
-        const unsigned long long done8 = *reinterpret_cast<const unsigned long long*>(sm.done);
-        const unsigned long long need8 = *reinterpret_cast<const unsigned long long*>(sm.need);
-        // a wait that gave up raised sm.abort; it is read here, after the CTA barrier that ends a
-        // round, so every thread of the CTA takes the same branch
-        if (done8 == 0x0101010101010101ull || sm.abort != 0) break;
-        const int needs = __popcll(need8), lives = 8 - __popcll(done8);
-        CL_STAMP(0);
-
-        if (need8 != 0ull) {
-            // ---- LSTM: gates of this CTA's 40 units = table row + h . w_hh^T + bias
-            lstm_compute_tmem<Cache>(lstm_taddr, &sm.ah[0][0], sm.part, warp, lane);
-            cp_async_wait_all();             // table rows / encoder rows requested at the last decision
-            __syncthreads();
-            CL_STAMP(1);
-            if (tid < kMaxUtt * kClUnits) {
-                const int slot = tid % kClUnits, u = tid / kClUnits;
-                if (u < U && sm.need[u]) {
-                    const float4 x = *reinterpret_cast<const float4*>(&sm.xg[u][slot * 4]);
-                    float gsum[4];
-                    if constexpr (Cache) {
-                        // exact integer dot products; order of decoder.cu:636-637: (recurrent + bias) + table
-                        float rec[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-                        for (int kg = 0; kg < LstmShape::KG; ++kg) {
-                            const float4 v = *reinterpret_cast<const float4*>(
-                                &sm.part[(kg * 8 + u) * LstmShape::kPitch + slot * 4]);
-                            rec[0] += v.x; rec[1] += v.y; rec[2] += v.z; rec[3] += v.w;
-                        }
-                        const float mul = sm.cache_mul[0];
-                        const float xin[4] = {x.x, x.y, x.z, x.w};
-                        // the scaled recurrent sum is rounded BEFORE the bias is added, as in the reference
-                        // (decoder.cu:113, :626-640: products rounded per lane, then summed): a fused
-                        // multiply-add here parts from the reference kernel's tokens after a few hundred steps
-#pragma unroll
-                        for (int g4 = 0; g4 < 4; ++g4)
-                            gsum[g4] = __fadd_rn(__fadd_rn(__fmul_rn(rec[g4], mul), sm.lstm_bias[slot][g4]), xin[g4]);
-                    } else {
-                        gsum[0] = sm.lstm_bias[slot][0] + x.x; gsum[1] = sm.lstm_bias[slot][1] + x.y;
-                        gsum[2] = sm.lstm_bias[slot][2] + x.z; gsum[3] = sm.lstm_bias[slot][3] + x.w;
-#pragma unroll
-                        for (int kg = 0; kg < LstmShape::KG; ++kg) {
-                            const float4 v = *reinterpret_cast<const float4*>(
-                                &sm.part[(kg * 8 + u) * LstmShape::kPitch + slot * 4]);
-                            gsum[0] += v.x; gsum[1] += v.y; gsum[2] += v.z; gsum[3] += v.w;
-                        }
-                    }
-                    cell_update(gsum, sm.cstate[u][slot], u, slot);
-                }
-            }
-            if (tid == 0) mbar_arrive_expect_tx(&sm.hbar, static_cast<uint32_t>(needs) * kHiddenTx);
-            __syncthreads();
-            CL_STAMP(2);
-            send_hidden(sm.hx, sm.ah, &sm.hbar);     // h slice -> every CTA's hx (and codes)
-            // the prediction weights of this warp are requested while the hidden state travels
-            [[maybe_unused]] FragRing<PredShape, 1> pred_ring;
-            if constexpr (Layers == 1 && !Cache) frag_prefetch<PredShape, true, 1, 0, 1>(wp, pred_ring, warp, lane);
-            mbar_wait_bounded(&sm.hbar, hphase, abort_flag);
-            hphase ^= 1u;
-            CL_STAMP(3);
-            const __half (*top_fresh)[kAct] = sm.hx;      // fresh hidden state of the top layer
-            __half (*top_committed)[kAct] = sm.ah;
-            if constexpr (Layers == 2) {
-                // ---- second LSTM layer: gates = [fresh h of layer 0 | own h] . [w_ih | w_hh]^T + bias
-                {
-                    FragRing<Lstm1Shape, 2> ring1;
-                    const int kg = warp / Lstm1Shape::NG;
-                    // k-groups 0, 1 read the 640 columns of hx (Cache: the fresh codes of layer 0 in
-                    // rows 8-15 of ah), groups 2, 3 those of ah1
-                    const __half* a = kg < 2 ? (Cache ? &sm.ah[8][0] : &sm.hx[0][0]) : &sm.second.ah1[0][0] - kHidden;
-                    frag_compute<Lstm1Shape, true, 2, 0, Cache>(wl1, a, sm.part, ring1, warp, lane);
-                }
-                __syncthreads();
-                if (tid < kMaxUtt * kClUnits) {
-                    const int slot = tid % kClUnits, u = tid / kClUnits;
-                    if (u < U && sm.need[u]) {
-                        float gsum[4] = {sm.second.lstm_bias1[slot][0], sm.second.lstm_bias1[slot][1],
-                                         sm.second.lstm_bias1[slot][2], sm.second.lstm_bias1[slot][3]};
-                        if constexpr (Cache) {
-                            // k-groups 0, 1: input codes (scale of w_ih[1]); 2, 3: recurrent codes;
-                            // decoder.cu:655-663 adds the bias last
-                            float in[4] = {0.0f, 0.0f, 0.0f, 0.0f}, rec[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-                            for (int kg = 0; kg < Lstm1Shape::KG; ++kg) {
-                                const float4 v = *reinterpret_cast<const float4*>(
-                                    &sm.part[(kg * 8 + u) * Lstm1Shape::kPitch + slot * 4]);
-                                float (&dst)[4] = kg < 2 ? in : rec;
-                                dst[0] += v.x; dst[1] += v.y; dst[2] += v.z; dst[3] += v.w;
-                            }
-#pragma unroll
-                            // rounded recurrent product first, the input product fused onto it (decoder.cu:113, :660)
-                            for (int g4 = 0; g4 < 4; ++g4)
-                                gsum[g4] = __fadd_rn(fmaf(in[g4], sm.cache_mul[2], __fmul_rn(rec[g4], sm.cache_mul[1])), gsum[g4]);
-                        } else {
-#pragma unroll
-                            for (int kg = 0; kg < Lstm1Shape::KG; ++kg) {
-                                const float4 v = *reinterpret_cast<const float4*>(
-                                    &sm.part[(kg * 8 + u) * Lstm1Shape::kPitch + slot * 4]);
-                                gsum[0] += v.x; gsum[1] += v.y; gsum[2] += v.z; gsum[3] += v.w;
-                            }
-                        }
-                        cell_update(gsum, sm.second.cstate1[u][slot], u, slot);
-                    }
-                } else {
-                    // meanwhile: commit the fresh state of layer 0
-                    commit_hidden(sm.hx, sm.ah, kMaxUtt * kClUnits);
-                }
-                if (tid == 0) mbar_arrive_expect_tx(&sm.second.hbar1, static_cast<uint32_t>(needs) * kHiddenTx);
-                __syncthreads();
-                send_hidden(sm.second.hx1, sm.second.ah1, &sm.second.hbar1);
-                if constexpr (!Cache) frag_prefetch<PredShape, true, 1, 0, 1>(wp, pred_ring, warp, lane);
-                mbar_wait_bounded(&sm.second.hbar1, h1phase, abort_flag);
-                h1phase ^= 1u;
-                top_fresh = sm.second.hx1;
-                top_committed = sm.second.ah1;
-            }
-            if constexpr (Cache) {
-                // ---- prediction projection in fp32 on the fp32 state, in the reference's summation
-                // order (decoder.cu:672-684): lane l takes elements 2l + 64w, w = 0..9, as one fma
-                // chain that starts from the bias in lane 0, then the shuffle tree of warp_sum
-                const float* hf = reinterpret_cast<const float*>(&top_fresh[0][0]);
-#pragma unroll
-                for (int it = 0; it < kClUnits / kClWarps; ++it) {
-                    const int n = warp + it * kClWarps;
-                    const uint32_t* wrow = reinterpret_cast<const uint32_t*>(
-                        p.w_pred + static_cast<size_t>(r * kClUnits + n) * kHidden);
-                    uint32_t words[10];
-#pragma unroll
-                    for (int w = 0; w < 10; ++w) words[w] = __ldg(wrow + lane + 32 * w);
-                    // the utterances run side by side: eight independent chains, each in its own order
-                    float sum[kMaxUtt];
-#pragma unroll
-                    for (int u = 0; u < kMaxUtt; ++u) sum[u] = lane == 0 ? sm.pred_bias[n] : 0.0f;
-#pragma unroll
-                    for (int w = 0; w < 10; ++w) {
-                        const float2 wv = __half22float2(*reinterpret_cast<const __half2*>(&words[w]));
-#pragma unroll
-                        for (int u = 0; u < kMaxUtt; ++u) {
-                            if (((need8 >> (8 * u)) & 1ull) == 0ull) continue;
-                            const float2 hv = *reinterpret_cast<const float2*>(hf + u * kHidden + 2 * lane + 64 * w);
-                            sum[u] = fmaf(wv.x, hv.x, sum[u]);
-                            sum[u] = fmaf(wv.y, hv.y, sum[u]);
-                        }
-                    }
-#pragma unroll
-                    for (int u = 0; u < kMaxUtt; ++u) {
-                        if (((need8 >> (8 * u)) & 1ull) == 0ull) continue;
-#pragma unroll
-                        for (int off = 16; off > 0; off /= 2) sum[u] += __shfl_down_sync(0xffffffffu, sum[u], off);
-                        if (lane == 0) sm.stage_p[u][n] = sum[u];
-                    }
-                }
-                CL_STAMP(4);
-                commit_hidden(top_fresh, top_committed, 0);
-            } else {
-            // ---- prediction projection of the new state (A operand: the fresh rows of the top layer)
-            frag_compute<PredShape, true, 1, 1>(wp, &top_fresh[0][0], sm.part, pred_ring, warp, lane);
-            __syncthreads();
-            CL_STAMP(4);
-            if (tid < kMaxUtt * kClUnits) {
-                const int row = tid % kClUnits, u = tid / kClUnits;
-                if (u < U && sm.need[u]) {
-                    float v = sm.pred_bias[row];
-#pragma unroll
-                    for (int kg = 0; kg < PredShape::KG; ++kg) v += sm.part[(kg * 8 + u) * PredShape::kPitch + row];
-                    sm.stage_p[u][row] = v;
-                }
-            } else {
-                // meanwhile the other threads commit the fresh hidden state for the next LSTM step
-                commit_hidden(top_fresh, top_committed, kMaxUtt * kClUnits);
-            }
-            }
-            if (tid == 0) mbar_arrive_expect_tx(&sm.pbar, static_cast<uint32_t>(needs) * kHidden * 4);
-            __syncthreads();
-            CL_STAMP(5);
-            {   // prediction slice (10 chunks of 4 floats per utterance) -> every CTA's pred
-                const uint32_t bar = map_to_cta(smem_u32(&sm.pbar), peer);
-#pragma unroll
-                for (int it = 0; it < 2; ++it) {
-                    const int item = item0 + it * kClUnits;         // 0..79
-                    const int u = item / 10, chunk = item % 10;
-                    if (u < U && sm.need[u]) {
-                        const uint4 v = *reinterpret_cast<const uint4*>(&sm.stage_p[u][chunk * 4]);
-                        st_async_v4(map_to_cta(smem_u32(&sm.pred[u][r * kClUnits + chunk * 4]), peer), v, bar);
-                    }
-                }
-            }
-            mbar_wait_bounded(&sm.pbar, pphase, abort_flag);
-            pphase ^= 1u;
-            CL_STAMP(6);
-        } else {
-            cp_async_wait_all();
-            __syncthreads();
-        }
-
-        // ---- joint input relu(enc + pred), one thread per column
-        {
-            float v[kMaxUtt];
-#pragma unroll
-            for (int u = 0; u < kMaxUtt; ++u) {
-                const bool live = ((done8 >> (8 * u)) & 1ull) == 0ull;
-                v[u] = live ? fmaxf(__half2float(sm.enc[u][tid]) + sm.pred[u][tid], 0.0f) : 0.0f;
-            }
-#pragma unroll
-            for (int u = 0; u < kMaxUtt; ++u) {
-                if (((done8 >> (8 * u)) & 1ull) != 0ull) continue;
-                if constexpr (Cache) reinterpret_cast<float*>(&sm.ax[0][0])[u * kHidden + tid] = v[u];   // ax as float[8][640]
-                else split_store(sm.ax, u, tid, v[u]);
-            }
-        }
-        __syncthreads();
-        CL_STAMP(7);
-        if constexpr (Cache) {
-            // joint rows in fp32 in the reference's summation order (decoder.cu:697-713): one row per
-            // half-warp, half-lane l takes elements 2l + 32s, s = 0..19, as one fma chain that starts from
-            // the bias in half-lane 0, then the shuffle tree of half_warp_sum.  The score (bias included)
-            // lands in the k-group-0 slot of `part`.  Rows come from the caller's [1030, 640] matrix.
-            const float* xf = reinterpret_cast<const float*>(&sm.ax[0][0]);
-            const int hw = tid / 16, hl = tid % 16;
-#pragma unroll 1
-            for (int it = 0; it < 2; ++it) {
-                const int n = hw + it * (kClThreads / 16);
-                const int row = r * kClJoint + n;
-                const bool owned = n < kClJoint && row < kJointRows;
-                const uint32_t* wrow = reinterpret_cast<const uint32_t*>(
-                    p.w_joint + static_cast<size_t>(owned ? row : 0) * kHidden);
-                uint32_t words[20];
-#pragma unroll
-                for (int st = 0; st < 20; ++st) words[st] = __ldg(wrow + hl + 16 * st);
-                const float bias = owned ? sm.joint_bias[n] : 0.0f;
-                float score[kMaxUtt];
-#pragma unroll
-                for (int u = 0; u < kMaxUtt; ++u) score[u] = hl == 0 ? bias : 0.0f;
-#pragma unroll
-                for (int st = 0; st < 20; ++st) {
-                    const float2 wv = __half22float2(*reinterpret_cast<const __half2*>(&words[st]));
-#pragma unroll
-                    for (int u = 0; u < kMaxUtt; ++u) {
-                        if (((done8 >> (8 * u)) & 1ull) != 0ull) continue;
-                        const float2 xv = *reinterpret_cast<const float2*>(xf + u * kHidden + 2 * hl + 32 * st);
-                        score[u] = fmaf(wv.x, xv.x, score[u]);
-                        score[u] = fmaf(wv.y, xv.y, score[u]);
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < kMaxUtt; ++u) {
-                    if (((done8 >> (8 * u)) & 1ull) != 0ull) continue;
-#pragma unroll
-                    for (int off = 8; off > 0; off /= 2) score[u] += __shfl_down_sync(0xffffffffu, score[u], off, 16);
-                    if (hl == 0 && owned) sm.part[u * JointShape::kPitch + n] = score[u];
-                }
-            }
-        } else {
-            FragRing<JointShape, 1> joint_ring;
-            if constexpr (Layers == 1) frag_compute<JointShape, false, 1, 0>(sm.wj, &sm.ax[0][0], sm.part, joint_ring, warp, lane);
-            else frag_compute<JointShape, true, 1, 0>(wjoint, &sm.ax[0][0], sm.part, joint_ring, warp, lane);
-        }
-        __syncthreads();
-        CL_STAMP(8);
-        const int par = static_cast<int>(round & 1u);
-        const uint32_t kbar_local = smem_u32(&sm.kbar[par]);
-        if (tid == 0) mbar_arrive_expect_tx(&sm.kbar[par], static_cast<uint32_t>(lives) * (kCl * 8 + kDurations * 4));
-        // warp u: this CTA's 65 rows of utterance u -> its best key, sent by the same warp (a version
-        // with two warps per utterance, a merge through shared memory and a CTA barrier before the
-        // send cost 0.3 us more per round)
-        if (warp < kMaxUtt) {
-            const int u = warp;
-            unsigned long long best = 0ull;
-            const bool live_u = u < U && !sm.done[u];
-            // three passes for every lane (the third covers row 64), so the warp stays converged up
-            // to the shuffle reduction
-#pragma unroll
-            for (int it = 0; it < 3; ++it) {
-                const int n = lane + it * 32;
-                const int row = r * kClJoint + n;
-                if (live_u && n < kClJoint && row < kJointRows) {
-                    float total;
-                    if constexpr (Cache) {
-                        total = sm.part[u * JointShape::kPitch + n];      // finished score of the fp32 joint
-                    } else {
-                        total = sm.joint_bias[n];
-#pragma unroll
-                        for (int kg = 0; kg < JointShape::KG; ++kg) total += sm.part[(kg * 8 + u) * JointShape::kPitch + n];
-                    }
-                    if (row >= kTokenOutputs) {
-                        const uint32_t local = smem_u32(&sm.dur[par][u][row - kTokenOutputs]);
-                        for (uint32_t d = 0; d < kCl; ++d)
-                            st_async_b32(map_to_cta(local, d), __float_as_uint(total), map_to_cta(kbar_local, d));
-                    } else if (total == total) {          // NaN never wins
-                        float sc = total;
-                        if (sc == 0.0f) sc = 0.0f;        // canonicalise -0
-                        const unsigned bits = __float_as_uint(sc);
-                        const unsigned ordered = (bits & 0x80000000u) ? ~bits : (bits ^ 0x80000000u);
-                        const unsigned long long key = (static_cast<unsigned long long>(ordered) << 32) |
-                                                       (static_cast<unsigned long long>(2047 - row) << 21) | 1ull;
-                        best = key > best ? key : best;
-                    }
-                }
-            }
-            __syncwarp();
-#pragma unroll
-            for (int off = 16; off > 0; off /= 2) {
-                const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, off);
-                best = other > best ? other : best;
-            }
-            // ---- this CTA's best row of utterance u -> every CTA of the cluster
-            if (live_u && lane < kCl) {
-                // a CTA whose rows all produced NaN still publishes a (losing) key
-                if (best == 0ull) best = (static_cast<unsigned long long>(2047 - kTokenOutputs) << 21) | 1ull;
-                st_async_b64(map_to_cta(smem_u32(&sm.keys[par][r][u]), static_cast<uint32_t>(lane)), best,
-                             map_to_cta(kbar_local, static_cast<uint32_t>(lane)));
-            }
-        }
-        CL_STAMP(9);
-        mbar_wait_bounded(&sm.kbar[par], kphase[par], abort_flag);
-        kphase[par] ^= 1u;
-        CL_STAMP(10);
-
-        // ---- decision (replicated in every CTA): warp u decides utterance u
-        if (warp < U && !sm.done[warp]) {
-            const int u = warp;
-            unsigned long long best = lane < kCl ? sm.keys[par][lane][u] : 0ull;
-#pragma unroll
-            for (int off = 16; off > 0; off /= 2) {
-                const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, off);
-                best = other > best ? other : best;
-            }
-            int token = 2047 - static_cast<int>((best >> 21) & 0x7FFull);
-            // keys not delivered (a wait gave up), or every token score of the round was NaN: a
-            // blank; the second case is reported as status bit 4
-            if (token > kBlank) {
-                token = kBlank;
-                if (r == 0 && lane == 0 && sm.abort == 0 && p.status != nullptr) atomicOr(p.status, 4);
-            }
-            // first strict maximum of the five duration logits
-            int duration = 0;
-            float best_dur = sm.dur[par][u][0];
-#pragma unroll
-            for (int i = 1; i < kDurations; ++i) {
-                const float v = sm.dur[par][u][i];
-                if (v > best_dur) { best_dur = v; duration = i; }
-            }
-            int frame = sm.frame[u] + duration;
-            int symbols = sm.symbols[u] + 1;
-            if (duration != 0 || symbols == kMaxSymbols) {
-                if (duration == 0) frame += 1;
-                symbols = 0;
-            }
-            const bool done = frame >= sm.total_frames[u];
-            // requests for the next round, in flight while the state is updated: the token's
-            // table row (this CTA's 4 x 40 gate inputs) and the encoder row of the new frame
-            if (token != kBlank) {
-                const float* row = xtab + static_cast<size_t>(token) * kGates + r * kClUnits;
-                for (int n = lane; n < kClUnits * 4; n += 32) cp_async_4(&sm.xg[u][n], row + (n % 4) * kHidden + n / 4);
-            }
-            if (!done && frame != sm.frame[u]) {
-                const __half* src = p.enc_proj + (static_cast<size_t>(u) * p.seg_stride + frame) * kHidden;
-                for (int c = lane; c < kEncChunks; c += 32) cp_async_16(&sm.enc[u][c * 8], src + c * 8);
-            }
-            __syncwarp();
-            if (lane == 0) {
-                if (sm.need[u]) sm.valid[u] = 1;        // this round's prediction is now current
-                if (token != kBlank) {
-                    if (r == 0 && sm.count[u] < p.max_tokens) {
-                        p.tokens[static_cast<size_t>(u) * p.max_tokens + sm.count[u]] = token;
-                        if (p.durations_out != nullptr)
-                            p.durations_out[static_cast<size_t>(u) * p.max_tokens + sm.count[u]] = duration;
-                    }
-                    sm.count[u] += 1;
-                    sm.valid[u] = 0;
-                }
-                sm.frame[u] = frame;
-                sm.symbols[u] = symbols;
-                sm.done[u] = done;
-                sm.need[u] = !done && !sm.valid[u];
-            }
-        }
-        __syncthreads();
-        CL_STAMP(11);
-        round += 1;
-    }
-    cp_async_wait_all();
-    tc_fence_before_sync();
-    __syncthreads();
-    if (warp == 1) {
-        tc_fence_after_sync();
-        tmem_dealloc(sm.tmem_base, kTmemColumns);
-    }
-    cluster_sync_all();      // no CTA leaves while a peer may still address its shared memory
-#ifdef PK100_DEC_PROFILE
-    if (r == 0 && tid == 0)
-        for (int i = 0; i < 16; ++i)
-            reinterpret_cast<volatile long long*>(p.workspace + xch_layout(U).abort)[2 + i] = sm.prof[i];
-#endif
-    if (r == 0 && tid < U && in_window(p, tid)) p.counts[tid] = min(sm.count[tid], p.max_tokens);
-    if (r == 0 && tid == 0) reinterpret_cast<volatile int*>(p.workspace + xch_layout(U).abort)[2] = static_cast<int>(round);
-    if (sm.abort != 0 && tid == 0 && p.status != nullptr) atomicExch(p.status, 2);
-}
+#include "decoder_cluster.cuh"
 
 }  // namespace pk100
 
@@ -2331,84 +1414,69 @@ namespace {
 
 // Can this device run a 16-CTA cluster of the cluster decoder?  Asked once per device and
 // kernel variant (one or two LSTM layers).
-template <int Layers, bool Cache>
-bool cluster_decoder_available(int* capacity = nullptr) {
-    static int cached[64] = {0};      // 0 = unknown, 1 = yes, 2 = no
-    static int resident[64] = {0};    // clusters of this kernel the device holds at once
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
-    if (cached[dev] != 0) {
-        if (capacity != nullptr) *capacity = resident[dev];
-        return cached[dev] == 1;
+// Calls f with the kernel for (layers, numerics, utterances of the call) and its shared-memory bytes.
+template <typename F>
+auto with_cluster_kernel(int layers, bool cache, int utterances, F&& f) {
+#define PK_PICK(L, C, N) return f(tdt_cluster_kernel<L, C, N>, static_cast<int>(sizeof(CSmem<L, C, N>)))
+    if (layers == 1) {
+        if (cache) { if (utterances <= 4) PK_PICK(1, true, 4); PK_PICK(1, true, 8); }
+        if (utterances <= 4) PK_PICK(1, false, 4);
+        PK_PICK(1, false, 8);
     }
-    bool ok = false;
-    do {
-        int max_smem = 0;
-        cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-        if (sizeof(CSmemT<Layers>) > static_cast<size_t>(max_smem)) break;
-        if (cudaFuncSetAttribute(tdt_cluster_kernel<Layers, Cache>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(sizeof(CSmemT<Layers>))) != cudaSuccess) break;
-        if (cudaFuncSetAttribute(tdt_cluster_kernel<Layers, Cache>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-            cudaSuccess) break;
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(kCl);
-        cfg.blockDim = dim3(kClThreads);
-        cfg.dynamicSmemBytes = sizeof(CSmemT<Layers>);
-        cudaLaunchAttribute attr{};
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = kCl;
-        attr.val.clusterDim.y = 1;
-        attr.val.clusterDim.z = 1;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
-        int clusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&clusters, tdt_cluster_kernel<Layers, Cache>, &cfg) != cudaSuccess) break;
-        ok = clusters >= 1;
-        resident[dev] = clusters;
-    } while (false);
-    cudaGetLastError();
-    cached[dev] = ok ? 1 : 2;
-    if (capacity != nullptr) *capacity = resident[dev];
-    return ok;
+    if (cache) { if (utterances <= 4) PK_PICK(2, true, 4); PK_PICK(2, true, 8); }
+    if (utterances <= 4) PK_PICK(2, false, 4);
+    PK_PICK(2, false, 8);
+#undef PK_PICK
 }
 
-bool cluster_decoder_available_for(int layers, bool cache) {
-    if (layers == 1) return cache ? cluster_decoder_available<1, true>() : cluster_decoder_available<1, false>();
-    if (layers == 2) return cache ? cluster_decoder_available<2, true>() : cluster_decoder_available<2, false>();
-    return false;
-}
-
-}  // namespace
-
-extern "C" int pk100_tdt_cluster_capacity(int lstm_layers) {
-    int clusters = 0;
-    bool ok = false;
-    if (lstm_layers == 1) ok = cluster_decoder_available<1, false>(&clusters);
-    else if (lstm_layers == 2) ok = cluster_decoder_available<2, false>(&clusters);
-    return ok ? clusters : 0;
-}
-
-namespace {
-
-template <int Layers, bool Cache>
-cudaError_t launch_cluster_kernel(cudaStream_t stream, const DecParams& p, const uint4* lstm, const uint4* pred,
-                                  const uint4* joint, const float* xtab, const uint4* lstm1) {
+cudaLaunchConfig_t cluster_config(cudaLaunchAttribute& attr, int smem, cudaStream_t stream) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(kCl);
     cfg.blockDim = dim3(kClThreads);
-    cfg.dynamicSmemBytes = sizeof(CSmemT<Layers>);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeClusterDimension;
     attr.val.clusterDim.x = kCl;
     attr.val.clusterDim.y = 1;
     attr.val.clusterDim.z = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, tdt_cluster_kernel<Layers, Cache>, p, lstm, pred, joint, xtab, lstm1);
+    return cfg;
+}
+
+// Can the current device host this variant?  Sets the kernel's attributes on the first call per device.
+bool cluster_decoder_available_for(int layers, bool cache, int utterances = 1, int* capacity = nullptr) {
+    static std::atomic<int> known[64][8];      // 0 = unknown, else 1 + clusters the device holds at once
+    int dev = 0;
+    if (layers < 1 || layers > 2 || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+    std::atomic<int>& slot = known[dev][(layers - 1) * 4 + (cache ? 2 : 0) + (utterances > 4 ? 1 : 0)];
+    if (slot.load() == 0) {
+        const int clusters = with_cluster_kernel(layers, cache, utterances, [&](auto kernel, int smem) {
+            int max_smem = 0, n = 0;
+            cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+            cudaLaunchAttribute attr{};
+            const cudaLaunchConfig_t cfg = cluster_config(attr, smem, nullptr);
+            if (smem > max_smem ||
+                cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+                cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+                cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess)
+                n = 0;
+            return n;
+        });
+        cudaGetLastError();
+        slot.store(1 + clusters);
+    }
+    const int clusters = slot.load() - 1;
+    if (capacity != nullptr) *capacity = clusters;
+    return clusters >= 1;
 }
 
 }  // namespace
+
+extern "C" int pk100_tdt_cluster_capacity(int lstm_layers) {
+    int clusters = 0;
+    return cluster_decoder_available_for(lstm_layers, false, 1, &clusters) ? clusters : 0;
+}
 
 namespace {
 int decode_cluster(void* stream_v, const pk100_decoder_weights* w, const void* enc_proj,
@@ -2421,7 +1489,7 @@ int decode_cluster(void* stream_v, const pk100_decoder_weights* w, const void* e
     if (utterances == 0) return PK100_OK;
     if (utterances < 0 || seg_stride <= 0 || max_tokens <= 0) return PK100_ERR_SHAPE;
     if (utterances > kMaxUtt) return PK100_ERR_LIMIT;
-    if (!cluster_decoder_available_for(w->layers, cache)) return PK100_ERR_UNSUPPORTED;
+    if (!cluster_decoder_available_for(w->layers, cache, utterances)) return PK100_ERR_UNSUPPORTED;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
     const ClLayout lay = cl_layout(utterances);
     uint8_t* ws = static_cast<uint8_t*>(workspace);
@@ -2435,22 +1503,27 @@ int decode_cluster(void* stream_v, const pk100_decoder_weights* w, const void* e
     uint4* packed_joint = reinterpret_cast<uint4*>(ws + lay.joint);
     uint4* packed_lstm1 = reinterpret_cast<uint4*>(ws + lay.lstm1);
     float* xtab = reinterpret_cast<float*>(ws + lay.xtab);
-    const __half* w_hh = static_cast<const __half*>(w->w_hh[0]);
     const __half* w_pred = static_cast<const __half*>(w->w_pred);
     const __half* w_joint = static_cast<const __half*>(w->w_joint);
     // weights -> fragment order (they may change between calls, so this is done every call)
-    tdt_pack_kernel<LstmShape, CLPACK_LSTM><<<(kCl * LstmShape::kPerCta + 255) / 256, 256, 0, stream>>>(
-        packed_lstm, w_hh, nullptr, absmax, 0, 0);
-    tdt_pack_kernel<PredShape, CLPACK_PRED><<<(kCl * PredShape::kPerCta + 255) / 256, 256, 0, stream>>>(
-        packed_pred, w_pred, nullptr, nullptr, 0, 0);
-    tdt_pack_kernel<JointShape, CLPACK_JOINT><<<(kCl * JointShape::kPerCta + 255) / 256, 256, 0, stream>>>(
-        packed_joint, w_joint, nullptr, nullptr, 0, 0);
-    pk100_count_launch();
-    pk100_count_launch();
-    pk100_count_launch();
+    const size_t slice1 = static_cast<size_t>(kCl) * Lstm1Split::kPerCta;
+    auto blocks = [](int per_cta) { return (kCl * per_cta + 255) / 256; };
+    auto gates = [&](uint4* dst, const void* src, bool second, int scale) {
+        const __half* m = static_cast<const __half*>(src);
+        if (cache) tdt_pack_kernel<CodeSplit, CLPACK_GATES, true><<<blocks(CodeSplit::kPerCta), 256, 0, stream>>>(dst, m, absmax, scale);
+        else if (second) tdt_pack_kernel<Lstm1Split, CLPACK_GATES, false><<<blocks(Lstm1Split::kPerCta), 256, 0, stream>>>(dst, m, nullptr, 0);
+        else tdt_pack_kernel<LstmSplit, CLPACK_GATES, false><<<blocks(LstmSplit::kPerCta), 256, 0, stream>>>(dst, m, nullptr, 0);
+        pk100_count_launch();
+    };
+    gates(packed_lstm, w->w_hh[0], false, 0);
     if (w->layers == 2) {
-        tdt_pack_kernel<Lstm1Shape, CLPACK_LSTM_IH_HH><<<(kCl * Lstm1Shape::kPerCta + 255) / 256, 256, 0, stream>>>(
-            packed_lstm1, static_cast<const __half*>(w->w_ih[1]), static_cast<const __half*>(w->w_hh[1]), absmax, 2, 1);
+        gates(packed_lstm1, w->w_ih[1], true, 2);
+        gates(packed_lstm1 + slice1, w->w_hh[1], true, 1);
+    }
+    if (!cache) {        // the long-request numerics read both matrices as the caller lays them out
+        tdt_pack_kernel<PredSplit, CLPACK_PRED, false><<<blocks(PredSplit::kPerCta), 256, 0, stream>>>(packed_pred, w_pred, nullptr, 0);
+        tdt_pack_kernel<JointSplit, CLPACK_JOINT, false><<<blocks(JointSplit::kPerCta), 256, 0, stream>>>(packed_joint, w_joint, nullptr, 0);
+        pk100_count_launch();
         pk100_count_launch();
     }
     cudaError_t err = cudaGetLastError();
@@ -2487,12 +1560,12 @@ int decode_cluster(void* stream_v, const pk100_decoder_weights* w, const void* e
     p.frames_lo = frames_lo;
     p.frames_hi = frames_hi;
 
-    if (w->layers == 1)
-        err = cache ? launch_cluster_kernel<1, true>(stream, p, packed_lstm, packed_pred, packed_joint, xtab, packed_lstm1)
-                    : launch_cluster_kernel<1, false>(stream, p, packed_lstm, packed_pred, packed_joint, xtab, packed_lstm1);
-    else
-        err = cache ? launch_cluster_kernel<2, true>(stream, p, packed_lstm, packed_pred, packed_joint, xtab, packed_lstm1)
-                    : launch_cluster_kernel<2, false>(stream, p, packed_lstm, packed_pred, packed_joint, xtab, packed_lstm1);
+    const ClWeights packed{packed_lstm, packed_pred, packed_joint, packed_lstm1, packed_lstm1 + slice1, xtab};
+    err = with_cluster_kernel(w->layers, cache, utterances, [&](auto kernel, int smem) {
+        cudaLaunchAttribute attr{};
+        const cudaLaunchConfig_t cfg = cluster_config(attr, smem, stream);
+        return cudaLaunchKernelEx(&cfg, kernel, p, packed);
+    });
     if (err != cudaSuccess) {
         cudaGetLastError();
         return static_cast<int>(err);
@@ -2523,7 +1596,7 @@ extern "C" int pk100_tdt_decode_long(void* stream_v, const pk100_decoder_weights
                                      int32_t* tokens, int32_t* durations, int32_t* counts, int max_tokens,
                                      int* status) {
     // the cluster kernel where a 16-CTA cluster can be hosted, else the grid-barrier kernel
-    if (w != nullptr && utterances > 0 && utterances <= kMaxUtt && cluster_decoder_available_for(w->layers, true))
+    if (w != nullptr && utterances > 0 && utterances <= kMaxUtt && cluster_decoder_available_for(w->layers, true, utterances))
         return pk100_tdt_decode_long_cluster(stream_v, w, enc_proj, utterances, seg_stride, frames, workspace,
                                              tokens, durations, counts, max_tokens, status);
     return pk100_tdt_decode_long_barrier(stream_v, w, enc_proj, utterances, seg_stride, frames, workspace, tokens,
@@ -2538,7 +1611,8 @@ extern "C" int pk100_tdt_decode_auto(void* stream_v, const pk100_decoder_weights
     // launches on the same stream, each decoding its own utterances and skipping the others
     constexpr int kLongRequestFrames = 1024;
     const bool cluster = w != nullptr && utterances > 0 && utterances <= kMaxUtt &&
-                         cluster_decoder_available_for(w->layers, false) && cluster_decoder_available_for(w->layers, true);
+                         cluster_decoder_available_for(w->layers, false, utterances) &&
+                         cluster_decoder_available_for(w->layers, true, utterances);
     auto run = cluster ? decode_cluster : decode_barrier;
     const int rc = run(stream_v, w, enc_proj, utterances, seg_stride, frames, workspace, tokens, durations, counts,
                        max_tokens, status, false, INT_MIN, kLongRequestFrames);
@@ -2553,7 +1627,7 @@ extern "C" int pk100_tdt_decode(void* stream_v, const pk100_decoder_weights* w, 
                                 int* status) {
     // a device that can host a 16-CTA cluster: the cluster kernel; anything else: the 148-CTA
     // exchange kernel
-    if (w != nullptr && utterances > 0 && utterances <= kMaxUtt && cluster_decoder_available_for(w->layers, false))
+    if (w != nullptr && utterances > 0 && utterances <= kMaxUtt && cluster_decoder_available_for(w->layers, false, utterances))
         return pk100_tdt_decode_cluster(stream_v, w, enc_proj, utterances, seg_stride, frames, workspace, tokens,
                                         durations, counts, max_tokens, status);
     return pk100_tdt_decode_exchange(stream_v, w, enc_proj, utterances, seg_stride, frames, workspace, tokens,
