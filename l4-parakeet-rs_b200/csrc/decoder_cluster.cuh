@@ -15,12 +15,14 @@
 //                recurrent weights only needs the new hidden state, not the next token, so it runs
 //                right behind the prediction GEMM, under the prediction exchange, and is ready when the
 //                next token is known.
-//   warps 20-23  control warps: LSTM cell, reductions of the K-split partial sums, all sends, the
-//                decision.  The prediction slice is turned into the joint input by its owner and
-//                travels as such; the fp32 prediction follows for the rounds after a blank, whose
-//                joint input is formed locally.
+//   control warps  one to four per utterance (their threads own its 40 units in registers): decision, LSTM
+//                cell, reductions of the K-split partial sums, all sends.  The token's table row and the
+//                new frame's encoder values go straight to the registers of the threads that use them.
+//                The prediction slice is turned into the joint input relu(enc + pred) by its owner and
+//                travels as such.
 // Weights are resident where they fit: recurrent weights (two layers: the critical input weights of the
-// second layer first) in tensor memory, joint rows in shared memory, prediction rows in
+// second layer first) in tensor memory, joint rows in shared memory (one fp16 layer: half of them in
+// tensor memory), prediction rows in
 // registers; with two fp16 layers the rest streams from L2 in "fragment order" (16 contiguous bytes per
 // lane and mma), off the critical path.  The input half of the first layer, W_ih . embedding[token],
 // is a table [1025, 2560] computed once per call by one GEMM; a round gathers 4 x 40 floats of it.
@@ -34,13 +36,11 @@ constexpr int kClUnits = kHidden / kCl;          // 40 hidden units / prediction
 constexpr int kClJoint = 65;                     // joint rows per CTA (16 x 65 >= 1030)
 constexpr int kMatrixWarps = 20;
 constexpr int kMatrixThreads = kMatrixWarps * 32;
-constexpr int kControlThreads = 128;
-constexpr int kClThreads = kMatrixThreads + kControlThreads;
-constexpr int kEncChunks = kHidden / 8;          // 16-byte chunks of one projected encoder row
+constexpr int cl_threads(int utts) { return kMatrixThreads + 32 * utts; }      // one control warp per utterance it is sized for
 constexpr uint32_t kTmemColumns = 512;
 
 // named barriers (0 is __syncthreads)
-enum : int { BAR_CONTROL = 1, BAR_PRED = 2, BAR_GO = 3, BAR_MATRIX = 4, BAR_LAYER1 = 5 };
+enum : int { BAR_CONTROL = 1, BAR_PRED = 2, BAR_GO = 3, BAR_LAYER1 = 4 };
 __device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 __device__ __forceinline__ void bar_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 
@@ -137,23 +137,18 @@ struct CSmem {
     alignas(16) uint8_t h1[Layers == 2 ? sizeof(Act) : 16];            // of layer 1
     alignas(16) float hf[Cache ? NU : 1][Cache ? kHidden : 4];         // Cache: fp32 state of the top layer
     alignas(16) uint8_t ax[Cache ? NU * kHidden * 4 : kActRows * kActPitch];   // joint input: hi / lo rows or fp32
-    alignas(16) float pred[NU][kHidden];                  // prediction vectors, written by all CTAs
-    alignas(16) __half enc[NU][kHidden];                  // projected encoder row of each utterance's frame
-    alignas(16) float xg[NU][4][kClUnits];                // W_ih . embedding[last token]: this CTA's gate inputs
     alignas(16) float gates0[kGateParts * NU * kGatePitch];            // partial sums of the recurrent product
     alignas(16) float gates1[Layers == 2 ? 4 * NU * kGatePitch : 4];   // layer 1: parts 0, 1 input, 2, 3 recurrent
     alignas(16) float part[Cache ? NU * kJointPitch : (20 * NU * kPredPitch > 10 * NU * kJointPitch ? 20 * NU * kPredPitch : 10 * NU * kJointPitch)];
-    float cell0[NU][kClUnits], cell1[Layers == 2 ? NU : 1][kClUnits];
     alignas(16) uint8_t stage_act[NU][2][kClUnits * 2];   // outgoing slice: hi / lo halves, Cache: codes (first 40 bytes)
     alignas(16) float stage_f[NU][kClUnits];              // outgoing fp32 slice (Cache: hidden state / joint input)
-    alignas(16) float stage_pred[NU][kClUnits];           // outgoing prediction slice
+    float pred[Cache ? NU : 1][kClUnits];                 // Cache: this CTA's prediction slice, finished by the matrix warps
     float bias0[kClUnits][4], bias1[Layers == 2 ? kClUnits : 1][4], pred_bias[kClUnits], joint_bias[kJointPitch];
     float cache_mul[3];                                   // scale / 127 of w_hh[0], w_hh[1], w_ih[1]
     unsigned long long keys[2][NU][3 * kCl];              // [round parity][utterance][source CTA, third of its rows]
     int dur[2][NU];                                       // [round parity][utterance] winning duration
-    uint64_t hbar0, hbar1, abar, pbar, kbar[2];           // exchange mbarriers (count 1 + transaction bytes)
+    uint64_t hbar0, hbar1, abar, kbar[2];           // exchange mbarriers (count 1 + transaction bytes)
     uint32_t tmem_base;
-    int frame[NU], symbols[NU], count[NU], total_frames[NU];
     alignas(8) unsigned char done[8], need[8];            // read as 64-bit words; done = 1 behind the last utterance
     int abort;
 #ifdef PK100_DEC_PROFILE
@@ -180,11 +175,6 @@ __device__ __forceinline__ void st_async_b32(uint32_t addr, unsigned v, uint32_t
     asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];"
                  ::"r"(addr), "r"(v), "r"(bar) : "memory");
 }
-__device__ __forceinline__ void cp_async_16(void* smem_dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
 __device__ __forceinline__ float fast_sigmoid(float x) { return __fdividef(1.0f, 1.0f + __expf(-x)); }
 __device__ __forceinline__ float fast_tanh(float x) { return 2.0f * fast_sigmoid(2.0f * x) - 1.0f; }
 
@@ -275,9 +265,10 @@ struct ClWeights {               // packed slices (see tdt_pack_kernel) and the 
 };
 
 template <int Layers, bool Cache, int NU>
-__global__ void __launch_bounds__(kClThreads, 1)
+__global__ void __launch_bounds__(cl_threads(NU), 1)
 tdt_cluster_kernel(const DecParams p, const ClWeights w) {
     using Smem = CSmem<Layers, Cache, NU>;
+    constexpr int kClThreads = cl_threads(NU), kControlThreads = kClThreads - kMatrixThreads;
     constexpr int NB = Cache ? 1 : NU / 4;                 // blocks of 8 B columns
     constexpr int kPitch = Smem::kActPitch;
     using Gates0 = typename std::conditional<Cache, CodeSplit, LstmSplit>::type;
@@ -286,7 +277,8 @@ tdt_cluster_kernel(const DecParams p, const ClWeights w) {
     constexpr int kCols0 = Layers == 2 && !Cache ? 16 : Gates0::KP * Gates0::NT * 8;      // w_hh[0] (two fp16 layers: one pair)
     constexpr int kCols1 = Layers == 2 ? Gates1::KP * 8 : 0;                              // w_ih[1]
     constexpr int kCols2 = Layers == 2 && Cache ? 16 : 0;                                 // w_hh[1]: two pairs
-    constexpr int kCols = kCols0 + kCols1 + kCols2;
+    constexpr int kColsJ = Layers == 1 && !Cache ? 16 : 0;                                // joint: the first pair of two tiles
+    constexpr int kCols = kCols0 + kCols1 + kCols2 + kColsJ;
     static_assert(5 * kCols <= static_cast<int>(kTmemColumns), "fits tensor memory");
 
     extern __shared__ __align__(16) uint8_t cs_raw[];
@@ -297,7 +289,7 @@ tdt_cluster_kernel(const DecParams p, const ClWeights w) {
     const int U = p.utts;
     volatile int* abort_flag = &sm.abort;
 
-    // ---- set-up: cleared state, biases, barriers, first encoder rows
+    // ---- set-up: cleared state, biases, barriers
     for (int i = tid; i < static_cast<int>(sizeof(Smem) / 16); i += kClThreads) reinterpret_cast<uint4*>(cs_raw)[i] = make_uint4(0, 0, 0, 0);
     __syncthreads();
     if (tid < kClUnits * 4) {
@@ -310,7 +302,6 @@ tdt_cluster_kernel(const DecParams p, const ClWeights w) {
     if (tid < kClJoint && r * kClJoint + tid < kJointRows) sm.joint_bias[tid] = p.b_joint[r * kClJoint + tid];
     if (tid < 8) {
         const bool done = tid >= U || p.frames[tid] <= 0 || !in_window(p, tid);
-        if (tid < NU) sm.total_frames[tid] = tid < U ? min(p.frames[tid], p.seg_stride) : 0;   // never past the utterance's block
         sm.done[tid] = done;
         sm.need[tid] = !done;
     }
@@ -318,7 +309,6 @@ tdt_cluster_kernel(const DecParams p, const ClWeights w) {
         mbar_init(&sm.hbar0, 1);
         mbar_init(&sm.hbar1, 1);
         mbar_init(&sm.abar, 1);
-        mbar_init(&sm.pbar, 1);
         mbar_init(&sm.kbar[0], 1);
         mbar_init(&sm.kbar[1], 1);
         fence_barrier_init();
@@ -330,10 +320,6 @@ tdt_cluster_kernel(const DecParams p, const ClWeights w) {
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    if (warp < U && !sm.done[warp]) {
-        const __half* src = p.enc_proj + static_cast<size_t>(warp) * p.seg_stride * kHidden;
-        for (int c = lane; c < kEncChunks; c += 32) cp_async_16(&sm.enc[warp][c * 8], src + c * 8);
-    }
     // resident joint rows
     if constexpr (Cache) {
         // row-major, 336 words per row (= 16 mod 32): the two half-warps of a warp read different rows
@@ -355,7 +341,6 @@ tdt_cluster_kernel(const DecParams p, const ClWeights w) {
             else if (rest % 32 < 4) dst[256 + (rest - 256) / 32 * 4 + rest % 32] = __ldg(src + i);   // fifth tile: row 64 only
         }
     }
-    cp_async_wait_all();
     __syncthreads();
     cluster_sync_all();      // every CTA's shared memory and mbarriers are ready before a peer writes
 
@@ -430,6 +415,12 @@ tdt_cluster_kernel(const DecParams p, const ClWeights w) {
             for (int i = 0; i < kCols1 / 8; ++i) fill(in1 + frag_index<Gates1>(kg1, i, tile1, 0, lane), kCols0 + i * 8);
 #pragma unroll
             for (int i = 0; i < kCols2 / 8; ++i) fill(rec1 + frag_index<Gates1>(kg1, i, tile1, 0, lane), kCols0 + kCols1 + i * 8);
+        }
+        if constexpr (kColsJ > 0) {
+            const uint4* src = w.joint + static_cast<size_t>(r) * JointSplit::kPerCta;
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+                fill(src + frag_index<JointSplit>(warp / JointSplit::NG, 0, (warp % JointSplit::NG) * 2 + j, 0, lane), kCols0 + j * 8);
         }
         tmem_st_wait();
         uint4* pairs = reinterpret_cast<uint4*>(sm.pairs);         // [pair][warp][tile][step][lane]
@@ -554,8 +545,8 @@ tdt_cluster_kernel(const DecParams p, const ClWeights w) {
                             s1 += __shfl_down_sync(0xffffffffu, s1, off);
                         }
                         if (lane == 0) {
-                            sm.stage_pred[u][warp] = s0;
-                            sm.stage_pred[u][warp + kMatrixWarps] = s1;
+                            sm.pred[u][warp] = s0;
+                            sm.pred[u][warp + kMatrixWarps] = s1;
                         }
                     }
                 } else {
@@ -575,26 +566,8 @@ tdt_cluster_kernel(const DecParams p, const ClWeights w) {
                 else
                     recurrent0();
             }
-            if ((~done8 & ~need8 & 0x0101010101010101ull) != 0ull) {
-                // utterances whose prediction did not change (their last token was a blank): joint input
-                // relu(enc + pred) of the new frame formed here, one thread per column
-                for (int u = 0; u < U; ++u) {
-                    if ((((done8 | need8) >> (8 * u)) & 1ull) != 0ull) continue;
-                    const float v = fmaxf(__half2float(sm.enc[u][tid]) + sm.pred[u][tid], 0.0f);
-                    if constexpr (Cache) {
-                        reinterpret_cast<float*>(sm.ax)[u * kHidden + tid] = v;
-                    } else {
-                        const __half hi = __float2half_rn(v);
-                        *reinterpret_cast<__half*>(sm.ax + (2 * u) * kPitch + tid * 2) = hi;
-                        *reinterpret_cast<__half*>(sm.ax + (2 * u + 1) * kPitch + tid * 2) = __float2half_rn(v - __half2float(hi));
-                    }
-                }
-                bar_sync(BAR_MATRIX, kMatrixThreads);
-            }
-            if (need8 != 0ull) {
-                mbar_wait_bounded(&sm.abar, hphase, abort_flag);
-                hphase ^= 1u;
-            }
+            mbar_wait_bounded(&sm.abar, round & 1u, abort_flag);
+            if (need8 != 0ull) hphase ^= 1u;
             // ---- joint rows
             if constexpr (Cache) {
                 // fp32 in the reference's summation order (decoder.cu:697-713): one row per half-warp, half-lane
@@ -635,8 +608,17 @@ tdt_cluster_kernel(const DecParams p, const ClWeights w) {
                     const uint4* block = Smem::kJointResident
                         ? reinterpret_cast<const uint4*>(sm.joint) + (kg * JointSplit::KP + kp) * (256 + 8)
                         : w.joint + static_cast<size_t>(r) * JointSplit::kPerCta + (kg * JointSplit::KP + kp) * 320;
+                    [[maybe_unused]] uint32_t f[16];
+                    if constexpr (kColsJ > 0)
+                        if (kp == 0) {
+                            tmem_ld_32x16(tm + kCols0, f);
+                            tmem_ld_wait();
+                        }
                     pair_mma<false, 3, NB>(acc, sm.ax + (kg * JointSplit::KP + kp) * 64 + lane_act, kPitch, ng == 0 ? 3 : 2,
                                            [&](int j, int step) {
+                        if constexpr (kColsJ > 0)
+                            if (kp == 0 && j < 2)
+                                return make_uint4(f[j * 8 + step * 4], f[j * 8 + step * 4 + 1], f[j * 8 + step * 4 + 2], f[j * 8 + step * 4 + 3]);
                         if (j < 2) return block[((ng * 2 + j) * 2 + step) * 32 + lane];
                         return lane < 4 ? block[256 + (Smem::kJointResident ? step * 4 : step * 32) + lane] : make_uint4(0, 0, 0, 0);
                     });
@@ -653,129 +635,152 @@ tdt_cluster_kernel(const DecParams p, const ClWeights w) {
     } else {
         // ============================================================ control warps
         const int ct = tid - kMatrixThreads, cw = ct / 32;
-        // sends: thread = (peer, item % 8); shared::cluster address of `x` in the peer = peer_base + offset of x
-        const uint32_t peer = static_cast<uint32_t>(ct % kCl);
+        // sends: thread = (peer, item % kSubs); shared::cluster address of `x` in the peer = peer_base + offset of x
+        constexpr int kSubs = kControlThreads / kCl;
+        const uint32_t local_base = smem_u32(cs_raw), peer_base = map_to_cta(local_base, static_cast<uint32_t>(ct % kCl));
         const int sub = ct / kCl;
-        const uint32_t local_base = smem_u32(cs_raw), peer_base = map_to_cta(local_base, peer);
         auto in_peer = [&](const void* x) { return peer_base + (smem_u32(x) - local_base); };
-        // 40 fp16 units as (hi, lo) rows 2u, 2u + 1 of `act`
-        auto send_halves = [&](uint8_t* act, uint64_t* bar_local, unsigned long long need8) {
+        // 40 fp16 units as (hi, lo) rows 2u, 2u + 1 of `act`; `who` = utterances that send, one byte each
+        auto send_halves = [&](uint8_t* act, uint64_t* bar_local, unsigned long long who) {
             const uint32_t bar = in_peer(bar_local);
             for (int u = 0; u < U; ++u) {
-                if (((need8 >> (8 * u)) & 1ull) == 0ull) continue;
-                for (int i = sub; i < 10; i += 8) {
+                if (((who >> (8 * u)) & 1ull) == 0ull) continue;
+                for (int i = sub; i < 10; i += kSubs) {
                     const int lo = i / 5, chunk = i % 5;
                     st_async_v4(in_peer(act + (2 * u + lo) * kPitch + r * kClUnits * 2 + chunk * 16),
                                 *reinterpret_cast<const uint4*>(&sm.stage_act[u][lo][chunk * 16]), bar);
                 }
             }
         };
-        auto send_floats = [&](float* dst, const float (*src)[kClUnits], uint64_t* bar_local, unsigned long long need8) {
+        auto send_floats = [&](float* dst, uint64_t* bar_local, unsigned long long who) {
             const uint32_t bar = in_peer(bar_local);
             for (int u = 0; u < U; ++u) {
-                if (((need8 >> (8 * u)) & 1ull) == 0ull) continue;
-                for (int i = sub; i < 10; i += 8)
-                    st_async_v4(in_peer(dst + u * kHidden + r * kClUnits + i * 4), *reinterpret_cast<const uint4*>(&src[u][i * 4]), bar);
+                if (((who >> (8 * u)) & 1ull) == 0ull) continue;
+                for (int i = sub; i < 10; i += kSubs)
+                    st_async_v4(in_peer(dst + u * kHidden + r * kClUnits + i * 4), *reinterpret_cast<const uint4*>(&sm.stage_f[u][i * 4]), bar);
             }
         };
-        auto send_codes = [&](uint8_t* act, uint64_t* bar_local, unsigned long long need8) {
+        auto send_codes = [&](uint8_t* act, uint64_t* bar_local, unsigned long long who) {
             const uint32_t bar = in_peer(bar_local);
             for (int u = 0; u < U; ++u) {
-                if (((need8 >> (8 * u)) & 1ull) == 0ull || sub >= 5) continue;
+                if (((who >> (8 * u)) & 1ull) == 0ull || sub >= 5) continue;
                 st_async_b64(in_peer(act + u * kPitch + r * kClUnits + sub * 8),
                              *reinterpret_cast<const unsigned long long*>(&sm.stage_act[u][0][sub * 8]), bar);
-            }
-        };
-        // LSTM cell of one (utterance, unit) from its four gate sums; stages h for the exchange
-        auto cell_update = [&](const float (&gsum)[4], float& cstate, int u, int slot) {
-            if constexpr (Cache) {
-                // the reference's approximations: h is rounded to 8 bits next, and a code that flips moves a gate
-                const float h = ref_lstm_cell(gsum, cstate);
-                sm.stage_act[u][0][slot] = static_cast<uint8_t>(quantize_i8(h * 127.0f));
-                sm.stage_f[u][slot] = h;
-            } else {
-                const float cell = fast_sigmoid(gsum[1]) * cstate + fast_sigmoid(gsum[0]) * fast_tanh(gsum[2]);
-                cstate = cell;
-                const float h = fast_sigmoid(gsum[3]) * fast_tanh(cell);
-                const __half hi = __float2half_rn(h);
-                reinterpret_cast<__half*>(sm.stage_act[u][0])[slot] = hi;
-                reinterpret_cast<__half*>(sm.stage_act[u][1])[slot] = __float2half_rn(h - __half2float(hi));
             }
         };
         auto gate_part = [&](const float* gates, int kg, int u, int slot) {
             return *reinterpret_cast<const float4*>(&gates[(kg * NU + u) * kGatePitch + slot * 4]);
         };
-        // bytes one stepping utterance contributes to the exchanges
+        // The warps of a team serve one utterance: its 40 slots (= this CTA's units) belong to fixed threads,
+        // so cell state, gate inputs, encoder values and the utterance's counters live in registers (the
+        // counters and the decision itself are replicated in the team's warps).
+        const int team = NU == 8 || U > 2 ? 1 : (U == 2 ? 2 : 4);          // warps per utterance
+        const int my = cw / team, first_slot = (cw % team) * 32 + lane, slot_step = team * 32;
+        constexpr int kPasses = 2;                                         // slots per thread at most
+        const bool serving = my < U;
+        const bool leader = serving && cw % team == 0 && lane == 0;
+        bool live = serving && !sm.done[serving ? my : 0];
+        bool need = live;
+        const int total_frames = live ? min(p.frames[my], p.seg_stride) : 0;   // never past the utterance's block
+        const __half* enc_rows = p.enc_proj + static_cast<size_t>(serving ? my : 0) * p.seg_stride * kHidden + r * kClUnits;
+        int frame = 0, symbols = 0, count = 0;
+        float cell0[kPasses] = {}, cell1[kPasses] = {}, pred[kPasses] = {}, xg[kPasses][4] = {}, enc[kPasses] = {};
+        auto for_slots = [&](auto&& f) {                                   // f(pass, slot)
+#pragma unroll
+            for (int i = 0; i < kPasses; ++i) {
+                const int slot = first_slot + i * slot_step;
+                if (slot < kClUnits) f(i, slot);
+            }
+        };
+        auto fetch_enc = [&]() {
+            for_slots([&](int i, int slot) { enc[i] = __half2float(enc_rows[static_cast<size_t>(frame) * kHidden + slot]); });
+        };
+        if (live) fetch_enc();
+        // LSTM cell of one unit from its four gate sums; stages h for the exchange
+        auto cell_update = [&](const float (&gsum)[4], float& cstate, int slot) {
+            if constexpr (Cache) {
+                // the reference's approximations: h is rounded to 8 bits next, and a code that flips moves a gate
+                const float h = ref_lstm_cell(gsum, cstate);
+                sm.stage_act[my][0][slot] = static_cast<uint8_t>(quantize_i8(h * 127.0f));
+                sm.stage_f[my][slot] = h;
+            } else {
+                const float cell = fast_sigmoid(gsum[1]) * cstate + fast_sigmoid(gsum[0]) * fast_tanh(gsum[2]);
+                cstate = cell;
+                const float h = fast_sigmoid(gsum[3]) * fast_tanh(cell);
+                const __half hi = __float2half_rn(h);
+                reinterpret_cast<__half*>(sm.stage_act[my][0])[slot] = hi;
+                reinterpret_cast<__half*>(sm.stage_act[my][1])[slot] = __float2half_rn(h - __half2float(hi));
+            }
+        };
+        // bytes one utterance contributes to the exchanges
         constexpr uint32_t kTopTx = Cache ? kHidden + kHidden * 4 : kHidden * 4, kLowTx = Cache ? kHidden : kHidden * 4;
-        uint32_t pphase = 0;
 #ifdef PK100_DEC_PROFILE
         if (ct == 0) sm.last_stamp = clock64();
 #endif
-        bar_sync(BAR_CONTROL, kControlThreads);
         while (true) {
-            const unsigned long long done8 = *reinterpret_cast<const unsigned long long*>(sm.done);
-            const unsigned long long need8 = *reinterpret_cast<const unsigned long long*>(sm.need);
-            bar_arrive(BAR_GO, kClThreads);
-            // a wait that gave up raised sm.abort; it is read here, behind the barriers that end a round
-            if (done8 == 0x0101010101010101ull || sm.abort != 0) break;
-            const uint32_t needs = static_cast<uint32_t>(__popcll(need8)), lives = 8u - static_cast<uint32_t>(__popcll(done8));
+            __syncwarp();
+            bar_arrive(BAR_GO, kClThreads);                // this round's flags are published
             const int par = static_cast<int>(round & 1u);
-            if (ct == 0) {
-                mbar_arrive_expect_tx(&sm.kbar[par], lives * (3 * kCl * 8 + 4));
-                if (need8 != 0ull) {
-                    mbar_arrive_expect_tx(&sm.hbar0, needs * (Layers == 1 ? kTopTx : kLowTx));
-                    if (Layers == 2) mbar_arrive_expect_tx(&sm.hbar1, needs * kTopTx);
-                    mbar_arrive_expect_tx(&sm.abar, needs * kHidden * 4);
-                    mbar_arrive_expect_tx(&sm.pbar, needs * kHidden * 4);
-                }
-            }
-            CL_STAMP(0);
-            if (need8 != 0ull) {
+            if (need) {
                 // ---- cell of layer 0: table row + h . w_hh^T + bias
-                for (int i = ct; i < U * kClUnits; i += kControlThreads) {
-                    const int u = i / kClUnits, slot = i % kClUnits;
-                    if (((need8 >> (8 * u)) & 1ull) == 0ull) continue;
+                for_slots([&](int i, int slot) {
                     float gsum[4];
                     if constexpr (Cache) {
                         // the scaled recurrent sum is rounded BEFORE the bias is added, as in the reference
                         // (decoder.cu:113, :626-640): a fused multiply-add here parts from the reference
                         // kernel's tokens after a few hundred steps
-                        const float4 a = gate_part(sm.gates0, 0, u, slot), b = gate_part(sm.gates0, 1, u, slot);
+                        const float4 a = gate_part(sm.gates0, 0, my, slot), b = gate_part(sm.gates0, 1, my, slot);
                         const float rec[4] = {a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w};
 #pragma unroll
                         for (int g = 0; g < 4; ++g)
-                            gsum[g] = __fadd_rn(__fadd_rn(__fmul_rn(rec[g], sm.cache_mul[0]), sm.bias0[slot][g]), sm.xg[u][g][slot]);
+                            gsum[g] = __fadd_rn(__fadd_rn(__fmul_rn(rec[g], sm.cache_mul[0]), sm.bias0[slot][g]), xg[i][g]);
                     } else {
 #pragma unroll
-                        for (int g = 0; g < 4; ++g) gsum[g] = sm.bias0[slot][g] + sm.xg[u][g][slot];
+                        for (int g = 0; g < 4; ++g) gsum[g] = sm.bias0[slot][g] + xg[i][g];
 #pragma unroll
                         for (int kg = 0; kg < LstmSplit::KG; ++kg) {
-                            const float4 v = gate_part(sm.gates0, kg, u, slot);
+                            const float4 v = gate_part(sm.gates0, kg, my, slot);
                             gsum[0] += v.x; gsum[1] += v.y; gsum[2] += v.z; gsum[3] += v.w;
                         }
                     }
-                    cell_update(gsum, sm.cell0[u][slot], u, slot);
-                }
-                cp_async_wait_all();                       // encoder rows of the new frames
-                bar_sync(BAR_CONTROL, kControlThreads);
-                CL_STAMP(1);
+                    cell_update(gsum, cell0[i], slot);
+                });
+            }
+            CL_STAMP(0);
+            bar_sync(BAR_CONTROL, kControlThreads);
+            const unsigned long long done8 = *reinterpret_cast<const unsigned long long*>(sm.done);
+            const unsigned long long need8 = *reinterpret_cast<const unsigned long long*>(sm.need);
+            const unsigned long long live8 = ~done8 & 0x0101010101010101ull;
+            // a wait that gave up raised sm.abort; it is read here, behind the barriers that end a round
+            if (live8 == 0ull || sm.abort != 0) break;
+            CL_STAMP(1);
+            if (need8 != 0ull) {
                 if constexpr (Cache) {
                     send_codes(sm.h0, &sm.hbar0, need8);
-                    if constexpr (Layers == 1) send_floats(&sm.hf[0][0], sm.stage_f, &sm.hbar0, need8);
+                    if constexpr (Layers == 1) send_floats(&sm.hf[0][0], &sm.hbar0, need8);
                 } else {
                     send_halves(sm.h0, &sm.hbar0, need8);
                 }
-                CL_STAMP(2);
+            }
+            if (ct == kControlThreads - 1) {               // (transaction counts may trail the transactions)
+                const uint32_t needs = static_cast<uint32_t>(__popcll(need8)), lives = static_cast<uint32_t>(__popcll(live8));
+                if (need8 != 0ull) {
+                    mbar_arrive_expect_tx(&sm.hbar0, needs * (Layers == 1 ? kTopTx : kLowTx));
+                    if (Layers == 2) mbar_arrive_expect_tx(&sm.hbar1, needs * kTopTx);
+                }
+                mbar_arrive_expect_tx(&sm.abar, lives * kHidden * 4);
+                mbar_arrive_expect_tx(&sm.kbar[par], lives * (3 * kCl * 8 + 4));
+            }
+            CL_STAMP(2);
+            if (need8 != 0ull) {
                 if constexpr (Layers == 2) {
                     bar_sync(BAR_LAYER1, kClThreads);
                     CL_STAMP(3);
                     // ---- cell of layer 1: [fresh h of layer 0 | own h] . [w_ih | w_hh]^T + bias
-                    for (int i = ct; i < U * kClUnits; i += kControlThreads) {
-                        const int u = i / kClUnits, slot = i % kClUnits;
-                        if (((need8 >> (8 * u)) & 1ull) == 0ull) continue;
+                    if (need) for_slots([&](int i, int slot) {
                         float gsum[4];
-                        const float4 a = gate_part(sm.gates1, 0, u, slot), b = gate_part(sm.gates1, 1, u, slot);
-                        const float4 c = gate_part(sm.gates1, 2, u, slot), d = gate_part(sm.gates1, 3, u, slot);
+                        const float4 a = gate_part(sm.gates1, 0, my, slot), b = gate_part(sm.gates1, 1, my, slot);
+                        const float4 c = gate_part(sm.gates1, 2, my, slot), d = gate_part(sm.gates1, 3, my, slot);
                         const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
                         const float cv[4] = {c.x, c.y, c.z, c.w}, dv[4] = {d.x, d.y, d.z, d.w};
 #pragma unroll
@@ -787,123 +792,107 @@ tdt_cluster_kernel(const DecParams p, const ClWeights w) {
                             else
                                 gsum[g] = (((sm.bias1[slot][g] + av[g]) + bv[g]) + cv[g]) + dv[g];
                         }
-                        cell_update(gsum, sm.cell1[u][slot], u, slot);
-                    }
+                        cell_update(gsum, cell1[i], slot);
+                    });
                     bar_sync(BAR_CONTROL, kControlThreads);
                     CL_STAMP(4);
                     if constexpr (Cache) {
                         send_codes(sm.h1, &sm.hbar1, need8);
-                        send_floats(&sm.hf[0][0], sm.stage_f, &sm.hbar1, need8);
+                        send_floats(&sm.hf[0][0], &sm.hbar1, need8);
                     } else {
                         send_halves(sm.h1, &sm.hbar1, need8);
                     }
                 }
                 bar_sync(BAR_PRED, kClThreads);
-                CL_STAMP(5);
-                // ---- prediction slice, and from it this CTA's 40 columns of the joint input relu(enc + pred)
-                for (int i = ct; i < U * kClUnits; i += kControlThreads) {
-                    const int u = i / kClUnits, n = i % kClUnits;
-                    if (((need8 >> (8 * u)) & 1ull) == 0ull) continue;
-                    float v;
+            } else {
+                bar_sync(BAR_CONTROL, kControlThreads);    // everyone has read the flags
+            }
+            CL_STAMP(5);
+            // ---- prediction slice where the state moved; this CTA's 40 columns of the joint input relu(enc + pred)
+            if (live) for_slots([&](int i, int slot) {
+                if (need) {
                     if constexpr (Cache) {
-                        v = sm.stage_pred[u][n];
+                        pred[i] = sm.pred[my][slot];
                     } else {
-                        v = sm.pred_bias[n];
+                        float part[PredSplit::KG];
 #pragma unroll
-                        for (int kg = 0; kg < PredSplit::KG; ++kg) v += sm.part[(kg * NU + u) * kPredPitch + n];
-                        sm.stage_pred[u][n] = v;
-                    }
-                    const float x = fmaxf(__half2float(sm.enc[u][r * kClUnits + n]) + v, 0.0f);
-                    if constexpr (Cache) {
-                        sm.stage_f[u][n] = x;
-                    } else {
-                        const __half hi = __float2half_rn(x);
-                        reinterpret_cast<__half*>(sm.stage_act[u][0])[n] = hi;
-                        reinterpret_cast<__half*>(sm.stage_act[u][1])[n] = __float2half_rn(x - __half2float(hi));
+                        for (int kg = 0; kg < PredSplit::KG; ++kg) part[kg] = sm.part[(kg * NU + my) * kPredPitch + slot];
+                        pred[i] = sm.pred_bias[slot];
+#pragma unroll
+                        for (int kg = 0; kg < PredSplit::KG; ++kg) pred[i] += part[kg];
                     }
                 }
-                bar_sync(BAR_CONTROL, kControlThreads);
-                CL_STAMP(6);
-                if constexpr (Cache) send_floats(reinterpret_cast<float*>(sm.ax), sm.stage_f, &sm.abar, need8);
-                else send_halves(sm.ax, &sm.abar, need8);
-                send_floats(&sm.pred[0][0], sm.stage_pred, &sm.pbar, need8);
-            }
+                const float x = fmaxf(enc[i] + pred[i], 0.0f);
+                if constexpr (Cache) {
+                    sm.stage_f[my][slot] = x;
+                } else {
+                    const __half hi = __float2half_rn(x);
+                    reinterpret_cast<__half*>(sm.stage_act[my][0])[slot] = hi;
+                    reinterpret_cast<__half*>(sm.stage_act[my][1])[slot] = __float2half_rn(x - __half2float(hi));
+                }
+            });
+            bar_sync(BAR_CONTROL, kControlThreads);
+            CL_STAMP(6);
+            if constexpr (Cache) send_floats(reinterpret_cast<float*>(sm.ax), &sm.abar, live8);
+            else send_halves(sm.ax, &sm.abar, live8);
             CL_STAMP(7);
             __syncthreads();                               // joint sums are complete
             CL_STAMP(8);
             publish_keys(done8);
             CL_STAMP(9);
             mbar_wait_bounded(&sm.kbar[par], (round >> 1) & 1u, abort_flag);
-            if (need8 != 0ull) {
-                mbar_wait_bounded(&sm.pbar, pphase, abort_flag);
-                pphase ^= 1u;
-            }
             CL_STAMP(10);
 
-            // ---- decision (replicated in every CTA): warp cw decides utterances cw, cw + 4
-            bool frame_now = false;
-            for (int u = cw; u < U; u += 4) {
-                if (((done8 >> (8 * u)) & 1ull) != 0ull) continue;
-                const unsigned long long k0 = sm.keys[par][u][lane], k1 = lane < kCl ? sm.keys[par][u][32 + lane] : 0ull;
+            // ---- decision (replicated in every CTA)
+            if (live) {
+                const unsigned long long k0 = sm.keys[par][my][lane], k1 = lane < kCl ? sm.keys[par][my][32 + lane] : 0ull;
                 const unsigned long long best = k1 > k0 ? k1 : k0;
                 const unsigned top = __reduce_max_sync(0xffffffffu, static_cast<unsigned>(best >> 32));
                 const unsigned low = __reduce_max_sync(0xffffffffu, static_cast<unsigned>(best >> 32) == top ? static_cast<unsigned>(best) : 0u);
                 int token = 2047 - static_cast<int>((low >> 21) & 0x7FFu);
                 // keys not delivered (a wait gave up), or every token score of the round was NaN: a
                 // blank; the second case is reported as status bit 4
-                if (token > kBlank) {
-                    token = kBlank;
-                    if (r == 0 && lane == 0 && sm.abort == 0 && p.status != nullptr) atomicOr(p.status, 4);
+                const bool no_score = token > kBlank;
+                if (no_score) token = kBlank;
+                need = token != kBlank;
+                // requests for the next round: the token's table row, then the encoder values of the new frame
+                if (need) {
+                    const float* row = w.xtab + static_cast<size_t>(token) * kGates + r * kClUnits;
+                    for_slots([&](int i, int slot) {
+#pragma unroll
+                        for (int g = 0; g < 4; ++g) xg[i][g] = __ldg(row + g * kHidden + slot);
+                    });
                 }
-                const int duration = sm.dur[par][u];
-                const int old_frame = sm.frame[u];
-                int frame = old_frame + duration;
-                int symbols = sm.symbols[u] + 1;
+                const int duration = sm.dur[par][my];
+                const int old_frame = frame;
+                frame += duration;
+                symbols += 1;
                 if (duration != 0 || symbols == kMaxSymbols) {
                     if (duration == 0) frame += 1;
                     symbols = 0;
                 }
-                const bool done = frame >= sm.total_frames[u];
-                // requests for the next round: the token's table row (this CTA's 4 x 40 gate inputs), then the
-                // encoder row of the new frame
-                if (token != kBlank && !done) {
-                    const float* row = w.xtab + static_cast<size_t>(token) * kGates + r * kClUnits;
-                    for (int n = lane; n < 40; n += 32) cp_async_16(&sm.xg[u][n / 10][(n % 10) * 4], row + (n / 10) * kHidden + (n % 10) * 4);
-                }
-                asm volatile("cp.async.commit_group;" ::: "memory");
-                if (!done && frame != old_frame) {
-                    const __half* src = p.enc_proj + (static_cast<size_t>(u) * p.seg_stride + frame) * kHidden;
-                    for (int c = lane; c < kEncChunks; c += 32) cp_async_16(&sm.enc[u][c * 8], src + c * 8);
-                }
-                asm volatile("cp.async.commit_group;" ::: "memory");
-                // the prediction of this round is current unless a token moves the state
-                frame_now = frame_now || (!done && token == kBlank);
-                __syncwarp();
-                if (lane == 0) {
-                    if (token != kBlank) {
-                        const int count = sm.count[u];
-                        if (r == 0 && count < p.max_tokens) {
-                            p.tokens[static_cast<size_t>(u) * p.max_tokens + count] = token;
-                            if (p.durations_out != nullptr) p.durations_out[static_cast<size_t>(u) * p.max_tokens + count] = duration;
+                live = frame < total_frames;
+                if (live && frame != old_frame) fetch_enc();
+                if (leader) {
+                    sm.done[my] = !live;
+                    sm.need[my] = live && need;
+                    if (r == 0) {
+                        if (no_score && sm.abort == 0 && p.status != nullptr) atomicOr(p.status, 4);
+                        if (need && count < p.max_tokens) {
+                            p.tokens[static_cast<size_t>(my) * p.max_tokens + count] = token;
+                            if (p.durations_out != nullptr) p.durations_out[static_cast<size_t>(my) * p.max_tokens + count] = duration;
                         }
-                        sm.count[u] = count + 1;
                     }
-                    sm.frame[u] = frame;
-                    sm.symbols[u] = symbols;
-                    sm.done[u] = done;
-                    sm.need[u] = !done && token != kBlank;
                 }
+                count += need ? 1 : 0;
+                need = need && live;
             }
-            // the table rows are needed now, the encoder rows only where the joint input is formed at once
-            if (frame_now || U > 4) cp_async_wait_all();
-            else asm volatile("cp.async.wait_group 1;" ::: "memory");
             round += 1;
-            bar_sync(BAR_CONTROL, kControlThreads);
             CL_STAMP(11);
         }
+        if (r == 0 && leader && in_window(p, my)) p.counts[my] = min(count, p.max_tokens);
     }
     // ---- teardown
-    cp_async_wait_all();
     tc_fence_before_sync();
     __syncthreads();
     if (warp == 1) {
@@ -916,7 +905,6 @@ tdt_cluster_kernel(const DecParams p, const ClWeights w) {
         for (int i = 0; i < 16; ++i)
             reinterpret_cast<volatile long long*>(p.workspace + xch_layout(U).abort)[2 + i] = sm.prof[i];
 #endif
-    if (r == 0 && tid < U && in_window(p, tid)) p.counts[tid] = min(sm.count[tid], p.max_tokens);
     if (r == 0 && tid == kMatrixThreads) reinterpret_cast<volatile int*>(p.workspace + xch_layout(U).abort)[2] = static_cast<int>(round);
     if (sm.abort != 0 && tid == 0 && p.status != nullptr) atomicExch(p.status, 2);
 }

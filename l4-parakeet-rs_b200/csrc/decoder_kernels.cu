@@ -1414,10 +1414,10 @@ namespace {
 
 // Can this device run a 16-CTA cluster of the cluster decoder?  Asked once per device and
 // kernel variant (one or two LSTM layers).
-// Calls f with the kernel for (layers, numerics, utterances of the call) and its shared-memory bytes.
+// Calls f with the kernel for (layers, numerics, utterances of the call) its threads and its shared-memory bytes.
 template <typename F>
 auto with_cluster_kernel(int layers, bool cache, int utterances, F&& f) {
-#define PK_PICK(L, C, N) return f(tdt_cluster_kernel<L, C, N>, static_cast<int>(sizeof(CSmem<L, C, N>)))
+#define PK_PICK(L, C, N) return f(tdt_cluster_kernel<L, C, N>, cl_threads(N), static_cast<int>(sizeof(CSmem<L, C, N>)))
     if (layers == 1) {
         if (cache) { if (utterances <= 4) PK_PICK(1, true, 4); PK_PICK(1, true, 8); }
         if (utterances <= 4) PK_PICK(1, false, 4);
@@ -1429,10 +1429,10 @@ auto with_cluster_kernel(int layers, bool cache, int utterances, F&& f) {
 #undef PK_PICK
 }
 
-cudaLaunchConfig_t cluster_config(cudaLaunchAttribute& attr, int smem, cudaStream_t stream) {
+cudaLaunchConfig_t cluster_config(cudaLaunchAttribute& attr, int threads, int smem, cudaStream_t stream) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(kCl);
-    cfg.blockDim = dim3(kClThreads);
+    cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     attr.id = cudaLaunchAttributeClusterDimension;
@@ -1451,11 +1451,11 @@ bool cluster_decoder_available_for(int layers, bool cache, int utterances = 1, i
     if (layers < 1 || layers > 2 || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
     std::atomic<int>& slot = known[dev][(layers - 1) * 4 + (cache ? 2 : 0) + (utterances > 4 ? 1 : 0)];
     if (slot.load() == 0) {
-        const int clusters = with_cluster_kernel(layers, cache, utterances, [&](auto kernel, int smem) {
+        const int clusters = with_cluster_kernel(layers, cache, utterances, [&](auto kernel, int threads, int smem) {
             int max_smem = 0, n = 0;
             cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
             cudaLaunchAttribute attr{};
-            const cudaLaunchConfig_t cfg = cluster_config(attr, smem, nullptr);
+            const cudaLaunchConfig_t cfg = cluster_config(attr, threads, smem, nullptr);
             if (smem > max_smem ||
                 cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
                 cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
@@ -1561,9 +1561,9 @@ int decode_cluster(void* stream_v, const pk100_decoder_weights* w, const void* e
     p.frames_hi = frames_hi;
 
     const ClWeights packed{packed_lstm, packed_pred, packed_joint, packed_lstm1, packed_lstm1 + slice1, xtab};
-    err = with_cluster_kernel(w->layers, cache, utterances, [&](auto kernel, int smem) {
+    err = with_cluster_kernel(w->layers, cache, utterances, [&](auto kernel, int threads, int smem) {
         cudaLaunchAttribute attr{};
-        const cudaLaunchConfig_t cfg = cluster_config(attr, smem, stream);
+        const cudaLaunchConfig_t cfg = cluster_config(attr, threads, smem, stream);
         return cudaLaunchKernelEx(&cfg, kernel, p, packed);
     });
     if (err != cudaSuccess) {
