@@ -126,9 +126,9 @@ struct CSmem {
     using Act = uint8_t[kActRows * kActPitch];
     static constexpr bool kJointResident = Cache || Layers == 1 || NU == 4;
     // K pairs of the streamed matrix that fit beside the rest (see weight placement below)
-    static constexpr int kSmemPairs = Layers == 2 && NU == 4 ? (Cache ? 3 : 1) : 0;
+    static constexpr int kSmemPairs = Layers == 1 ? 0 : Cache ? (NU == 4 ? 3 : 2) : (NU == 4 ? 1 : 2);
     static constexpr int kPairBytes = kMatrixWarps * (Cache ? 1 : 2) * 1024;
-    static constexpr int kJointBytes = !kJointResident ? 0 : Cache ? kClJoint * 1344 : 10 * 2 * (4 * 1024 + 128);
+    static constexpr int kJointBytes = !kJointResident ? 0 : Cache ? kClJoint * 1280 : 10 * 2 * (4 * 1024 + 128);
     static constexpr int kGateParts = Cache ? 2 : 4;
 
     alignas(16) uint8_t joint[kJointBytes > 0 ? kJointBytes : 16];
@@ -322,15 +322,15 @@ tdt_cluster_kernel(const DecParams p, const ClWeights w) {
     tc_fence_after_sync();
     // resident joint rows
     if constexpr (Cache) {
-        // row-major, 336 words per row (= 16 mod 32): the two half-warps of a warp read different rows
+        // half-lane hl reads words hl + 16 s, s = 0..19: four of them per 16-byte group [row][s / 4][hl]
         for (int i = tid; i < kClJoint * 80; i += kClThreads) {
             const int n = i / 80, c = i % 80, row = r * kClJoint + n;
             uint4 v = make_uint4(0, 0, 0, 0);
             if (row < kJointRows) {
-                const uint32_t* src = reinterpret_cast<const uint32_t*>(p.w_joint + static_cast<size_t>(row) * kHidden) + c * 4;
-                v = make_uint4(__ldg(src), __ldg(src + 1), __ldg(src + 2), __ldg(src + 3));
+                const uint32_t* src = reinterpret_cast<const uint32_t*>(p.w_joint + static_cast<size_t>(row) * kHidden) + (c / 16) * 64 + c % 16;
+                v = make_uint4(__ldg(src), __ldg(src + 16), __ldg(src + 32), __ldg(src + 48));
             }
-            *reinterpret_cast<uint4*>(sm.joint + n * 1344 + c * 16) = v;
+            *reinterpret_cast<uint4*>(sm.joint + n * 1280 + c * 16) = v;
         }
     } else if constexpr (Smem::kJointResident) {
         const uint4* src = w.joint + static_cast<size_t>(r) * JointSplit::kPerCta;
@@ -566,6 +566,30 @@ tdt_cluster_kernel(const DecParams p, const ClWeights w) {
                 else
                     recurrent0();
             }
+            // the joint rows' fragments do not depend on the activations: requested before the wait (all of them
+            // where the registers allow it)
+            constexpr int kAhead = Cache || (Layers == 2 && NU == 4) ? 0 : NU == 4 ? JointSplit::KP : 1;
+            [[maybe_unused]] const int jkg = warp / JointSplit::NG, jng = warp % JointSplit::NG;
+            [[maybe_unused]] uint4 jf[JointSplit::KP][3][2];
+            [[maybe_unused]] uint32_t jt[16];                      // the pair that lives in tensor memory
+            auto joint_fetch = [&](int kp) {
+                const uint4* block = Smem::kJointResident
+                    ? reinterpret_cast<const uint4*>(sm.joint) + (jkg * JointSplit::KP + kp) * (256 + 8)
+                    : w.joint + static_cast<size_t>(r) * JointSplit::kPerCta + (jkg * JointSplit::KP + kp) * 320;
+                if (kColsJ > 0 && kp == 0) tmem_ld_32x16(tm + kCols0, jt);
+#pragma unroll
+                for (int step = 0; step < 2; ++step) {
+#pragma unroll
+                    for (int j = 0; j < 2; ++j)
+                        if (kColsJ == 0 || kp > 0) jf[kp][j][step] = block[((jng * 2 + j) * 2 + step) * 32 + lane];
+                    jf[kp][2][step] = jng == 0 && lane < 4 ? block[256 + (Smem::kJointResident ? step * 4 : step * 32) + lane]
+                                                           : make_uint4(0, 0, 0, 0);
+                }
+            };
+            if constexpr (!Cache) {
+#pragma unroll
+                for (int kp = 0; kp < kAhead; ++kp) joint_fetch(kp);
+            }
             mbar_wait_bounded(&sm.abar, round & 1u, abort_flag);
             if (need8 != 0ull) hphase ^= 1u;
             // ---- joint rows
@@ -575,20 +599,24 @@ tdt_cluster_kernel(const DecParams p, const ClWeights w) {
                 // then a shuffle tree.  Rows hw and hw + 40 share the loads of x.
                 const int hw = tid / 16, hl = tid % 16;
                 const bool second = hw + 40 < kClJoint;
-                const uint32_t* w0 = reinterpret_cast<const uint32_t*>(sm.joint + hw * 1344) + hl;
-                const uint32_t* w1 = reinterpret_cast<const uint32_t*>(sm.joint + (second ? hw + 40 : hw) * 1344) + hl;
+                const uint4* w0 = reinterpret_cast<const uint4*>(sm.joint + hw * 1280) + hl;
+                const uint4* w1 = reinterpret_cast<const uint4*>(sm.joint + (second ? hw + 40 : hw) * 1280) + hl;
                 for (int u = 0; u < U; ++u) {
                     if (((done8 >> (8 * u)) & 1ull) != 0ull) continue;
                     const float* x = reinterpret_cast<const float*>(sm.ax) + u * kHidden + 2 * hl;
                     float s0 = hl == 0 ? sm.joint_bias[hw] : 0.0f, s1 = hl == 0 && second ? sm.joint_bias[hw + 40] : 0.0f;
 #pragma unroll
-                    for (int st = 0; st < 20; ++st) {
-                        const float2 xv = *reinterpret_cast<const float2*>(x + 32 * st);
-                        const uint32_t a = w0[16 * st], b = w1[16 * st];
-                        const float2 av = __half22float2(*reinterpret_cast<const __half2*>(&a));
-                        const float2 bv = __half22float2(*reinterpret_cast<const __half2*>(&b));
-                        s0 = fmaf(av.y, xv.y, fmaf(av.x, xv.x, s0));
-                        s1 = fmaf(bv.y, xv.y, fmaf(bv.x, xv.x, s1));
+                    for (int q = 0; q < 5; ++q) {
+                        const uint4 a4 = w0[16 * q], b4 = w1[16 * q];
+                        const uint32_t a[4] = {a4.x, a4.y, a4.z, a4.w}, b[4] = {b4.x, b4.y, b4.z, b4.w};
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const float2 xv = *reinterpret_cast<const float2*>(x + 32 * (4 * q + i));
+                            const float2 av = __half22float2(*reinterpret_cast<const __half2*>(&a[i]));
+                            const float2 bv = __half22float2(*reinterpret_cast<const __half2*>(&b[i]));
+                            s0 = fmaf(av.y, xv.y, fmaf(av.x, xv.x, s0));
+                            s1 = fmaf(bv.y, xv.y, fmaf(bv.x, xv.x, s1));
+                        }
                     }
 #pragma unroll
                     for (int off = 8; off > 0; off /= 2) {
@@ -601,32 +629,21 @@ tdt_cluster_kernel(const DecParams p, const ClWeights w) {
                     }
                 }
             } else {
-                const int kg = warp / JointSplit::NG, ng = warp % JointSplit::NG;
                 float acc[3][NB][4] = {};
 #pragma unroll
                 for (int kp = 0; kp < JointSplit::KP; ++kp) {
-                    const uint4* block = Smem::kJointResident
-                        ? reinterpret_cast<const uint4*>(sm.joint) + (kg * JointSplit::KP + kp) * (256 + 8)
-                        : w.joint + static_cast<size_t>(r) * JointSplit::kPerCta + (kg * JointSplit::KP + kp) * 320;
-                    [[maybe_unused]] uint32_t f[16];
-                    if constexpr (kColsJ > 0)
-                        if (kp == 0) {
-                            tmem_ld_32x16(tm + kCols0, f);
-                            tmem_ld_wait();
-                        }
-                    pair_mma<false, 3, NB>(acc, sm.ax + (kg * JointSplit::KP + kp) * 64 + lane_act, kPitch, ng == 0 ? 3 : 2,
+                    if (kp >= kAhead) joint_fetch(kp);
+                    if (kColsJ > 0 && kp == 0) tmem_ld_wait();
+                    pair_mma<false, 3, NB>(acc, sm.ax + (jkg * JointSplit::KP + kp) * 64 + lane_act, kPitch, jng == 0 ? 3 : 2,
                                            [&](int j, int step) {
-                        if constexpr (kColsJ > 0)
-                            if (kp == 0 && j < 2)
-                                return make_uint4(f[j * 8 + step * 4], f[j * 8 + step * 4 + 1], f[j * 8 + step * 4 + 2], f[j * 8 + step * 4 + 3]);
-                        if (j < 2) return block[((ng * 2 + j) * 2 + step) * 32 + lane];
-                        return lane < 4 ? block[256 + (Smem::kJointResident ? step * 4 : step * 32) + lane] : make_uint4(0, 0, 0, 0);
+                        const int i = (j * 2 + step) * 4;
+                        return kColsJ > 0 && kp == 0 && j < 2 ? make_uint4(jt[i], jt[i + 1], jt[i + 2], jt[i + 3]) : jf[kp][j][step];
                     });
                 }
 #pragma unroll
                 for (int j = 0; j < 3; ++j)
-                    if (j < 2 || ng == 0)
-                        store_part<false, NB, NU>(acc[j], sm.part, kg, (j < 2 ? ng * 2 + j : 4) * 16, kClJoint, kJointPitch, lane);
+                    if (j < 2 || jng == 0)
+                        store_part<false, NB, NU>(acc[j], sm.part, jkg, (j < 2 ? jng * 2 + j : 4) * 16, kClJoint, kJointPitch, lane);
             }
             __syncthreads();
             publish_keys(done8);
@@ -684,7 +701,8 @@ tdt_cluster_kernel(const DecParams p, const ClWeights w) {
         const int total_frames = live ? min(p.frames[my], p.seg_stride) : 0;   // never past the utterance's block
         const __half* enc_rows = p.enc_proj + static_cast<size_t>(serving ? my : 0) * p.seg_stride * kHidden + r * kClUnits;
         int frame = 0, symbols = 0, count = 0;
-        float cell0[kPasses] = {}, cell1[kPasses] = {}, pred[kPasses] = {}, xg[kPasses][4] = {}, enc[kPasses] = {};
+        float cell0[kPasses] = {}, cell1[kPasses] = {}, pred[kPasses] = {}, xg[kPasses][4] = {};
+        __half enc[kPasses] = {};                                          // (converted where used: the load stays in flight)
         auto for_slots = [&](auto&& f) {                                   // f(pass, slot)
 #pragma unroll
             for (int i = 0; i < kPasses; ++i) {
@@ -693,7 +711,7 @@ tdt_cluster_kernel(const DecParams p, const ClWeights w) {
             }
         };
         auto fetch_enc = [&]() {
-            for_slots([&](int i, int slot) { enc[i] = __half2float(enc_rows[static_cast<size_t>(frame) * kHidden + slot]); });
+            for_slots([&](int i, int slot) { enc[i] = __ldg(enc_rows + static_cast<size_t>(frame) * kHidden + slot); });
         };
         if (live) fetch_enc();
         // LSTM cell of one unit from its four gate sums; stages h for the exchange
@@ -822,7 +840,7 @@ tdt_cluster_kernel(const DecParams p, const ClWeights w) {
                         for (int kg = 0; kg < PredSplit::KG; ++kg) pred[i] += part[kg];
                     }
                 }
-                const float x = fmaxf(enc[i] + pred[i], 0.0f);
+                const float x = fmaxf(__half2float(enc[i]) + pred[i], 0.0f);
                 if constexpr (Cache) {
                     sm.stage_f[my][slot] = x;
                 } else {

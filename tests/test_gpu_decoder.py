@@ -301,3 +301,33 @@ def test_rounds_whose_scores_are_all_nan_decode_as_blank(pk, cuda, kernel):
     assert int(dec.status.item()) & 4
     dec.status.zero_()
     assert not host(counts).any()
+
+
+@pytest.mark.parametrize("cache", ["fp16", "int8"])
+@pytest.mark.parametrize("layers", [1, 2])
+def test_team_sizes_give_the_tokens_of_single_utterances(pk, cuda, layers, cache):
+    """The cluster kernel serves an utterance with 4, 2 or 1 control warps and has variants for up to 4
+    and up to 8 utterances: every batch size decodes like its utterances alone (ragged lengths, one of
+    them empty), with random blanks in between."""
+    w = pk.synth.decoder_weights(21, layers)
+    w["b_joint"] = w["b_joint"].copy()
+    w["b_joint"][1024] += 0.8                        # blanks often enough to cover rounds without an LSTM step
+    dec = pk.decoder.TdtDecoder(w, cuda)
+    frames, stride = [90, 41, 128, 1, 77, 0, 120, 63], 128
+    rng = np.random.default_rng(9)
+    proj = dev16(rng.standard_normal((8 * stride, 640)) * 0.7)
+    alone = []
+    for u, f in enumerate(frames):
+        t, d, c = dec.decode(proj[u * stride:(u + 1) * stride], 1, stride, torch.tensor([f], dtype=torch.int32, device=cuda),
+                             1280, kernel="cluster", lstm_cache=cache)
+        n = int(c[0])
+        alone.append((host(t)[0, :n], host(d)[0, :n]))
+    assert any(len(t) > 20 for t, _ in alone)
+    for n in (2, 3, 4, 5, 8):
+        t, d, c = dec.decode(proj[:n * stride], n, stride, torch.tensor(frames[:n], dtype=torch.int32, device=cuda), 1280,
+                             kernel="cluster", lstm_cache=cache)
+        torch.cuda.synchronize()
+        assert int(dec.status.item()) == 0
+        for u in range(n):
+            k = int(c[u])
+            assert np.array_equal(host(t)[u, :k], alone[u][0]) and np.array_equal(host(d)[u, :k], alone[u][1])
