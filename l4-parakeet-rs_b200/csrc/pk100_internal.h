@@ -47,6 +47,26 @@ static inline void pk100_launch_chained(void (*kernel)(Params...), dim3 grid, di
     cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
 }
 
+// Row geometry of a batch: uniform blocks of seg_stride rows per utterance (tiles == nullptr), or a packed
+// batch in which every utterance takes whole 128-row tiles: tiles[row / 128] = {first row of the tile's
+// utterance, its valid rows}.
+struct pk100_rows {
+    const int2* tiles;
+    int seg_stride, valid_rows;
+    const int* seg_valid;
+};
+
+// The row-wise operators behind the C entry points, on either geometry (total_rows: a multiple of 128 when
+// packed).  Arguments are the entry points', already checked.
+int pk100_layer_norm_rows(void* stream, const void* input, const void* gamma, const void* beta, void* output, float* scales,
+                          int mode, float inv_scale, int total_rows, const pk100_rows& geometry, float eps);
+int pk100_layer_norm_pair_rows(void* stream, const void* input, const void* gamma, const void* beta, void* output,
+                               const void* next_gamma, const void* next_beta, void* next_output, float* next_scales,
+                               int next_mode, float next_inv_scale, int total_rows, const pk100_rows& geometry, float eps);
+int pk100_depthwise_bn_silu_rows(void* stream, const void* input, const void* dw_weight, const float* bn_gamma, const float* bn_beta,
+                                 const float* bn_mean, const float* bn_var, void* output, float* row_scales, int quantize,
+                                 int total_rows, int segments, const pk100_rows& geometry, float eps);
+
 // 2-D TMA descriptor of a row-major matrix [rows, cols] (`ld` elements between rows) with a box of
 // [box_rows, swizzle_bytes / elem_bytes] elements; served from the library's descriptor cache
 // (gemm_host.cu).  `map` points to a CUtensorMap.

@@ -7,8 +7,11 @@
 #include <cuda_fp8.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "pk100_internal.h"
 #include "ptx_sm100.cuh"
+#include "row_quant.cuh"
 
 namespace pk100 {
 
@@ -73,10 +76,41 @@ __device__ __forceinline__ int segment_valid(const int* seg_valid, int seg, int 
     return seg_valid != nullptr ? seg_valid[seg] : valid_rows;
 }
 
+// Where a row lies in its utterance.  Uniform batches: segment s owns rows [s*seg_stride, (s+1)*seg_stride),
+// its first seg_valid[s] (or the uniform valid_rows) rows carry data.  Packed batches: `tiles` gives per
+// 128-row tile the first row of the utterance it belongs to and that utterance's row count.
+__device__ __forceinline__ bool row_live(const pk100_rows& g, int row) {
+    if (g.tiles != nullptr) {
+        const int2 t = __ldg(g.tiles + row / 128);
+        return row - t.x < t.y;
+    }
+    const int seg = row / g.seg_stride;
+    return row - seg * g.seg_stride < segment_valid(g.seg_valid, seg, g.valid_rows);
+}
+
 // ------------------------------------------------------------- LayerNorm
-// Normalise one row held as 4 x 8 values per lane; returns f16-rounded values.
-__device__ __forceinline__ void normalise_row(float (&x)[4][8], const __half* gamma,
-                                              const __half* beta, int lane, float eps) {
+// gamma and beta of this lane's 32 columns (column i * 256 + lane * 8 + j), packed
+struct NormVectors {
+    uint4 g[4], b[4];
+    // `volatile`: stays where it is written, so that the second norm's vectors are fetched per row (from L1)
+    // instead of being held across the row loop, which spills
+    static __device__ __forceinline__ uint4 fetch(const __half* p) {
+        uint4 v;
+        asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+        return v;
+    }
+    __device__ __forceinline__ void load(const __half* gamma, const __half* beta, int lane) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            g[i] = fetch(gamma + i * 256 + lane * 8);
+            b[i] = fetch(beta + i * 256 + lane * 8);
+        }
+    }
+};
+
+// Normalise one row held as 4 x 8 values per lane; the results are rounded to fp16 (`h`, packed) and
+// left in x.  The order of the sums (a lane's 32 values in column order, then the butterfly) is fixed.
+__device__ __forceinline__ void normalise_row(float (&x)[4][8], uint4 (&h)[4], const NormVectors& v, float eps) {
     float sum = 0.0f;
 #pragma unroll
     for (int i = 0; i < 4; ++i)
@@ -88,37 +122,56 @@ __device__ __forceinline__ void normalise_row(float (&x)[4][8], const __half* ga
     for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            const float d = x[i][j] - mean;
-            sq = fmaf(d, d, sq);
+            x[i][j] -= mean;
+            sq = fmaf(x[i][j], x[i][j], sq);
         }
     const float rstd = rsqrtf(warp_sum_all(sq) * (1.0f / kWidth) + eps);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        const int col = i * 256 + lane * 8;
         float g[8], b[8];
-        unpack8(*reinterpret_cast<const uint4*>(gamma + col), g);
-        unpack8(*reinterpret_cast<const uint4*>(beta + col), b);
+        unpack8(v.g[i], g);
+        unpack8(v.b[i], b);
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-            x[i][j] = __half2float(__float2half_rn((x[i][j] - mean) * rstd * g[j] + b[j]));
+        for (int j = 0; j < 8; ++j) x[i][j] = fmaf(x[i][j] * rstd, g[j], b[j]);
+        h[i] = pack8(x[i]);
+        unpack8(h[i], x[i]);
     }
 }
 
+// largest |value| of the row from the packed fp16 values
+__device__ __forceinline__ float row_absmax(const uint4 (&h)[4]) {
+    __half2 mx = __habs2(*reinterpret_cast<const __half2*>(&h[0].x));
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t w[4] = {h[i].x, h[i].y, h[i].z, h[i].w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) mx = __hmax2(mx, __habs2(*reinterpret_cast<const __half2*>(&w[j])));
+    }
+    // non-negative floats order like their bits
+    const float2 m = __half22float2(mx);
+    return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(m.x, m.y))));
+}
+
+// four INT8 codes rne(q) of |q| <= 127 in one word: adding 1.5 * 2^23 leaves the integer in the low mantissa bits
+__device__ __forceinline__ uint32_t codes_s8x4(float a, float b, float c, float d) {
+    constexpr float kMagic = 12582912.0f;
+    const uint32_t lo = __byte_perm(__float_as_uint(a + kMagic), __float_as_uint(b + kMagic), 0x0040);
+    const uint32_t hi = __byte_perm(__float_as_uint(c + kMagic), __float_as_uint(d + kMagic), 0x0040);
+    return __byte_perm(lo, hi, 0x5410);
+}
+
 // Write one normalised row in the requested encoding.
-__device__ __forceinline__ void emit_row(const float (&x)[4][8], int mode, float inv_scale,
+template <int Mode>
+__device__ __forceinline__ void emit_row(const float (&x)[4][8], const uint4 (&h)[4], float inv_scale,
                                          void* out, float* scales, size_t row, int lane) {
-    if (mode == PK100_LN_F16) {
+    if constexpr (Mode == PK100_LN_F16) {
         __half* o = reinterpret_cast<__half*>(out) + row * kWidth;
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-            *reinterpret_cast<uint4*>(o + i * 256 + lane * 8) = pack8(x[i]);
+        for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(o + i * 256 + lane * 8) = h[i];
         return;
     }
     uint8_t* o = reinterpret_cast<uint8_t*>(out) + row * kWidth;
-    float mult = inv_scale;
-    bool divide = false;
-    float scale = 1.0f;
-    if (mode == PK100_LN_S4_ROW) {
+    if constexpr (Mode == PK100_LN_S4_ROW) {
         // every signed 4-bit code is used: the scale is the larger of max/7 and -min/8
         float mx = 0.0f;
 #pragma unroll
@@ -126,7 +179,7 @@ __device__ __forceinline__ void emit_row(const float (&x)[4][8], int mode, float
 #pragma unroll
             for (int j = 0; j < 8; ++j) mx = fmaxf(mx, fmaxf(__fdiv_rn(x[i][j], 7.0f), __fdiv_rn(-x[i][j], 8.0f)));
         mx = warp_max_all(mx);
-        scale = mx > 0.0f ? mx : 1.0f;
+        const float scale = mx > 0.0f ? mx : 1.0f;
         if (lane == 0) scales[row] = scale;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -138,78 +191,83 @@ __device__ __forceinline__ void emit_row(const float (&x)[4][8], int mode, float
             }
             *reinterpret_cast<uint2*>(o + i * 256 + lane * 8) = make_uint2(w[0], w[1]);
         }
-        return;
-    }
-    if (mode == PK100_LN_E4M3_ROW || mode == PK100_LN_S8_ROW) {
-        float mx = 0.0f;
+    } else if constexpr (Mode == PK100_LN_E4M3_FIXED) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < 4; ++i) {
+            float q[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) mx = fmaxf(mx, fabsf(x[i][j]));
-        mx = warp_max_all(mx);
-        const float top = mode == PK100_LN_E4M3_ROW ? 448.0f : 127.0f;
-        scale = mx > 0.0f ? __fdiv_rn(mx, top) : 1.0f;
-        if (lane == 0) scales[row] = scale;
-        divide = true;
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        float q[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) q[j] = divide ? __fdiv_rn(x[i][j], scale) : x[i][j] * mult;
-        const uint2 bytes = (mode == PK100_LN_S8_ROW) ? s8x8(q) : e4m3x8(q);
-        *reinterpret_cast<uint2*>(o + i * 256 + lane * 8) = bytes;
-    }
-}
-
-__device__ __forceinline__ void emit_zero_row(int mode, void* out, float* scales, size_t row,
-                                              int lane) {
-    if (mode == PK100_LN_F16) {
-        __half* o = reinterpret_cast<__half*>(out) + row * kWidth;
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-            *reinterpret_cast<uint4*>(o + i * 256 + lane * 8) = make_uint4(0, 0, 0, 0);
+            for (int j = 0; j < 8; ++j) q[j] = x[i][j] * inv_scale;
+            *reinterpret_cast<uint2*>(o + i * 256 + lane * 8) = e4m3x8(q);
+        }
     } else {
-        uint8_t* o = reinterpret_cast<uint8_t*>(out) + row * kWidth;
+        const float mx = row_absmax(h);
+        const float scale = mx > 0.0f ? __fdiv_rn(mx, Mode == PK100_LN_E4M3_ROW ? 448.0f : 127.0f) : 1.0f;
+        if (lane == 0) scales[row] = scale;
+        const RowDivisor div(scale);
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-            *reinterpret_cast<uint2*>(o + i * 256 + lane * 8) = make_uint2(0, 0);
-        if (scales != nullptr && lane == 0) scales[row] = 1.0f;
+        for (int i = 0; i < 4; ++i) {
+            float q[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) q[j] = div(x[i][j]);
+            *reinterpret_cast<uint2*>(o + i * 256 + lane * 8) = Mode == PK100_LN_S8_ROW
+                ? make_uint2(codes_s8x4(q[0], q[1], q[2], q[3]), codes_s8x4(q[4], q[5], q[6], q[7])) : e4m3x8(q);
+        }
     }
 }
 
-// mode / second_mode: PK100_LN_*.  When gamma2 != nullptr a second LayerNorm is
-// applied to the f16-rounded first result and written to out2 (the "pair" form:
-// block-output norm + next block's first norm in one pass over the row).
-__global__ void __launch_bounds__(256)
+template <int Mode>
+__device__ __forceinline__ void emit_zero_row(void* out, float* scales, size_t row, int lane) {
+    constexpr int kBytes = Mode == PK100_LN_F16 ? 2 : 1;
+    uint8_t* o = reinterpret_cast<uint8_t*>(out) + row * kWidth * kBytes;
+#pragma unroll
+    for (int i = 0; i < 2 * kBytes; ++i) *reinterpret_cast<uint4*>(o + i * 512 + lane * 16) = make_uint4(0, 0, 0, 0);
+    if (Mode >= PK100_LN_E4M3_ROW && lane == 0) scales[row] = 1.0f;
+}
+
+// One warp per row, walking the rows of the grid; the next row is requested before the current one is
+// reduced.  Mode / Mode2: PK100_LN_*.  Mode2 >= 0: a second LayerNorm is applied to the f16-rounded
+// first result and written to out2 (the "pair" form: block-output norm + next block's first norm in
+// one pass over the row).  Bound by HBM for large row counts (45 056 rows, 138 MB: INT8 57 -> 38 us, E4M3 43 -> 31 us, pair 69 -> 54 us against one row per
+// warp with full divisions and gamma / beta fetched per row) and by the latency of
+// load, two reductions and store for a few hundred rows.
+template <int Mode, int Mode2>
+__global__ void __launch_bounds__(256, 2)
 layer_norm_kernel(const __half* __restrict__ in, const __half* __restrict__ gamma,
-                  const __half* __restrict__ beta, void* __restrict__ out, float* scales,
-                  int mode, float inv_scale, const __half* __restrict__ gamma2,
-                  const __half* __restrict__ beta2, void* __restrict__ out2, float* scales2,
-                  int mode2, float inv_scale2, int total_rows, int seg_stride, int valid_rows,
-                  const int* __restrict__ seg_valid, float eps) {
+                  const __half* __restrict__ beta, void* __restrict__ out, float* scales, float inv_scale,
+                  const __half* __restrict__ gamma2, const __half* __restrict__ beta2, void* __restrict__ out2,
+                  float* scales2, float inv_scale2, int total_rows, const pk100_rows geometry, float eps) {
+    const int lane = threadIdx.x % 32;
+    const int first = blockIdx.x * 8 + threadIdx.x / 32, step = gridDim.x * 8;
     grid_dependents_launch();
     grid_dependency_wait();
-    const int lane = threadIdx.x % 32;
-    const int row = blockIdx.x * 8 + threadIdx.x / 32;
-    if (row >= total_rows) return;
-    const int seg = row / seg_stride;
-    const int local = row - seg * seg_stride;
-    if (local >= segment_valid(seg_valid, seg, valid_rows)) {
-        emit_zero_row(mode, out, scales, row, lane);
-        if (gamma2 != nullptr) emit_zero_row(mode2, out2, scales2, row, lane);
-        return;
-    }
-    float x[4][8];
-    const __half* src = in + static_cast<size_t>(row) * kWidth;
+    NormVectors v;
+    v.load(gamma, beta, lane);
+    uint4 raw[4];
+    auto request = [&](int row) {
+        const uint4* src = reinterpret_cast<const uint4*>(in + static_cast<size_t>(row) * kWidth) + lane;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-        unpack8(*reinterpret_cast<const uint4*>(src + i * 256 + lane * 8), x[i]);
-    normalise_row(x, gamma, beta, lane, eps);
-    emit_row(x, mode, inv_scale, out, scales, row, lane);
-    if (gamma2 != nullptr) {
-        normalise_row(x, gamma2, beta2, lane, eps);
-        emit_row(x, mode2, inv_scale2, out2, scales2, row, lane);
+        for (int i = 0; i < 4; ++i) raw[i] = src[i * 32];
+    };
+    if (first < total_rows) request(first);
+    for (int row = first; row < total_rows; row += step) {
+        float x[4][8];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) unpack8(raw[i], x[i]);
+        if (row + step < total_rows) request(row + step);
+        if (!row_live(geometry, row)) {
+            emit_zero_row<Mode>(out, scales, row, lane);
+            if constexpr (Mode2 >= 0) emit_zero_row<Mode2>(out2, scales2, row, lane);
+            continue;
+        }
+        uint4 h[4];
+        normalise_row(x, h, v, eps);
+        emit_row<Mode>(x, h, inv_scale, out, scales, row, lane);
+        if constexpr (Mode2 >= 0) {
+            NormVectors v2;
+            v2.load(gamma2, beta2, lane);
+            normalise_row(x, h, v2, eps);
+            emit_row<Mode2>(x, h, inv_scale2, out2, scales2, row, lane);
+        }
     }
 }
 
@@ -443,130 +501,160 @@ __global__ void glu_masked_kernel(const __half* __restrict__ in, __half* __restr
 }
 
 // ------------------------------------------------- depthwise + BN + SiLU
-// One CTA = 256 threads x 4 channels = all 1024 channels of a strip of 8 rows (short strips:
-// 768 CTAs at 6144 rows keep enough loads in flight; the 8 halo rows come from L2).
-// A 9-row window of the thread's 4 channels slides down the strip in registers.
-constexpr int kDwStrip = 8;
+// One CTA = 256 threads x 4 channels = all 1024 channels of a strip of kStrip rows; the 8 halo rows come
+// from L2.  Two neighbouring channels share every packed fp32 instruction (fma.rn.f32x2 and friends,
+// each half rounds like the scalar one).  A window of 9 rows slides down the strip in registers;
+// the row's E4M3 scale takes one warp reduction and one exchange through shared memory.  Long strips read
+// fewer halo rows, short ones keep every SM busy: 16 rows where that gives the device two CTAs per SM,
+// else 8.  Bound by issue slots (convolution, BatchNorm, SiLU and E4M3 rounding of every element).  45 056
+// rows: 155 us with scalar instructions and full divisions, 91 us now; 768 rows: 10.6 -> 6.2 us.
+using Pair = unsigned long long;
+__device__ __forceinline__ Pair pair_of(float lo, float hi) {
+    Pair r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 halves_of(Pair v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ Pair pair_fma(Pair a, Pair b, Pair c) {
+    Pair d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ Pair pair_mul(Pair a, Pair b) {
+    Pair d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ Pair pair_add(Pair a, Pair b) {
+    Pair d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
 
-__global__ void __launch_bounds__(256)
+template <bool Quantize, int kStrip>
+__global__ void __launch_bounds__(256, 2)
 depthwise_bn_silu_kernel(const __half* __restrict__ in, const __half* __restrict__ wdw,
                          const float* __restrict__ bn_gamma, const float* __restrict__ bn_beta,
                          const float* __restrict__ bn_mean, const float* __restrict__ bn_var,
-                         void* __restrict__ out, float* __restrict__ row_scales, int quantize,
-                         int seg_stride, int valid_rows, const int* __restrict__ seg_valid,
-                         float eps) {
-    __shared__ float s_max[8][8];
+                         void* __restrict__ out, float* __restrict__ row_scales, const pk100_rows geometry, float eps) {
+    __shared__ float s_max[kStrip / 8][8][8];
     grid_dependents_launch();
     grid_dependency_wait();
     const int tid = threadIdx.x;
     const int lane = tid % 32, warp = tid / 32;
     const int c0 = tid * 4;
-    const int strips_per_seg = (seg_stride + kDwStrip - 1) / kDwStrip;
-    const int seg = blockIdx.x / strips_per_seg;
-    const int r0 = (blockIdx.x % strips_per_seg) * kDwStrip;
-    const int rows = segment_valid(seg_valid, seg, valid_rows);
-    const size_t base = static_cast<size_t>(seg) * seg_stride;
+    size_t base;                                       // first row of the utterance
+    int r0, rows, stride;                              // this strip's first row in it, its valid rows, its block
+    if (geometry.tiles != nullptr) {
+        const int2 t = __ldg(geometry.tiles + blockIdx.x / (128 / kStrip));
+        base = t.x;
+        r0 = blockIdx.x * kStrip - t.x;
+        rows = t.y;
+        stride = r0 + kStrip;                          // tiles are whole
+    } else {
+        const int strips = (geometry.seg_stride + kStrip - 1) / kStrip, seg = blockIdx.x / strips;
+        base = static_cast<size_t>(seg) * geometry.seg_stride;
+        r0 = (blockIdx.x % strips) * kStrip;
+        rows = segment_valid(geometry.seg_valid, seg, geometry.valid_rows);
+        stride = geometry.seg_stride;
+    }
 
     // this thread's 4 x 9 taps are 72 contiguous bytes (8-byte aligned): 9 vector loads
-    float w[4][9], rstd[4], gam[4], add[4], mean[4];
+    Pair w[9][2], rstd[2], gam[2], add[2], neg_mean[2];
     {
-        __half taps[36];
+        alignas(8) __half taps[36];
         const uint2* src = reinterpret_cast<const uint2*>(wdw + static_cast<size_t>(c0) * 9);
 #pragma unroll
         for (int i = 0; i < 9; ++i) reinterpret_cast<uint2*>(taps)[i] = __ldg(src + i);
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
+        for (int t = 0; t < 9; ++t)
 #pragma unroll
-            for (int t = 0; t < 9; ++t) w[c][t] = __half2float(taps[c * 9 + t]);
+            for (int c = 0; c < 2; ++c) w[t][c] = pair_of(__half2float(taps[(2 * c) * 9 + t]), __half2float(taps[(2 * c + 1) * 9 + t]));
         const float4 var = __ldg(reinterpret_cast<const float4*>(bn_var + c0));
         const float4 g4 = __ldg(reinterpret_cast<const float4*>(bn_gamma + c0));
         const float4 b4 = __ldg(reinterpret_cast<const float4*>(bn_beta + c0));
         const float4 m4 = __ldg(reinterpret_cast<const float4*>(bn_mean + c0));
-        rstd[0] = rsqrtf(var.x + eps); rstd[1] = rsqrtf(var.y + eps);
-        rstd[2] = rsqrtf(var.z + eps); rstd[3] = rsqrtf(var.w + eps);
-        gam[0] = g4.x; gam[1] = g4.y; gam[2] = g4.z; gam[3] = g4.w;
-        add[0] = b4.x; add[1] = b4.y; add[2] = b4.z; add[3] = b4.w;
-        mean[0] = m4.x; mean[1] = m4.y; mean[2] = m4.z; mean[3] = m4.w;
+        rstd[0] = pair_of(rsqrtf(var.x + eps), rsqrtf(var.y + eps)); rstd[1] = pair_of(rsqrtf(var.z + eps), rsqrtf(var.w + eps));
+        gam[0] = pair_of(g4.x, g4.y); gam[1] = pair_of(g4.z, g4.w);
+        add[0] = pair_of(b4.x, b4.y); add[1] = pair_of(b4.z, b4.w);
+        neg_mean[0] = pair_of(-m4.x, -m4.y); neg_mean[1] = pair_of(-m4.z, -m4.w);
     }
 
-    auto load_row = [&](int r, float (&dst)[4]) {
-        if (r >= 0 && r < rows) {
-            const uint2 raw = *reinterpret_cast<const uint2*>(in + (base + r) * kWidth + c0);
-            const __half2* h = reinterpret_cast<const __half2*>(&raw);
-            const float2 a = __half22float2(h[0]), b = __half22float2(h[1]);
-            dst[0] = a.x; dst[1] = a.y; dst[2] = b.x; dst[3] = b.y;
-        } else {
-            dst[0] = dst[1] = dst[2] = dst[3] = 0.0f;
-        }
+    // rows r0 - 4 .. of the window arrive as packed halves; the strip's loads are issued 8 rows at a time
+    auto load_row = [&](int r) {
+        return r >= 0 && r < rows ? *reinterpret_cast<const uint2*>(in + (base + r) * kWidth + c0) : make_uint2(0, 0);
     };
-
-    float win[9][4];
+    auto widen = [&](uint2 raw, Pair (&dst)[2]) {
+        const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&raw.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
+        dst[0] = pair_of(a.x, a.y);
+        dst[1] = pair_of(b.x, b.y);
+    };
+    Pair win[9][2];
+    uint2 ahead[8];
 #pragma unroll
-    for (int t = 0; t < 8; ++t) load_row(r0 - 4 + t, win[t + 1]);   // slots 1..8 = rows r0-4..r0+3
+    for (int t = 0; t < 8; ++t) ahead[t] = load_row(r0 - 4 + t);
+#pragma unroll
+    for (int t = 0; t < 8; ++t) widen(ahead[t], win[t + 1]);            // slots 1..8 = rows r0-4..r0+3
+#pragma unroll
+    for (int t = 0; t < 8; ++t) ahead[t] = load_row(r0 + 4 + t);
 
-    for (int blk = 0; blk < kDwStrip / 8; ++blk) {
-        float y[8][4];
-        float mx[8];
+#pragma unroll 1
+    for (int blk = 0; blk < kStrip / 8; ++blk) {
+        __half2 y[8][2];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const int r = r0 + blk * 8 + i;
-            // slide: drop the oldest row, fetch row r+4
+            // slide: drop the oldest row, take row r + 4
 #pragma unroll
-            for (int t = 0; t < 8; ++t)
+            for (int t = 0; t < 8; ++t) {
+                win[t][0] = win[t + 1][0];
+                win[t][1] = win[t + 1][1];
+            }
+            widen(ahead[i], win[8]);
+            if (blk + 1 < kStrip / 8) ahead[i] = load_row(r + 12);
+            __half2 top = __half2half2(__ushort_as_half(0));
 #pragma unroll
-                for (int c = 0; c < 4; ++c) win[t][c] = win[t + 1][c];
-            load_row(r + 4, win[8]);
-            mx[i] = 0.0f;
+            for (int c = 0; c < 2; ++c) {
+                Pair acc = 0ull;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                float acc = 0.0f;
-#pragma unroll
-                for (int t = 0; t < 9; ++t) acc = fmaf(win[t][c], w[c][t], acc);
-                float v = (acc - mean[c]) * rstd[c] * gam[c] + add[c];
-                v = __fdividef(v, 1.0f + __expf(-v));
-                v = __half2float(__float2half_rn(v));
-                if (r >= rows) v = 0.0f;
-                y[i][c] = v;
-                mx[i] = fmaxf(mx[i], fabsf(v));
+                for (int t = 0; t < 9; ++t) acc = pair_fma(win[t][c], w[t][c], acc);
+                acc = pair_fma(pair_mul(pair_add(acc, neg_mean[c]), rstd[c]), gam[c], add[c]);
+                const float2 v = halves_of(acc);
+                y[i][c] = __floats2half2_rn(__fdividef(v.x, 1.0f + __expf(-v.x)), __fdividef(v.y, 1.0f + __expf(-v.y)));
+                if (r >= rows) y[i][c] = __half2half2(__ushort_as_half(0));
+                top = __hmax2(top, __habs2(y[i][c]));
+            }
+            if constexpr (Quantize) {
+                const float2 m = __half22float2(top);
+                // non-negative floats order like their bits
+                const unsigned mx = __reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(m.x, m.y)));
+                if (lane == 0) s_max[blk][i][warp] = __uint_as_float(mx);
             }
         }
-        if (quantize) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                mx[i] = warp_max_all(mx[i]);
-                if (lane == 0) s_max[warp][i] = mx[i];
-            }
-            __syncthreads();
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                float m = 0.0f;
-#pragma unroll
-                for (int q = 0; q < 8; ++q) m = fmaxf(m, s_max[q][i]);
-                mx[i] = m;
-            }
-            __syncthreads();
-        }
+        if constexpr (Quantize) __syncthreads();
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const int r = r0 + blk * 8 + i;
-            if (r >= seg_stride) continue;
+            if (r >= stride) continue;
             const size_t grow = base + r;
-            if (quantize) {
-                const float scale = mx[i] > 0.0f ? __fdiv_rn(mx[i], 448.0f) : 1.0f;
+            if constexpr (Quantize) {
+                const float4 a = *reinterpret_cast<const float4*>(&s_max[blk][i][0]), b = *reinterpret_cast<const float4*>(&s_max[blk][i][4]);
+                const float mx = fmaxf(fmaxf(fmaxf(a.x, a.y), fmaxf(a.z, a.w)), fmaxf(fmaxf(b.x, b.y), fmaxf(b.z, b.w)));
+                const float scale = mx > 0.0f ? __fdiv_rn(mx, 448.0f) : 1.0f;
+                const RowDivisor div(scale);
                 if (tid == 0) row_scales[grow] = scale;
-                const uint32_t lo = __nv_cvt_float2_to_fp8x2(
-                    make_float2(__fdiv_rn(y[i][0], scale), __fdiv_rn(y[i][1], scale)),
-                    __NV_SATFINITE, __NV_E4M3);
-                const uint32_t hi = __nv_cvt_float2_to_fp8x2(
-                    make_float2(__fdiv_rn(y[i][2], scale), __fdiv_rn(y[i][3], scale)),
-                    __NV_SATFINITE, __NV_E4M3);
-                *reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(out) + grow * kWidth + c0) =
-                    lo | (hi << 16);
+                const float2 p = __half22float2(y[i][0]), q = __half22float2(y[i][1]);
+                const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(div(p.x), div(p.y)), __NV_SATFINITE, __NV_E4M3);
+                const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(div(q.x), div(q.y)), __NV_SATFINITE, __NV_E4M3);
+                *reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(out) + grow * kWidth + c0) = lo | (hi << 16);
             } else {
                 uint2 raw;
-                __half2* h = reinterpret_cast<__half2*>(&raw);
-                h[0] = __floats2half2_rn(y[i][0], y[i][1]);
-                h[1] = __floats2half2_rn(y[i][2], y[i][3]);
+                raw.x = *reinterpret_cast<const uint32_t*>(&y[i][0]);
+                raw.y = *reinterpret_cast<const uint32_t*>(&y[i][1]);
                 *reinterpret_cast<uint2*>(reinterpret_cast<__half*>(out) + grow * kWidth + c0) = raw;
             }
         }
@@ -578,6 +666,50 @@ depthwise_bn_silu_kernel(const __half* __restrict__ in, const __half* __restrict
 // ------------------------------------------------------------ C-ABI entry
 using namespace pk100;
 
+// Rows per launch beyond one per resident warp are walked by the same warps.
+template <int Mode, int Mode2>
+static int launch_layer_norm(void* stream, const void* input, const void* gamma, const void* beta, void* output, float* scales,
+                             float inv_scale, const void* gamma2, const void* beta2, void* output2, float* scales2,
+                             float inv_scale2, int total_rows, const pk100_rows& geometry, float eps) {
+    auto kernel = layer_norm_kernel<Mode, Mode2>;
+    static std::atomic<int> resident{0};
+    if (resident.load(std::memory_order_relaxed) == 0) {
+        int per_sm = 0;
+        const cudaError_t err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 256, 0);
+        if (err != cudaSuccess) return static_cast<int>(err);
+        resident.store(148 * (per_sm > 0 ? per_sm : 1), std::memory_order_relaxed);
+    }
+    const int blocks = (total_rows + 7) / 8, cap = resident.load(std::memory_order_relaxed);
+    pk100_launch_chained(kernel, dim3(blocks < cap ? blocks : cap), dim3(256), 0, static_cast<cudaStream_t>(stream),
+        static_cast<const __half*>(input), static_cast<const __half*>(gamma), static_cast<const __half*>(beta), output, scales,
+        inv_scale, static_cast<const __half*>(gamma2), static_cast<const __half*>(beta2), output2, scales2, inv_scale2,
+        total_rows, geometry, eps);
+    return pk100_launch_status();
+}
+
+int pk100_layer_norm_rows(void* stream, const void* input, const void* gamma, const void* beta, void* output, float* scales,
+                          int mode, float inv_scale, int total_rows, const pk100_rows& geometry, float eps) {
+#define PK_LN(M) case M: return launch_layer_norm<M, -1>(stream, input, gamma, beta, output, scales, inv_scale, nullptr, \
+                                                         nullptr, nullptr, nullptr, 0.0f, total_rows, geometry, eps)
+    switch (mode) {
+    PK_LN(PK100_LN_F16); PK_LN(PK100_LN_E4M3_FIXED); PK_LN(PK100_LN_E4M3_ROW); PK_LN(PK100_LN_S8_ROW); PK_LN(PK100_LN_S4_ROW);
+    default: return PK100_ERR_SHAPE;
+    }
+#undef PK_LN
+}
+
+int pk100_layer_norm_pair_rows(void* stream, const void* input, const void* gamma, const void* beta, void* output,
+                               const void* next_gamma, const void* next_beta, void* next_output, float* next_scales,
+                               int next_mode, float next_inv_scale, int total_rows, const pk100_rows& geometry, float eps) {
+#define PK_LN(M) case M: return launch_layer_norm<PK100_LN_F16, M>(stream, input, gamma, beta, output, nullptr, 0.0f, next_gamma, \
+                                                                   next_beta, next_output, next_scales, next_inv_scale, total_rows, geometry, eps)
+    switch (next_mode) {
+    PK_LN(PK100_LN_F16); PK_LN(PK100_LN_E4M3_FIXED); PK_LN(PK100_LN_E4M3_ROW); PK_LN(PK100_LN_S8_ROW); PK_LN(PK100_LN_S4_ROW);
+    default: return PK100_ERR_SHAPE;
+    }
+#undef PK_LN
+}
+
 extern "C" int pk100_layer_norm(void* stream, const void* input, const void* gamma,
                                 const void* beta, void* output, float* scales, int mode,
                                 float inv_scale, int total_rows, int seg_stride, int valid_rows,
@@ -586,11 +718,8 @@ extern "C" int pk100_layer_norm(void* stream, const void* input, const void* gam
     if (total_rows <= 0) return total_rows == 0 ? PK100_OK : PK100_ERR_SHAPE;
     if (seg_stride <= 0 || mode < 0 || mode > PK100_LN_S4_ROW) return PK100_ERR_SHAPE;
     if (mode >= PK100_LN_E4M3_ROW && !scales) return PK100_ERR_NULL;
-    pk100_launch_chained(layer_norm_kernel, dim3((total_rows + 7) / 8), dim3(256), 0, static_cast<cudaStream_t>(stream),
-        static_cast<const __half*>(input), static_cast<const __half*>(gamma),
-        static_cast<const __half*>(beta), output, scales, mode, inv_scale, nullptr, nullptr,
-        nullptr, nullptr, 0, 0.0f, total_rows, seg_stride, valid_rows, seg_valid, eps);
-    return pk100_launch_status();
+    return pk100_layer_norm_rows(stream, input, gamma, beta, output, scales, mode, inv_scale, total_rows,
+                                 pk100_rows{nullptr, seg_stride, valid_rows, seg_valid}, eps);
 }
 
 extern "C" int pk100_layer_norm_pair(void* stream, const void* input, const void* gamma,
@@ -605,12 +734,9 @@ extern "C" int pk100_layer_norm_pair(void* stream, const void* input, const void
     if (seg_stride <= 0 || next_mode < 0 || next_mode > PK100_LN_S4_ROW) return PK100_ERR_SHAPE;
     if (next_mode >= PK100_LN_E4M3_ROW && !next_scales)
         return PK100_ERR_NULL;
-    pk100_launch_chained(layer_norm_kernel, dim3((total_rows + 7) / 8), dim3(256), 0, static_cast<cudaStream_t>(stream),
-        static_cast<const __half*>(input), static_cast<const __half*>(gamma),
-        static_cast<const __half*>(beta), output, nullptr, PK100_LN_F16, 0.0f,
-        static_cast<const __half*>(next_gamma), static_cast<const __half*>(next_beta), next_output,
-        next_scales, next_mode, next_inv_scale, total_rows, seg_stride, valid_rows, seg_valid, eps);
-    return pk100_launch_status();
+    return pk100_layer_norm_pair_rows(stream, input, gamma, beta, output, next_gamma, next_beta, next_output, next_scales,
+                                      next_mode, next_inv_scale, total_rows,
+                                      pk100_rows{nullptr, seg_stride, valid_rows, seg_valid}, eps);
 }
 
 extern "C" int pk100_quantize_fp8_fixed(void* stream, const void* input, void* output,
@@ -709,6 +835,22 @@ extern "C" int pk100_glu_masked(void* stream, const void* input, void* output, i
     return pk100_launch_status();
 }
 
+int pk100_depthwise_bn_silu_rows(void* stream, const void* input, const void* dw_weight, const float* bn_gamma, const float* bn_beta,
+                                 const float* bn_mean, const float* bn_var, void* output, float* row_scales, int quantize,
+                                 int total_rows, int segments, const pk100_rows& geometry, float eps) {
+    auto launch = [&](auto kernel, int strip) {
+        const int per_segment = geometry.tiles != nullptr ? 0 : (geometry.seg_stride + strip - 1) / strip;
+        const int blocks = geometry.tiles != nullptr ? total_rows / strip : segments * per_segment;
+        pk100_launch_chained(kernel, dim3(blocks), dim3(256), 0, static_cast<cudaStream_t>(stream),
+            static_cast<const __half*>(input), static_cast<const __half*>(dw_weight), bn_gamma, bn_beta, bn_mean, bn_var, output,
+            row_scales, geometry, eps);
+        return pk100_launch_status();
+    };
+    const bool wide = total_rows >= 2 * 148 * 16;
+    if (quantize) return wide ? launch(depthwise_bn_silu_kernel<true, 16>, 16) : launch(depthwise_bn_silu_kernel<true, 8>, 8);
+    return wide ? launch(depthwise_bn_silu_kernel<false, 16>, 16) : launch(depthwise_bn_silu_kernel<false, 8>, 8);
+}
+
 extern "C" int pk100_depthwise_bn_silu(void* stream, const void* input, const void* dw_weight,
                                        const float* bn_gamma, const float* bn_beta,
                                        const float* bn_mean, const float* bn_var, void* output,
@@ -724,10 +866,6 @@ extern "C" int pk100_depthwise_bn_silu(void* stream, const void* input, const vo
     if (misaligned(dw_weight, 7) || misaligned(bn_gamma, 15) || misaligned(bn_beta, 15) ||
         misaligned(bn_mean, 15) || misaligned(bn_var, 15) || misaligned(input, 7))
         return PK100_ERR_ALIGN;      // the kernel reads taps 8 bytes and BatchNorm vectors 16 bytes at a time
-    const int strips = (seg_stride + kDwStrip - 1) / kDwStrip;
-    pk100_launch_chained(depthwise_bn_silu_kernel, dim3(segments * strips), dim3(256), 0, static_cast<cudaStream_t>(stream),
-        static_cast<const __half*>(input), static_cast<const __half*>(dw_weight), bn_gamma,
-        bn_beta, bn_mean, bn_var, output, row_scales, quantize, seg_stride, valid_rows, seg_valid,
-        eps);
-    return pk100_launch_status();
+    return pk100_depthwise_bn_silu_rows(stream, input, dw_weight, bn_gamma, bn_beta, bn_mean, bn_var, output, row_scales, quantize,
+                                        segments * seg_stride, segments, pk100_rows{nullptr, seg_stride, valid_rows, seg_valid}, eps);
 }

@@ -177,3 +177,43 @@ def test_depthwise_bn_silu(pk, cuda, seg_stride, valid):
         wq, ws = O.quant_rows_fp8_dynamic(got[blk], valid)
         assert np.array_equal(gs[blk], ws)
         assert np.array_equal(gq[blk], wq)
+
+
+@pytest.mark.parametrize("rows,stride,valid", [(9, 9, 9), (2369, 2369, 2368), (5120, 640, 601)])
+def test_row_codes_are_those_of_a_full_division(pk, cuda, rows, stride, valid):
+    """The per-row quantisers of LayerNorm divide by three multiply-adds per element; pack_weight_rows divides
+    in full: codes and scales of both must be equal bit for bit, for one row per warp and for several
+    (2368 = the rows of one row per resident warp)."""
+    L = pk.lib
+    g, b = _affine(5)
+    g[:64], b[:64] = 0.0, -0.0                      # exact zeros of both signs among the values
+    x = dev16(_rows(rows, rows, 2.0))
+    args = dict(seg_stride=stride, valid_rows=valid)
+    y, _ = pk.ops.layer_norm(x, dev16(g), dev16(b), L.LN_F16, **args)
+    for mode, fmt in ((L.LN_E4M3_ROW, L.PACK_E4M3), (L.LN_S8_ROW, L.PACK_S8)):
+        q, s = pk.ops.layer_norm(x, dev16(g), dev16(b), mode, **args)
+        want, ws = pk.ops.pack_weight_rows(y, fmt)
+        assert torch.equal(s, ws) and torch.equal(q.view(torch.uint8), want.view(torch.uint8))
+        y1, q2, s2 = pk.ops.layer_norm_pair(x, dev16(g), dev16(b), dev16(g), dev16(b), mode, **args)
+        again, sa = pk.ops.layer_norm(y, dev16(g), dev16(b), mode, **args)
+        assert torch.equal(y1, y) and torch.equal(q2, again) and torch.equal(s2, sa)
+
+
+@pytest.mark.parametrize("segments,stride,valid", [(1, 24, 21), (3, 136, 130), (1, 4736, 4733), (37, 133, 129)])
+def test_depthwise_strips_and_codes(pk, cuda, segments, stride, valid):
+    """8-row strips below 4736 rows, 16-row strips from there on, strides that cut a strip: the fp16 output
+    of a batch equals that of its segments alone, and the codes are those of a full division."""
+    L = pk.lib
+    rng = np.random.default_rng(stride)
+    x = dev16(rng.standard_normal((segments * stride, 1024)))
+    w = dev16(rng.standard_normal((1024, 9)) * 0.3)
+    bn = [dev(a.astype(np.float32)) for a in (1 + 0.1 * rng.standard_normal(1024), 0.1 * rng.standard_normal(1024),
+                                              0.1 * rng.standard_normal(1024), 1 + 0.2 * rng.random(1024))]
+    y, _ = pk.ops.depthwise_bn_silu(x, w, *bn, seg_stride=stride, valid_rows=valid)
+    q, s = pk.ops.depthwise_bn_silu(x, w, *bn, quantize=True, seg_stride=stride, valid_rows=valid)
+    want, ws = pk.ops.pack_weight_rows(y, L.PACK_E4M3)
+    assert torch.equal(s, ws) and torch.equal(q, want)
+    for u in (0, segments - 1):
+        rows = slice(u * stride, u * stride + valid)
+        alone, _ = pk.ops.depthwise_bn_silu(x[rows].contiguous(), w, *bn)
+        assert torch.equal(alone, y[rows]) and not bool(y[u * stride + valid:(u + 1) * stride].any())
