@@ -5,22 +5,32 @@
 //   ctx = sum_k p . V_k  (definition: local_attention_simple_kernel; reference:
 //   kernels/sm89/encoder.cu:1338-1461, tensor-core form :1500-2035).
 //
-// One CTA = 128 consecutive queries of one head of one utterance; their keys lie in a window of
-// 384 rows.  The three contractions run as tcgen05.mma kind::f16 (M = 128) with fp32 accumulators in
-// tensor memory:
+// A tile = 128 consecutive queries of one head of one utterance; their keys lie in a window of three
+// 128-key blocks, of which the ones outside the utterance are left out.  The kernel is persistent: a CTA
+// takes a contiguous range of (head, tile) items.  The contractions run as tcgen05.mma kind::f16 (M = 128)
+// with fp32 accumulators in tensor memory:
 //     QP = Q . P_h^T   (N = 128 + 128 + 16: the 257 position rows)   TMEM columns [0, 272)
-//     S  = Q . K^T     (three key blocks of N = 128)                 [384, 512), [0, 128), [128, 256)
-//     O  = Pr . V      (Pr = softmax probabilities, fp16, K = keys)  [256, 384)
+//     S  = Q . K^T     (key blocks of N = 128)                       [384, 512), [0, 128), [128, 256)
+//     O  = Pr . V      (Pr = softmax probabilities, fp16, K = keys)  [384, 512), when S_0 has been read
 // Operands arrive by TMA (cp.async.bulk.tensor, 128-byte swizzle, no multicast) into three 32 KB slots
 // that hold blocks of P_h, then K, then V in turn, each load issued as soon as its slot is free.  Q, P
 // and K are K-major operands; V is used as it lies in memory (rows = keys = the K dimension of
 // Pr . V, features contiguous), i.e. as an MN-major B operand: instruction-descriptor bit 16, and a
 // shared-memory descriptor whose leading-dimension offset is the distance between the two 64-feature
 // atoms and whose stride is the 1024 bytes between 8-key groups.  The u / v biases are added in fp32
-// outside the MMAs (u . K_k and v . P_j are per-column constants).  QP is drained to shared memory as fp16 so that the relative shift is a plain
-// gather (key kk of query ql reads column kk - ql).  The softmax is two passes over the S accumulators
-// (row maximum, then exponentials) by sixteen warps, four per TMEM lane quadrant; the probabilities go
-// back through swizzled shared memory as the A operand of the last contraction.
+// outside the MMAs (u . K_k and v . P_j are per-column constants; v . P_j is formed once per head, u . K_k
+// once per key block while the tiles of a CTA follow each other).  QP is drained to shared memory as fp16
+// so that the relative shift is a plain gather (key kk of query ql reads column kk - ql).  The softmax is
+// two passes by sixteen warps, four per TMEM lane quadrant: the first forms the scaled, masked scores,
+// writes them back over the accumulators and takes the row maximum, the second reads them and writes the
+// probabilities through swizzled shared memory (the space the position scores had) as the A operand of
+// the last contraction.
+//
+// What bounds it: one tile is a chain of about ten dependent steps with one tile in flight per SM (tensor
+// memory and shared memory are full), so what counts is the length of the chain and what the next tile can
+// start meanwhile.  Q, P and the first key block of the next tile are loaded, and its QP product is issued,
+// while the softmax warps finish this one.
+// ATT_FIGURES
 // Every wait is a bounded mbarrier wait; when one expires the kernel raises the status word and all
 // roles leave through the common teardown (tensor memory freed).
 #include <cuda.h>
@@ -55,32 +65,34 @@ constexpr int kTailBytes = 2 * 16 * 128;  // position rows 256..271
 constexpr int kQpPitch = 274;             // halves per QP row: 137 words, odd, so that the 32 rows of a
                                           // warp fall into 32 different banks
 
-// barrier indices
+// barrier indices; each completes once per tile, the ones of a key block once per tile that has the block
 enum : int {
-    B_IN = 0, B_QP_DONE, B_BIAS_DONE, B_QP_DRAINED,
+    B_Q_IN = 0, B_P_IN, B_VP_DONE, B_QP_DONE, B_QP_DRAINED, B_PASS0_DONE, B_CTX_READ,
     B_K_IN,                    // 3
     B_UK_DONE = B_K_IN + 3,    // 3
     B_S_DONE = B_UK_DONE + 3,  // 3
     B_V_IN = B_S_DONE + 3,     // 3
     B_P_READY = B_V_IN + 3,    // 3
     B_PV_DONE = B_P_READY + 3, // 3
-    B_MAX = B_PV_DONE + 3,     // 4 (one per lane quadrant)
-    B_SUM = B_MAX + 4,         // 4
+    B_SUM = B_PV_DONE + 3,     // 4 (one per lane quadrant)
     B_COUNT = B_SUM + 4
 };
 
-// Operand staging: three 32 KB slots take, in turn, the position rows (slots 0, 1 and the 4 KB tail),
-// the key blocks (K0 -> slot 2 at once, K1 / K2 -> slots 0 / 1 when the position rows are done with)
-// and the value blocks (V_b -> the slot K_b had, when S_b and its bias term are done).
+// Operand staging: three 32 KB slots take, in turn, the position rows (slots 0, 1 and the 4 KB tail), the
+// key blocks (K0 -> slot 2 at once, K1 / K2 -> slots 0 / 1 when the position rows are done with) and the
+// value blocks (V_b -> slot b, when the key block there and its bias term are done).  P_V frees slot 0
+// first, so the next tile's position rows follow the value blocks in order.
 struct Smem {
-    alignas(1024) uint8_t q[kSlotBytes];              // Q tile, later the probability block
+    alignas(1024) uint8_t q[kSlotBytes];
     alignas(1024) uint8_t slot[3][kSlotBytes];
     alignas(1024) uint8_t tail[kTailBytes];
-    alignas(16) __half qp[kTile * kQpPitch + 8];
+    union {
+        alignas(1024) __half qp[kTile * kQpPitch + 8];    // position scores, until the first pass is over
+        alignas(1024) uint8_t pr[2][kSlotBytes];          // probabilities of two key blocks
+    };
     float vp[288];
-    float uk[kWindow];
+    float uk[3][128];                                     // key block i of the utterance -> row i % 3
     alignas(16) float bias_u[kDim];
-    alignas(16) float bias_v[kDim];
     float rowmax[kParts][kTile];
     float rowsum[kParts][kTile];
     uint64_t bar[B_COUNT];
@@ -92,10 +104,52 @@ struct Params {
     const __half* bias_u;     // [8, 128]
     const __half* bias_v;
     __half* out; int ldo;
-    int segments, seg_stride, valid_rows;
-    const int* seg_valid;
+    int tiles;                // 128-row tiles of the batch
+    pk100_rows rows;
     int* status;
 };
+
+// Place of a tile: first row of its utterance, first query inside it, the utterance's valid rows.
+struct TilePlace {
+    int base, q0, valid;
+    __device__ __forceinline__ TilePlace(const pk100_rows& g, int tile) {
+        if (g.tiles != nullptr) {
+            const int2 t = __ldg(g.tiles + tile);
+            base = t.x;
+            valid = t.y;
+        } else {
+            const int seg = tile / (g.seg_stride / kTile);
+            base = seg * g.seg_stride;
+            valid = min(g.seg_valid != nullptr ? __ldg(g.seg_valid + seg) : g.valid_rows, g.seg_stride);
+        }
+        q0 = tile * kTile - base;
+    }
+    __device__ __forceinline__ bool padding() const { return q0 >= valid; }
+    // key blocks that have keys: bit b = rows q0 - 128 + 128 b .. of the utterance
+    __device__ __forceinline__ uint32_t blocks() const {
+        return 2u | (q0 > 0 ? 1u : 0u) | (q0 + kTile < valid ? 4u : 0u);
+    }
+};
+
+// two fp32 values per instruction, each half rounded like the scalar operation
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+    uint64_t v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
+    return v;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
 
 // byte offset of 16-byte chunk `chunk` (0..7) of row `row` inside a [rows x 64 halves] swizzled atom
 __device__ __forceinline__ int swz(int row, int chunk) {
@@ -120,13 +174,12 @@ __device__ __forceinline__ float bias_dot32(const uint8_t* atom, int row, int fi
     return acc0 + acc1;
 }
 
-// One copy of the polling loop for the whole kernel: the code of a CTA runs once, front to back,
-// so its time is largely instruction fetch; every loop below is kept rolled for the same reason.
-__device__ __noinline__ bool att_wait(uint64_t* bar, volatile int* abort_flag) {
-    return mbar_wait_bounded(bar, 0u, abort_flag);
+// One copy of the polling loop for the whole kernel (it is inlined nowhere: the roles wait at some thirty places).
+__device__ __noinline__ bool att_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+    return mbar_wait_bounded(bar, parity, abort_flag);
 }
-#define ATT_WAIT(index)                                                         \
-    if (!att_wait(&sm.bar[index], abort_flag)) break
+#define ATT_WAIT(index, parity)                                                         \
+    if (!(ok = att_wait(&sm.bar[index], (parity), abort_flag))) break
 
 __global__ void __launch_bounds__(kThreads, 1)
 local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
@@ -135,32 +188,21 @@ local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const 
     extern __shared__ uint8_t att5_raw[];
     Smem& sm = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(att5_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-    const int head = blockIdx.y, seg = blockIdx.z;
-    const int q0 = blockIdx.x * kTile;
-    int valid = p.seg_valid != nullptr ? p.seg_valid[seg] : p.valid_rows;
-    valid = min(valid, p.seg_stride);
-    const int base = seg * p.seg_stride;
-    const int rows_here = min(kTile, p.seg_stride - q0);
+    // (head, tile) items of this CTA, heads outermost: a range meets two heads at most a few times
+    const long long items = static_cast<long long>(kHeads) * p.tiles;
+    const int first_item = static_cast<int>(items * blockIdx.x / gridDim.x);
+    const int last_item = static_cast<int>(items * (blockIdx.x + 1) / gridDim.x);
 
-    // (the segment lengths, biases and position rows are constant over the kernel chain)
     grid_dependents_launch();
-    if (q0 >= valid) {                       // the whole tile is padding: zero-fill and leave
-        grid_dependency_wait();
-        for (int c = tid; c < rows_here * 16; c += kThreads)
-            *reinterpret_cast<uint4*>(p.out + static_cast<size_t>(base + q0 + c / 16) * p.ldo + head * kDim + (c % 16) * 8) =
-                make_uint4(0, 0, 0, 0);
-        return;
-    }
-
     volatile int* abort_flag = &sm.abort;
     if (tid == 0) {
         sm.abort = 0;
         for (int i = 0; i < B_COUNT; ++i) {
             int count = 1;                                             // TMA arrive / tcgen05.commit
-            if (i == B_BIAS_DONE || i == B_QP_DRAINED || (i >= B_UK_DONE && i < B_UK_DONE + 3) ||
-                (i >= B_P_READY && i < B_P_READY + 3))
+            if (i == B_VP_DONE || i == B_QP_DRAINED || i == B_PASS0_DONE || i == B_CTX_READ ||
+                (i >= B_UK_DONE && i < B_UK_DONE + 3) || (i >= B_P_READY && i < B_P_READY + 3))
                 count = kSoftmaxWarps;
-            if (i >= B_MAX) count = kParts;
+            if (i >= B_SUM) count = kParts;
             mbar_init(&sm.bar[i], count);
         }
         fence_barrier_init();
@@ -169,10 +211,6 @@ local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const 
         prefetch_tensormap(&map_p);
         prefetch_tensormap(&map_p16);
         prefetch_tensormap(&map_v);
-    }
-    if (tid < kDim) {
-        sm.bias_u[tid] = __half2float(p.bias_u[head * kDim + tid]);
-        sm.bias_v[tid] = __half2float(p.bias_v[head * kDim + tid]);
     }
     if (warp == kSoftmaxWarps + 1) {
         tmem_alloc(&sm.tmem_base, 512);
@@ -183,59 +221,92 @@ local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const 
     tc_fence_after_sync();
     const uint32_t tmem = sm.tmem_base;
     grid_dependency_wait();                  // Q, K and V come from the kernel before
-    const int key_first = q0 - kReach;       // window index kk <-> key key_first + kk
-    // slot of key block b, and of value block b after it
-    auto slot_of = [](int b) { return b == 0 ? 2 : b - 1; };
+    // slot of key block b (value block b: slot b)
+    auto slot_of_key = [](int b) { return b == 0 ? 2 : b - 1; };
     // TMEM columns of the score block b and of the context
     auto score_col = [](int b) { return b == 0 ? 384u : (b == 1 ? 0u : 128u); };
-    constexpr uint32_t kCtxCol = 256u;
+    constexpr uint32_t kCtxCol = 384u;
+    bool ok = true;
+    // Parities of the current tile's phases.  Bit 1 is that of every barrier that completes once per tile
+    // (the middle key block is in every tile), bits 0 and 2 those of the first and last key block.
+    uint32_t ph = 0;
 
     if (warp == kSoftmaxWarps) {
         // ------------------------------------------------------------ TMA producer
         if (lane == 0) {
-            do {
-                mbar_arrive_expect_tx(&sm.bar[B_IN], 3 * kSlotBytes + kTailBytes);
-                for (int a = 0; a < 2; ++a) {
-                    tma_load_2d(sm.q + a * kAtomBytes, &map_q, &sm.bar[B_IN], head * kDim + a * 64, base + q0);
-                    for (int b = 0; b < 2; ++b)
-                        tma_load_2d(sm.slot[b] + a * kAtomBytes, &map_p, &sm.bar[B_IN], a * 64, head * kPosRows + b * 128);
-                    tma_load_2d(sm.tail + a * (kTailBytes / 2), &map_p16, &sm.bar[B_IN], a * 64, head * kPosRows + 256);
-                }
-                auto load_keys = [&](int b) {
-                    mbar_arrive_expect_tx(&sm.bar[B_K_IN + b], kSlotBytes);
+            uint32_t before = 0, ph_before = 0;        // key blocks and parities of the tile before (0: none)
+            for (int item = first_item; ok && item < last_item; ++item) {
+                const TilePlace at(p.rows, item % p.tiles);
+                if (at.padding()) continue;
+                const int head = item / p.tiles;
+                const uint32_t blocks = at.blocks(), par = (ph >> 1) & 1u;
+                const int key_row = at.base + at.q0 - kReach;
+                auto load_block = [&](int slot, const CUtensorMap* map, int bar, int b) {
+                    mbar_arrive_expect_tx(&sm.bar[bar], kSlotBytes);
                     for (int a = 0; a < 2; ++a)
-                        tma_load_2d(sm.slot[slot_of(b)] + a * kAtomBytes, &map_k, &sm.bar[B_K_IN + b],
-                                    head * kDim + a * 64, base + key_first + b * 128);
+                        tma_load_2d(sm.slot[slot] + a * kAtomBytes, map, &sm.bar[bar], head * kDim + a * 64, key_row + b * 128);
                 };
-                load_keys(0);                       // slot 2 is free from the start
+                // the score products of the tile before have retired (waited for below)
+                mbar_arrive_expect_tx(&sm.bar[B_Q_IN], kSlotBytes);
+                for (int a = 0; a < 2; ++a)
+                    tma_load_2d(sm.q + a * kAtomBytes, &map_q, &sm.bar[B_Q_IN], head * kDim + a * 64, at.base + at.q0);
+                // position rows: slot 0 held V0 (or K1), slot 1 held V1 of the tile before
+                mbar_arrive_expect_tx(&sm.bar[B_P_IN], 2 * kSlotBytes + kTailBytes);
+                for (int a = 0; a < 2; ++a)
+                    tma_load_2d(sm.tail + a * (kTailBytes / 2), &map_p16, &sm.bar[B_P_IN], a * 64, head * kPosRows + 256);
+                if (before & 1u) ATT_WAIT(B_PV_DONE + 0, ph_before & 1u);
+                if (before != 0 && !(before & 1u)) ATT_WAIT(B_PV_DONE + 1, (ph_before >> 1) & 1u);
+                for (int a = 0; a < 2; ++a)
+                    tma_load_2d(sm.slot[0] + a * kAtomBytes, &map_p, &sm.bar[B_P_IN], a * 64, head * kPosRows);
+                if (before != 0) ATT_WAIT(B_PV_DONE + 1, (ph_before >> 1) & 1u);
+                for (int a = 0; a < 2; ++a)
+                    tma_load_2d(sm.slot[1] + a * kAtomBytes, &map_p, &sm.bar[B_P_IN], a * 64, head * kPosRows + 128);
+                if (before & 4u) ATT_WAIT(B_PV_DONE + 2, (ph_before >> 2) & 1u);
+                if (blocks & 1u) load_block(slot_of_key(0), &map_k, B_K_IN + 0, 0);
                 // the other key blocks: once the position rows have been multiplied
-                ATT_WAIT(B_QP_DONE);
-                ATT_WAIT(B_BIAS_DONE);
-                load_keys(1);
-                load_keys(2);
-                // values follow their key block into its slot
-                bool ok = true;
-                for (int b = 0; b < 3 && ok; ++b) {
-                    ok = att_wait(&sm.bar[B_S_DONE + b], abort_flag) &&
-                         att_wait(&sm.bar[B_UK_DONE + b], abort_flag);
-                    if (!ok) break;
-                    mbar_arrive_expect_tx(&sm.bar[B_V_IN + b], kSlotBytes);
-                    // rows = keys, 64 features per atom: the MN-major form of the B operand of Pr.V
-                    for (int a = 0; a < 2; ++a)
-                        tma_load_2d(sm.slot[slot_of(b)] + a * kAtomBytes, &map_v, &sm.bar[B_V_IN + b],
-                                    head * kDim + a * 64, base + key_first + b * 128);
+                ATT_WAIT(B_QP_DONE, par);
+                ATT_WAIT(B_VP_DONE, par);
+                load_block(slot_of_key(1), &map_k, B_K_IN + 1, 1);
+                if (blocks & 4u) load_block(slot_of_key(2), &map_k, B_K_IN + 2, 2);
+                // values: V0 after K1, V1 after K2 (or the position rows), V2 after K0
+                ATT_WAIT(B_S_DONE + 1, par);
+                ATT_WAIT(B_UK_DONE + 1, par);
+                if (blocks & 1u) load_block(0, &map_v, B_V_IN + 0, 0);
+                if (blocks & 4u) {
+                    ATT_WAIT(B_S_DONE + 2, (ph >> 2) & 1u);
+                    ATT_WAIT(B_UK_DONE + 2, (ph >> 2) & 1u);
                 }
-            } while (false);
+                load_block(1, &map_v, B_V_IN + 1, 1);
+                if (blocks & 4u) {
+                    if (blocks & 1u) {
+                        ATT_WAIT(B_S_DONE + 0, ph & 1u);
+                        ATT_WAIT(B_UK_DONE + 0, ph & 1u);
+                    }
+                    load_block(2, &map_v, B_V_IN + 2, 2);
+                }
+                before = blocks;
+                ph_before = ph;
+                ph ^= blocks;
+            }
         }
     } else if (warp == kSoftmaxWarps + 1) {
         // ------------------------------------------------------------- MMA issuer
         if (lane == 0) {
-            do {
-                constexpr uint32_t idesc128 = make_instr_desc<KIND_F16>(128, 128);
-                constexpr uint32_t idesc16 = make_instr_desc<KIND_F16>(128, 16);
-                const uint32_t q_addr = smem_u32(sm.q);
-                ATT_WAIT(B_IN);
+            constexpr uint32_t idesc128 = make_instr_desc<KIND_F16>(128, 128);
+            constexpr uint32_t idesc16 = make_instr_desc<KIND_F16>(128, 16);
+            // B = V[keys, features] as it lies in memory: MN-major (features contiguous),
+            // 8-key groups 1024 bytes apart, the second 64 features 16 KB on; 16 keys = 2048 bytes
+            constexpr uint32_t idesc_v = idesc128 | (1u << 16);
+            const uint32_t q_addr = smem_u32(sm.q);
+            bool any = false;
+            for (int item = first_item; ok && item < last_item; ++item) {
+                const TilePlace at(p.rows, item % p.tiles);
+                if (at.padding()) continue;
+                const uint32_t blocks = at.blocks(), par = (ph >> 1) & 1u;
+                ATT_WAIT(B_Q_IN, par);
+                ATT_WAIT(B_P_IN, par);
                 tc_fence_after_sync();
+                // (columns [0, 272) are free: P_READY of the tile before came after their last read)
                 for (int ks = 0; ks < 8; ++ks) {           // 16 features per MMA
                     const int a = ks / 4, j = ks % 4;
                     const uint64_t da = make_smem_desc<128>(q_addr + a * kAtomBytes) + 2u * j;
@@ -246,13 +317,15 @@ local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const 
                                      make_smem_desc<128>(smem_u32(sm.tail) + a * (kTailBytes / 2)) + 2u * j, idesc16, ks > 0);
                 }
                 tc_commit(&sm.bar[B_QP_DONE]);
-                bool ok = true;
-                for (int b = 0; b < 3 && ok; ++b) {
-                    if (b == 1) ok = att_wait(&sm.bar[B_QP_DRAINED], abort_flag);   // columns [0, 272) are free
-                    if (ok) ok = att_wait(&sm.bar[B_K_IN + b], abort_flag);
-                    if (!ok) break;
+                // S_0 and the context share their columns
+                if (any) ATT_WAIT(B_CTX_READ, par ^ 1u);
+                any = true;
+                for (int b = 0; b < 3; ++b) {
+                    if (!((blocks >> b) & 1u)) continue;
+                    if (b == 1) ATT_WAIT(B_QP_DRAINED, par);   // columns [0, 272) are free
+                    ATT_WAIT(B_K_IN + b, (ph >> b) & 1u);
                     tc_fence_after_sync();
-                    const uint32_t k_addr = smem_u32(sm.slot[slot_of(b)]);
+                    const uint32_t k_addr = smem_u32(sm.slot[slot_of_key(b)]);
                     for (int ks = 0; ks < 8; ++ks) {
                         const int a = ks / 4, j = ks % 4;
                         tc_mma<KIND_F16>(tmem + score_col(b), make_smem_desc<128>(q_addr + a * kAtomBytes) + 2u * j,
@@ -261,26 +334,26 @@ local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const 
                     tc_commit(&sm.bar[B_S_DONE + b]);
                 }
                 if (!ok) break;
-                for (int b = 0; b < 3 && ok; ++b) {
-                    ok = att_wait(&sm.bar[B_V_IN + b], abort_flag) &&
-                         att_wait(&sm.bar[B_P_READY + b], abort_flag);
-                    if (!ok) break;
+                uint32_t accumulate = 0;
+                for (int b = 0; b < 3; ++b) {
+                    if (!((blocks >> b) & 1u)) continue;
+                    ATT_WAIT(B_V_IN + b, (ph >> b) & 1u);
+                    ATT_WAIT(B_P_READY + b, (ph >> b) & 1u);
                     tc_fence_after_sync();
-                    const uint32_t v_addr = smem_u32(sm.slot[slot_of(b)]);
+                    const uint32_t v_addr = smem_u32(sm.slot[b]), p_addr = smem_u32(sm.pr[b & 1]);
                     for (int ks = 0; ks < 8; ++ks) {       // 16 keys per MMA
                         const int a = ks / 4, j = ks % 4;
-                        // B = V[keys, features] as it lies in memory: MN-major (features contiguous),
-                        // 8-key groups 1024 bytes apart, the second 64 features 16 KB on; 16 keys = 2048 bytes
-                        constexpr uint32_t idesc_v = idesc128 | (1u << 16);
                         const uint64_t dv = static_cast<uint64_t>(((v_addr + ks * 2048u) & 0x3FFFFu) >> 4) |
                                             (static_cast<uint64_t>(kAtomBytes >> 4) << 16) | (64ull << 32) |
                                             (1ull << 46) | (2ull << 61);
-                        tc_mma<KIND_F16>(tmem + kCtxCol, make_smem_desc<128>(q_addr + a * kAtomBytes) + 2u * j,
-                                         dv, idesc_v, (b > 0 || ks > 0) ? 1u : 0u);
+                        tc_mma<KIND_F16>(tmem + kCtxCol, make_smem_desc<128>(p_addr + a * kAtomBytes) + 2u * j,
+                                         dv, idesc_v, accumulate);
+                        accumulate = 1;
                     }
                     tc_commit(&sm.bar[B_PV_DONE + b]);
                 }
-            } while (false);
+                ph ^= blocks;
+            }
         }
     } else {
         // ------------------------------------------ bias terms, QP drain, softmax, output
@@ -289,42 +362,58 @@ local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const 
         const uint32_t lane_addr = tmem + (static_cast<uint32_t>(quad * 32) << 16);
         constexpr float kLog2e = 1.4426950408889634f;
         const float scale2 = kSoftmaxScale * kLog2e;
-        const bool q_live = q0 + ql < valid;
-        do {
-            // v . P_j for the 272 position rows (per-column constant of QP): four threads per row,
-            // 32 features each, from the staged operand tiles
-            ATT_WAIT(B_IN);
-            const int qt = tid % 4;                                // this thread's features: 32 * qt ..
-            float bias[32];
+        const uint64_t scale22 = pack2(scale2, scale2);
+        const int qt = tid % 4;                                // features of the bias terms: 32 * qt ..
+        int head_now = -1, base_now = -1, q0_now = 0;          // what vp and uk in shared memory belong to
+        for (int item = first_item; ok && item < last_item; ++item) {
+            const TilePlace at(p.rows, item % p.tiles);
+            const int head = item / p.tiles;
+            const int q0 = at.q0, valid = at.valid;
+            if (at.padding()) {                  // the whole tile is padding: zeros
+                for (int c = tid; c < kTile * 16; c += kSoftmaxThreads)
+                    *reinterpret_cast<uint4*>(p.out + static_cast<size_t>(at.base + q0 + c / 16) * p.ldo + head * kDim + (c % 16) * 8) =
+                        make_uint4(0, 0, 0, 0);
+                continue;
+            }
+            const uint32_t blocks = at.blocks(), par = (ph >> 1) & 1u;
+            const bool q_live = q0 + ql < valid;
+            const int key_first = q0 - kReach;       // window index kk <-> key key_first + kk
+            // u . K of the first two key blocks is there when the tile in front of this one was done last
+            const bool follows = head == head_now && at.base == base_now && q0 == q0_now + kTile;
+            if (head != head_now) {
+                // v . P_j for the 272 position rows (per-column constant of QP): four threads per row,
+                // 32 features each, from the staged operand tiles
+                if (tid < kDim) sm.bias_u[tid] = __half2float(p.bias_u[head * kDim + tid]);
+                float bias[32];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const float4 t = *reinterpret_cast<const float4*>(&sm.bias_v[32 * qt + 4 * i]);
-                bias[4 * i] = t.x; bias[4 * i + 1] = t.y; bias[4 * i + 2] = t.z; bias[4 * i + 3] = t.w;
-            }
+                for (int i = 0; i < 32; ++i) bias[i] = __half2float(p.bias_v[head * kDim + 32 * qt + i]);
+                ATT_WAIT(B_P_IN, par);
 #pragma unroll 1
-            for (int item = tid; item < 4 * kPosRows; item += kSoftmaxThreads) {
-                const int row = item / 4;
-                const uint8_t* atom = row < 256 ? sm.slot[row / 128] + (qt / 2) * kAtomBytes
-                                                : sm.tail + (qt / 2) * (kTailBytes / 2);
-                float acc = bias_dot32(atom, row < 256 ? row % 128 : row - 256, 4 * (qt % 2), bias);
-                acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-                acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-                if (qt == 0) sm.vp[row] = acc;
+                for (int i = tid; i < 4 * kPosRows; i += kSoftmaxThreads) {
+                    const int row = i / 4;
+                    const uint8_t* atom = row < 256 ? sm.slot[row / 128] + (qt / 2) * kAtomBytes
+                                                    : sm.tail + (qt / 2) * (kTailBytes / 2);
+                    float acc = bias_dot32(atom, row < 256 ? row % 128 : row - 256, 4 * (qt % 2), bias);
+                    acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+                    acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+                    if (qt == 0) sm.vp[row] = acc;
+                }
+                __syncwarp();
             }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&sm.bar[B_BIAS_DONE]);
-            ATT_WAIT(B_BIAS_DONE);
+            head_now = head; base_now = at.base; q0_now = q0;
+            if (lane == 0) mbar_arrive(&sm.bar[B_VP_DONE]);
+            ATT_WAIT(B_VP_DONE, par);
             // QP: tensor memory -> fp16 rows in shared memory, bias term added.  Row ql is stored shifted
             // right by (ql & 1) halves, so that the run of position columns a key piece needs (kk0 - ql ...)
             // starts on a 32-bit word for every thread.  Part p drains columns [64p, 64p + 64), the last
             // part the 16 columns beyond as well.
-            ATT_WAIT(B_QP_DONE);
+            ATT_WAIT(B_QP_DONE, par);
             tc_fence_after_sync();
             {
                 uint32_t* row = reinterpret_cast<uint32_t*>(&sm.qp[ql * kQpPitch]);
                 const bool odd = (ql & 1) != 0;
                 // 32 columns per step (part 3: a last step of 16 columns, the load still 32 wide: the columns
-                // beyond 272 hold stale accumulators that are never stored)
+                // beyond 272 are never stored)
                 const int steps = part == kParts - 1 ? 3 : 2;
 #pragma unroll 1
                 for (int st = 0; st < steps; ++st) {
@@ -362,145 +451,165 @@ local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const 
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) mbar_arrive(&sm.bar[B_QP_DRAINED]);
-            // u . K_kk for the keys of each block, as soon as the block has landed: four threads per key
+            // u . K_kk for the keys of each new block, as soon as the block has landed: four threads per key
+            const int ring = q0 / kTile + 2;                   // key block b of the tile: row (ring + b) % 3
             {
+                float bias[32];
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                     const float4 t = *reinterpret_cast<const float4*>(&sm.bias_u[32 * qt + 4 * i]);
                     bias[4 * i] = t.x; bias[4 * i + 1] = t.y; bias[4 * i + 2] = t.z; bias[4 * i + 3] = t.w;
                 }
-                bool ok = true;
 #pragma unroll 1
-                for (int b = 0; b < 3 && ok; ++b) {
-                    ok = att_wait(&sm.bar[B_K_IN + b], abort_flag);
-                    if (!ok) break;
-                    const int row = tid / 4;
-                    float acc = bias_dot32(sm.slot[slot_of(b)] + (qt / 2) * kAtomBytes, row, 4 * (qt % 2), bias);
-                    acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-                    acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-                    if (qt == 0) sm.uk[b * 128 + row] = acc;
-                    __syncwarp();
+                for (int b = 0; b < 3; ++b) {
+                    if (!((blocks >> b) & 1u)) continue;
+                    if (b == 2 || !follows) {
+                        ATT_WAIT(B_K_IN + b, (ph >> b) & 1u);
+                        const int row = tid / 4;
+                        float acc = bias_dot32(sm.slot[slot_of_key(b)] + (qt / 2) * kAtomBytes, row, 4 * (qt % 2), bias);
+                        acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+                        acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+                        if (qt == 0) sm.uk[(ring + b) % 3][row] = acc;
+                        __syncwarp();
+                    }
                     if (lane == 0) mbar_arrive(&sm.bar[B_UK_DONE + b]);
                 }
-                for (int b = 0; b < 3 && ok; ++b) ok = att_wait(&sm.bar[B_UK_DONE + b], abort_flag);
                 if (!ok) break;
             }
-            ATT_WAIT(B_QP_DRAINED);
-            {
-                bool ok = true;
-                for (int b = 0; b < 3 && ok; ++b) ok = att_wait(&sm.bar[B_S_DONE + b], abort_flag);
-                if (!ok) break;
-            }
-            tc_fence_after_sync();
+            ATT_WAIT(B_QP_DRAINED, par);
 
             // keys this query sees, in window coordinates: [lo, hi] (empty for a padding row)
             const int lo = max(ql, -key_first);
             const int hi = q_live ? min(ql + 2 * kReach, valid - 1 - key_first) : -1;
-            // the same for the whole warp: pieces outside [w_lo, w_hi] are skipped
-            const int w_lo = max(quad * 32, -key_first), w_hi = min(quad * 32 + 31 + 2 * kReach, valid - 1 - key_first);
             const unsigned span = static_cast<unsigned>(hi - lo);          // hi < lo: nothing passes
-            // A piece = 16 consecutive columns of this thread's scores; this warp owns two pieces (32
-            // columns) of every block.  Pass 0 finds the row maximum, pass 1 writes the probabilities,
-            // block by block, into the A operand of the last contraction (one rolled loop for both).
+            // the same for the whole warp: pieces outside [w_lo, w_hi] are skipped, pieces inside
+            // [a_lo, a_hi] are seen whole by every row
+            const int w_lo = max(quad * 32, -key_first), w_hi = min(quad * 32 + 31 + 2 * kReach, valid - 1 - key_first);
+            const int a_lo = max(quad * 32 + 31, -key_first);
+            const int a_hi = q0 + quad * 32 + 31 < valid ? min(quad * 32 + 2 * kReach, valid - 1 - key_first) : -1;
+            // A piece = 32 consecutive columns of this thread's scores, one per block.  Pass 0 writes the
+            // scaled and masked scores back over the accumulators and finds the row maximum.
             float mx = -INFINITY, sum = 0.0f;
-            bool ok = true;
 #pragma unroll 1
-            for (int pass = 0; pass < 2 && ok; ++pass) {
+            for (int b = 0; b < 3; ++b) {
+                if (!((blocks >> b) & 1u)) continue;
+                ATT_WAIT(B_UK_DONE + b, (ph >> b) & 1u);
+                ATT_WAIT(B_S_DONE + b, (ph >> b) & 1u);
+                tc_fence_after_sync();
+                const int kk0 = b * 128 + part * 32;
+                if (kk0 + 31 < w_lo || kk0 > w_hi) continue;
+                uint32_t r[32];
+                tmem_ld_32x32(lane_addr + score_col(b) + static_cast<uint32_t>(part * 32), r);
+                // position scores of columns kk0 - ql .. + 31: stored from half (ql & 1) on, so the
+                // run starts at a word of the row (kk0 is even)
+                const __half2* qp2 = reinterpret_cast<const __half2*>(&sm.qp[ql * kQpPitch + kk0 - ql + (ql & 1)]);
+                const float4* uk4 = reinterpret_cast<const float4*>(&sm.uk[(ring + b) % 3][part * 32]);
+                uint64_t t2[16];
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    const float4 u = uk4[c];
+                    const float2 a = __half22float2(qp2[2 * c]), bb = __half22float2(qp2[2 * c + 1]);
+                    t2[2 * c] = add2(pack2(a.x, a.y), pack2(u.x, u.y));
+                    t2[2 * c + 1] = add2(pack2(bb.x, bb.y), pack2(u.z, u.w));
+                }
+                tmem_ld_wait();
+                float s[32];
+#pragma unroll
+                for (int i = 0; i < 16; ++i)
+                    unpack2(mul2(add2(pack2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), t2[i]), scale22),
+                            s[2 * i], s[2 * i + 1]);
+                if (kk0 < a_lo || kk0 + 31 > a_hi) {
+                    const int off = kk0 - lo;
+                    const bool some = hi >= lo;
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) s[i] = some && static_cast<unsigned>(off + i) <= span ? s[i] : -INFINITY;
+                }
+#pragma unroll
+                for (int i = 0; i < 32; ++i) mx = fmaxf(mx, s[i]);
+#pragma unroll
+                for (int hf = 0; hf < 2; ++hf) {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(s[16 * hf + i]);
+                    tmem_st_32x16(lane_addr + score_col(b) + static_cast<uint32_t>(part * 32 + 16 * hf),
+                                  *reinterpret_cast<const uint32_t(*)[16]>(&r[0]));
+                }
+            }
+            if (!ok) break;
+            tmem_st_wait();
+            sm.rowmax[part][ql] = mx;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sm.bar[B_PASS0_DONE]);
+            // all warps are done with the position scores: their space takes the probabilities
+            ATT_WAIT(B_PASS0_DONE, par);
+            mx = fmaxf(fmaxf(sm.rowmax[0][ql], sm.rowmax[1][ql]), fmaxf(sm.rowmax[2][ql], sm.rowmax[3][ql]));
+            if (mx == -INFINITY) mx = 0.0f;            // a query without keys: every probability is 0
+            const uint64_t minus_mx2 = pack2(-mx, -mx);
+            // Pass 1: probabilities, block by block, into the A operand of the last contraction.
 #pragma unroll 1
-                for (int b = 0; b < 3 && ok; ++b) {
-                    uint32_t w[16];
-                    const int kk0 = b * 128 + part * 32;
-                    float s[32];
-                    const bool live = !(kk0 + 31 < w_lo || kk0 > w_hi);
-                    if (live) {
-                        uint32_t r[32];
-                        tmem_ld_32x32(lane_addr + score_col(b) + static_cast<uint32_t>(kk0 % 128), r);
-                        // position scores of columns kk0 - ql .. + 31: stored from half (ql & 1) on, so the
-                        // run starts at a word of the row (kk0 is even)
-                        const __half2* qp2 = reinterpret_cast<const __half2*>(&sm.qp[ql * kQpPitch + kk0 - ql + (ql & 1)]);
-                        const float4* uk4 = reinterpret_cast<const float4*>(&sm.uk[kk0]);
+            for (int b = 0; b < 3; ++b) {
+                if (!((blocks >> b) & 1u)) continue;
+                uint32_t w[16];
+                const int kk0 = b * 128 + part * 32;
+                if (kk0 + 31 < w_lo || kk0 > w_hi) {
 #pragma unroll
-                        for (int c = 0; c < 8; ++c) {
-                            const float4 u = uk4[c];
-                            const float2 a = __half22float2(qp2[2 * c]), bb = __half22float2(qp2[2 * c + 1]);
-                            s[4 * c + 0] = a.x + u.x; s[4 * c + 1] = a.y + u.y; s[4 * c + 2] = bb.x + u.z; s[4 * c + 3] = bb.y + u.w;
-                        }
-                        tmem_ld_wait();
-                        const int off = kk0 - lo;
+                    for (int e = 0; e < 16; ++e) w[e] = 0u;
+                } else {
+                    uint32_t r[32];
+                    tmem_ld_32x32(lane_addr + score_col(b) + static_cast<uint32_t>(part * 32), r);
+                    tmem_ld_wait();
 #pragma unroll
-                        for (int i = 0; i < 32; ++i) {
-                            const bool in = hi >= lo && static_cast<unsigned>(off + i) <= span;
-                            s[i] = in ? (__uint_as_float(r[i]) + s[i]) * scale2 : -INFINITY;
-                        }
-                    }
-                    if (pass == 0) {
-                        if (live) {
-#pragma unroll
-                            for (int i = 0; i < 32; ++i) mx = fmaxf(mx, s[i]);
-                        }
-                    } else {
-#pragma unroll
-                        for (int e = 0; e < 16; ++e) {
-                            float p0 = 0.0f, p1 = 0.0f;                     // ex2(-inf) = 0
-                            if (live) {
-                                asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(p0) : "f"(s[2 * e] - mx));
-                                asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(p1) : "f"(s[2 * e + 1] - mx));
-                            }
-                            sum += p0 + p1;
-                            const __half2 h = __floats2half2_rn(p0, p1);
-                            w[e] = *reinterpret_cast<const uint32_t*>(&h);
-                        }
-                    }
-                    if (pass == 1) {
-                        if (b > 0) ok = att_wait(&sm.bar[B_PV_DONE + b - 1], abort_flag);   // the buffer is free
-                        if (ok) {
-                            uint8_t* atom = sm.q + (part / 2) * kAtomBytes;   // keys 64 * (part / 2) .. + 63 of the block
-#pragma unroll
-                            for (int e = 0; e < 4; ++e)
-                                *reinterpret_cast<uint4*>(atom + swz(ql, 4 * (part % 2) + e)) =
-                                    make_uint4(w[4 * e], w[4 * e + 1], w[4 * e + 2], w[4 * e + 3]);
-                            fence_proxy_async_smem();
-                            __syncwarp();
-                            if (lane == 0) mbar_arrive(&sm.bar[B_P_READY + b]);
-                        }
+                    for (int e = 0; e < 16; ++e) {
+                        float p0, p1;                                       // ex2(-inf) = 0
+                        unpack2(add2(pack2(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1])), minus_mx2), p0, p1);
+                        asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(p0));
+                        asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(p1));
+                        sum += p0 + p1;
+                        const __half2 h = __floats2half2_rn(p0, p1);
+                        w[e] = *reinterpret_cast<const uint32_t*>(&h);
                     }
                 }
-                if (pass == 0) {
-                    sm.rowmax[part][ql] = mx;
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&sm.bar[B_MAX + quad]);
-                    ok = att_wait(&sm.bar[B_MAX + quad], abort_flag);
-                    mx = fmaxf(fmaxf(sm.rowmax[0][ql], sm.rowmax[1][ql]), fmaxf(sm.rowmax[2][ql], sm.rowmax[3][ql]));
-                    if (mx == -INFINITY) mx = 0.0f;            // a query without keys: every probability is 0
-                }
+                // the third block takes the first one's buffer
+                if (b == 2 && (blocks & 1u)) ATT_WAIT(B_PV_DONE + 0, ph & 1u);
+                uint8_t* atom = sm.pr[b & 1] + (part / 2) * kAtomBytes;   // keys 64 * (part / 2) .. + 63 of the block
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    *reinterpret_cast<uint4*>(atom + swz(ql, 4 * (part % 2) + e)) =
+                        make_uint4(w[4 * e], w[4 * e + 1], w[4 * e + 2], w[4 * e + 3]);
+                fence_proxy_async_smem();
+                tc_fence_before_sync();                                   // the scores have been read
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&sm.bar[B_P_READY + b]);
             }
             if (!ok) break;
             sm.rowsum[part][ql] = sum;
             __syncwarp();
             if (lane == 0) mbar_arrive(&sm.bar[B_SUM + quad]);
-            ATT_WAIT(B_SUM + quad);
+            ATT_WAIT(B_SUM + quad, par);
             sum = (sm.rowsum[0][ql] + sm.rowsum[1][ql]) + (sm.rowsum[2][ql] + sm.rowsum[3][ql]);
             const float inv = sum > 0.0f ? 1.0f / sum : 0.0f;
-            ATT_WAIT(B_PV_DONE + 2);
+            const int last = (blocks & 4u) ? 2 : 1;
+            ATT_WAIT(B_PV_DONE + last, (ph >> last) & 1u);
             tc_fence_after_sync();
             // context: this warp writes features [32 * part, +32) of its 32 queries
             {
                 uint32_t r[32];
                 tmem_ld_32x32(lane_addr + kCtxCol + static_cast<uint32_t>(part * 32), r);
                 tmem_ld_wait();
-                if (ql < rows_here) {
-                    uint32_t w[16];
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&sm.bar[B_CTX_READ]);
+                uint32_t w[16];
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        const __half2 h = __floats2half2_rn(__uint_as_float(r[2 * i]) * inv, __uint_as_float(r[2 * i + 1]) * inv);
-                        w[i] = q_live ? *reinterpret_cast<const uint32_t*>(&h) : 0u;
-                    }
-                    uint4* dst = reinterpret_cast<uint4*>(p.out + static_cast<size_t>(base + q0 + ql) * p.ldo + head * kDim + part * 32);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) dst[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+                for (int i = 0; i < 16; ++i) {
+                    const __half2 h = __floats2half2_rn(__uint_as_float(r[2 * i]) * inv, __uint_as_float(r[2 * i + 1]) * inv);
+                    w[i] = q_live ? *reinterpret_cast<const uint32_t*>(&h) : 0u;
                 }
+                uint4* dst = reinterpret_cast<uint4*>(p.out + static_cast<size_t>(at.base + q0 + ql) * p.ldo + head * kDim + part * 32);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) dst[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
             }
-        } while (false);
+            ph ^= blocks;
+        }
     }
 
     // ------------------------------------------------------------------- teardown
@@ -523,23 +632,12 @@ local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const 
 
 using namespace pk100;
 
-extern "C" int pk100_local_relpos_attention_tcgen05(
-    void* stream_v, const void* query, int ldq, const void* key, int ldk, const void* value, int ldv,
-    const void* position, const void* bias_u, const void* bias_v, void* output, int ldo, int segments,
-    int seg_stride, int valid_rows, const int* seg_valid, int* status) {
+int pk100_local_attention_rows(void* stream_v, const void* query, int ldq, const void* key, int ldk, const void* value, int ldv,
+                               const void* position, const void* bias_u, const void* bias_v, void* output, int ldo,
+                               int total_rows, const pk100_rows& geometry, int* status) {
     using namespace att5;
-    if (!query || !key || !value || !position || !bias_u || !bias_v || !output) return PK100_ERR_NULL;
-    if (segments < 0 || seg_stride <= 0) return PK100_ERR_SHAPE;
-    if (seg_stride % kTile != 0) return PK100_ERR_SHAPE;          // whole 128-query tiles
-    if (ldq < 1024 || ldk < 1024 || ldv < 1024 || ldo < 1024 || (ldq | ldk | ldv | ldo) % 8 != 0) return PK100_ERR_SHAPE;
-    const uintptr_t bits = reinterpret_cast<uintptr_t>(query) | reinterpret_cast<uintptr_t>(key) |
-                           reinterpret_cast<uintptr_t>(value) | reinterpret_cast<uintptr_t>(position) |
-                           reinterpret_cast<uintptr_t>(output);
-    if (bits & 15u) return PK100_ERR_ALIGN;
-    if (segments == 0) return PK100_OK;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
-    const unsigned long long rows = static_cast<unsigned long long>(segments) * seg_stride;
-
+    const unsigned long long rows = static_cast<unsigned long long>(total_rows);
     CUtensorMap map_q, map_k, map_p, map_p16, map_v;
     int rc = pk100_tensor_map_2d(&map_q, query, 2, rows, 1024, ldq, kTile, 128);
     if (rc == PK100_OK) rc = pk100_tensor_map_2d(&map_k, key, 2, rows, 1024, ldk, 128, 128);
@@ -556,9 +654,30 @@ extern "C" int pk100_local_relpos_attention_tcgen05(
         if (err != cudaSuccess) return static_cast<int>(err);
         configured = true;
     }
+    const int tiles = total_rows / kTile;
     Params p{static_cast<const __half*>(bias_u), static_cast<const __half*>(bias_v), static_cast<__half*>(output), ldo,
-             segments, seg_stride, valid_rows, seg_valid, status};
-    dim3 grid(seg_stride / kTile, kHeads, segments);
-    pk100_launch_chained(local_attention_tcgen05_kernel, grid, dim3(kThreads), smem_bytes, stream, map_q, map_k, map_p, map_p16, map_v, p);
+             tiles, geometry, status};
+    // one persistent CTA per SM; fewer while decoder clusters of earlier batches hold some of them
+    const long long items = static_cast<long long>(kHeads) * tiles;
+    const int ctas = static_cast<int>(items < pk100_cta_budget() ? items : pk100_cta_budget());
+    pk100_launch_chained(local_attention_tcgen05_kernel, dim3(ctas), dim3(kThreads), smem_bytes, stream, map_q, map_k, map_p, map_p16, map_v, p);
     return pk100_launch_status();
+}
+
+extern "C" int pk100_local_relpos_attention_tcgen05(
+    void* stream_v, const void* query, int ldq, const void* key, int ldk, const void* value, int ldv,
+    const void* position, const void* bias_u, const void* bias_v, void* output, int ldo, int segments,
+    int seg_stride, int valid_rows, const int* seg_valid, int* status) {
+    using namespace att5;
+    if (!query || !key || !value || !position || !bias_u || !bias_v || !output) return PK100_ERR_NULL;
+    if (segments < 0 || seg_stride <= 0) return PK100_ERR_SHAPE;
+    if (seg_stride % kTile != 0) return PK100_ERR_SHAPE;          // whole 128-query tiles
+    if (ldq < 1024 || ldk < 1024 || ldv < 1024 || ldo < 1024 || (ldq | ldk | ldv | ldo) % 8 != 0) return PK100_ERR_SHAPE;
+    const uintptr_t bits = reinterpret_cast<uintptr_t>(query) | reinterpret_cast<uintptr_t>(key) |
+                           reinterpret_cast<uintptr_t>(value) | reinterpret_cast<uintptr_t>(position) |
+                           reinterpret_cast<uintptr_t>(output);
+    if (bits & 15u) return PK100_ERR_ALIGN;
+    if (segments == 0) return PK100_OK;
+    return pk100_local_attention_rows(stream_v, query, ldq, key, ldk, value, ldv, position, bias_u, bias_v, output, ldo,
+                                      segments * seg_stride, pk100_rows{nullptr, seg_stride, valid_rows, seg_valid}, status);
 }

@@ -142,11 +142,11 @@ extern "C" void pk100_set_gemm_cta_pairs(int enable) { g_use_pairs.store(enable 
 static std::atomic<int> g_dependent_launch{1};
 static std::atomic<int> g_cta_cap{0};
 extern "C" void pk100_set_gemm_cta_cap(int ctas) { g_cta_cap.store(ctas > 0 ? ctas : 0); }
-static int cta_budget(const pk100_gemm_args& a) {
-    if (a.max_ctas > 0) return a.max_ctas;
+static int shared_budget() {
     const int cap = g_cta_cap.load(std::memory_order_relaxed);
     return cap > 0 && cap < sm_count() ? cap : sm_count();
 }
+static int cta_budget(const pk100_gemm_args& a) { return a.max_ctas > 0 ? a.max_ctas : shared_budget(); }
 extern "C" void pk100_set_dependent_launch(int enable) { g_dependent_launch.store(enable != 0); }
 extern "C" void pk100_tensor_map_cache_stats(long long* hits, long long* misses) {
     if (hits != nullptr) *hits = g_map_hits.load(std::memory_order_relaxed);
@@ -266,6 +266,8 @@ int pk100_tensor_map_2d(void* map, const void* base, int elem_bytes, unsigned lo
                         unsigned long long cols, unsigned long long ld, int box_rows, int swizzle_bytes) {
     return make_map(static_cast<CUtensorMap*>(map), base, elem_bytes, rows, cols, ld, box_rows, swizzle_bytes);
 }
+
+int pk100_cta_budget() { return pk100::shared_budget(); }
 
 bool pk100_dependent_launch_enabled() { return pk100::g_dependent_launch.load(std::memory_order_relaxed) != 0; }
 

@@ -67,6 +67,14 @@ int pk100_depthwise_bn_silu_rows(void* stream, const void* input, const void* dw
                                  const float* bn_mean, const float* bn_var, void* output, float* row_scales, int quantize,
                                  int total_rows, int segments, const pk100_rows& geometry, float eps);
 
+// Local attention behind pk100_local_relpos_attention_tcgen05 on either geometry (total_rows: a multiple of 128).
+int pk100_local_attention_rows(void* stream, const void* query, int ldq, const void* key, int ldk, const void* value, int ldv,
+                               const void* position, const void* bias_u, const void* bias_v, void* output, int ldo,
+                               int total_rows, const pk100_rows& geometry, int* status);
+
+// SMs a persistent kernel may use: all of them, or the cap set by pk100_set_gemm_cta_cap.
+int pk100_cta_budget();
+
 // 2-D TMA descriptor of a row-major matrix [rows, cols] (`ld` elements between rows) with a box of
 // [box_rows, swizzle_bytes / elem_bytes] elements; served from the library's descriptor cache
 // (gemm_host.cu).  `map` points to a CUtensorMap.

@@ -106,3 +106,21 @@ def test_tcgen05_kernel_segments_strides_and_large_scores(pk, cuda):
     # a stride that is no multiple of 128 is refused (the caller takes the other kernel)
     with pytest.raises(pk.lib.Pk100Error):
         pk.ops.local_attention_tcgen05(dev16(q[:200]), dev16(k[:200]), dev16(v[:200]), dev16(pos), dev16(u), dev16(bv))
+
+
+@pytest.mark.parametrize("ctas", [1, 3, 5, 0])
+def test_tcgen05_tile_ranges_of_persistent_ctas(pk, cuda, ctas):
+    """Several tiles per CTA: tiles that follow each other, a new utterance, a new head and padding tiles
+    inside one CTA's range; utterances that end on, just behind and just before a tile edge."""
+    seg, valid = 512, [512, 129, 0, 128, 385, 1]
+    q, k, v, pos, u, bv = _case(9, seg * len(valid))
+    sv = torch.tensor(valid, dtype=torch.int32, device=cuda)
+    st = torch.zeros(1, dtype=torch.int32, device=cuda)
+    pk.lib.lib.pk100_set_gemm_cta_cap(ctas)
+    try:
+        got = host(pk.ops.local_attention_tcgen05(dev16(q), dev16(k), dev16(v), dev16(pos), dev16(u), dev16(bv),
+                                                  seg_stride=seg, seg_valid=sv, status=st))
+    finally:
+        pk.lib.lib.pk100_set_gemm_cta_cap(0)
+    assert int(st.item()) == 0
+    _check_segments(got, q, k, v, pos, u, bv, seg, valid)
