@@ -90,7 +90,7 @@ struct Smem {
         alignas(1024) __half qp[kTile * kQpPitch + 8];    // position scores, until the first pass is over
         alignas(1024) uint8_t pr[2][kSlotBytes];          // probabilities of two key blocks
     };
-    float vp[288];
+    float vp[288];                                        // 272 used, the rest read and dropped
     float uk[3][128];                                     // key block i of the utterance -> row i % 3
     alignas(16) float bias_u[kDim];
     float rowmax[kParts][kTile];
@@ -106,6 +106,7 @@ struct Params {
     __half* out; int ldo;
     int tiles;                // 128-row tiles of the batch
     pk100_rows rows;
+    int early;                // the kernel before writes none of position, bias_u, bias_v, rows
     int* status;
 };
 
@@ -174,9 +175,13 @@ __device__ __forceinline__ float bias_dot32(const uint8_t* atom, int row, int fi
     return acc0 + acc1;
 }
 
-// One copy of the polling loop for the whole kernel (it is inlined nowhere: the roles wait at some thirty places).
-__device__ __noinline__ bool att_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+// The first poll is inlined (most waits of a tile find their phase complete; a call cost 250 cycles), the
+// polling loop exists once.
+__device__ __noinline__ bool att_poll(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
     return mbar_wait_bounded(bar, parity, abort_flag);
+}
+__device__ __forceinline__ bool att_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+    return mbar_try_wait(bar, parity) || att_poll(bar, parity, abort_flag);
 }
 #define ATT_WAIT(index, parity)                                                         \
     if (!(ok = att_wait(&sm.bar[index], (parity), abort_flag))) break
@@ -184,7 +189,7 @@ __device__ __noinline__ bool att_wait(uint64_t* bar, uint32_t parity, volatile i
 __global__ void __launch_bounds__(kThreads, 1)
 local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                                const __grid_constant__ CUtensorMap map_p, const __grid_constant__ CUtensorMap map_p16,
-                               const __grid_constant__ CUtensorMap map_v, const Params p) {
+                               const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_out, const Params p) {
     extern __shared__ uint8_t att5_raw[];
     Smem& sm = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(att5_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
@@ -192,6 +197,7 @@ local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const 
     const long long items = static_cast<long long>(kHeads) * p.tiles;
     const int first_item = static_cast<int>(items * blockIdx.x / gridDim.x);
     const int last_item = static_cast<int>(items * (blockIdx.x + 1) / gridDim.x);
+    const int first_head = first_item / p.tiles, first_tile = first_item % p.tiles;
 
     grid_dependents_launch();
     volatile int* abort_flag = &sm.abort;
@@ -220,7 +226,8 @@ local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const 
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = sm.tmem_base;
-    grid_dependency_wait();                  // Q, K and V come from the kernel before
+    // Q, K and V come from the kernel before: the roles wait for it where they first need it (p.early: the
+    // position rows and biases do not, so the first tile's are fetched and multiplied in its shadow)
     // slot of key block b (value block b: slot b)
     auto slot_of_key = [](int b) { return b == 0 ? 2 : b - 1; };
     // TMEM columns of the score block b and of the context
@@ -235,10 +242,12 @@ local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const 
         // ------------------------------------------------------------ TMA producer
         if (lane == 0) {
             uint32_t before = 0, ph_before = 0;        // key blocks and parities of the tile before (0: none)
+            if (!p.early) grid_dependency_wait();
+            int head = first_head, tile = first_tile - 1;
             for (int item = first_item; ok && item < last_item; ++item) {
-                const TilePlace at(p.rows, item % p.tiles);
+                if (++tile == p.tiles) { tile = 0; ++head; }
+                const TilePlace at(p.rows, tile);
                 if (at.padding()) continue;
-                const int head = item / p.tiles;
                 const uint32_t blocks = at.blocks(), par = (ph >> 1) & 1u;
                 const int key_row = at.base + at.q0 - kReach;
                 auto load_block = [&](int slot, const CUtensorMap* map, int bar, int b) {
@@ -246,10 +255,12 @@ local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const 
                     for (int a = 0; a < 2; ++a)
                         tma_load_2d(sm.slot[slot] + a * kAtomBytes, map, &sm.bar[bar], head * kDim + a * 64, key_row + b * 128);
                 };
-                // the score products of the tile before have retired (waited for below)
-                mbar_arrive_expect_tx(&sm.bar[B_Q_IN], kSlotBytes);
-                for (int a = 0; a < 2; ++a)
-                    tma_load_2d(sm.q + a * kAtomBytes, &map_q, &sm.bar[B_Q_IN], head * kDim + a * 64, at.base + at.q0);
+                auto load_queries = [&] {
+                    mbar_arrive_expect_tx(&sm.bar[B_Q_IN], kSlotBytes);
+                    for (int a = 0; a < 2; ++a)
+                        tma_load_2d(sm.q + a * kAtomBytes, &map_q, &sm.bar[B_Q_IN], head * kDim + a * 64, at.base + at.q0);
+                };
+                if (before != 0) load_queries();       // the score products of the tile before have retired
                 // position rows: slot 0 held V0 (or K1), slot 1 held V1 of the tile before
                 mbar_arrive_expect_tx(&sm.bar[B_P_IN], 2 * kSlotBytes + kTailBytes);
                 for (int a = 0; a < 2; ++a)
@@ -262,6 +273,10 @@ local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const 
                 for (int a = 0; a < 2; ++a)
                     tma_load_2d(sm.slot[1] + a * kAtomBytes, &map_p, &sm.bar[B_P_IN], a * 64, head * kPosRows + 128);
                 if (before & 4u) ATT_WAIT(B_PV_DONE + 2, (ph_before >> 2) & 1u);
+                if (before == 0) {
+                    if (p.early) grid_dependency_wait();
+                    load_queries();
+                }
                 if (blocks & 1u) load_block(slot_of_key(0), &map_k, B_K_IN + 0, 0);
                 // the other key blocks: once the position rows have been multiplied
                 ATT_WAIT(B_QP_DONE, par);
@@ -299,8 +314,11 @@ local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const 
             constexpr uint32_t idesc_v = idesc128 | (1u << 16);
             const uint32_t q_addr = smem_u32(sm.q);
             bool any = false;
+            int tile = first_tile - 1;
+            if (!p.early) grid_dependency_wait();              // (the geometry)
             for (int item = first_item; ok && item < last_item; ++item) {
-                const TilePlace at(p.rows, item % p.tiles);
+                if (++tile == p.tiles) tile = 0;
+                const TilePlace at(p.rows, tile);
                 if (at.padding()) continue;
                 const uint32_t blocks = at.blocks(), par = (ph >> 1) & 1u;
                 ATT_WAIT(B_Q_IN, par);
@@ -365,11 +383,16 @@ local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const 
         const uint64_t scale22 = pack2(scale2, scale2);
         const int qt = tid % 4;                                // features of the bias terms: 32 * qt ..
         int head_now = -1, base_now = -1, q0_now = 0;          // what vp and uk in shared memory belong to
+        int head = first_head, tile = first_tile - 1;
+        if (!p.early) grid_dependency_wait();
+        bool waited = !p.early;
         for (int item = first_item; ok && item < last_item; ++item) {
-            const TilePlace at(p.rows, item % p.tiles);
-            const int head = item / p.tiles;
+            if (++tile == p.tiles) { tile = 0; ++head; }
+            const TilePlace at(p.rows, tile);
             const int q0 = at.q0, valid = at.valid;
             if (at.padding()) {                  // the whole tile is padding: zeros
+                if (!waited) grid_dependency_wait();
+                waited = true;
                 for (int c = tid; c < kTile * 16; c += kSoftmaxThreads)
                     *reinterpret_cast<uint4*>(p.out + static_cast<size_t>(at.base + q0 + c / 16) * p.ldo + head * kDim + (c % 16) * 8) =
                         make_uint4(0, 0, 0, 0);
@@ -401,7 +424,12 @@ local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const 
                 __syncwarp();
             }
             head_now = head; base_now = at.base; q0_now = q0;
-            if (lane == 0) mbar_arrive(&sm.bar[B_VP_DONE]);
+            if (!waited) grid_dependency_wait();
+            waited = true;
+            if (lane == 0) {
+                bulk_wait_read_all();            // the staged context of the tile before has left
+                mbar_arrive(&sm.bar[B_VP_DONE]);
+            }
             ATT_WAIT(B_VP_DONE, par);
             // QP: tensor memory -> fp16 rows in shared memory, bias term added.  Row ql is stored shifted
             // right by (ql & 1) halves, so that the run of position columns a key piece needs (kk0 - ql ...)
@@ -410,72 +438,50 @@ local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const 
             ATT_WAIT(B_QP_DONE, par);
             tc_fence_after_sync();
             {
-                uint32_t* row = reinterpret_cast<uint32_t*>(&sm.qp[ql * kQpPitch]);
+                uint32_t* row = reinterpret_cast<uint32_t*>(&sm.qp[ql * kQpPitch]) + 32 * part;
                 const bool odd = (ql & 1) != 0;
-                // 32 columns per step (part 3: a last step of 16 columns, the load still 32 wide: the columns
-                // beyond 272 are never stored)
+                // An odd row's words hold (column 2m - 1, column 2m): one byte permute per word with a
+                // selector per lane; the two words shared with the neighbouring parts are written as halves.
+                const uint32_t sel = odd ? 0x5432u : 0x7654u;
+                uint32_t carry = 0;
+                // 32 columns per step (part 3: a last step of 16 columns)
                 const int steps = part == kParts - 1 ? 3 : 2;
 #pragma unroll 1
                 for (int st = 0; st < steps; ++st) {
                     const int c0 = 64 * part + 32 * st;
-                    const int words = st == 2 ? 8 : 16;
                     uint32_t r[32], w[16];
-                    tmem_ld_32x32(lane_addr + static_cast<uint32_t>(c0), r);
+                    tmem_ld_32x32(lane_addr + static_cast<uint32_t>(c0), r);    // (beyond column 272: never stored)
                     tmem_ld_wait();
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
-                        float4 t = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                        if (4 * i < 2 * words) t = *reinterpret_cast<const float4*>(&sm.vp[c0 + 4 * i]);
+                        const float4 t = *reinterpret_cast<const float4*>(&sm.vp[c0 + 4 * i]);
                         const __half2 h0 = __floats2half2_rn(__uint_as_float(r[4 * i + 0]) + t.x, __uint_as_float(r[4 * i + 1]) + t.y);
                         const __half2 h1 = __floats2half2_rn(__uint_as_float(r[4 * i + 2]) + t.z, __uint_as_float(r[4 * i + 3]) + t.w);
                         w[2 * i + 0] = *reinterpret_cast<const uint32_t*>(&h0);
                         w[2 * i + 1] = *reinterpret_cast<const uint32_t*>(&h1);
                     }
-                    // an odd row's words hold (column 2m - 1, column 2m): shifted by one half, the two
-                    // words shared with the neighbouring chunks are written as halves
-                    uint32_t* dst = row + c0 / 2;
-                    if (!odd) {
-#pragma unroll
-                        for (int i = 0; i < 16; ++i)
-                            if (i < words) dst[i] = w[i];
-                    } else {
+                    uint32_t* dst = row + 16 * st;
+                    if (st == 0 && odd)
                         reinterpret_cast<__half*>(dst)[1] = __ushort_as_half(static_cast<unsigned short>(w[0] & 0xFFFFu));
+                    else
+                        dst[0] = __byte_perm(carry, w[0], sel);
 #pragma unroll
-                        for (int i = 1; i < 16; ++i)
-                            if (i < words) dst[i] = __byte_perm(w[i - 1], w[i], 0x5432);
-                        const uint32_t last = words == 16 ? w[15] : w[7];
-                        reinterpret_cast<__half*>(dst + words)[0] = __ushort_as_half(static_cast<unsigned short>(last >> 16));
+                    for (int i = 1; i < 8; ++i) dst[i] = __byte_perm(w[i - 1], w[i], sel);
+                    if (st < 2) {
+#pragma unroll
+                        for (int i = 8; i < 16; ++i) dst[i] = __byte_perm(w[i - 1], w[i], sel);
+                        carry = w[15];
+                    } else {
+                        carry = w[7];
                     }
                 }
+                if (odd)
+                    reinterpret_cast<__half*>(row + (part == kParts - 1 ? 40 : 32))[0] =
+                        __ushort_as_half(static_cast<unsigned short>(carry >> 16));
             }
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) mbar_arrive(&sm.bar[B_QP_DRAINED]);
-            // u . K_kk for the keys of each new block, as soon as the block has landed: four threads per key
-            const int ring = q0 / kTile + 2;                   // key block b of the tile: row (ring + b) % 3
-            {
-                float bias[32];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const float4 t = *reinterpret_cast<const float4*>(&sm.bias_u[32 * qt + 4 * i]);
-                    bias[4 * i] = t.x; bias[4 * i + 1] = t.y; bias[4 * i + 2] = t.z; bias[4 * i + 3] = t.w;
-                }
-#pragma unroll 1
-                for (int b = 0; b < 3; ++b) {
-                    if (!((blocks >> b) & 1u)) continue;
-                    if (b == 2 || !follows) {
-                        ATT_WAIT(B_K_IN + b, (ph >> b) & 1u);
-                        const int row = tid / 4;
-                        float acc = bias_dot32(sm.slot[slot_of_key(b)] + (qt / 2) * kAtomBytes, row, 4 * (qt % 2), bias);
-                        acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-                        acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-                        if (qt == 0) sm.uk[(ring + b) % 3][row] = acc;
-                        __syncwarp();
-                    }
-                    if (lane == 0) mbar_arrive(&sm.bar[B_UK_DONE + b]);
-                }
-                if (!ok) break;
-            }
             ATT_WAIT(B_QP_DRAINED, par);
 
             // keys this query sees, in window coordinates: [lo, hi] (empty for a padding row)
@@ -487,13 +493,32 @@ local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const 
             const int w_lo = max(quad * 32, -key_first), w_hi = min(quad * 32 + 31 + 2 * kReach, valid - 1 - key_first);
             const int a_lo = max(quad * 32 + 31, -key_first);
             const int a_hi = q0 + quad * 32 + 31 < valid ? min(quad * 32 + 2 * kReach, valid - 1 - key_first) : -1;
+            const int ring = q0 / kTile + 2;                   // u . K of key block b of the tile: row (ring + b) % 3
             // A piece = 32 consecutive columns of this thread's scores, one per block.  Pass 0 writes the
             // scaled and masked scores back over the accumulators and finds the row maximum.
             float mx = -INFINITY, sum = 0.0f;
 #pragma unroll 1
             for (int b = 0; b < 3; ++b) {
                 if (!((blocks >> b) & 1u)) continue;
-                ATT_WAIT(B_UK_DONE + b, (ph >> b) & 1u);
+                if (b < 2 && follows) {
+                    if (lane == 0) mbar_arrive(&sm.bar[B_UK_DONE + b]);
+                } else {
+                    // u . K_kk for the 128 keys of a new block: four threads per key, 32 features each
+                    float bias[32];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const float4 t = *reinterpret_cast<const float4*>(&sm.bias_u[32 * qt + 4 * i]);
+                        bias[4 * i] = t.x; bias[4 * i + 1] = t.y; bias[4 * i + 2] = t.z; bias[4 * i + 3] = t.w;
+                    }
+                    ATT_WAIT(B_K_IN + b, (ph >> b) & 1u);
+                    float acc = bias_dot32(sm.slot[slot_of_key(b)] + (qt / 2) * kAtomBytes, tid / 4, 4 * (qt % 2), bias);
+                    acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+                    acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+                    if (qt == 0) sm.uk[(ring + b) % 3][tid / 4] = acc;
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&sm.bar[B_UK_DONE + b]);
+                    ATT_WAIT(B_UK_DONE + b, (ph >> b) & 1u);
+                }
                 ATT_WAIT(B_S_DONE + b, (ph >> b) & 1u);
                 tc_fence_after_sync();
                 const int kk0 = b * 128 + part * 32;
@@ -604,12 +629,23 @@ local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const 
                     const __half2 h = __floats2half2_rn(__uint_as_float(r[2 * i]) * inv, __uint_as_float(r[2 * i + 1]) * inv);
                     w[i] = q_live ? *reinterpret_cast<const uint32_t*>(&h) : 0u;
                 }
-                uint4* dst = reinterpret_cast<uint4*>(p.out + static_cast<size_t>(at.base + q0 + ql) * p.ldo + head * kDim + part * 32);
+                // out through shared memory (64-byte rows, 64-byte swizzle; the probabilities there are done
+                // with) and one TMA store per warp: 16-byte stores a row apart took 4.5k of a tile's 25k cycles
+                uint8_t* stage = sm.pr[1] + warp * 2048;
 #pragma unroll
-                for (int i = 0; i < 4; ++i) dst[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+                for (int i = 0; i < 4; ++i)
+                    *reinterpret_cast<uint4*>(stage + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4)) =
+                        make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) {
+                    tma_store_2d(&map_out, stage, head * kDim + part * 32, at.base + q0 + quad * 32);
+                    bulk_commit_group();
+                }
             }
             ph ^= blocks;
         }
+        if (lane == 0) bulk_wait_all();          // this warp's stores have landed
     }
 
     // ------------------------------------------------------------------- teardown
@@ -634,16 +670,17 @@ using namespace pk100;
 
 int pk100_local_attention_rows(void* stream_v, const void* query, int ldq, const void* key, int ldk, const void* value, int ldv,
                                const void* position, const void* bias_u, const void* bias_v, void* output, int ldo,
-                               int total_rows, const pk100_rows& geometry, int* status) {
+                               int total_rows, const pk100_rows& geometry, bool constants_settled, int* status) {
     using namespace att5;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
     const unsigned long long rows = static_cast<unsigned long long>(total_rows);
-    CUtensorMap map_q, map_k, map_p, map_p16, map_v;
+    CUtensorMap map_q, map_k, map_p, map_p16, map_v, map_out;
     int rc = pk100_tensor_map_2d(&map_q, query, 2, rows, 1024, ldq, kTile, 128);
     if (rc == PK100_OK) rc = pk100_tensor_map_2d(&map_k, key, 2, rows, 1024, ldk, 128, 128);
     if (rc == PK100_OK) rc = pk100_tensor_map_2d(&map_p, position, 2, kHeads * kPosRows, kDim, kDim, 128, 128);
     if (rc == PK100_OK) rc = pk100_tensor_map_2d(&map_p16, position, 2, kHeads * kPosRows, kDim, kDim, 16, 128);
     if (rc == PK100_OK) rc = pk100_tensor_map_2d(&map_v, value, 2, rows, 1024, ldv, 128, 128);
+    if (rc == PK100_OK) rc = pk100_tensor_map_2d(&map_out, output, 2, rows, 1024, ldo, 32, 64);
     if (rc != PK100_OK) return rc;
 
     constexpr int smem_bytes = static_cast<int>(sizeof(Smem)) + 1024;
@@ -656,11 +693,11 @@ int pk100_local_attention_rows(void* stream_v, const void* query, int ldq, const
     }
     const int tiles = total_rows / kTile;
     Params p{static_cast<const __half*>(bias_u), static_cast<const __half*>(bias_v), static_cast<__half*>(output), ldo,
-             tiles, geometry, status};
+             tiles, geometry, constants_settled ? 1 : 0, status};
     // one persistent CTA per SM; fewer while decoder clusters of earlier batches hold some of them
     const long long items = static_cast<long long>(kHeads) * tiles;
     const int ctas = static_cast<int>(items < pk100_cta_budget() ? items : pk100_cta_budget());
-    pk100_launch_chained(local_attention_tcgen05_kernel, dim3(ctas), dim3(kThreads), smem_bytes, stream, map_q, map_k, map_p, map_p16, map_v, p);
+    pk100_launch_chained(local_attention_tcgen05_kernel, dim3(ctas), dim3(kThreads), smem_bytes, stream, map_q, map_k, map_p, map_p16, map_v, map_out, p);
     return pk100_launch_status();
 }
 
@@ -679,5 +716,5 @@ extern "C" int pk100_local_relpos_attention_tcgen05(
     if (bits & 15u) return PK100_ERR_ALIGN;
     if (segments == 0) return PK100_OK;
     return pk100_local_attention_rows(stream_v, query, ldq, key, ldk, value, ldv, position, bias_u, bias_v, output, ldo,
-                                      segments * seg_stride, pk100_rows{nullptr, seg_stride, valid_rows, seg_valid}, status);
+                                      segments * seg_stride, pk100_rows{nullptr, seg_stride, valid_rows, seg_valid}, false, status);
 }

@@ -150,10 +150,13 @@ extern "C" int pk100_run_layers(void* stream, const pk100_layer_weights* layers,
                     w.position, w.bias_u, w.bias_v, ws.att, kWidth, segments, seg_stride, valid_rows,
                     seg_valid));
             } else if (attention_impl == 0 && seg_stride % 128 == 0) {
-                PK_TRY(pk100_local_relpos_attention_tcgen05(
+                if (!w.position || !w.bias_u || !w.bias_v) return PK100_ERR_NULL;
+                if ((reinterpret_cast<uintptr_t>(ws.qkv) | reinterpret_cast<uintptr_t>(w.position) |
+                     reinterpret_cast<uintptr_t>(ws.att)) & 15u) return PK100_ERR_ALIGN;
+                PK_TRY(pk100_local_attention_rows(
                     stream, qkv, 3 * kWidth, qkv + kWidth, 3 * kWidth, qkv + 2 * kWidth, 3 * kWidth,
-                    w.position, w.bias_u, w.bias_v, ws.att, kWidth, segments, seg_stride, valid_rows,
-                    seg_valid, ws.status));
+                    w.position, w.bias_u, w.bias_v, ws.att, kWidth, g.rows,
+                    pk100_rows{nullptr, seg_stride, valid_rows, seg_valid}, true, ws.status));
             } else {
                 PK_TRY(pk100_local_relpos_attention(
                     stream, qkv, 3 * kWidth, qkv + kWidth, 3 * kWidth, qkv + 2 * kWidth, 3 * kWidth,

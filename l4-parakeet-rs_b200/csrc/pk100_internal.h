@@ -68,9 +68,10 @@ int pk100_depthwise_bn_silu_rows(void* stream, const void* input, const void* dw
                                  int total_rows, int segments, const pk100_rows& geometry, float eps);
 
 // Local attention behind pk100_local_relpos_attention_tcgen05 on either geometry (total_rows: a multiple of 128).
+// constants_settled: the kernel before it in the stream writes neither position, biases nor the geometry.
 int pk100_local_attention_rows(void* stream, const void* query, int ldq, const void* key, int ldk, const void* value, int ldv,
                                const void* position, const void* bias_u, const void* bias_v, void* output, int ldo,
-                               int total_rows, const pk100_rows& geometry, int* status);
+                               int total_rows, const pk100_rows& geometry, bool constants_settled, int* status);
 
 // SMs a persistent kernel may use: all of them, or the cap set by pk100_set_gemm_cta_cap.
 int pk100_cta_budget();
