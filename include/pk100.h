@@ -329,6 +329,14 @@ int pk100_run_layers(void* stream, const pk100_layer_weights* layers, int n_laye
                      int seg_stride, int valid_rows, const int* seg_valid, float* tile_stats,
                      int attention_impl, void** output);
 
+/* The same on a packed batch: every utterance takes whole 128-row tiles and only as many as it needs, so a
+ * batch of unequal utterances carries no padding tiles.  rows: a multiple of 128; tiles (device, 8-byte
+ * aligned): rows / 128 pairs {first row of the tile's utterance, valid rows of that utterance}, written
+ * before the kernel in front of this call in the stream.  Same results per utterance as pk100_run_layers. */
+int pk100_run_layers_packed(void* stream, const pk100_layer_weights* layers, int n_layers, void* state_a,
+                            void* state_b, const pk100_encoder_workspace* workspace, int rows, const int* tiles,
+                            void** output);
+
 /* ------------------------------------------------------------------------
  * TDT greedy decoder.  Replaces DecoderWeights (src/cuda/decoder.rs:227-271),
  * launch_decode (:274-353) and the persistent kernels pk_sm89_tdt_persistent_v2
@@ -508,6 +516,14 @@ long long pk100_subsampling_fp8_workspace_bytes(int utterances, int frames, int 
 int pk100_run_subsampling_fp8(void* stream, const pk100_subsampling_weights* weights,
                               const pk100_subsampling_fp8* fp8, const float* mel, int utterances, int frames,
                               const int* mel_frames, void* workspace, void* output, int seg_stride, int* status);
+
+/* Either variant (q == NULL: fp16) with `mel_stride` >= frames mel rows between utterances and, when row_base
+ * (device, one int per utterance) is given, a packed output: utterance u fills whole 128-row tiles from row
+ * row_base[u] on, `rows` rows in all.  row_base == NULL: rows = utterances * seg_stride.  The workspace is that
+ * of (utterances, frames, seg_stride). */
+int pk100_run_subsampling_rows(void* stream, const pk100_subsampling_weights* weights, const pk100_subsampling_fp8* q,
+                               const float* mel, int mel_stride, int utterances, int frames, const int* mel_frames,
+                               void* workspace, void* output, int seg_stride, const int* row_base, int rows, int* status);
 
 /* ------------------------------------------------------------------------
  * ".pkl4" weight artifact: reader and layout packers (host code, no GPU).

@@ -51,7 +51,6 @@ constexpr int kHeads = 8;
 constexpr int kDim = 128;                 // head width
 constexpr int kTile = 128;                // queries per CTA
 constexpr int kReach = 128;               // keys on each side
-constexpr int kWindow = kTile + 2 * kReach;          // 384 keys seen by a tile
 constexpr int kPosRows = 272;             // position rows per head (257 used)
 constexpr float kSoftmaxScale = 0.08838834764831845f;
 constexpr int kParts = 4;                 // softmax warps per TMEM lane quadrant: 32 columns of a block each
@@ -92,7 +91,7 @@ struct Smem {
     };
     float vp[288];                                        // 272 used, the rest read and dropped
     float uk[3][128];                                     // key block i of the utterance -> row i % 3
-    alignas(16) float bias_u[kDim];
+    alignas(16) float bias_u[4][36];                      // 32 features a row, rows in different banks
     float rowmax[kParts][kTile];
     float rowsum[kParts][kTile];
     uint64_t bar[B_COUNT];
@@ -155,6 +154,13 @@ __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
 // byte offset of 16-byte chunk `chunk` (0..7) of row `row` inside a [rows x 64 halves] swizzled atom
 __device__ __forceinline__ int swz(int row, int chunk) {
     return (row >> 3) * 1024 + (row & 7) * 128 + ((chunk ^ (row & 7)) << 4);
+}
+
+// a + b in fp32, a widened inside the instruction
+__device__ __forceinline__ float add_half(__half a, float b) {
+    float d;
+    asm("add.rn.f32.f16 %0, %1, %2;" : "=f"(d) : "h"(__half_as_ushort(a)), "f"(b));
+    return d;
 }
 
 // dot product of 32 fp32 bias values (in registers) with 32 consecutive halves (chunks first ..
@@ -252,6 +258,7 @@ local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const 
                 const int key_row = at.base + at.q0 - kReach;
                 auto load_block = [&](int slot, const CUtensorMap* map, int bar, int b) {
                     mbar_arrive_expect_tx(&sm.bar[bar], kSlotBytes);
+#pragma unroll 1
                     for (int a = 0; a < 2; ++a)
                         tma_load_2d(sm.slot[slot] + a * kAtomBytes, map, &sm.bar[bar], head * kDim + a * 64, key_row + b * 128);
                 };
@@ -312,7 +319,10 @@ local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const 
             // B = V[keys, features] as it lies in memory: MN-major (features contiguous),
             // 8-key groups 1024 bytes apart, the second 64 features 16 KB on; 16 keys = 2048 bytes
             constexpr uint32_t idesc_v = idesc128 | (1u << 16);
-            const uint32_t q_addr = smem_u32(sm.q);
+            const uint64_t desc_q = make_smem_desc<128>(smem_u32(sm.q)), desc_tail = make_smem_desc<128>(smem_u32(sm.tail));
+            const uint64_t desc_slot[2] = {make_smem_desc<128>(smem_u32(sm.slot[0])), make_smem_desc<128>(smem_u32(sm.slot[1]))};
+            // K step of 16 halves inside a K-major operand block, in descriptor units of 16 bytes
+            auto k_offset = [](int ks) { return static_cast<uint32_t>((ks / 4) * (kAtomBytes / 16) + 2 * (ks % 4)); };
             bool any = false;
             int tile = first_tile - 1;
             if (!p.early) grid_dependency_wait();              // (the geometry)
@@ -325,47 +335,44 @@ local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const 
                 ATT_WAIT(B_P_IN, par);
                 tc_fence_after_sync();
                 // (columns [0, 272) are free: P_READY of the tile before came after their last read)
+#pragma unroll 1
                 for (int ks = 0; ks < 8; ++ks) {           // 16 features per MMA
-                    const int a = ks / 4, j = ks % 4;
-                    const uint64_t da = make_smem_desc<128>(q_addr + a * kAtomBytes) + 2u * j;
-                    for (int b = 0; b < 2; ++b)
-                        tc_mma<KIND_F16>(tmem + 128u * b, da,
-                                         make_smem_desc<128>(smem_u32(sm.slot[b]) + a * kAtomBytes) + 2u * j, idesc128, ks > 0);
-                    tc_mma<KIND_F16>(tmem + 256u, da,
-                                     make_smem_desc<128>(smem_u32(sm.tail) + a * (kTailBytes / 2)) + 2u * j, idesc16, ks > 0);
+                    const uint32_t off = k_offset(ks);
+                    tc_mma<KIND_F16>(tmem, desc_q + off, desc_slot[0] + off, idesc128, ks > 0);
+                    tc_mma<KIND_F16>(tmem + 128u, desc_q + off, desc_slot[1] + off, idesc128, ks > 0);
+                    tc_mma<KIND_F16>(tmem + 256u, desc_q + off, desc_tail + (ks / 4) * (kTailBytes / 32) + 2u * (ks % 4), idesc16, ks > 0);
                 }
                 tc_commit(&sm.bar[B_QP_DONE]);
                 // S_0 and the context share their columns
                 if (any) ATT_WAIT(B_CTX_READ, par ^ 1u);
                 any = true;
+#pragma unroll 1
                 for (int b = 0; b < 3; ++b) {
                     if (!((blocks >> b) & 1u)) continue;
                     if (b == 1) ATT_WAIT(B_QP_DRAINED, par);   // columns [0, 272) are free
                     ATT_WAIT(B_K_IN + b, (ph >> b) & 1u);
                     tc_fence_after_sync();
-                    const uint32_t k_addr = smem_u32(sm.slot[slot_of_key(b)]);
-                    for (int ks = 0; ks < 8; ++ks) {
-                        const int a = ks / 4, j = ks % 4;
-                        tc_mma<KIND_F16>(tmem + score_col(b), make_smem_desc<128>(q_addr + a * kAtomBytes) + 2u * j,
-                                         make_smem_desc<128>(k_addr + a * kAtomBytes) + 2u * j, idesc128, ks > 0);
-                    }
+                    const uint64_t desc_k = desc_slot[0] + static_cast<uint32_t>(slot_of_key(b) * (kSlotBytes / 16));
+#pragma unroll 1
+                    for (int ks = 0; ks < 8; ++ks)
+                        tc_mma<KIND_F16>(tmem + score_col(b), desc_q + k_offset(ks), desc_k + k_offset(ks), idesc128, ks > 0);
                     tc_commit(&sm.bar[B_S_DONE + b]);
                 }
                 if (!ok) break;
                 uint32_t accumulate = 0;
+#pragma unroll 1
                 for (int b = 0; b < 3; ++b) {
                     if (!((blocks >> b) & 1u)) continue;
                     ATT_WAIT(B_V_IN + b, (ph >> b) & 1u);
                     ATT_WAIT(B_P_READY + b, (ph >> b) & 1u);
                     tc_fence_after_sync();
-                    const uint32_t v_addr = smem_u32(sm.slot[b]), p_addr = smem_u32(sm.pr[b & 1]);
-                    for (int ks = 0; ks < 8; ++ks) {       // 16 keys per MMA
-                        const int a = ks / 4, j = ks % 4;
-                        const uint64_t dv = static_cast<uint64_t>(((v_addr + ks * 2048u) & 0x3FFFFu) >> 4) |
+                    const uint64_t desc_v = static_cast<uint64_t>((smem_u32(sm.slot[b]) & 0x3FFFFu) >> 4) |
                                             (static_cast<uint64_t>(kAtomBytes >> 4) << 16) | (64ull << 32) |
                                             (1ull << 46) | (2ull << 61);
-                        tc_mma<KIND_F16>(tmem + kCtxCol, make_smem_desc<128>(p_addr + a * kAtomBytes) + 2u * j,
-                                         dv, idesc_v, accumulate);
+                    const uint64_t desc_p = make_smem_desc<128>(smem_u32(sm.pr[b & 1]));
+#pragma unroll 1
+                    for (int ks = 0; ks < 8; ++ks) {       // 16 keys per MMA
+                        tc_mma<KIND_F16>(tmem + kCtxCol, desc_p + k_offset(ks), desc_v + ks * 128u, idesc_v, accumulate);
                         accumulate = 1;
                     }
                     tc_commit(&sm.bar[B_PV_DONE + b]);
@@ -381,7 +388,9 @@ local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const 
         constexpr float kLog2e = 1.4426950408889634f;
         const float scale2 = kSoftmaxScale * kLog2e;
         const uint64_t scale22 = pack2(scale2, scale2);
-        const int qt = tid % 4;                                // features of the bias terms: 32 * qt ..
+        // Bias terms: four lanes per operand row, 32 features each (32 * qt ..).  The eight lanes of a
+        // 16-byte shared-memory access are four rows of one 64-feature atom: eight different chunks.
+        const int qt = (lane & 1) | ((lane >> 2) & 2), bias_row = warp * 8 + (((lane >> 1) & 3) | ((lane >> 2) & 4));
         int head_now = -1, base_now = -1, q0_now = 0;          // what vp and uk in shared memory belong to
         int head = first_head, tile = first_tile - 1;
         if (!p.early) grid_dependency_wait();
@@ -406,19 +415,18 @@ local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const 
             if (head != head_now) {
                 // v . P_j for the 272 position rows (per-column constant of QP): four threads per row,
                 // 32 features each, from the staged operand tiles
-                if (tid < kDim) sm.bias_u[tid] = __half2float(p.bias_u[head * kDim + tid]);
+                if (tid < kDim) sm.bias_u[tid / 32][tid % 32] = __half2float(p.bias_u[head * kDim + tid]);
                 float bias[32];
 #pragma unroll
                 for (int i = 0; i < 32; ++i) bias[i] = __half2float(p.bias_v[head * kDim + 32 * qt + i]);
                 ATT_WAIT(B_P_IN, par);
 #pragma unroll 1
-                for (int i = tid; i < 4 * kPosRows; i += kSoftmaxThreads) {
-                    const int row = i / 4;
+                for (int row = bias_row; row < kPosRows; row += kSoftmaxThreads / 4) {   // (whole warps)
                     const uint8_t* atom = row < 256 ? sm.slot[row / 128] + (qt / 2) * kAtomBytes
                                                     : sm.tail + (qt / 2) * (kTailBytes / 2);
                     float acc = bias_dot32(atom, row < 256 ? row % 128 : row - 256, 4 * (qt % 2), bias);
                     acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-                    acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+                    acc += __shfl_xor_sync(0xffffffffu, acc, 8);
                     if (qt == 0) sm.vp[row] = acc;
                 }
                 __syncwarp();
@@ -507,14 +515,14 @@ local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const 
                     float bias[32];
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
-                        const float4 t = *reinterpret_cast<const float4*>(&sm.bias_u[32 * qt + 4 * i]);
+                        const float4 t = *reinterpret_cast<const float4*>(&sm.bias_u[qt][4 * i]);
                         bias[4 * i] = t.x; bias[4 * i + 1] = t.y; bias[4 * i + 2] = t.z; bias[4 * i + 3] = t.w;
                     }
                     ATT_WAIT(B_K_IN + b, (ph >> b) & 1u);
-                    float acc = bias_dot32(sm.slot[slot_of_key(b)] + (qt / 2) * kAtomBytes, tid / 4, 4 * (qt % 2), bias);
+                    float acc = bias_dot32(sm.slot[slot_of_key(b)] + (qt / 2) * kAtomBytes, bias_row, 4 * (qt % 2), bias);
                     acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-                    acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-                    if (qt == 0) sm.uk[(ring + b) % 3][tid / 4] = acc;
+                    acc += __shfl_xor_sync(0xffffffffu, acc, 8);
+                    if (qt == 0) sm.uk[(ring + b) % 3][bias_row] = acc;
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&sm.bar[B_UK_DONE + b]);
                     ATT_WAIT(B_UK_DONE + b, (ph >> b) & 1u);
@@ -523,40 +531,43 @@ local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const 
                 tc_fence_after_sync();
                 const int kk0 = b * 128 + part * 32;
                 if (kk0 + 31 < w_lo || kk0 > w_hi) continue;
-                uint32_t r[32];
-                tmem_ld_32x32(lane_addr + score_col(b) + static_cast<uint32_t>(part * 32), r);
-                // position scores of columns kk0 - ql .. + 31: stored from half (ql & 1) on, so the
-                // run starts at a word of the row (kk0 is even)
-                const __half2* qp2 = reinterpret_cast<const __half2*>(&sm.qp[ql * kQpPitch + kk0 - ql + (ql & 1)]);
-                const float4* uk4 = reinterpret_cast<const float4*>(&sm.uk[(ring + b) % 3][part * 32]);
-                uint64_t t2[16];
+                const bool whole = kk0 >= a_lo && kk0 + 31 <= a_hi;
+                // two halves of 16 columns: 32 at a time spilled
+#pragma unroll 1
+                for (int c0 = 0; c0 < 32; c0 += 16) {
+                    uint32_t r[16];
+                    const uint32_t taddr = lane_addr + score_col(b) + static_cast<uint32_t>(part * 32 + c0);
+                    tmem_ld_32x16(taddr, r);
+                    // position scores of columns kk0 + c0 - ql ..: stored from half (ql & 1) on, so the
+                    // run starts at a word of the row (kk0 is even)
+                    const __half2* qp2 = reinterpret_cast<const __half2*>(&sm.qp[ql * kQpPitch + kk0 + c0 - ql + (ql & 1)]);
+                    const float4* uk4 = reinterpret_cast<const float4*>(&sm.uk[(ring + b) % 3][part * 32 + c0]);
+                    float s[16];
 #pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    const float4 u = uk4[c];
-                    const float2 a = __half22float2(qp2[2 * c]), bb = __half22float2(qp2[2 * c + 1]);
-                    t2[2 * c] = add2(pack2(a.x, a.y), pack2(u.x, u.y));
-                    t2[2 * c + 1] = add2(pack2(bb.x, bb.y), pack2(u.z, u.w));
-                }
-                tmem_ld_wait();
-                float s[32];
+                    for (int c = 0; c < 4; ++c) {
+                        const float4 u = uk4[c];
+                        s[4 * c + 0] = add_half(__low2half(qp2[2 * c]), u.x);
+                        s[4 * c + 1] = add_half(__high2half(qp2[2 * c]), u.y);
+                        s[4 * c + 2] = add_half(__low2half(qp2[2 * c + 1]), u.z);
+                        s[4 * c + 3] = add_half(__high2half(qp2[2 * c + 1]), u.w);
+                    }
+                    tmem_ld_wait();
 #pragma unroll
-                for (int i = 0; i < 16; ++i)
-                    unpack2(mul2(add2(pack2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), t2[i]), scale22),
-                            s[2 * i], s[2 * i + 1]);
-                if (kk0 < a_lo || kk0 + 31 > a_hi) {
-                    const int off = kk0 - lo;
-                    const bool some = hi >= lo;
+                    for (int i = 0; i < 8; ++i)
+                        unpack2(mul2(add2(pack2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), pack2(s[2 * i], s[2 * i + 1])), scale22),
+                                s[2 * i], s[2 * i + 1]);
+                    if (!whole) {
+                        const int off = kk0 + c0 - lo;
+                        const bool some = hi >= lo;
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) s[i] = some && static_cast<unsigned>(off + i) <= span ? s[i] : -INFINITY;
-                }
+                        for (int i = 0; i < 16; ++i) s[i] = some && static_cast<unsigned>(off + i) <= span ? s[i] : -INFINITY;
+                    }
 #pragma unroll
-                for (int i = 0; i < 32; ++i) mx = fmaxf(mx, s[i]);
-#pragma unroll
-                for (int hf = 0; hf < 2; ++hf) {
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(s[16 * hf + i]);
-                    tmem_st_32x16(lane_addr + score_col(b) + static_cast<uint32_t>(part * 32 + 16 * hf),
-                                  *reinterpret_cast<const uint32_t(*)[16]>(&r[0]));
+                    for (int i = 0; i < 16; ++i) {
+                        mx = fmaxf(mx, s[i]);
+                        r[i] = __float_as_uint(s[i]);
+                    }
+                    tmem_st_32x16(taddr, r);
                 }
             }
             if (!ok) break;

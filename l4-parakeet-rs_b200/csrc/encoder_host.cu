@@ -20,6 +20,7 @@ long long align256(long long v) { return (v + 255) / 256 * 256; }
 struct Geometry {
     int rows, segments, seg_stride, valid_rows;
     const int* seg_valid;
+    const int2* tiles;        // packed batch: place of every 128-row tile (pk100_rows), else nullptr
 };
 
 #define PK_TRY(expr)                 \
@@ -102,21 +103,28 @@ extern "C" int pk100_encoder_workspace_carve(void* base, int rows, pk100_encoder
     return PK100_OK;
 }
 
-extern "C" int pk100_run_layers(void* stream, const pk100_layer_weights* layers, int n_layers,
-                                void* state_a, void* state_b, const pk100_encoder_workspace* wsp,
-                                int segments, int seg_stride, int valid_rows, const int* seg_valid,
-                                float* tile_stats, int attention_impl, void** output) {
+static int run_layers(void* stream, const pk100_layer_weights* layers, int n_layers, void* state_a, void* state_b,
+                      const pk100_encoder_workspace* wsp, const Geometry& g, float* tile_stats, int attention_impl,
+                      void** output) {
     if (!layers || !state_a || !state_b || !wsp) return PK100_ERR_NULL;
-    if (n_layers < 0 || segments < 0 || seg_stride <= 0) return PK100_ERR_SHAPE;
+    const int segments = g.segments, seg_stride = g.seg_stride, valid_rows = g.valid_rows;
+    const int* const seg_valid = g.seg_valid;
+    const pk100_rows place{g.tiles, seg_stride, valid_rows, seg_valid};
     const pk100_encoder_workspace& ws = *wsp;
     if (!ws.q8 || !ws.row_scales || !ws.hidden8 || !ws.keep || !ws.qkv || !ws.att || !ws.glu ||
         !ws.dw8 || !ws.dw_scales)
         return PK100_ERR_NULL;
-    Geometry g{segments * seg_stride, segments, seg_stride, valid_rows, seg_valid};
     void* x = state_a;
     void* other = state_b;
     if (output) *output = x;
     if (g.rows == 0 || n_layers == 0) return PK100_OK;
+    // the row-wise operators of a packed batch have no entry points of their own
+    auto norm = [&](const void* in, const void* gamma, const void* beta, void* out, float* scales, int mode, float inv_scale) {
+        if (g.tiles == nullptr)
+            return pk100_layer_norm(stream, in, gamma, beta, out, scales, mode, inv_scale, g.rows, seg_stride, valid_rows, seg_valid, kEps);
+        if (!gamma || !beta) return static_cast<int>(PK100_ERR_NULL);
+        return pk100_layer_norm_rows(stream, in, gamma, beta, out, scales, mode, inv_scale, g.rows, place, kEps);
+    };
     const long long stats_stride = static_cast<long long>((g.rows + 127) / 128) * 64;
 
     for (int i = 0; i < n_layers; ++i) {
@@ -127,16 +135,12 @@ extern "C" int pk100_run_layers(void* stream, const pk100_layer_weights* layers,
 
         // ---- feed-forward module 1 (its LayerNorm was fused into the previous block's output norm)
         if (i == 0) {
-            PK_TRY(pk100_layer_norm(stream, x, w.ff1.ln_gamma, w.ff1.ln_beta, ws.q8, nullptr,
-                                    PK100_LN_E4M3_FIXED, kFp8InputInv, g.rows, seg_stride,
-                                    valid_rows, seg_valid, kEps));
+            PK_TRY(norm(x, w.ff1.ln_gamma, w.ff1.ln_beta, ws.q8, nullptr, PK100_LN_E4M3_FIXED, kFp8InputInv));
         }
         PK_TRY(ff_module(stream, w.ff1, x, ws, g, stats1, 2 * i));
 
         // ---- self-attention
-        PK_TRY(pk100_layer_norm(stream, x, w.ln_att_gamma, w.ln_att_beta, ws.q8, ws.row_scales,
-                                PK100_LN_S8_ROW, 0.0f, g.rows, seg_stride, valid_rows, seg_valid,
-                                kEps));
+        PK_TRY(norm(x, w.ln_att_gamma, w.ln_att_beta, ws.q8, ws.row_scales, PK100_LN_S8_ROW, 0.0f));
         gemm_base(a, PK100_KIND_S8, g.rows, 3 * kWidth, kWidth, ws.q8, w.wqkv);
         a.row_scales = ws.row_scales;
         a.col_scales = w.wqkv_scales;
@@ -149,14 +153,14 @@ extern "C" int pk100_run_layers(void* stream, const pk100_layer_weights* layers,
                     stream, qkv, 3 * kWidth, qkv + kWidth, 3 * kWidth, qkv + 2 * kWidth, 3 * kWidth,
                     w.position, w.bias_u, w.bias_v, ws.att, kWidth, segments, seg_stride, valid_rows,
                     seg_valid));
-            } else if (attention_impl == 0 && seg_stride % 128 == 0) {
+            } else if (attention_impl == 0 && (g.tiles != nullptr || seg_stride % 128 == 0)) {
                 if (!w.position || !w.bias_u || !w.bias_v) return PK100_ERR_NULL;
                 if ((reinterpret_cast<uintptr_t>(ws.qkv) | reinterpret_cast<uintptr_t>(w.position) |
                      reinterpret_cast<uintptr_t>(ws.att)) & 15u) return PK100_ERR_ALIGN;
                 PK_TRY(pk100_local_attention_rows(
                     stream, qkv, 3 * kWidth, qkv + kWidth, 3 * kWidth, qkv + 2 * kWidth, 3 * kWidth,
                     w.position, w.bias_u, w.bias_v, ws.att, kWidth, g.rows,
-                    pk100_rows{nullptr, seg_stride, valid_rows, seg_valid}, true, ws.status));
+                    place, true, ws.status));
             } else {
                 PK_TRY(pk100_local_relpos_attention(
                     stream, qkv, 3 * kWidth, qkv + kWidth, 3 * kWidth, qkv + 2 * kWidth, 3 * kWidth,
@@ -175,9 +179,7 @@ extern "C" int pk100_run_layers(void* stream, const pk100_layer_weights* layers,
         PK_TRY(pk100_gemm(stream, &a));
 
         // ---- convolution module
-        PK_TRY(pk100_layer_norm(stream, x, w.ln_conv_gamma, w.ln_conv_beta, ws.q8, ws.row_scales,
-                                PK100_LN_E4M3_ROW, 0.0f, g.rows, seg_stride, valid_rows, seg_valid,
-                                kEps));
+        PK_TRY(norm(x, w.ln_conv_gamma, w.ln_conv_beta, ws.q8, ws.row_scales, PK100_LN_E4M3_ROW, 0.0f));
         gemm_base(a, PK100_KIND_E4M3, g.rows, 2 * kWidth, kWidth, ws.q8, w.wpw1);
         a.epilogue = PK100_EPI_GLU;
         a.row_scales = ws.row_scales;
@@ -186,9 +188,15 @@ extern "C" int pk100_run_layers(void* stream, const pk100_layer_weights* layers,
         // the pad mask is per utterance: handled by the depthwise kernel's row bound, and the
         // LayerNorm above already zero-filled pad rows, so GLU(0, 0) = 0 there
         PK_TRY(pk100_gemm(stream, &a));
-        PK_TRY(pk100_depthwise_bn_silu(stream, ws.glu, w.dw_weight, w.bn_gamma, w.bn_beta, w.bn_mean,
-                                       w.bn_var, ws.dw8, ws.dw_scales, 1, segments, seg_stride,
-                                       valid_rows, seg_valid, kEps));
+        if (g.tiles == nullptr) {
+            PK_TRY(pk100_depthwise_bn_silu(stream, ws.glu, w.dw_weight, w.bn_gamma, w.bn_beta, w.bn_mean,
+                                           w.bn_var, ws.dw8, ws.dw_scales, 1, segments, seg_stride,
+                                           valid_rows, seg_valid, kEps));
+        } else {
+            if (!w.dw_weight || !w.bn_gamma || !w.bn_beta || !w.bn_mean || !w.bn_var) return PK100_ERR_NULL;
+            PK_TRY(pk100_depthwise_bn_silu_rows(stream, ws.glu, w.dw_weight, w.bn_gamma, w.bn_beta, w.bn_mean,
+                                                w.bn_var, ws.dw8, ws.dw_scales, 1, g.rows, segments, place, kEps));
+        }
         gemm_base(a, PK100_KIND_E4M3, g.rows, kWidth, kWidth, ws.dw8, w.wpw2);
         a.row_scales = ws.dw_scales;
         a.col_scales = w.wpw2_scales;
@@ -196,25 +204,49 @@ extern "C" int pk100_run_layers(void* stream, const pk100_layer_weights* layers,
         PK_TRY(pk100_gemm(stream, &a));
 
         // ---- feed-forward module 2
-        PK_TRY(pk100_layer_norm(stream, x, w.ff2.ln_gamma, w.ff2.ln_beta, ws.q8, nullptr,
-                                PK100_LN_E4M3_FIXED, kFp8InputInv, g.rows, seg_stride, valid_rows,
-                                seg_valid, kEps));
+        PK_TRY(norm(x, w.ff2.ln_gamma, w.ff2.ln_beta, ws.q8, nullptr, PK100_LN_E4M3_FIXED, kFp8InputInv));
         PK_TRY(ff_module(stream, w.ff2, x, ws, g, stats2, 2 * i + 1));
 
         // ---- output norm, fused with the next block's first norm
         if (i + 1 < n_layers) {
             const pk100_layer_weights& nx = layers[i + 1];
-            PK_TRY(pk100_layer_norm_pair(stream, x, w.ln_out_gamma, w.ln_out_beta, other,
-                                         nx.ff1.ln_gamma, nx.ff1.ln_beta, ws.q8, nullptr,
-                                         PK100_LN_E4M3_FIXED, kFp8InputInv, g.rows, seg_stride,
-                                         valid_rows, seg_valid, kEps));
+            if (g.tiles == nullptr) {
+                PK_TRY(pk100_layer_norm_pair(stream, x, w.ln_out_gamma, w.ln_out_beta, other,
+                                             nx.ff1.ln_gamma, nx.ff1.ln_beta, ws.q8, nullptr,
+                                             PK100_LN_E4M3_FIXED, kFp8InputInv, g.rows, seg_stride,
+                                             valid_rows, seg_valid, kEps));
+            } else {
+                if (!w.ln_out_gamma || !w.ln_out_beta || !nx.ff1.ln_gamma || !nx.ff1.ln_beta) return PK100_ERR_NULL;
+                PK_TRY(pk100_layer_norm_pair_rows(stream, x, w.ln_out_gamma, w.ln_out_beta, other,
+                                                  nx.ff1.ln_gamma, nx.ff1.ln_beta, ws.q8, nullptr,
+                                                  PK100_LN_E4M3_FIXED, kFp8InputInv, g.rows, place, kEps));
+            }
         } else {
-            PK_TRY(pk100_layer_norm(stream, x, w.ln_out_gamma, w.ln_out_beta, other, nullptr,
-                                    PK100_LN_F16, 0.0f, g.rows, seg_stride, valid_rows, seg_valid,
-                                    kEps));
+            PK_TRY(norm(x, w.ln_out_gamma, w.ln_out_beta, other, nullptr, PK100_LN_F16, 0.0f));
         }
         void* t = x; x = other; other = t;
         if (output) *output = x;
     }
     return PK100_OK;
+}
+
+extern "C" int pk100_run_layers(void* stream, const pk100_layer_weights* layers, int n_layers,
+                                void* state_a, void* state_b, const pk100_encoder_workspace* wsp,
+                                int segments, int seg_stride, int valid_rows, const int* seg_valid,
+                                float* tile_stats, int attention_impl, void** output) {
+    if (!layers || !state_a || !state_b || !wsp) return PK100_ERR_NULL;
+    if (n_layers < 0 || segments < 0 || seg_stride <= 0) return PK100_ERR_SHAPE;
+    const Geometry g{segments * seg_stride, segments, seg_stride, valid_rows, seg_valid, nullptr};
+    return run_layers(stream, layers, n_layers, state_a, state_b, wsp, g, tile_stats, attention_impl, output);
+}
+
+extern "C" int pk100_run_layers_packed(void* stream, const pk100_layer_weights* layers, int n_layers,
+                                       void* state_a, void* state_b, const pk100_encoder_workspace* wsp,
+                                       int rows, const int* tiles, void** output) {
+    if (!layers || !state_a || !state_b || !wsp || !tiles) return PK100_ERR_NULL;
+    if (n_layers < 0 || rows < 0 || rows % 128 != 0) return PK100_ERR_SHAPE;
+    if (reinterpret_cast<uintptr_t>(tiles) & 7u) return PK100_ERR_ALIGN;
+    if ((reinterpret_cast<uintptr_t>(state_a) | reinterpret_cast<uintptr_t>(state_b)) & 15u) return PK100_ERR_ALIGN;
+    const Geometry g{rows, 1, rows, rows, nullptr, reinterpret_cast<const int2*>(tiles)};
+    return run_layers(stream, layers, n_layers, state_a, state_b, wsp, g, nullptr, 0, output);
 }

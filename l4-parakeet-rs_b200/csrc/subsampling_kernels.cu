@@ -345,18 +345,20 @@ subsample_depthwise_kernel(const __half* __restrict__ in, const __half* __restri
 
 // [utt][cap][16][256] -> rows [utt*seg_stride + frame][channel*16 + feature]; rows at or
 // beyond the utterance's output length are zero (kernels/sm89/subsampling.cu:202-226).
+// row_base != nullptr (packed batch): utterance utt starts at row row_base[utt] and has whole 128-row tiles.
 // 128 threads per row, thread = two neighbouring channels: their 32 features are contiguous in the row.
 // Fp8: the row leaves as E4M3 codes with one scale (absmax / 448).
 template <bool Fp8>
 __global__ void __launch_bounds__(128)
 subsample_flatten_kernel(const __half* __restrict__ in, void* __restrict__ out, float* __restrict__ out_scales,
                          int in_cap, int seg_stride, int mel_frames_uniform,
-                         const int* __restrict__ mel_frames_per_utt) {
+                         const int* __restrict__ mel_frames_per_utt, const int* __restrict__ row_base) {
     __shared__ float warp_max[4];
     const int frame = blockIdx.x, utt = blockIdx.y, tid = threadIdx.x;
     int valid = frames_of(mel_frames_per_utt, utt, mel_frames_uniform);
     for (int l = 0; l < 3; ++l) valid = (valid + 1) / 2;
-    const size_t row = static_cast<size_t>(utt) * seg_stride + frame;
+    if (row_base != nullptr && frame >= (valid + 127) / 128 * 128) return;
+    const size_t row = (row_base != nullptr ? static_cast<size_t>(row_base[utt]) : static_cast<size_t>(utt) * seg_stride) + frame;
     const __half2* src = reinterpret_cast<const __half2*>(in + (static_cast<size_t>(utt) * in_cap + frame) * 16 * kChannels) + tid;
     __half2 v[16];
 #pragma unroll
@@ -437,15 +439,27 @@ extern "C" long long pk100_subsampling_fp8_workspace_bytes(int utterances, int f
 }
 
 static int run_subsampling(void* stream_v, const pk100_subsampling_weights* w, const pk100_subsampling_fp8* q,
-                           const float* mel, int utterances, int frames, const int* mel_frames, void* workspace,
-                           void* output, int seg_stride, int* status);
+                           const float* mel, int mel_stride, int utterances, int frames, const int* mel_frames,
+                           void* workspace, void* output, int seg_stride, const int* row_base, int rows, int* status);
 
 extern "C" int pk100_run_subsampling(void* stream_v, const pk100_subsampling_weights* w,
                                      const float* mel, int utterances, int frames,
                                      const int* mel_frames, void* workspace, void* output,
                                      int seg_stride, int* status) {
-    return run_subsampling(stream_v, w, nullptr, mel, utterances, frames, mel_frames, workspace, output, seg_stride,
-                           status);
+    return run_subsampling(stream_v, w, nullptr, mel, frames, utterances, frames, mel_frames, workspace, output, seg_stride,
+                           nullptr, utterances * seg_stride, status);
+}
+
+extern "C" int pk100_run_subsampling_rows(void* stream_v, const pk100_subsampling_weights* w, const pk100_subsampling_fp8* q,
+                                          const float* mel, int mel_stride, int utterances, int frames, const int* mel_frames,
+                                          void* workspace, void* output, int seg_stride, const int* row_base, int rows,
+                                          int* status) {
+    if (q != nullptr && (!q->pw1_q || !q->pw1_scales || !q->proj_q || !q->proj_scales)) return PK100_ERR_NULL;
+    if (utterances < 0 || mel_stride < frames) return PK100_ERR_SHAPE;
+    if (row_base == nullptr ? rows != utterances * seg_stride : (rows <= 0 || rows % 128 != 0 || rows > utterances * seg_stride))
+        return PK100_ERR_SHAPE;
+    return run_subsampling(stream_v, w, q, mel, mel_stride, utterances, frames, mel_frames, workspace, output, seg_stride,
+                           row_base, rows, status);
 }
 
 extern "C" int pk100_run_subsampling_fp8(void* stream_v, const pk100_subsampling_weights* w,
@@ -453,12 +467,13 @@ extern "C" int pk100_run_subsampling_fp8(void* stream_v, const pk100_subsampling
                                          int frames, const int* mel_frames, void* workspace, void* output,
                                          int seg_stride, int* status) {
     if (!q || !q->pw1_q || !q->pw1_scales || !q->proj_q || !q->proj_scales) return PK100_ERR_NULL;
-    return run_subsampling(stream_v, w, q, mel, utterances, frames, mel_frames, workspace, output, seg_stride, status);
+    return run_subsampling(stream_v, w, q, mel, frames, utterances, frames, mel_frames, workspace, output, seg_stride,
+                           nullptr, utterances * seg_stride, status);
 }
 
 static int run_subsampling(void* stream_v, const pk100_subsampling_weights* w, const pk100_subsampling_fp8* q,
-                           const float* mel, int utterances, int frames, const int* mel_frames, void* workspace,
-                           void* output, int seg_stride, int* status) {
+                           const float* mel, int mel_stride, int utterances, int frames, const int* mel_frames,
+                           void* workspace, void* output, int seg_stride, const int* row_base, int rows, int* status) {
     if (!w || !mel || !workspace || !output) return PK100_ERR_NULL;
     if (!w->conv0_w || !w->conv0_b || !w->dw1_w || !w->dw1_b || !w->pw1_w || !w->pw1_b || !w->dw2_w ||
         !w->dw2_b || !w->pw2_w || !w->pw2_b || !w->proj_w || !w->proj_b)
@@ -497,7 +512,7 @@ static int run_subsampling(void* stream_v, const pk100_subsampling_weights* w, c
                                                  sizeof(float2) * kFirstPitch * first_rows(kFirstMaxFrames));
     if (err != cudaSuccess) return static_cast<int>(err);
     first_kernel<<<first_grid, kFirstThreads, first_bytes, stream>>>(mel, w0, b0, w1, b1, q != nullptr ? static_cast<void*>(q2) : s2,
-                                                                     q2_scales, frames, frames, mel_frames, c.f2, run);
+                                                                     q2_scales, mel_stride, frames, mel_frames, c.f2, run);
     int rc = pk100_launch_status();
     if (rc != PK100_OK) return rc;
 
@@ -525,13 +540,13 @@ static int run_subsampling(void* stream_v, const pk100_subsampling_weights* w, c
 
     if (q != nullptr)
         subsample_flatten_kernel<true><<<dim3(seg_stride, utterances), 128, 0, stream>>>(s5, qflat, qflat_scales, c.f3, seg_stride,
-                                                                                         frames, mel_frames);
+                                                                                         frames, mel_frames, row_base);
     else
         subsample_flatten_kernel<false><<<dim3(seg_stride, utterances), 128, 0, stream>>>(s5, flat, nullptr, c.f3, seg_stride,
-                                                                                          frames, mel_frames);
+                                                                                          frames, mel_frames, row_base);
     if ((rc = pk100_launch_status()) != PK100_OK) return rc;
 
-    a.m = static_cast<int>(u * seg_stride); a.n = 1024; a.k = 4096;
+    a.m = rows; a.n = 1024; a.k = 4096;
     a.a = flat; a.lda = 4096; a.b = w->proj_w; a.ldb = 4096; a.bias = w->proj_b; a.act = PK100_ACT_NONE;
     a.out = output; a.ld_out = 1024;
     if (q != nullptr) {

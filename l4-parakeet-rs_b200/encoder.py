@@ -50,6 +50,9 @@ L.lib.pk100_encoder_workspace_carve.restype = C.c_int
 L.lib.pk100_run_layers.argtypes = [vp, C.POINTER(LayerWeights), C.c_int, vp, vp, C.POINTER(Workspace),
                                    C.c_int, C.c_int, C.c_int, vp, vp, C.c_int, C.POINTER(vp)]
 L.lib.pk100_run_layers.restype = C.c_int
+L.lib.pk100_run_layers_packed.argtypes = [vp, C.POINTER(LayerWeights), C.c_int, vp, vp, C.POINTER(Workspace), C.c_int, vp,
+                                          C.POINTER(vp)]
+L.lib.pk100_run_layers_packed.restype = C.c_int
 
 
 def relative_position_encoding() -> np.ndarray:
@@ -164,6 +167,17 @@ class EncoderLayers:
             None if seg_valid is None else seg_valid.data_ptr(),
             None if tile_stats is None else tile_stats.data_ptr(), attention_impl, C.byref(out))
         L.check(rc, "pk100_run_layers")
+        return state_a if out.value == state_a.data_ptr() else state_b
+
+    def run_packed(self, state_a, state_b, ws, rows, tiles):
+        """All layers on a packed batch: `rows` rows in whole 128-row tiles, tiles int32 CUDA [rows / 128, 2]
+        = (first row of the tile's utterance, its valid rows).  Returns the tensor holding the result."""
+        arr = (LayerWeights * len(self.layers))(*self.layers)
+        out = vp()
+        rc = L.lib.pk100_run_layers_packed(
+            torch.cuda.current_stream().cuda_stream, arr, len(self.layers), state_a.data_ptr(), state_b.data_ptr(),
+            C.byref(ws), rows, tiles.data_ptr(), C.byref(out))
+        L.check(rc, "pk100_run_layers_packed")
         return state_a if out.value == state_a.data_ptr() else state_b
 
     def status(self, ws_arena, ws):

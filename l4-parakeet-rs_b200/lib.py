@@ -60,6 +60,7 @@ SIGNATURES = {
     "pk100_encoder_workspace_bytes": None,
     "pk100_encoder_workspace_carve": None,
     "pk100_run_layers": None,
+    "pk100_run_layers_packed": None,
     "pk100_tdt_workspace_bytes": None,
     "pk100_tdt_rounds_offset": None,
     "pk100_tdt_cluster_capacity": None,
@@ -91,6 +92,7 @@ SIGNATURES = {
     "pk100_mel_frontend": None,
     "pk100_subsampling_workspace_bytes": None,
     "pk100_run_subsampling": None,
+    "pk100_run_subsampling_rows": None,
     "pk100_subsampling_fp8_workspace_bytes": None,
     "pk100_run_subsampling_fp8": None,
     "pk100_launch_count": None,

@@ -55,6 +55,7 @@ class _Slot:
         self.out_frames_host = torch.full((n,), eng.frames_out, dtype=torch.int32)
         self.longest_out_frames = eng.frames_out
         self._lengths = tuple([eng.mel_frames] * n)
+        self.place = torch.zeros(eng.place.shape, dtype=torch.int32, device=dev)
         self.enc_proj = torch.zeros_like(eng.enc_proj)
         self.tokens, self.durations, self.counts = (torch.zeros_like(t) for t in (eng.tokens, eng.durations, eng.counts))
         self.tokens_host = torch.zeros_like(eng.tokens_host).pin_memory()
@@ -104,6 +105,8 @@ class PipelineEngine:
         self.calibrated = False
         self._events = None
         self._lengths = tuple([mel_frames] * max_utterances)
+        # packed batches: first row of every utterance, then (utterance's first row, its rows) per 128-row tile
+        self.place = torch.zeros(2 * (max_utterances + self.rows // 128), dtype=torch.int32, device=dev)
         # one side stream, scratch and event set per decode group
         self.dec_streams = [torch.cuda.Stream(device=self.device, priority=-1) for _ in range(self.decode_groups)]
         self.dec_scratch = [None] + [self.dec.make_scratch() for _ in range(self.decode_groups - 1)]
@@ -127,9 +130,9 @@ class PipelineEngine:
     def gemm_times_ms(self):
         """[(milliseconds, rows of that launch)] for every FF-expand launch of the last request."""
         out = []
-        for e, (u0, u1) in enumerate(self.last_encode_groups):
+        for e in range(len(self.last_encode_groups)):
             ev = self._events[e]
-            out += [(ev[2 * i].elapsed_time(ev[2 * i + 1]), (u1 - u0) * self.seg_stride) for i in range(len(ev) // 2)]
+            out += [(ev[2 * i].elapsed_time(ev[2 * i + 1]), self.last_encode_rows[e]) for i in range(len(ev) // 2)]
         return out
 
     # ---- stages
@@ -164,6 +167,14 @@ class PipelineEngine:
         b.out_frames_dev[:len(of)].copy_(of)
         b.out_frames_host[:len(of)].copy_(of)
         b.longest_out_frames = int(b.out_frames_host.max())
+        # where the utterances lie when the batch is packed
+        place, row = [0] * (2 * self.max_utterances), 0
+        for u, f in enumerate(b._lengths):
+            f = min(sub_mod.output_frames(f), self.frames_out)
+            place[u] = row
+            place += [row, f] * (seg_stride_for(f) // 128)
+            row += seg_stride_for(f)
+        b.place[:len(place)].copy_(torch.tensor(place, dtype=torch.int32))
 
     def encode(self, utterances):
         self.sub.run(self.mel_dev[:utterances], self.seg_stride, mel_frames=self.mel_frames_dev,
@@ -204,13 +215,24 @@ class PipelineEngine:
             plan.append(((decs[g0][0], decs[g1 - 1][1]), decs[g0:g1]))
         return plan
 
-    def run_resident(self, utterances, slot=None, join=True, clusters_in_flight=0, decode_groups=None):
+    def _geometry(self, lengths):
+        """(mel frames, rows per utterance, rows of the packed form or None) of a request: utterances at the
+        distance that the longest one needs, and without any padding tiles where their lengths differ."""
+        rows = [seg_stride_for(sub_mod.output_frames(f)) for f in lengths]
+        seg = max(max(rows), 128)
+        packed = sum(rows) if self.encode_groups == 1 and 0 < sum(rows) < seg * len(rows) else None
+        return max(max(lengths), 1), seg, packed
+
+    def run_resident(self, utterances, slot=None, join=True, clusters_in_flight=0, decode_groups=None, fitted=False):
         """Hot path with the inputs already in HBM: subsampling -> encoder -> projection -> decode,
         group by group (see the module text); returns with everything queued on the caller's
         stream, which waits for the side streams (join=False: it does not, and the decode groups'
         streams are returned).  slot: the buffers of the batch (default: the engine's own);
-        clusters_in_flight: decoder clusters of an earlier batch still running beside this one."""
+        clusters_in_flight: decoder clusters of an earlier batch still running beside this one;
+        fitted: rows laid out for the lengths of `set_lengths` instead of for the engine's capacity (the
+        rows of an utterance in enc_proj then lie at that distance, the same numbers in them)."""
         b = self if slot is None else slot
+        frames, seg, packed = self._geometry(b._lengths[:utterances]) if fitted else (self.mel_frames, self.seg_stride, None)
         # the reference switches decoder kernels (and numerics) at 1024 frames per request
         # (src/cuda/decoder.rs:88); a batch of short utterances needs one launch only
         cache = "auto" if b.longest_out_frames >= dec_mod.LONG_REQUEST_FRAMES else "fp16"
@@ -220,7 +242,7 @@ class PipelineEngine:
         self.last_groups = [d for _, decs in plan for d in decs]
         self.last_encode_of = [e for e, (_, decs) in enumerate(plan) for _ in decs]
         single = len(self.last_groups) == 1 and join
-        seg = self.seg_stride
+        self.last_encode_rows = []
         g = 0
         for e, ((a0, a1), decs) in enumerate(plan):
             ev = self._stage_events if slot is None else None
@@ -232,10 +254,21 @@ class PipelineEngine:
                 ev["enc"][e][0].record(main)
             if self._events is not None and slot is None:
                 self.ws.profile_events = C.cast(self._event_arrays[e], C.POINTER(C.c_void_p))
-            self.sub.run(b.mel_dev[a0:a1], seg, mel_frames=b.mel_frames_dev[a0:a1], out=self.state_a[r0:r1])
-            encoded = self.enc.run(self.state_a[r0:r1], self.state_b[r0:r1], self.ws, a1 - a0, seg,
-                                   self.frames_out, seg_valid=b.out_frames_dev[a0:a1])
-            self.dec.project(encoded, out=b.enc_proj[r0:r1])
+            self.last_encode_rows.append(r1 - r0 if packed is None else packed)
+            if packed is None:
+                self.sub.run_rows(b.mel_dev[a0:a1], frames, seg, b.mel_frames_dev[a0:a1], self.state_a[r0:r1])
+                encoded = self.enc.run(self.state_a[r0:r1], self.state_b[r0:r1], self.ws, a1 - a0, seg,
+                                       min(seg, self.frames_out), seg_valid=b.out_frames_dev[a0:a1])
+                self.dec.project(encoded, out=b.enc_proj[r0:r1])
+            else:
+                self.sub.run_rows(b.mel_dev[:utterances], frames, seg, b.mel_frames_dev, self.state_a, row_base=b.place, rows=packed)
+                encoded = self.enc.run_packed(self.state_a, self.state_b, self.ws, packed, b.place[2 * self.max_utterances:])
+                row = 0
+                for u, f in enumerate(b._lengths[:utterances]):       # back to the decoder's fixed distance
+                    n = seg_stride_for(sub_mod.output_frames(f))
+                    if n > 0:
+                        self.dec.project(encoded[row:row + n], out=b.enc_proj[u * seg:u * seg + n])
+                    row += n
             if ev:
                 ev["enc"][e][1].record(main)
             for (u0, u1) in decs:
@@ -272,7 +305,7 @@ class PipelineEngine:
         if lengths != self._lengths[:utterances]:
             self.set_lengths(lengths)          # never reuse the lengths an earlier request left behind
         self.mel_dev[:utterances, :mel_host.shape[1]].copy_(mel_host, non_blocking=True)
-        self.run_resident(utterances)
+        self.run_resident(utterances, fitted=True)
         self.counts_host.copy_(self.counts, non_blocking=True)
         self.tokens_host.copy_(self.tokens, non_blocking=True)
         self._queue_status()
@@ -333,7 +366,8 @@ class PipelineEngine:
                 self.set_lengths(lengths, slot=b)
             b.mel_dev[:utterances, :mel_host.shape[1]].copy_(mel_host, non_blocking=True)
             streams = self.run_resident(utterances, slot=b, join=False,
-                                        clusters_in_flight=sum(e[3] for e in pending), decode_groups=decode_groups)
+                                        clusters_in_flight=sum(e[3] for e in pending), decode_groups=decode_groups,
+                                        fitted=True)
             collect = self._collect_streams[k]
             for st in streams:
                 collect.wait_stream(st)
@@ -400,7 +434,7 @@ class PipelineEngine:
         self.frontend.compute(self.pcm_dev[:utterances], self.pcm_counts_dev[:utterances], frame_cap=self.mel_frames,
                               out=self.mel_dev[:utterances])
         self.set_lengths([n // fe_mod.HOP for n in sample_counts])       # valid frames are known on the host
-        self.run_resident(utterances)
+        self.run_resident(utterances, fitted=True)
         self.counts_host.copy_(self.counts, non_blocking=True)
         self.tokens_host.copy_(self.tokens, non_blocking=True)
         self._queue_status()

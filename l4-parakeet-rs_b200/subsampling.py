@@ -34,6 +34,9 @@ L.lib.pk100_subsampling_fp8_workspace_bytes.restype = C.c_longlong
 L.lib.pk100_run_subsampling_fp8.argtypes = [vp, C.POINTER(SubsamplingWeightsC), C.POINTER(SubsamplingFp8C), vp, C.c_int,
                                             C.c_int, vp, vp, vp, C.c_int, vp]
 L.lib.pk100_run_subsampling_fp8.restype = C.c_int
+L.lib.pk100_run_subsampling_rows.argtypes = [vp, C.POINTER(SubsamplingWeightsC), C.POINTER(SubsamplingFp8C), vp, C.c_int,
+                                             C.c_int, C.c_int, vp, vp, vp, C.c_int, vp, C.c_int, vp]
+L.lib.pk100_run_subsampling_rows.restype = C.c_int
 
 
 def output_frames(mel_frames: int) -> int:
@@ -97,4 +100,17 @@ class Subsampling:
         else:
             L.check(L.lib.pk100_run_subsampling_fp8(stream, C.byref(self.c), C.byref(self.q), *args),
                     "pk100_run_subsampling_fp8")
+        return out
+
+    def run_rows(self, mel, frames, seg_stride, mel_frames, out, row_base=None, rows=None):
+        """The first `frames` mel rows of every utterance of `mel` (fp32 CUDA [utterances, capacity, 128], the
+        utterances at the capacity's distance); row_base (int32 CUDA) and rows: the packed form of the output."""
+        utterances, capacity, bins = mel.shape
+        assert bins == 128 and mel.dtype == torch.float32 and mel.is_contiguous() and frames <= capacity
+        ws = self.workspace(utterances, frames, seg_stride)
+        L.check(L.lib.pk100_run_subsampling_rows(
+            torch.cuda.current_stream().cuda_stream, C.byref(self.c), None if self.q is None else C.byref(self.q),
+            mel.data_ptr(), capacity, utterances, frames, mel_frames.data_ptr(), ws.data_ptr(), out.data_ptr(), seg_stride,
+            None if row_base is None else row_base.data_ptr(), utterances * seg_stride if row_base is None else rows,
+            self.status.data_ptr()), "pk100_run_subsampling_rows")
         return out

@@ -109,3 +109,30 @@ def test_streamed_batches_return_what_single_requests_return(pk, cuda, engine):
         for g, w in zip(got, want):
             assert len(g) == len(w) and all(np.array_equal(x, y) for x, y in zip(g, w))
     assert any(len(t) > 0 for batch in got for t in batch)
+
+
+@pytest.mark.parametrize("frames", [[3100, 1024, 1025], [8, 3100, 2049], [40, 40, 40], [0, 2100, 1], [3100, 3100, 1]])
+def test_rows_fitted_to_the_request_give_the_same_bits(pk, cuda, frames):
+    """Rows laid out for the request's lengths (a smaller distance between utterances, or a packed batch without
+    padding tiles; utterances that end on and just behind a tile edge) against the engine's full capacity."""
+    eng = pk.pipeline.PipelineEngine(cuda, layers=2, decoder_layers=1, seed=9, max_utterances=3, mel_frames=3100)
+    for l in range(2):
+        eng.enc.set_tau(l, 0.4, 0.4)
+    eng.mel_dev.normal_(generator=torch.Generator(device=cuda).manual_seed(3))
+    eng.set_lengths(frames)
+    got = []
+    for fitted in (False, True):
+        eng.enc_proj.fill_(float("nan"))
+        eng.run_resident(3, fitted=fitted)
+        torch.cuda.synchronize()
+        seg = eng._geometry(frames)[1] if fitted else eng.seg_stride
+        rows = [eng.enc_proj[u * seg:u * seg + pk.subsampling.output_frames(f)].cpu() for u, f in enumerate(frames)]
+        got.append((rows, eng.tokens.cpu().clone(), eng.counts.cpu().clone(), seg))
+    assert eng.status() == 0
+    for a, b in zip(got[0][0], got[1][0]):
+        assert torch.isfinite(b).all() and torch.equal(a, b)
+    assert torch.equal(got[0][2], got[1][2])
+    for u in range(3):
+        assert torch.equal(got[0][1][u, :got[0][2][u]], got[1][1][u, :got[0][2][u]])
+    packed = eng._geometry(frames)[2]
+    assert (packed is None) == (len({pk.pipeline.seg_stride_for(pk.subsampling.output_frames(f)) for f in frames}) == 1)
