@@ -275,7 +275,9 @@ static std::atomic<long long> g_launches{0};
 void pk100_count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 extern "C" long long pk100_launch_count(void) { return g_launches.load(std::memory_order_relaxed); }
 
-extern "C" int pk100_gemm(void* stream_v, const pk100_gemm_args* a) {
+extern "C" int pk100_gemm(void* stream_v, const pk100_gemm_args* a) { return pk100_gemm_chained(stream_v, a, false); }
+
+int pk100_gemm_chained(void* stream_v, const pk100_gemm_args* a, bool b_settled) {
     if (a == nullptr || a->a == nullptr || a->b == nullptr || a->out == nullptr) return PK100_ERR_NULL;
     if (a->m < 0 || a->n <= 0 || a->k <= 0) return PK100_ERR_SHAPE;
     if (a->m == 0) return PK100_OK;
@@ -336,6 +338,7 @@ extern "C" int pk100_gemm(void* stream_v, const pk100_gemm_args* a) {
     p.w4_codes = w4 ? static_cast<const uint8_t*>(a->b) : nullptr;
     p.w4_scales = w4 ? static_cast<const __half*>(a->b_group_scales) : nullptr;
     p.status = a->status;
+    p.b_settled = b_settled ? 1 : 0;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
 
     // Tile width: the one with the shorter schedule, counting whole waves over the CTAs available and a

@@ -57,6 +57,9 @@ struct GemmParams {
     // Bytes of one output row in a warp's 32-row slice when the slices leave through shared
     // memory and a TMA store (64 or 128); 0 = each thread stores its row piece directly.
     int store_row_bytes;
+    // B is not written by the kernel in front of this one in the stream: the first stages of the weights are
+    // requested before the wait for that kernel.
+    int b_settled;
 };
 
 constexpr int kBlockM = 128;
@@ -390,7 +393,31 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     if constexpr (CtaGroup == 2) cluster_sync_all();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_ptr_smem;
-    // everything above touched only shared / tensor memory and kernel parameters: under a
+    // Weights of the first work item's first stages: requested while the previous kernel drains, so that the
+    // DRAM latency of a layer's weights (read once per pass) is not on the chain of small launches.
+    int b_ahead = 0;
+    if constexpr (CtaGroup == 1 && BSrc == BSRC_TMA) {
+        if (p.b_settled != 0 && p.keep_in == nullptr) b_ahead = k_blocks < kStages ? k_blocks : kStages;
+    }
+    auto load_b = [&](int stage, int nt_, int kb) {
+        uint8_t* sb = smem + stage * Smem::kStageBytes + Smem::kStageA;
+        const int n_first = Epi == EPI_GLU ? nt_ * kBHalf : nt_ * BlockN;
+        const int n_second = Epi == EPI_GLU ? p.n / 2 + nt_ * kBHalf : n_first + kBHalf;
+        tma_load_2d(sb, &map_b, full_bar + stage, kb * kBlockK, n_first);
+        tma_load_2d(sb + kBHalf * SwizzleBytes, &map_b, full_bar + stage, kb * kBlockK, n_second);
+    };
+    if constexpr (CtaGroup == 1 && BSrc == BSRC_TMA) {
+        if (b_ahead > 0 && threadIdx.x == 0) {
+            int mg, nt;
+            if (work_item(0, mg, nt)) {
+                for (int s = 0; s < b_ahead; ++s) {
+                    mbar_arrive_expect_tx(full_bar + s, Smem::kStageBytes);
+                    load_b(s, nt, s);
+                }
+            }
+        }
+    }
+    // everything above touched only shared / tensor memory, kernel parameters and settled weights: under a
     // programmatic dependent launch it overlapped the previous kernel's tail
     grid_dependency_wait();
     if (balanced) {
@@ -429,7 +456,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                         break;
                     }
                     uint8_t* sa = smem + stage * Smem::kStageBytes;
-                    uint8_t* sb = sa + Smem::kStageA;
+                    [[maybe_unused]] uint8_t* sb = sa + Smem::kStageA;
                     if constexpr (CtaGroup == 2) {
                         // the leader's barrier counts the bytes of both CTAs
                         if (rank == 0) mbar_arrive_expect_tx(full_bar + stage, 2 * Smem::kStageBytes);
@@ -443,19 +470,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                         tma_load_2d_pair(sa, &map_a, bar, kb * kBlockK, m0);
                         tma_load_2d_pair(sb, &map_b, bar, kb * kBlockK, n_rows);
                     } else if constexpr (BSrc == BSRC_TMA) {
-                        mbar_arrive_expect_tx(full_bar + stage, Smem::kStageBytes);
+                        const bool ahead = it == 0 && kb < b_ahead;      // (stage kb: its B is on the way)
+                        if (!ahead) mbar_arrive_expect_tx(full_bar + stage, Smem::kStageBytes);
                         tma_load_2d(sa, &map_a, full_bar + stage, kb * kBlockK, m0);
-                        int n_first, n_second;
-                        if constexpr (Epi == EPI_GLU) {
-                            n_first = nt * kBHalf;
-                            n_second = p.n / 2 + nt * kBHalf;
-                        } else {
-                            n_first = nt * BlockN;
-                            n_second = n_first + kBHalf;
-                        }
-                        tma_load_2d(sb, &map_b, full_bar + stage, kb * kBlockK, n_first);
-                        tma_load_2d(sb + kBHalf * SwizzleBytes, &map_b, full_bar + stage,
-                                    kb * kBlockK, n_second);
+                        if (!ahead) load_b(stage, nt, kb);
                     } else {
                         // 128-row boxes of A, one per accumulator that has rows
                         const bool second = m0 + kBlockM < p.m;

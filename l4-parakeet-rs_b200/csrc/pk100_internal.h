@@ -73,6 +73,9 @@ int pk100_local_attention_rows(void* stream, const void* query, int ldq, const v
                                const void* position, const void* bias_u, const void* bias_v, void* output, int ldo,
                                int total_rows, const pk100_rows& geometry, bool constants_settled, int* status);
 
+// pk100_gemm for a caller who knows that the kernel in front of it in the stream does not write B.
+int pk100_gemm_chained(void* stream, const pk100_gemm_args* args, bool b_settled);
+
 // SMs a persistent kernel may use: all of them, or the cap set by pk100_set_gemm_cta_cap.
 int pk100_cta_budget();
 

@@ -527,7 +527,7 @@ static int run_subsampling(void* stream_v, const pk100_subsampling_weights* w, c
         first.kind = PK100_KIND_E4M3; first.a = q2; first.b = q->pw1_q; first.row_scales = q2_scales;
         first.col_scales = q->pw1_scales;
     }
-    if ((rc = pk100_gemm(stream, &first)) != PK100_OK) return rc;
+    if ((rc = pk100_gemm_chained(stream, &first, true)) != PK100_OK) return rc;
 
     subsample_depthwise_kernel<<<dim3(16 / (4 * kDepthwiseRun), c.f3, utterances), 128, 0, stream>>>(
         s3, static_cast<const __half*>(w->dw2_w), static_cast<const __half*>(w->dw2_b), s4, c.f2, 32,
@@ -536,7 +536,7 @@ static int run_subsampling(void* stream_v, const pk100_subsampling_weights* w, c
 
     a.m = static_cast<int>(u * c.f3 * 16);
     a.a = s4; a.b = w->pw2_w; a.bias = w->pw2_b; a.out = s5;
-    if ((rc = pk100_gemm(stream, &a)) != PK100_OK) return rc;
+    if ((rc = pk100_gemm_chained(stream, &a, true)) != PK100_OK) return rc;
 
     if (q != nullptr)
         subsample_flatten_kernel<true><<<dim3(seg_stride, utterances), 128, 0, stream>>>(s5, qflat, qflat_scales, c.f3, seg_stride,
@@ -553,5 +553,5 @@ static int run_subsampling(void* stream_v, const pk100_subsampling_weights* w, c
         a.kind = PK100_KIND_E4M3; a.a = qflat; a.b = q->proj_q; a.row_scales = qflat_scales;
         a.col_scales = q->proj_scales;
     }
-    return pk100_gemm(stream, &a);
+    return pk100_gemm_chained(stream, &a, true);
 }
