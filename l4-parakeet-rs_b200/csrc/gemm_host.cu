@@ -346,6 +346,12 @@ int pk100_gemm_chained(void* stream_v, const pk100_gemm_args* a, bool b_settled)
     // takes 17.6 us against 20.3 us for two waves of 192 narrow ones; at 6144 x 1024 two wide waves
     // take 24.3 us against 28.7 us for three narrow ones; a single partial wave prefers the narrow tile).
     const int m_tiles = (a->m + kBlockM - 1) / kBlockM;
+    // 64-column tiles where they still fit one wave: such a launch is bound by the round trips of its operand
+    // ring (1.7 us each, the weights come from DRAM), and eight 24 KB stages hold a K of 1024 bytes whole where
+    // the 128-column tile has five stages, for twice the CTAs and half the epilogue.  Encoder of a 4 s request
+    // (128 rows, 24 layers, GLU rule below included) 340 us shorter, of a 60 s one (768 rows) 210 us; FF contract
+    // with a 30 % live K at 128 .. 1024 rows 14.0 -> 12.6 us per call.
+    const bool tiny = a->n % 64 == 0 && static_cast<long long>(m_tiles) * (a->n / 64) <= cta_budget(*a);
     bool narrow = a->n % 256 != 0;
     if (!narrow) {
         const long long ctas = cta_budget(*a);
@@ -357,6 +363,11 @@ int pk100_gemm_chained(void* stream_v, const pk100_gemm_args* a, bool b_settled)
     if (w4) return launch_w4(*a, p, stream);
     switch (a->epilogue) {
     case PK100_EPI_LINEAR:
+        if (tiny) {
+            if (a->kind == PK100_KIND_F16) return launch<KIND_F16, 64, 128, EPI_LINEAR>(*a, p, stream);
+            if (a->kind == PK100_KIND_E4M3) return launch<KIND_F8, 64, 128, EPI_LINEAR>(*a, p, stream);
+            return launch<KIND_I8, 64, 128, EPI_LINEAR>(*a, p, stream);
+        }
         if (a->kind == PK100_KIND_F16) {
             return narrow ? launch<KIND_F16, 128, 128, EPI_LINEAR>(*a, p, stream)
                           : launch<KIND_F16, 256, 128, EPI_LINEAR>(*a, p, stream);
@@ -371,16 +382,19 @@ int pk100_gemm_chained(void* stream_v, const pk100_gemm_args* a, bool b_settled)
         // measured 14 % slower: TMA moves rows of a box at the same rate whatever their width.
         return narrow ? launch<KIND_I8, 128, 128, EPI_LINEAR>(*a, p, stream)
                       : launch<KIND_I8, 256, 128, EPI_LINEAR>(*a, p, stream);
-    case PK100_EPI_GLU:
+    case PK100_EPI_GLU: {
+        // 128-column tiles (64 values and their gates) likewise only in one wave
+        const bool thin_glu = a->n % 256 != 0 || static_cast<long long>(m_tiles) * (a->n / 128) <= cta_budget(*a);
         if (a->kind == PK100_KIND_E4M3) {
-            return (a->n % 256 != 0) ? launch<KIND_F8, 128, 128, EPI_GLU>(*a, p, stream)
+            return thin_glu ? launch<KIND_F8, 128, 128, EPI_GLU>(*a, p, stream)
                                      : launch<KIND_F8, 256, 128, EPI_GLU>(*a, p, stream);
         }
         if (a->kind == PK100_KIND_F16) {
-            return (a->n % 256 != 0) ? launch<KIND_F16, 128, 128, EPI_GLU>(*a, p, stream)
+            return thin_glu ? launch<KIND_F16, 128, 128, EPI_GLU>(*a, p, stream)
                                      : launch<KIND_F16, 256, 128, EPI_GLU>(*a, p, stream);
         }
         return PK100_ERR_UNSUPPORTED;
+    }
     case PK100_EPI_SPARSE_OUT:
         if (a->kind == PK100_KIND_E4M3) return launch<KIND_F8, 256, 128, EPI_SPARSE_OUT>(*a, p, stream);
         if (a->kind == PK100_KIND_F16) return launch<KIND_F16, 256, 128, EPI_SPARSE_OUT>(*a, p, stream);

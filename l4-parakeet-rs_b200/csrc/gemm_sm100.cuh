@@ -660,7 +660,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         // biases (GLU: value columns first, their gate columns after).  Warp-private, so staging
         // a tile's constants needs no CTA-wide barrier.
         constexpr int kSlice = BlockN / kParts;
-        constexpr int kPer = kSlice / 32;
+        constexpr int kPer = (kSlice + 31) / 32;       // (64-column tiles: half a warp's lanes)
         float* my_scale = s_cols + ew * 2 * kSlice;
         float* my_bias = my_scale + kSlice;
         float pre_s[kPer], pre_b[kPer];
@@ -675,7 +675,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                 } else {
                     src = nt_ * BlockN + part * kColsPerWarp + i;
                 }
-                const bool in = src < p.n;
+                const bool in = src < p.n && i < kSlice;
                 pre_s[u] = (p.col_scales != nullptr && in) ? __ldg(p.col_scales + src) : 1.0f;
                 pre_b[u] = (p.bias != nullptr && in) ? __ldg(p.bias + src) : 0.0f;
             }
@@ -695,8 +695,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
             __syncwarp();
 #pragma unroll
             for (int u = 0; u < kPer; ++u) {
-                my_scale[u * 32 + lane] = pre_s[u];
-                my_bias[u * 32 + lane] = pre_b[u];
+                if (kSlice % 32 == 0 || lane < kSlice) {
+                    my_scale[u * 32 + lane] = pre_s[u];
+                    my_bias[u * 32 + lane] = pre_b[u];
+                }
             }
             __syncwarp();
             {

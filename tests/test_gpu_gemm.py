@@ -397,3 +397,39 @@ def test_sparse_out_reports_clamped_codes(pk, cuda):
         torch.cuda.synchronize()
         assert bool(int(st.item()) & 8) == clipped and not int(st.item()) & 1
         assert int(host(hq).max()) == (127 if clipped else int(host(hq).max()))
+
+
+@pytest.mark.parametrize("kind", ["f16", "e4m3", "s8"])
+@pytest.mark.parametrize("m,n,k", [(128, 1024, 1024), (77, 64, 64), (750, 1024, 4096), (257, 640, 1024), (1, 3072, 512)])
+def test_one_wave_tiles_give_the_bits_of_wide_tiles(pk, cuda, kind, m, n, k):
+    """Small problems run on 64-column tiles (128-column GLU tiles), one per CTA; with one CTA the same call
+    takes the wide tiles.  The sums over K are the same, so every output and residual form must agree bit for bit."""
+    L = pk.lib
+    g = torch.Generator(device=cuda).manual_seed(m * n + k)
+    dt = torch.float16 if kind == "f16" else torch.int8
+    new = lambda r: (torch.randn((r, k), generator=g, device=cuda).half() if kind == "f16" else
+                     torch.randint(-100, 100, (r, k), generator=g, device=cuda, dtype=dt))
+    a, b = new(m), new(n)
+    if kind == "e4m3":
+        a, b = (t & ~0x40 for t in (a, b))                      # (codes of finite values below 2)
+    kw = dict(kind=dict(f16=L.KIND_F16, e4m3=L.KIND_E4M3, s8=L.KIND_S8)[kind])
+    rs, cs = (torch.rand(r, generator=g, device=cuda) * 0.01 for r in (m, n))
+    bias = torch.randn(n, generator=g, device=cuda)
+    res = torch.randn((m, n), generator=g, device=cuda).half()
+    forms = [dict(), dict(row_scales=rs, col_scales=cs, bias=bias, act=L.ACT_SILU, valid_rows=max(1, m - 30)),
+             dict(row_scale=0.01, residual=res, alpha=0.5), dict(out_type=L.OUT_F32, act=L.ACT_RELU),
+             dict(out_type=L.OUT_S8, row_scale=0.001, out_scale=32.0), dict(out_type=L.OUT_E4M3, row_scale=0.001)]
+    if kind == "s8" and k % 64 == 0:
+        keep = (torch.rand(((m + 127) // 128, k // 64), generator=g, device=cuda) < 0.3).to(torch.uint8)
+        forms.append(dict(keep_in=keep, residual=res, row_scale=0.01))
+    if kind != "s8" and n % 128 == 0:
+        forms.append(dict(epilogue=L.EPI_GLU, row_scales=rs, col_scales=cs))
+    dtypes = {L.OUT_F16: torch.float16, L.OUT_F32: torch.float32, L.OUT_S8: torch.int8, L.OUT_E4M3: torch.uint8}
+    st = _status(cuda)
+    for form in forms:
+        cols = n // 2 if "epilogue" in form else n
+        outs = [torch.zeros((m, cols), dtype=dtypes[form.get("out_type", L.OUT_F16)], device=cuda) for _ in range(2)]
+        for out, ctas in zip(outs, (0, 1)):
+            pk.ops.gemm(a, b, out=out, status=st, max_ctas=ctas, **form, **kw)
+        assert int(st.item()) == 0
+        assert torch.equal(outs[0].view(torch.uint8), outs[1].view(torch.uint8)), form
