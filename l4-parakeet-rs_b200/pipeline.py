@@ -351,6 +351,9 @@ class PipelineEngine:
             counts = b.counts_host.numpy()
             return [b.tokens_host[u, :int(counts[u])].numpy().copy() for u in range(utterances)]
 
+        # The last batch of a sequence of known length has nothing behind it to leave SMs for: it is decoded on
+        # all clusters that the batches in flight do not hold (6 batches of 8 x 60 s: see the note above).
+        last = len(batches) - 1 if hasattr(batches, "__len__") else -1
         pending = []                              # oldest first: (slot index, utterances, event, clusters)
         for i, item in enumerate(batches):
             mel_host, lengths = item if isinstance(item, (tuple, list)) else (item, None)
@@ -365,8 +368,9 @@ class PipelineEngine:
             if lengths != b._lengths[:utterances]:
                 self.set_lengths(lengths, slot=b)
             b.mel_dev[:utterances, :mel_host.shape[1]].copy_(mel_host, non_blocking=True)
-            streams = self.run_resident(utterances, slot=b, join=False,
-                                        clusters_in_flight=sum(e[3] for e in pending), decode_groups=decode_groups,
+            busy = sum(e[3] for e in pending)
+            groups = decode_groups if i != last else max(decode_groups, self.decode_groups - busy)
+            streams = self.run_resident(utterances, slot=b, join=False, clusters_in_flight=busy, decode_groups=groups,
                                         fitted=True)
             collect = self._collect_streams[k]
             for st in streams:
