@@ -160,21 +160,27 @@ class PipelineEngine:
 
     def set_lengths(self, mel_frames_per_utt, slot=None):
         b = self if slot is None else slot
-        b._lengths = tuple(int(f) for f in mel_frames_per_utt) + b._lengths[len(mel_frames_per_utt):]
-        mf = torch.tensor(mel_frames_per_utt, dtype=torch.int32)
-        of = torch.tensor([sub_mod.output_frames(int(f)) for f in mel_frames_per_utt], dtype=torch.int32)
+        given = [int(f) for f in mel_frames_per_utt]
+        # refused before anything is written: an engine whose buffers and recorded lengths disagree would lay
+        # the rows of the next request out wrongly
+        if len(given) > self.max_utterances or any(f > self.mel_frames for f in given):
+            raise ValueError("more utterances, or a longer one, than the engine was sized for")
+        lengths = tuple(given) + b._lengths[len(given):]
+        mf = torch.tensor(given, dtype=torch.int32)
+        of = torch.tensor([sub_mod.output_frames(f) for f in given], dtype=torch.int32)
+        # where the utterances lie when the batch is packed
+        place, row = [0] * (2 * self.max_utterances), 0
+        for u, f in enumerate(lengths):
+            f = sub_mod.output_frames(f)
+            place[u] = row
+            place += [row, f] * (seg_stride_for(f) // 128)
+            row += seg_stride_for(f)
         b.mel_frames_dev[:len(mf)].copy_(mf)
         b.out_frames_dev[:len(of)].copy_(of)
         b.out_frames_host[:len(of)].copy_(of)
         b.longest_out_frames = int(b.out_frames_host.max())
-        # where the utterances lie when the batch is packed
-        place, row = [0] * (2 * self.max_utterances), 0
-        for u, f in enumerate(b._lengths):
-            f = min(sub_mod.output_frames(f), self.frames_out)
-            place[u] = row
-            place += [row, f] * (seg_stride_for(f) // 128)
-            row += seg_stride_for(f)
         b.place[:len(place)].copy_(torch.tensor(place, dtype=torch.int32))
+        b._lengths = lengths
 
     def encode(self, utterances):
         self.sub.run(self.mel_dev[:utterances], self.seg_stride, mel_frames=self.mel_frames_dev,
@@ -300,8 +306,8 @@ class PipelineEngine:
         utterances = mel_host.shape[0]
         lengths = tuple([int(mel_host.shape[1])] * utterances if mel_frames_per_utt is None
                         else [int(f) for f in mel_frames_per_utt])
-        if max(lengths) > mel_host.shape[1] or mel_host.shape[1] > self.mel_frames:
-            raise ValueError("utterance longer than the engine was sized for")
+        if utterances > self.max_utterances or max(lengths) > mel_host.shape[1] or mel_host.shape[1] > self.mel_frames:
+            raise ValueError("more utterances, or a longer one, than the engine was sized for")
         if lengths != self._lengths[:utterances]:
             self.set_lengths(lengths)          # never reuse the lengths an earlier request left behind
         self.mel_dev[:utterances, :mel_host.shape[1]].copy_(mel_host, non_blocking=True)
@@ -430,8 +436,8 @@ class PipelineEngine:
         Frontend -> subsampling -> encoder -> decode; returns token arrays like transcribe_batch."""
         from . import frontend as fe_mod
         utterances, samples = pcm_host.shape
-        if samples > self.pcm_capacity or max(sample_counts) > samples:
-            raise ValueError("utterance longer than the engine was sized for")
+        if utterances > self.max_utterances or samples > self.pcm_capacity or max(sample_counts) > samples:
+            raise ValueError("more utterances, or a longer one, than the engine was sized for")
         self.pcm_dev[:utterances, :samples].copy_(pcm_host, non_blocking=True)
         if samples < self.pcm_capacity:
             self.pcm_dev[:utterances, samples:].zero_()

@@ -136,3 +136,20 @@ def test_rows_fitted_to_the_request_give_the_same_bits(pk, cuda, frames):
         assert torch.equal(got[0][1][u, :got[0][2][u]], got[1][1][u, :got[0][2][u]])
     packed = eng._geometry(frames)[2]
     assert (packed is None) == (len({pk.pipeline.seg_stride_for(pk.subsampling.output_frames(f)) for f in frames}) == 1)
+
+
+def test_a_refused_request_changes_no_later_result(pk, cuda):
+    """Requests that the engine is too small for are refused before anything is queued; ragged requests after
+    them (sent twice: the second finds its lengths recorded) decode like those of an engine that saw none."""
+    engines = [pk.pipeline.PipelineEngine(cuda, layers=1, decoder_layers=1, seed=9, max_utterances=3, mel_frames=3100)
+               for _ in range(2)]
+    mel = torch.randn((4, 3100, 128), generator=torch.Generator().manual_seed(7)).pin_memory()
+    frames = [3100, 1025, 40]
+    want = engines[0].transcribe_batch(mel[:3], frames)
+    assert engines[1]._geometry(frames)[2] is not None and any(len(t) > 0 for t in want)
+    for lengths in ([3100] * 4, frames + [1]):
+        with pytest.raises(ValueError):
+            engines[1].transcribe_batch(mel, lengths)
+        for _ in range(2):
+            got = engines[1].transcribe_batch(mel[:3], frames)
+            assert all(np.array_equal(a, b) for a, b in zip(got, want))
