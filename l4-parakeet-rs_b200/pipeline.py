@@ -160,7 +160,7 @@ class PipelineEngine:
 
     def set_lengths(self, mel_frames_per_utt, slot=None):
         b = self if slot is None else slot
-        given = [int(f) for f in mel_frames_per_utt]
+        given = [max(int(f), 0) for f in mel_frames_per_utt]      # (no frames, no rows)
         # refused before anything is written: an engine whose buffers and recorded lengths disagree would lay
         # the rows of the next request out wrongly
         if len(given) > self.max_utterances or any(f > self.mel_frames for f in given):

@@ -41,3 +41,12 @@ def test_a_refused_request_leaves_the_engine_as_it_was(pk):
         for e in (eng, fresh):
             e.set_lengths(lengths)
         assert _state(eng) == _state(fresh) and eng._lengths[:len(lengths)] == tuple(lengths)
+
+
+@pytest.mark.parametrize("negative", [-1, -8, -2000, -20000])
+def test_a_negative_length_is_an_empty_utterance(pk, negative):
+    eng, fresh = _engine(pk), _engine(pk)
+    eng.set_lengths([3000, negative, 6000, 40])
+    fresh.set_lengths([3000, 0, 6000, 40])
+    assert _state(eng) == _state(fresh)
+    assert eng._geometry(eng._lengths[:4]) == fresh._geometry(fresh._lengths[:4])
