@@ -217,11 +217,17 @@ __device__ __forceinline__ void emit_row(const float (&x)[4][8], const uint4 (&h
 
 template <int Mode>
 __device__ __forceinline__ void emit_zero_row(void* out, float* scales, size_t row, int lane) {
-    constexpr int kBytes = Mode == PK100_LN_F16 ? 2 : 1;
-    uint8_t* o = reinterpret_cast<uint8_t*>(out) + row * kWidth * kBytes;
+    if constexpr (Mode == PK100_LN_F16) {
+        __half* o = reinterpret_cast<__half*>(out) + row * kWidth;
 #pragma unroll
-    for (int i = 0; i < 2 * kBytes; ++i) *reinterpret_cast<uint4*>(o + i * 512 + lane * 16) = make_uint4(0, 0, 0, 0);
-    if (Mode >= PK100_LN_E4M3_ROW && lane == 0) scales[row] = 1.0f;
+        for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(o + i * 256 + lane * 8) = make_uint4(0, 0, 0, 0);
+    } else {
+        // (8 bytes at a time like the codes of a live row: the output need not be aligned to more)
+        uint8_t* o = reinterpret_cast<uint8_t*>(out) + row * kWidth;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) *reinterpret_cast<uint2*>(o + i * 256 + lane * 8) = make_uint2(0, 0);
+        if (Mode >= PK100_LN_E4M3_ROW && lane == 0) scales[row] = 1.0f;
+    }
 }
 
 // One warp per row, walking the rows of the grid; the next row is requested before the current one is

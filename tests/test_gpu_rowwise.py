@@ -217,3 +217,22 @@ def test_depthwise_strips_and_codes(pk, cuda, segments, stride, valid):
         rows = slice(u * stride, u * stride + valid)
         alone, _ = pk.ops.depthwise_bn_silu(x[rows].contiguous(), w, *bn)
         assert torch.equal(alone, y[rows]) and not bool(y[u * stride + valid:(u + 1) * stride].any())
+
+
+@pytest.mark.parametrize("mode", ["E4M3_FIXED", "E4M3_ROW", "S8_ROW", "S4_ROW"])
+def test_codes_in_an_output_aligned_to_8_bytes(pk, cuda, mode):
+    """8-bit outputs need 8-byte alignment, in live and in padding rows, of one norm and of the pair form."""
+    L = pk.lib
+    mode = getattr(L, "LN_" + mode)
+    g, b = (dev16(t) for t in _affine(11))
+    x = dev16(_rows(12, 40, 2.0))
+    args = dict(seg_stride=20, valid_rows=13)
+    at8 = lambda like: torch.full((like.numel() + 8,), 0x55, dtype=torch.uint8, device=cuda).view(like.dtype)[8:].view(like.shape)
+    want, ws = pk.ops.layer_norm(x, g, b, mode, inv_scale=56.0, **args)
+    out = at8(want)
+    assert out.data_ptr() % 16 == 8
+    got, gs = pk.ops.layer_norm(x, g, b, mode, inv_scale=56.0, out=out, **args)
+    assert torch.equal(got, want) and (ws is None or torch.equal(gs, ws)) and not bool(got[13:20].any())
+    _, want, ws = pk.ops.layer_norm_pair(x, g, b, g, b, mode, next_inv_scale=56.0, **args)
+    _, got, gs = pk.ops.layer_norm_pair(x, g, b, g, b, mode, next_inv_scale=56.0, next_out=at8(want), **args)
+    assert torch.equal(got, want) and (ws is None or torch.equal(gs, ws)) and not bool(got[33:].any())
