@@ -226,7 +226,7 @@ __device__ __forceinline__ void emit_zero_row(void* out, float* scales, size_t r
         uint8_t* o = reinterpret_cast<uint8_t*>(out) + row * kWidth;
 #pragma unroll
         for (int i = 0; i < 4; ++i) *reinterpret_cast<uint2*>(o + i * 256 + lane * 8) = make_uint2(0, 0);
-        if (Mode >= PK100_LN_E4M3_ROW && lane == 0) scales[row] = 1.0f;
+        if (scales != nullptr && lane == 0) scales[row] = 1.0f;      // (fixed scale: only where the caller gives an array)
     }
 }
 

@@ -236,3 +236,16 @@ def test_codes_in_an_output_aligned_to_8_bytes(pk, cuda, mode):
     _, want, ws = pk.ops.layer_norm_pair(x, g, b, g, b, mode, next_inv_scale=56.0, **args)
     _, got, gs = pk.ops.layer_norm_pair(x, g, b, g, b, mode, next_inv_scale=56.0, next_out=at8(want), **args)
     assert torch.equal(got, want) and (ws is None or torch.equal(gs, ws)) and not bool(got[33:].any())
+
+
+def test_padding_rows_take_scale_1_wherever_scales_are_given(pk, cuda):
+    """Padding rows write scale 1 in every 8-bit mode, also where the live rows' scale is the caller's constant."""
+    L = pk.lib
+    g, b = (dev16(t) for t in _affine(11))
+    x = dev16(_rows(12, 40, 2.0))
+    want = torch.full((40,), 7.0, device=cuda)
+    want[13:20] = want[33:] = 1.0
+    scales = [torch.full((40,), 7.0, device=cuda) for _ in range(2)]
+    pk.ops.layer_norm(x, g, b, L.LN_E4M3_FIXED, inv_scale=56.0, scales=scales[0], seg_stride=20, valid_rows=13)
+    pk.ops.layer_norm_pair(x, g, b, g, b, L.LN_E4M3_FIXED, next_inv_scale=56.0, next_scales=scales[1], seg_stride=20, valid_rows=13)
+    assert all(torch.equal(s, want) for s in scales)
