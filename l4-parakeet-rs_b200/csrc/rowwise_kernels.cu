@@ -138,21 +138,21 @@ __device__ __forceinline__ void normalise_row(float (&x)[4][8], uint4 (&h)[4], c
     }
 }
 
-// largest |value| of the row from the packed fp16 values
-__device__ __forceinline__ float row_absmax(const uint4 (&h)[4]) {
+// bits of the row's largest |value| from the packed fp16 values, those of a NaN where the row has one
+__device__ __forceinline__ unsigned row_absmax_bits(const uint4 (&h)[4]) {
     __half2 mx = __habs2(*reinterpret_cast<const __half2*>(&h[0].x));
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const uint32_t w[4] = {h[i].x, h[i].y, h[i].z, h[i].w};
 #pragma unroll
-        for (int j = 0; j < 4; ++j) mx = __hmax2(mx, __habs2(*reinterpret_cast<const __half2*>(&w[j])));
+        for (int j = 0; j < 4; ++j) mx = __hmax2_nan(mx, __habs2(*reinterpret_cast<const __half2*>(&w[j])));
     }
-    // non-negative floats order like their bits
+    // non-negative floats order like their bits, infinity and then NaN last
     const float2 m = __half22float2(mx);
-    return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(m.x, m.y))));
+    return __reduce_max_sync(0xffffffffu, max(__float_as_uint(m.x), __float_as_uint(m.y)));
 }
 
-// four INT8 codes rne(q) of |q| <= 127 in one word: adding 1.5 * 2^23 leaves the integer in the low mantissa bits
+// four INT8 codes rne(q) of |q| <= 127 (no NaN) in one word: adding 1.5 * 2^23 leaves the integer in the low mantissa bits
 __device__ __forceinline__ uint32_t codes_s8x4(float a, float b, float c, float d) {
     constexpr float kMagic = 12582912.0f;
     const uint32_t lo = __byte_perm(__float_as_uint(a + kMagic), __float_as_uint(b + kMagic), 0x0040);
@@ -160,9 +160,9 @@ __device__ __forceinline__ uint32_t codes_s8x4(float a, float b, float c, float 
     return __byte_perm(lo, hi, 0x5410);
 }
 
-// Write one normalised row in the requested encoding.
+// Write one normalised row in the requested encoding (x is used up).
 template <int Mode>
-__device__ __forceinline__ void emit_row(const float (&x)[4][8], const uint4 (&h)[4], float inv_scale,
+__device__ __forceinline__ void emit_row(float (&x)[4][8], const uint4 (&h)[4], float inv_scale,
                                          void* out, float* scales, size_t row, int lane) {
     if constexpr (Mode == PK100_LN_F16) {
         __half* o = reinterpret_cast<__half*>(out) + row * kWidth;
@@ -200,7 +200,19 @@ __device__ __forceinline__ void emit_row(const float (&x)[4][8], const uint4 (&h
             *reinterpret_cast<uint2*>(o + i * 256 + lane * 8) = e4m3x8(q);
         }
     } else {
-        const float mx = row_absmax(h);
+        float mx = __uint_as_float(row_absmax_bits(h));
+        if (!isfinite(mx)) {                               // (the whole warp or none of it)
+            // the maximum is taken over what is a number; INT8 codes of NaN and of infinity / infinity are 0
+            float top = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    top = fmaxf(top, fabsf(x[i][j]));
+                    if (Mode == PK100_LN_S8_ROW && !isfinite(x[i][j])) x[i][j] = 0.0f;
+                }
+            mx = warp_max_all(top);
+        }
         const float scale = mx > 0.0f ? __fdiv_rn(mx, Mode == PK100_LN_E4M3_ROW ? 448.0f : 127.0f) : 1.0f;
         if (lane == 0) scales[row] = scale;
         const RowDivisor div(scale);

@@ -249,3 +249,31 @@ def test_padding_rows_take_scale_1_wherever_scales_are_given(pk, cuda):
     pk.ops.layer_norm(x, g, b, L.LN_E4M3_FIXED, inv_scale=56.0, scales=scales[0], seg_stride=20, valid_rows=13)
     pk.ops.layer_norm_pair(x, g, b, g, b, L.LN_E4M3_FIXED, next_inv_scale=56.0, next_scales=scales[1], seg_stride=20, valid_rows=13)
     assert all(torch.equal(s, want) for s in scales)
+
+
+def test_row_codes_of_rows_with_nan_and_infinity(pk, cuda):
+    """The row quantisers of LayerNorm take the maximum over what is a number and code a NaN as 0 (INT8) or NaN
+    (E4M3), like pack_weight_rows on the same fp16 values: single NaN columns, all 32 columns of a lane, a row
+    of NaN only, values that overflow fp16, and both at once."""
+    L = pk.lib
+    g, b = _affine(5)
+    x = _rows(7, 24, 2.0)
+    x[3, 100] = np.nan                                            # the whole row's mean is NaN
+    lane = np.array([i * 256 + 40 + j for i in range(4) for j in range(8)])
+    cases = []
+    for nan_cols, big_cols in (([17], []), (lane, []), ([], [3, 900]), (lane, [44]), (lane, [3]), (np.arange(1024), [])):
+        g2, b2 = g.copy(), b.copy()
+        g2[big_cols] = 60000.0
+        b2[nan_cols] = np.nan
+        cases.append((dev16(g2), dev16(b2)))
+    xd = dev16(x)
+    for gd, bd in cases:
+        y, _ = pk.ops.layer_norm(xd, gd, bd, L.LN_F16)
+        for mode, fmt in ((L.LN_E4M3_ROW, L.PACK_E4M3), (L.LN_S8_ROW, L.PACK_S8)):
+            want, ws = pk.ops.pack_weight_rows(y, fmt)
+            q, s = pk.ops.layer_norm(xd, gd, bd, mode)
+            assert torch.equal(s, ws) and torch.equal(q.view(torch.uint8), want.view(torch.uint8))
+            _, q2, s2 = pk.ops.layer_norm_pair(xd, dev16(np.ones(1024)), dev16(np.zeros(1024)), gd, bd, mode)
+            y1, _ = pk.ops.layer_norm(xd, dev16(np.ones(1024)), dev16(np.zeros(1024)), L.LN_F16)
+            want2, ws2 = pk.ops.pack_weight_rows(pk.ops.layer_norm(y1, gd, bd, L.LN_F16)[0], fmt)
+            assert torch.equal(s2, ws2) and torch.equal(q2.view(torch.uint8), want2.view(torch.uint8))
