@@ -45,12 +45,11 @@ __device__ __forceinline__ Pair half2_pair(__half2 h) {
     return make_pair(f.x, f.y);
 }
 
-// both halves through ReLU and rounded to fp16
+// both halves rounded to fp16 and through ReLU; a NaN becomes 0 (max.f16x2 returns the operand that is a number,
+// the .relu form of the conversion would keep it)
 __device__ __forceinline__ __half2 relu_half2(Pair v) {
     const float2 f = split_pair(v);
-    uint32_t r;
-    asm("cvt.rn.relu.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(f.y), "f"(f.x));
-    return *reinterpret_cast<const __half2*>(&r);
+    return __hmax2(__floats2half2_rn(f.x, f.y), __half2half2(__ushort_as_half(0)));
 }
 
 // E4M3 codes of one row, absmax / 448 per row: the arithmetic of pk100_pack_weight_rows

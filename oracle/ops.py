@@ -488,8 +488,9 @@ def subsampling(mel, w, fp8=False, collect=None):
     per-row E4M3 weights (pk_sm89_quantize_rows256, pk_sm89_subsample_pointwise_fp8: + bias, ReLU);
     the second stage stays fp16; the flattened rows are quantised per row (pk_sm89_quantize_ffn_contract)
     and the projection is an E4M3 GEMM (pk_sm89_subsample_projection_fp8: + bias)."""
-    x = f16_round(np.maximum(_conv_s2(np.asarray(mel, dtype=F32)[:, :, None], w["conv0_w"].reshape(256, 3, 3),
-                                      w["conv0_b"]), 0))
+    # (fmax: a NaN sum becomes 0, like fmaxf(sum, 0))
+    x = f16_round(np.fmax(_conv_s2(np.asarray(mel, dtype=F32)[:, :, None], w["conv0_w"].reshape(256, 3, 3),
+                                   w["conv0_b"]), 0))
     for stage in (1, 2):
         x = f16_round(_conv_s2(x, w[f"dw{stage}_w"].reshape(256, 3, 3), w[f"dw{stage}_b"]))
         f, t, c = x.shape

@@ -53,3 +53,19 @@ def test_frames_per_cta_do_not_change_a_bit(pk, cuda, frames_list, precision):
         alone = sub.run(batch[i:i + 1, :f].contiguous(), stride)
         rows = pk.subsampling.output_frames(f)
         assert torch.equal(alone[:rows], together[i * stride:i * stride + rows]) and bool(alone[:rows].any())
+
+
+@pytest.mark.parametrize("precision", ["fp16", "fp8"])
+def test_nan_mel_values_end_at_the_first_relu(pk, cuda, precision):
+    """max(NaN, 0) = 0: a NaN mel value removes the first-layer features it reaches and nothing else."""
+    w = pk.synth.subsampling_weights(2)
+    sub = pk.subsampling.Subsampling(w, cuda, precision=precision)
+    mel = pk.synth.mel_input(8, 203)
+    for f, t in ((0, 0), (0, 127), (57, 64), (58, 33), (202, 5)):
+        mel[f, t] = np.nan
+    mel[120] = np.nan
+    got = host(sub.run(dev(mel[None]), 128))[:26]
+    want = O.subsampling(mel, w, fp8=precision == "fp8")
+    assert np.isfinite(got).all() and np.isfinite(want).all()
+    max_abs, max_nrmse = (2e-2, 2e-3) if precision == "fp16" else (4e-2, 1e-2)      # as without NaN
+    assert np.max(np.abs(got - want)) <= max_abs and nrmse(got, want) <= max_nrmse
