@@ -65,8 +65,8 @@ __device__ __forceinline__ float e4m3_row_scale(float absmax) { return absmax > 
 // both channels.  Intermediate rows are walked in order; the row shared by two output frames
 // (2*f2 + 1) is computed once and scattered into both, so a frame costs two rows of the first
 // convolution, not three.  The accumulation order of both convolutions (bias, then taps row by row)
-// is the reference's (kernels/sm89/subsampling.cu:11-179); the out-of-range taps it skips read
-// zeros here.
+// is the reference's (kernels/sm89/subsampling.cu:11-179); the out-of-range taps it skips are zero
+// taps on zero values here.
 // Bound by its fp32 multiply-adds (about 6000 packed warp instructions per output frame).  8 x 60 s: 405 us
 // with one frame per CTA, one channel per thread and three rows per frame, 330 us now (E4M3 372 us, where
 // a quantising pass of 270 us followed before).
@@ -128,6 +128,16 @@ subsample_first_fused_kernel(const float* __restrict__ in, const __half* __restr
     auto walk_row = [&](int k, __half2 (&v)[2 * kFirstOuts + 1]) {
         Pair w[9];
         load_taps(w, 0);
+        // taps on rows in front of the first or behind the last frame
+        const int f1 = 2 * first - 1 + k;                  // its mel rows: 2*f1 - 1 .. 2*f1 + 1
+        if (f1 == 0 || 2 * f1 + 1 >= in_frames) [[unlikely]] {
+            const bool head = f1 == 0, tail = 2 * f1 + 1 >= in_frames;
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                w[i] = head ? 0ull : w[i];
+                w[6 + i] = tail ? 0ull : w[6 + i];
+            }
+        }
         const float2* base[3];
         Pair c0[3], c1[3];                                 // columns 2*m1 - 1, 2*m1 of the sliding window
 #pragma unroll
@@ -154,7 +164,8 @@ subsample_first_fused_kernel(const float* __restrict__ in, const __half* __restr
             for (int a = 0; a < 3; ++a) {
                 // columns 2*m1 + 1 and 2*m1 + 2: 16-byte aligned, because an even column sits at an odd index
                 const ulonglong2 nx = *reinterpret_cast<const ulonglong2*>(base[a] + 2 * m + 2);
-                acc = fma_pair(c0[a], w[a * 3 + 0], acc);
+                // (column -1 is outside)
+                acc = fma_pair(c0[a], m == 0 && part == 0 ? 0ull : w[a * 3 + 0], acc);
                 acc = fma_pair(c1[a], w[a * 3 + 1], acc);
                 acc = fma_pair(nx.x, w[a * 3 + 2], acc);
                 c0[a] = nx.x;

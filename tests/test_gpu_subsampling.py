@@ -69,3 +69,16 @@ def test_nan_mel_values_end_at_the_first_relu(pk, cuda, precision):
     assert np.isfinite(got).all() and np.isfinite(want).all()
     max_abs, max_nrmse = (2e-2, 2e-3) if precision == "fp16" else (4e-2, 1e-2)      # as without NaN
     assert np.max(np.abs(got - want)) <= max_abs and nrmse(got, want) <= max_nrmse
+
+
+@pytest.mark.parametrize("frames,rows", [(1, (0, 2)), (2, (0,))])
+def test_taps_outside_the_utterance_are_not_multiplied(pk, cuda, frames, rows):
+    """Taps of the first convolution that lie in front of or behind every frame: infinite weights there change
+    nothing (multiplied with a zero they would give NaN)."""
+    w = pk.synth.subsampling_weights(2)
+    mel = dev(pk.synth.mel_input(9, frames)[None])
+    want = pk.subsampling.Subsampling(w, cuda).run(mel, 128).clone()
+    taps = w["conv0_w"] = w["conv0_w"].copy()
+    taps.reshape(256, 3, 3)[:, rows, :] = np.inf
+    got = pk.subsampling.Subsampling(w, cuda).run(mel, 128)
+    assert torch.equal(got, want) and bool(got[:1].any())
