@@ -86,6 +86,8 @@ class PipelineEngine:
             self.enc.add_layer(synth.layer_weights(seed, l, randomize_norms=randomize_norms))
         self.dec = dec_mod.TdtDecoder(synth.decoder_weights(seed, decoder_layers), self.device)
         self.arena, self.ws = self.enc.make_workspace(self.rows)
+        # (128 rows more per utterance: what encode_chunk adds for the rows it drops)
+        self.sub.workspace(max_utterances, mel_frames, self.seg_stride + 128)
         dev = self.device
         self.state_a = torch.zeros((self.rows, 1024), dtype=torch.float16, device=dev)
         self.state_b = torch.zeros((self.rows, 1024), dtype=torch.float16, device=dev)

@@ -153,3 +153,18 @@ def test_a_refused_request_changes_no_later_result(pk, cuda):
         for _ in range(2):
             got = engines[1].transcribe_batch(mel[:3], frames)
             assert all(np.array_equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("precision", ["fp16", "fp8"])
+def test_requests_allocate_no_device_memory_of_their_own(pk, cuda, precision):
+    """The stages' workspaces hold the engine's capacity from the start: a request longer than all before it,
+    or of more utterances, allocates nothing, nor does a chunk of a long utterance."""
+    eng = pk.pipeline.PipelineEngine(cuda, layers=1, decoder_layers=1, seed=9, max_utterances=3, mel_frames=1200,
+                                     subsampling_precision=precision)
+    mel = torch.randn((3, 1200, 128), generator=torch.Generator().manual_seed(7)).pin_memory()
+    held = eng.sub._ws.data_ptr(), eng.sub._ws.numel()
+    for n, frames in ((1, 40), (1, 900), (2, 400), (3, 1200)):
+        eng.transcribe_batch(mel[:n, :frames])
+        assert (eng.sub._ws.data_ptr(), eng.sub._ws.numel()) == held
+    eng.encode_chunk(mel[0, :640], 2, 70)
+    assert (eng.sub._ws.data_ptr(), eng.sub._ws.numel()) == held
