@@ -331,8 +331,8 @@ int pk100_run_layers(void* stream, const pk100_layer_weights* layers, int n_laye
 
 /* The same on a packed batch: every utterance takes whole 128-row tiles and only as many as it needs, so a
  * batch of unequal utterances carries no padding tiles.  rows: a multiple of 128; tiles (device, 8-byte
- * aligned): rows / 128 pairs {first row of the tile's utterance, valid rows of that utterance}, written
- * before the kernel in front of this call in the stream.  Same results per utterance as pk100_run_layers. */
+ * aligned): rows / 128 pairs {first row of the tile's utterance, valid rows of that utterance}.  Same results
+ * per utterance as pk100_run_layers. */
 int pk100_run_layers_packed(void* stream, const pk100_layer_weights* layers, int n_layers, void* state_a,
                             void* state_b, const pk100_encoder_workspace* workspace, int rows, const int* tiles,
                             void** output);

@@ -108,7 +108,7 @@ struct Params {
     __half* out; int ldo;
     int tiles;                // 128-row tiles of the batch
     pk100_rows rows;
-    int early;                // the kernel before writes none of position, bias_u, bias_v, rows
+    int early;                // position, bias_u, bias_v and rows were complete before the chain of launches began
     int* status;
 };
 

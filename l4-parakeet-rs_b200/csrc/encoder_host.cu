@@ -46,8 +46,6 @@ int gemm_base(pk100_gemm_args& a, int kind, int m, int n, int k, const void* x, 
 // LN (already applied) -> FP8 expand + SiLU + tile threshold -> INT8 contract, x += 0.5*y
 int ff_module(void* stream, const pk100_ff_weights& w, void* x, const pk100_encoder_workspace& ws,
               const Geometry& g, float* stats, int profile_slot) {
-    // (what the caller queued right before the first module may have written its weights)
-    const bool w1_settled = profile_slot > 0;
     pk100_gemm_args a;
     const bool timed = ws.profile_events != nullptr && 2 * profile_slot + 1 < ws.profile_events_len;
     if (timed) cudaEventRecord(static_cast<cudaEvent_t>(ws.profile_events[2 * profile_slot]),
@@ -58,7 +56,7 @@ int ff_module(void* stream, const pk100_ff_weights& w, void* x, const pk100_enco
     a.col_scales = w.w1_scales;
     a.out = ws.hidden8; a.ld_out = kFf; a.out_type = PK100_OUT_S8; a.out_scale = kHiddenInv;
     a.tau = w.tau; a.keep_out = ws.keep; a.stats_out = stats; a.status = ws.status;
-    PK_TRY(pk100_gemm_chained(stream, &a, w1_settled));
+    PK_TRY(pk100_gemm_chained(stream, &a, true));
     if (timed) cudaEventRecord(static_cast<cudaEvent_t>(ws.profile_events[2 * profile_slot + 1]),
                                static_cast<cudaStream_t>(stream));
 
@@ -120,12 +118,11 @@ static int run_layers(void* stream, const pk100_layer_weights* layers, int n_lay
     void* other = state_b;
     if (output) *output = x;
     if (g.rows == 0 || n_layers == 0) return PK100_OK;
-    // the row-wise operators of a packed batch have no entry points of their own
-    auto norm = [&](const void* in, const void* gamma, const void* beta, void* out, float* scales, int mode, float inv_scale) {
-        if (g.tiles == nullptr)
-            return pk100_layer_norm(stream, in, gamma, beta, out, scales, mode, inv_scale, g.rows, seg_stride, valid_rows, seg_valid, kEps);
+    if (g.rows < 0) return PK100_ERR_SHAPE;
+    auto norm = [&](const void* in, const void* gamma, const void* beta, void* out, float* scales, int mode, float inv_scale,
+                    bool dependent = true) {
         if (!gamma || !beta) return static_cast<int>(PK100_ERR_NULL);
-        return pk100_layer_norm_rows(stream, in, gamma, beta, out, scales, mode, inv_scale, g.rows, place, kEps);
+        return pk100_layer_norm_rows(stream, in, gamma, beta, out, scales, mode, inv_scale, g.rows, place, kEps, dependent);
     };
     const long long stats_stride = static_cast<long long>((g.rows + 127) / 128) * 64;
 
@@ -137,7 +134,9 @@ static int run_layers(void* stream, const pk100_layer_weights* layers, int n_lay
 
         // ---- feed-forward module 1 (its LayerNorm was fused into the previous block's output norm)
         if (i == 0) {
-            PK_TRY(norm(x, w.ff1.ln_gamma, w.ff1.ln_beta, ws.q8, nullptr, PK100_LN_E4M3_FIXED, kFp8InputInv));
+            // Plainly launched: all that the caller queued in front of this call, weights and geometry among it,
+            // is complete before any kernel of the chain starts, so their prologues may read both.
+            PK_TRY(norm(x, w.ff1.ln_gamma, w.ff1.ln_beta, ws.q8, nullptr, PK100_LN_E4M3_FIXED, kFp8InputInv, false));
         }
         PK_TRY(ff_module(stream, w.ff1, x, ws, g, stats1, 2 * i));
 

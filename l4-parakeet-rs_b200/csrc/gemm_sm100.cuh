@@ -57,8 +57,8 @@ struct GemmParams {
     // Bytes of one output row in a warp's 32-row slice when the slices leave through shared
     // memory and a TMA store (64 or 128); 0 = each thread stores its row piece directly.
     int store_row_bytes;
-    // B is not written by the kernel in front of this one in the stream: the first stages of the weights are
-    // requested before the wait for that kernel.
+    // B was complete before the chain of dependent launches began: the first stages of the weights are
+    // requested before the wait for the kernel in front.
     int b_settled;
 };
 

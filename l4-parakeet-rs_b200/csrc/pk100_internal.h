@@ -29,11 +29,18 @@ static inline int pk100_launch_status() {
 // latency and the prologue (barrier set-up, tensor-memory allocation, descriptor prefetch) leave
 // the critical path; the data dependency is still the whole predecessor grid.  On by default;
 // pk100_set_dependent_launch(0) restores plain stream order.
+//
+// A chain of such launches reaches further back than its last link: every kernel lets the next one start
+// before it has itself waited, so the prologue of the n-th may run while whatever stands in front of the
+// first still does.  What a prologue reads (weights, geometry: b_settled, constants_settled below) must
+// therefore have been written in front of a PLAIN launch that opens the chain; pk100_run_layers and the
+// subsampling stage open theirs with one.
 bool pk100_dependent_launch_enabled();
 
+// dependent: as above where enabled; false = plain stream order for this launch
 template <typename... Params, typename... Args>
-static inline void pk100_launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem_bytes,
-                                        cudaStream_t stream, Args&&... args) {
+static inline void pk100_launch(bool dependent, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem_bytes,
+                                cudaStream_t stream, Args&&... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -43,8 +50,14 @@ static inline void pk100_launch_chained(void (*kernel)(Params...), dim3 grid, di
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &attr;
-    cfg.numAttrs = pk100_dependent_launch_enabled() ? 1 : 0;
+    cfg.numAttrs = dependent && pk100_dependent_launch_enabled() ? 1 : 0;
     cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
+template <typename... Params, typename... Args>
+static inline void pk100_launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem_bytes,
+                                        cudaStream_t stream, Args&&... args) {
+    pk100_launch(true, kernel, grid, block, smem_bytes, stream, args...);
 }
 
 // Row geometry of a batch: uniform blocks of seg_stride rows per utterance (tiles == nullptr), or a packed
@@ -57,9 +70,9 @@ struct pk100_rows {
 };
 
 // The row-wise operators behind the C entry points, on either geometry (total_rows: a multiple of 128 when
-// packed).  Arguments are the entry points', already checked.
+// packed).  Arguments are the entry points', already checked.  dependent = false opens a chain (see above).
 int pk100_layer_norm_rows(void* stream, const void* input, const void* gamma, const void* beta, void* output, float* scales,
-                          int mode, float inv_scale, int total_rows, const pk100_rows& geometry, float eps);
+                          int mode, float inv_scale, int total_rows, const pk100_rows& geometry, float eps, bool dependent = true);
 int pk100_layer_norm_pair_rows(void* stream, const void* input, const void* gamma, const void* beta, void* output,
                                const void* next_gamma, const void* next_beta, void* next_output, float* next_scales,
                                int next_mode, float next_inv_scale, int total_rows, const pk100_rows& geometry, float eps);
@@ -68,12 +81,12 @@ int pk100_depthwise_bn_silu_rows(void* stream, const void* input, const void* dw
                                  int total_rows, int segments, const pk100_rows& geometry, float eps);
 
 // Local attention behind pk100_local_relpos_attention_tcgen05 on either geometry (total_rows: a multiple of 128).
-// constants_settled: the kernel before it in the stream writes neither position, biases nor the geometry.
+// constants_settled: position, biases and geometry were written in front of the plain launch that opened the chain.
 int pk100_local_attention_rows(void* stream, const void* query, int ldq, const void* key, int ldk, const void* value, int ldv,
                                const void* position, const void* bias_u, const void* bias_v, void* output, int ldo,
                                int total_rows, const pk100_rows& geometry, bool constants_settled, int* status);
 
-// pk100_gemm for a caller who knows that the kernel in front of it in the stream does not write B.
+// pk100_gemm; b_settled: B was written in front of the plain launch that opened the chain.
 int pk100_gemm_chained(void* stream, const pk100_gemm_args* args, bool b_settled);
 
 // SMs a persistent kernel may use: all of them, or the cap set by pk100_set_gemm_cta_cap.

@@ -688,7 +688,7 @@ using namespace pk100;
 template <int Mode, int Mode2>
 static int launch_layer_norm(void* stream, const void* input, const void* gamma, const void* beta, void* output, float* scales,
                              float inv_scale, const void* gamma2, const void* beta2, void* output2, float* scales2,
-                             float inv_scale2, int total_rows, const pk100_rows& geometry, float eps) {
+                             float inv_scale2, int total_rows, const pk100_rows& geometry, float eps, bool dependent = true) {
     auto kernel = layer_norm_kernel<Mode, Mode2>;
     static std::atomic<int> resident{0};
     if (resident.load(std::memory_order_relaxed) == 0) {
@@ -698,7 +698,7 @@ static int launch_layer_norm(void* stream, const void* input, const void* gamma,
         resident.store(148 * (per_sm > 0 ? per_sm : 1), std::memory_order_relaxed);
     }
     const int blocks = (total_rows + 7) / 8, cap = resident.load(std::memory_order_relaxed);
-    pk100_launch_chained(kernel, dim3(blocks < cap ? blocks : cap), dim3(256), 0, static_cast<cudaStream_t>(stream),
+    pk100_launch(dependent, kernel, dim3(blocks < cap ? blocks : cap), dim3(256), 0, static_cast<cudaStream_t>(stream),
         static_cast<const __half*>(input), static_cast<const __half*>(gamma), static_cast<const __half*>(beta), output, scales,
         inv_scale, static_cast<const __half*>(gamma2), static_cast<const __half*>(beta2), output2, scales2, inv_scale2,
         total_rows, geometry, eps);
@@ -706,9 +706,9 @@ static int launch_layer_norm(void* stream, const void* input, const void* gamma,
 }
 
 int pk100_layer_norm_rows(void* stream, const void* input, const void* gamma, const void* beta, void* output, float* scales,
-                          int mode, float inv_scale, int total_rows, const pk100_rows& geometry, float eps) {
+                          int mode, float inv_scale, int total_rows, const pk100_rows& geometry, float eps, bool dependent) {
 #define PK_LN(M) case M: return launch_layer_norm<M, -1>(stream, input, gamma, beta, output, scales, inv_scale, nullptr, \
-                                                         nullptr, nullptr, nullptr, 0.0f, total_rows, geometry, eps)
+                                                         nullptr, nullptr, nullptr, 0.0f, total_rows, geometry, eps, dependent)
     switch (mode) {
     PK_LN(PK100_LN_F16); PK_LN(PK100_LN_E4M3_FIXED); PK_LN(PK100_LN_E4M3_ROW); PK_LN(PK100_LN_S8_ROW); PK_LN(PK100_LN_S4_ROW);
     default: return PK100_ERR_SHAPE;

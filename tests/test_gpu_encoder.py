@@ -237,3 +237,29 @@ def test_three_layer_stack_dense_hidden(pk, cuda):
     for w in ws_list:
         cur = O.encoder_layer(cur, O.prepare_layer(w), valid, 0.0, 0.0)
     assert nrmse(got[:valid], cur[:valid]) <= 3e-2
+
+
+def test_weights_written_by_a_kernel_right_in_front(pk, cuda):
+    """Plain stream order for everything a block reads: a long product on one SM, which lets dependent launches
+    start at once, writes the output projection's weights right in front of the call."""
+    L = pk.lib
+    enc = pk.encoder.EncoderLayers(cuda)
+    lw = enc.add_layer(pk.synth.layer_weights(3, 0, randomize_norms=True))
+    gen = torch.Generator(device=cuda).manual_seed(5)
+    a, b = ((torch.randn((1024, 16384), generator=gen, device=cuda) * 0.02).half() for _ in range(2))
+    wo = torch.zeros((1024, 1024), dtype=torch.float16, device=cuda)
+    lw.wo_f16 = wo.data_ptr()
+    arena, ws = enc.make_workspace(128)
+    x = dev16(_input(1, 128, 100))
+    got = []
+    for wait in (True, False):
+        state, other = x.clone(), torch.zeros_like(x)
+        wo.zero_()
+        torch.cuda.synchronize()
+        pk.ops.gemm(a, b, kind=L.KIND_F16, out=wo, max_ctas=1)
+        if wait:
+            torch.cuda.synchronize()
+        got.append(enc.run(state, other, ws, 1, 128, 100).clone())
+    torch.cuda.synchronize()
+    assert enc.status(arena, ws) == 0 and bool(wo.any())
+    assert torch.isfinite(got[0]).all() and torch.equal(got[0], got[1])
