@@ -362,7 +362,10 @@ class PipelineEngine:
         # The last batch of a sequence of known length has nothing behind it to leave SMs for: it is decoded on
         # all clusters that the batches in flight do not hold (6 batches of 8 x 60 s: 1.20 -> 1.34 times the rate
         # of the code before the persistent attention kernel, measured beside it).
-        last = len(batches) - 1 if hasattr(batches, "__len__") else -1
+        try:
+            last = len(batches) - 1
+        except (TypeError, NotImplementedError):          # (no length, or an iterable that does not know it)
+            last = -1
         pending = []                              # oldest first: (slot index, utterances, event, clusters)
         for i, item in enumerate(batches):
             mel_host, lengths = item if isinstance(item, (tuple, list)) else (item, None)

@@ -168,3 +168,23 @@ def test_requests_allocate_no_device_memory_of_their_own(pk, cuda, precision):
         assert (eng.sub._ws.data_ptr(), eng.sub._ws.numel()) == held
     eng.encode_chunk(mel[0, :640], 2, 70)
     assert (eng.sub._ws.data_ptr(), eng.sub._ws.numel()) == held
+
+
+class _Unsized:
+    """Iterable whose length is not known, like a loader over a stream."""
+
+    def __init__(self, items):
+        self.items = items
+
+    def __iter__(self):
+        return iter(self.items)
+
+    def __len__(self):
+        raise TypeError("no length")
+
+
+def test_a_stream_of_unknown_length_is_accepted(pk, cuda, engine):
+    mel = torch.randn((2, 400, 128), generator=torch.Generator().manual_seed(2)).pin_memory()
+    want = engine.transcribe_batch(mel)
+    for got in engine.transcribe_stream(_Unsized([mel, mel]), depth=2):
+        assert all(np.array_equal(a, b) for a, b in zip(got, want))
