@@ -130,11 +130,13 @@ int pk100_gemm(void* stream, const pk100_gemm_args* args);
  * 256 x 256 tiles); default 0 = one CTA per 128 x 256 tile, which measured faster on B200. */
 void pk100_set_gemm_cta_pairs(int enable);
 
-/* Process-wide cap on the persistent CTAs of every pk100_gemm launch whose own max_ctas is <= 0
- * (the sequencers pk100_run_layers / pk100_run_subsampling included); 0 = one CTA per SM.  For a
- * host that keeps another persistent kernel resident beside the encoder (the cluster decoder holds
- * 16 SMs per call): persistent GEMM CTAs that cannot be placed at once queue behind the first wave
- * and double the kernel's time, a smaller grid does not.  Takes effect on launches issued after it. */
+/* Process-wide cap on the persistent CTAs of every pk100_gemm launch whose own max_ctas is <= 0 and of the
+ * tcgen05 attention kernel (the sequencers pk100_run_layers / pk100_run_subsampling included); 0 = one CTA
+ * per SM.  The LayerNorm, depthwise, subsampling and frontend launches size their grids or tiles for that many
+ * SMs as well.  For a host that keeps another persistent kernel resident beside the encoder (the cluster
+ * decoder holds 16 SMs per call): persistent CTAs that cannot be placed at once queue behind the first wave
+ * and double the kernel's time, a smaller grid does not.  No result depends on it.  Takes effect on launches
+ * issued after it. */
 void pk100_set_gemm_cta_cap(int ctas);
 
 /* Programmatic dependent launch of the kernels of the per-block chain (LayerNorm, GEMMs,

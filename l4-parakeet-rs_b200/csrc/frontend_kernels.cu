@@ -334,7 +334,7 @@ extern "C" int pk100_mel_frontend(void* stream_v, const pk100_frontend_weights* 
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
     // 8-frame tiles while 32-frame ones would not give every SM two CTAs
     const long long frames = static_cast<long long>(frame_cap) * utterances;
-    const int frc = frames >= 32LL * 2 * 148
+    const int frc = frames >= 32LL * 2 * pk100_cta_budget()
         ? launch_mel_frames<32>(stream, w, samples, utterances, sample_stride, sample_counts, mel, frame_cap)
         : launch_mel_frames<8>(stream, w, samples, utterances, sample_stride, sample_counts, mel, frame_cap);
     if (frc != PK100_OK) return frc;

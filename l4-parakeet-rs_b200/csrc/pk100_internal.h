@@ -89,7 +89,7 @@ int pk100_local_attention_rows(void* stream, const void* query, int ldq, const v
 // pk100_gemm; b_settled: B was written in front of the plain launch that opened the chain.
 int pk100_gemm_chained(void* stream, const pk100_gemm_args* args, bool b_settled);
 
-// SMs a persistent kernel may use: all of them, or the cap set by pk100_set_gemm_cta_cap.
+// SMs a launch may count on: all of them, or the cap set by pk100_set_gemm_cta_cap.
 int pk100_cta_budget();
 
 // 2-D TMA descriptor of a row-major matrix [rows, cols] (`ld` elements between rows) with a box of

@@ -690,14 +690,14 @@ static int launch_layer_norm(void* stream, const void* input, const void* gamma,
                              float inv_scale, const void* gamma2, const void* beta2, void* output2, float* scales2,
                              float inv_scale2, int total_rows, const pk100_rows& geometry, float eps, bool dependent = true) {
     auto kernel = layer_norm_kernel<Mode, Mode2>;
-    static std::atomic<int> resident{0};
+    static std::atomic<int> resident{0};                   // CTAs per SM
     if (resident.load(std::memory_order_relaxed) == 0) {
         int per_sm = 0;
         const cudaError_t err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 256, 0);
         if (err != cudaSuccess) return static_cast<int>(err);
-        resident.store(148 * (per_sm > 0 ? per_sm : 1), std::memory_order_relaxed);
+        resident.store(per_sm > 0 ? per_sm : 1, std::memory_order_relaxed);
     }
-    const int blocks = (total_rows + 7) / 8, cap = resident.load(std::memory_order_relaxed);
+    const int blocks = (total_rows + 7) / 8, cap = pk100_cta_budget() * resident.load(std::memory_order_relaxed);
     pk100_launch(dependent, kernel, dim3(blocks < cap ? blocks : cap), dim3(256), 0, static_cast<cudaStream_t>(stream),
         static_cast<const __half*>(input), static_cast<const __half*>(gamma), static_cast<const __half*>(beta), output, scales,
         inv_scale, static_cast<const __half*>(gamma2), static_cast<const __half*>(beta2), output2, scales2, inv_scale2,
@@ -864,7 +864,7 @@ int pk100_depthwise_bn_silu_rows(void* stream, const void* input, const void* dw
             row_scales, geometry, eps);
         return pk100_launch_status();
     };
-    const bool wide = total_rows >= 2 * 148 * 16;
+    const bool wide = total_rows >= 2 * pk100_cta_budget() * 16;
     if (quantize) return wide ? launch(depthwise_bn_silu_kernel<true, 16>, 16) : launch(depthwise_bn_silu_kernel<true, 8>, 8);
     return wide ? launch(depthwise_bn_silu_kernel<false, 16>, 16) : launch(depthwise_bn_silu_kernel<false, 8>, 8);
 }

@@ -513,8 +513,8 @@ static int run_subsampling(void* stream_v, const pk100_subsampling_weights* w, c
     const auto *w1 = static_cast<const __half*>(w->dw1_w), *b1 = static_cast<const __half*>(w->dw1_b);
     // frames per CTA: whole waves over the 2 resident CTAs of every SM (a frame range takes two CTAs, one per
     // half of the features), each CTA with at most kFirstMaxFrames frames
-    const long long total = u * c.f2, waves = (total + 148 * kFirstMaxFrames - 1) / (148 * kFirstMaxFrames);
-    const int run = static_cast<int>((total + 148 * waves - 1) / (148 * waves));
+    const long long sms = pk100_cta_budget(), total = u * c.f2, waves = (total + sms * kFirstMaxFrames - 1) / (sms * kFirstMaxFrames);
+    const int run = static_cast<int>((total + sms * waves - 1) / (sms * waves));
     const dim3 first_grid((c.f2 + run - 1) / run, utterances, 32 / (2 * kFirstOuts));
     const size_t first_bytes = sizeof(float2) * kFirstPitch * first_rows(run);
     auto first_kernel = q != nullptr ? subsample_first_fused_kernel<true> : subsample_first_fused_kernel<false>;

@@ -277,3 +277,25 @@ def test_row_codes_of_rows_with_nan_and_infinity(pk, cuda):
             y1, _ = pk.ops.layer_norm(xd, dev16(np.ones(1024)), dev16(np.zeros(1024)), L.LN_F16)
             want2, ws2 = pk.ops.pack_weight_rows(pk.ops.layer_norm(y1, gd, bd, L.LN_F16)[0], fmt)
             assert torch.equal(s2, ws2) and torch.equal(q2.view(torch.uint8), want2.view(torch.uint8))
+
+
+@pytest.mark.parametrize("cap", [1, 37])
+def test_launch_sizes_follow_the_cta_cap_and_change_no_bit(pk, cuda, cap):
+    """Row-wise and subsampling launches are sized by the SMs left free; the results do not depend on it."""
+    L = pk.lib
+    g, b = (dev16(t) for t in _affine(5))
+    x = dev16(_rows(3, 5000, 2.0))
+    w = dev16(np.random.default_rng(4).standard_normal((1024, 9)) * 0.3)
+    bn = [torch.ones(1024, device=cuda) for _ in range(4)]
+    sub = pk.subsampling.Subsampling(pk.synth.subsampling_weights(2), cuda)
+    mel = dev(pk.synth.mel_input(8, 1203)[None])
+    def run():
+        return (*pk.ops.layer_norm(x, g, b, L.LN_S8_ROW, seg_stride=1000, valid_rows=990),
+                *pk.ops.depthwise_bn_silu(x, w, *bn, quantize=True, seg_stride=1000, valid_rows=990), sub.run(mel, 256).clone())
+    want = run()
+    L.lib.pk100_set_gemm_cta_cap(cap)
+    try:
+        got = run()
+    finally:
+        L.lib.pk100_set_gemm_cta_cap(0)
+    assert all(torch.equal(p, q) for p, q in zip(got, want))
