@@ -188,3 +188,28 @@ def test_a_stream_of_unknown_length_is_accepted(pk, cuda, engine):
     want = engine.transcribe_batch(mel)
     for got in engine.transcribe_stream(_Unsized([mel, mel]), depth=2):
         assert all(np.array_equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("decode_groups,depth", [(1, 2), (2, 2), (1, 4)])
+def test_last_batch_of_a_known_number_takes_the_free_clusters(pk, cuda, engine, decode_groups, depth):
+    """A list knows its last batch, an iterator does not: the last batch is decoded on the clusters that the
+    batches in flight do not hold, with the same tokens, more batches than buffer sets and ragged lengths."""
+    eng, rng = engine, np.random.default_rng(6)
+    batches = []
+    for i, n in enumerate((3, 1, 2, 3, 2, 3)):
+        frames = [int(f) for f in rng.integers(40, 1001, size=n)]
+        mels = np.zeros((n, 1000, 128), np.float32)
+        for u, f in enumerate(frames):
+            mels[u, :f] = pk.synth.mel_input(400 + 10 * i + u, f)
+        batches.append((torch.from_numpy(mels).pin_memory(), frames))
+    want = [eng.transcribe_batch(mel, frames) for mel, frames in batches]
+    assert eng.decode_groups == 3 and any(len(t) > 0 for t in want[-1])
+    groups = []
+    for source in (batches, iter(batches)):
+        got = list(eng.transcribe_stream(source, decode_groups=decode_groups, depth=depth))
+        assert eng.status() == 0 and len(got) == len(want)
+        for g, w in zip(got, want):
+            assert len(g) == len(w) and all(np.array_equal(x, y) for x, y in zip(g, w))
+        groups.append(len(eng.last_groups))
+    busy = (depth - 1) * decode_groups if depth == 2 else 3          # (at depth 4: batches of at least one cluster each)
+    assert groups[1] == decode_groups and groups[0] == max(decode_groups, 3 - busy)

@@ -82,3 +82,25 @@ def test_taps_outside_the_utterance_are_not_multiplied(pk, cuda, frames, rows):
     taps.reshape(256, 3, 3)[:, rows, :] = np.inf
     got = pk.subsampling.Subsampling(w, cuda).run(mel, 128)
     assert torch.equal(got, want) and bool(got[:1].any())
+
+
+@pytest.mark.parametrize("precision", ["fp16", "fp8"])
+@pytest.mark.parametrize("frames_list", [[3100, 1024, 1025], [8, 3100, 0, 2049], [1, 1, 1024]])
+def test_packed_rows_are_the_rows_of_the_uniform_layout(pk, cuda, precision, frames_list):
+    """row_base: every utterance in whole 128-row tiles, at its own place, padding rows included; utterances at
+    the distance of a larger buffer."""
+    sub = pk.subsampling.Subsampling(pk.synth.subsampling_weights(2), cuda, precision=precision)
+    n, cap, frames = len(frames_list), 3300, max(frames_list)
+    mel = torch.randn((n, cap, 128), generator=torch.Generator(device=cuda).manual_seed(n), device=cuda)
+    mf = torch.tensor(frames_list, dtype=torch.int32, device=cuda)
+    seg = pk.pipeline.seg_stride_for(pk.subsampling.output_frames(frames))
+    want = sub.run(mel[:, :frames].contiguous(), seg, mel_frames=mf).clone()
+    rows = [pk.pipeline.seg_stride_for(pk.subsampling.output_frames(f)) for f in frames_list]
+    base = np.concatenate([[0], np.cumsum(rows)[:-1]])
+    out = torch.full((sum(rows), 1024), float("nan"), dtype=torch.float16, device=cuda)
+    sub.run_rows(mel, frames, seg, mf, out, row_base=torch.tensor(base, dtype=torch.int32, device=cuda), rows=sum(rows))
+    assert int(sub.status.item()) == 0
+    for u in range(n):
+        assert torch.equal(out[base[u]:base[u] + rows[u]], want[u * seg:u * seg + rows[u]])
+    uniform = sub.run_rows(mel, frames, seg, mf, torch.empty_like(want))
+    assert torch.equal(uniform, want) and bool(want.any())
