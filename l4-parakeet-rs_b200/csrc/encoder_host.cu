@@ -194,7 +194,6 @@ static int run_layers(void* stream, const pk100_layer_weights* layers, int n_lay
                                            w.bn_var, ws.dw8, ws.dw_scales, 1, segments, seg_stride,
                                            valid_rows, seg_valid, kEps));
         } else {
-            if (!w.dw_weight || !w.bn_gamma || !w.bn_beta || !w.bn_mean || !w.bn_var) return PK100_ERR_NULL;
             PK_TRY(pk100_depthwise_bn_silu_rows(stream, ws.glu, w.dw_weight, w.bn_gamma, w.bn_beta, w.bn_mean,
                                                 w.bn_var, ws.dw8, ws.dw_scales, 1, g.rows, segments, place, kEps));
         }

@@ -70,7 +70,8 @@ struct pk100_rows {
 };
 
 // The row-wise operators behind the C entry points, on either geometry (total_rows: a multiple of 128 when
-// packed).  Arguments are the entry points', already checked.  dependent = false opens a chain (see above).
+// packed).  Arguments are the entry points', already checked (pointers of the depthwise form excepted: it
+// checks them itself).  dependent = false opens a chain (see above).
 int pk100_layer_norm_rows(void* stream, const void* input, const void* gamma, const void* beta, void* output, float* scales,
                           int mode, float inv_scale, int total_rows, const pk100_rows& geometry, float eps, bool dependent = true);
 int pk100_layer_norm_pair_rows(void* stream, const void* input, const void* gamma, const void* beta, void* output,

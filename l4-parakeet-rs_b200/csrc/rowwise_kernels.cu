@@ -856,6 +856,12 @@ extern "C" int pk100_glu_masked(void* stream, const void* input, void* output, i
 int pk100_depthwise_bn_silu_rows(void* stream, const void* input, const void* dw_weight, const float* bn_gamma, const float* bn_beta,
                                  const float* bn_mean, const float* bn_var, void* output, float* row_scales, int quantize,
                                  int total_rows, int segments, const pk100_rows& geometry, float eps) {
+    if (!input || !dw_weight || !bn_gamma || !bn_beta || !bn_mean || !bn_var || !output || (quantize && !row_scales))
+        return PK100_ERR_NULL;
+    auto misaligned = [](const void* ptr, uintptr_t mask) { return (reinterpret_cast<uintptr_t>(ptr) & mask) != 0; };
+    if (misaligned(dw_weight, 7) || misaligned(bn_gamma, 15) || misaligned(bn_beta, 15) ||
+        misaligned(bn_mean, 15) || misaligned(bn_var, 15) || misaligned(input, 7))
+        return PK100_ERR_ALIGN;      // the kernel reads taps 8 bytes and BatchNorm vectors 16 bytes at a time
     auto launch = [&](auto kernel, int strip) {
         const int per_segment = geometry.tiles != nullptr ? 0 : (geometry.seg_stride + strip - 1) / strip;
         const int blocks = geometry.tiles != nullptr ? total_rows / strip : segments * per_segment;
@@ -875,15 +881,10 @@ extern "C" int pk100_depthwise_bn_silu(void* stream, const void* input, const vo
                                        float* row_scales, int quantize, int segments,
                                        int seg_stride, int valid_rows, const int* seg_valid,
                                        float eps) {
-    if (!input || !dw_weight || !bn_gamma || !bn_beta || !bn_mean || !bn_var || !output)
+    if (!input || !dw_weight || !bn_gamma || !bn_beta || !bn_mean || !bn_var || !output || (quantize && !row_scales))
         return PK100_ERR_NULL;
-    if (quantize && !row_scales) return PK100_ERR_NULL;
     if (segments <= 0) return segments == 0 ? PK100_OK : PK100_ERR_SHAPE;
     if (seg_stride <= 0) return PK100_ERR_SHAPE;
-    auto misaligned = [](const void* ptr, uintptr_t mask) { return (reinterpret_cast<uintptr_t>(ptr) & mask) != 0; };
-    if (misaligned(dw_weight, 7) || misaligned(bn_gamma, 15) || misaligned(bn_beta, 15) ||
-        misaligned(bn_mean, 15) || misaligned(bn_var, 15) || misaligned(input, 7))
-        return PK100_ERR_ALIGN;      // the kernel reads taps 8 bytes and BatchNorm vectors 16 bytes at a time
     return pk100_depthwise_bn_silu_rows(stream, input, dw_weight, bn_gamma, bn_beta, bn_mean, bn_var, output, row_scales, quantize,
                                         segments * seg_stride, segments, pk100_rows{nullptr, seg_stride, valid_rows, seg_valid}, eps);
 }

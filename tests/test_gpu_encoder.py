@@ -263,3 +263,22 @@ def test_weights_written_by_a_kernel_right_in_front(pk, cuda):
     torch.cuda.synchronize()
     assert enc.status(arena, ws) == 0 and bool(wo.any())
     assert torch.isfinite(got[0]).all() and torch.equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("packed", [False, True])
+def test_misaligned_convolution_weights_are_refused(pk, cuda, packed):
+    """Taps are read 8 bytes and BatchNorm vectors 16 bytes at a time: PK100_ERR_ALIGN on either geometry."""
+    enc = pk.encoder.EncoderLayers(cuda)
+    lw = enc.add_layer(pk.synth.layer_weights(3, 0))
+    arena, ws = enc.make_workspace(128)
+    x = dev16(_input(1, 128, 100))
+    tiles = torch.tensor([[0, 100]], dtype=torch.int32, device=cuda)
+    for name, off in (("dw_weight", 2), ("bn_gamma", 4), ("bn_beta", 4), ("bn_mean", 4), ("bn_var", 8)):
+        right = getattr(lw, name)
+        setattr(lw, name, right + off)
+        with pytest.raises(pk.lib.Pk100Error, match=str(pk.lib.ERR_ALIGN)):
+            if packed:
+                enc.run_packed(x.clone(), torch.zeros_like(x), ws, 128, tiles)
+            else:
+                enc.run(x.clone(), torch.zeros_like(x), ws, 1, 128, 100)
+        setattr(lw, name, right)
