@@ -2,10 +2,11 @@
 // (a round = LSTM -> prediction projection for the utterances that just emitted a token, then
 // joint + argmax for all live ones).  Three kernels share one contract and one set of decision
 // rules:
-//   tdt_cluster_kernel   one 16-CTA thread-block cluster; vectors are exchanged through
-//                        distributed shared memory (st.async + mbarrier complete_tx), layer 0's
-//                        recurrent weights live in tensor memory, the joint rows in shared
-//                        memory, the rest streams from L2.  The kernel of the hot path.
+//   tdt_cluster_kernel   one 16-CTA thread-block cluster (decoder_cluster.cuh); vectors are
+//                        exchanged through distributed shared memory (st.async + mbarrier
+//                        complete_tx), weights resident in tensor memory, shared memory and
+//                        registers as far as they fit, the rest from L2 off the critical path.
+//                        The kernel of the hot path.
 //   tdt_exchange_kernel  one CTA per SM, all weights resident in shared memory, exchanges
 //                        through tagged 64-bit global-memory slots (no cluster needed).
 //   tdt_greedy_kernel    one persistent cooperative kernel with the reference's structure: per

@@ -93,7 +93,8 @@ __device__ __forceinline__ bool row_live(const pk100_rows& g, int row) {
 struct NormVectors {
     uint4 g[4], b[4];
     // `volatile`: stays where it is written, so that the second norm's vectors are fetched per row (from L1)
-    // instead of being held across the row loop, which spills
+    // and not held across the row loop beside the first norm's.  (The pair form spills 112 to 128 bytes a
+    // thread at its 128 registers all the same.)
     static __device__ __forceinline__ uint4 fetch(const __half* p) {
         uint4 v;
         asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));

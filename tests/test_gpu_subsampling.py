@@ -41,7 +41,7 @@ def test_subsampling_matches_oracle(pk, cuda, frames_list, precision):
 @pytest.mark.parametrize("frames_list", [[2501, 97, 2], [6000] * 3])
 def test_frames_per_cta_do_not_change_a_bit(pk, cuda, frames_list, precision):
     """The first kernel walks 1 to 8 output frames per CTA depending on the batch: an utterance in a
-    batch (5 and 8 frames per CTA here) gives the bits of the utterance alone (1 to 6)."""
+    batch (7 and 8 frames per CTA here) gives the bits of the utterance alone (1 to 6)."""
     sub = pk.subsampling.Subsampling(pk.synth.subsampling_weights(2), cuda, precision=precision)
     cap = max(frames_list)
     batch = torch.zeros((len(frames_list), cap, 128), dtype=torch.float32, device=cuda)
