@@ -134,26 +134,6 @@ struct TilePlace {
     }
 };
 
-// two fp32 values per instruction, each half rounded like the scalar operation
-__device__ __forceinline__ uint64_t pack2(float a, float b) {
-    uint64_t v;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
-    return v;
-}
-__device__ __forceinline__ void unpack2(uint64_t v, float& a, float& b) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-
 // byte offset of 16-byte chunk `chunk` (0..7) of row `row` inside a [rows x 64 halves] swizzled atom
 __device__ __forceinline__ int swz(int row, int chunk) {
     return (row >> 3) * 1024 + (row & 7) * 128 + ((chunk ^ (row & 7)) << 4);
@@ -390,7 +370,7 @@ local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const 
         const uint32_t lane_addr = tmem + (static_cast<uint32_t>(quad * 32) << 16);
         constexpr float kLog2e = 1.4426950408889634f;
         const float scale2 = kSoftmaxScale * kLog2e;
-        const uint64_t scale22 = pack2(scale2, scale2);
+        const Pair scale22 = pair_of(scale2, scale2);
         // Bias terms: four lanes per operand row, 32 features each (32 * qt ..).  The eight lanes of a
         // 16-byte shared-memory access are four rows of one 64-feature atom: eight different chunks.
         const int qt = (lane & 1) | ((lane >> 2) & 2), bias_row = warp * 8 + (((lane >> 1) & 3) | ((lane >> 2) & 4));
@@ -556,9 +536,12 @@ local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const 
                     }
                     tmem_ld_wait();
 #pragma unroll
-                    for (int i = 0; i < 8; ++i)
-                        unpack2(mul2(add2(pack2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), pack2(s[2 * i], s[2 * i + 1])), scale22),
-                                s[2 * i], s[2 * i + 1]);
+                    for (int i = 0; i < 8; ++i) {
+                        const Pair sum2 = pair_add(pair_of(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), pair_of(s[2 * i], s[2 * i + 1]));
+                        const float2 scaled = halves_of(pair_mul(sum2, scale22));
+                        s[2 * i] = scaled.x;
+                        s[2 * i + 1] = scaled.y;
+                    }
                     if (!whole) {
                         const int off = kk0 + c0 - lo;
                         const bool some = hi >= lo;
@@ -582,7 +565,7 @@ local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const 
             ATT_WAIT(B_PASS0_DONE, par);
             mx = fmaxf(fmaxf(sm.rowmax[0][ql], sm.rowmax[1][ql]), fmaxf(sm.rowmax[2][ql], sm.rowmax[3][ql]));
             if (mx == -INFINITY) mx = 0.0f;            // a query without keys: every probability is 0
-            const uint64_t minus_mx2 = pack2(-mx, -mx);
+            const Pair minus_mx2 = pair_of(-mx, -mx);
             // Pass 1: probabilities, block by block, into the A operand of the last contraction.
 #pragma unroll 1
             for (int b = 0; b < 3; ++b) {
@@ -598,12 +581,11 @@ local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const 
                     tmem_ld_wait();
 #pragma unroll
                     for (int e = 0; e < 16; ++e) {
-                        float p0, p1;                                       // ex2(-inf) = 0
-                        unpack2(add2(pack2(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1])), minus_mx2), p0, p1);
-                        asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(p0));
-                        asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(p1));
-                        sum += p0 + p1;
-                        const __half2 h = __floats2half2_rn(p0, p1);
+                        float2 pr = halves_of(pair_add(pair_of(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1])), minus_mx2));
+                        asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(pr.x));     // ex2(-inf) = 0
+                        asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(pr.y));
+                        sum += pr.x + pr.y;
+                        const __half2 h = __floats2half2_rn(pr.x, pr.y);
                         w[e] = *reinterpret_cast<const uint32_t*>(&h);
                     }
                 }

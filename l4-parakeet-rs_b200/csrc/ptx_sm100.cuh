@@ -11,6 +11,38 @@
 
 namespace pk100 {
 
+// Two fp32 values in one 64-bit register; the packed instructions round each half like the scalar one.
+using Pair = unsigned long long;
+__device__ __forceinline__ Pair pair_of(float lo, float hi) {
+    Pair r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ Pair pair_of(__half2 h) {
+    const float2 f = __half22float2(h);
+    return pair_of(f.x, f.y);
+}
+__device__ __forceinline__ float2 halves_of(Pair v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ Pair pair_fma(Pair a, Pair b, Pair c) {
+    Pair d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ Pair pair_mul(Pair a, Pair b) {
+    Pair d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ Pair pair_add(Pair a, Pair b) {
+    Pair d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }

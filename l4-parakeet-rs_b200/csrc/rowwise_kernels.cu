@@ -527,33 +527,6 @@ __global__ void glu_masked_kernel(const __half* __restrict__ in, __half* __restr
 // fewer halo rows, short ones keep every SM busy: 16 rows where that gives the device two CTAs per SM,
 // else 8.  Bound by issue slots (convolution, BatchNorm, SiLU and E4M3 rounding of every element).  45 056
 // rows: 155 us with scalar instructions and full divisions, 91 us now; 768 rows: 10.6 -> 6.2 us.
-using Pair = unsigned long long;
-__device__ __forceinline__ Pair pair_of(float lo, float hi) {
-    Pair r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ float2 halves_of(Pair v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ Pair pair_fma(Pair a, Pair b, Pair c) {
-    Pair d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ Pair pair_mul(Pair a, Pair b) {
-    Pair d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ Pair pair_add(Pair a, Pair b) {
-    Pair d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-
 template <bool Quantize, int kStrip>
 __global__ void __launch_bounds__(256, 2)
 depthwise_bn_silu_kernel(const __half* __restrict__ in, const __half* __restrict__ wdw,

@@ -23,32 +23,10 @@ __device__ __forceinline__ int frames_of(const int* per_utt, int utt, int unifor
     return per_utt != nullptr ? per_utt[utt] : uniform;
 }
 
-// Two fp32 values handled by one packed instruction (fma.rn.f32x2: each half rounds like fmaf).
-using Pair = unsigned long long;
-__device__ __forceinline__ Pair make_pair(float lo, float hi) {
-    Pair r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ Pair fma_pair(Pair a, Pair b, Pair c) {
-    Pair d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ float2 split_pair(Pair v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ Pair half2_pair(__half2 h) {
-    const float2 f = __half22float2(h);
-    return make_pair(f.x, f.y);
-}
-
 // both halves rounded to fp16 and through ReLU; a NaN becomes 0 (max.f16x2 returns the operand that is a number,
 // the .relu form of the conversion would keep it)
 __device__ __forceinline__ __half2 relu_half2(Pair v) {
-    const float2 f = split_pair(v);
+    const float2 f = halves_of(v);
     return __hmax2(__floats2half2_rn(f.x, f.y), __half2half2(__ushort_as_half(0)));
 }
 
@@ -109,11 +87,11 @@ subsample_first_fused_kernel(const float* __restrict__ in, const __half* __restr
     }
     for (int i = tid; i < kChannels / 2 * 9; i += kFirstThreads) {
         const int pair = i / 9, tap = i % 9;
-        taps[0][tap][pair] = make_pair(__half2float(w0[pair * 18 + tap]), __half2float(w0[pair * 18 + 9 + tap]));
-        taps[1][tap][pair] = make_pair(__half2float(w1[pair * 18 + tap]), __half2float(w1[pair * 18 + 9 + tap]));
+        taps[0][tap][pair] = pair_of(__half2float(w0[pair * 18 + tap]), __half2float(w0[pair * 18 + 9 + tap]));
+        taps[1][tap][pair] = pair_of(__half2float(w1[pair * 18 + tap]), __half2float(w1[pair * 18 + 9 + tap]));
     }
-    const Pair bias0 = make_pair(__half2float(b0[ch]), __half2float(b0[ch + 1]));
-    const Pair bias1 = make_pair(__half2float(b1[ch]), __half2float(b1[ch + 1]));
+    const Pair bias0 = pair_of(__half2float(b0[ch]), __half2float(b0[ch + 1]));
+    const Pair bias1 = pair_of(__half2float(b1[ch]), __half2float(b1[ch + 1]));
     __syncthreads();
     // Nine taps as registers.  Reloaded per intermediate row and convolution (`volatile` keeps the
     // compiler from holding all 18 pairs across the loop, which spills the sums).
@@ -151,9 +129,9 @@ subsample_first_fused_kernel(const float* __restrict__ in, const __half* __restr
             Pair acc = bias0;
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
-                acc = fma_pair(*reinterpret_cast<const Pair*>(base[a] - 2), w[a * 3 + 0], acc);
-                acc = fma_pair(*reinterpret_cast<const Pair*>(base[a] - 1), w[a * 3 + 1], acc);
-                acc = fma_pair(c0[a], w[a * 3 + 2], acc);
+                acc = pair_fma(*reinterpret_cast<const Pair*>(base[a] - 2), w[a * 3 + 0], acc);
+                acc = pair_fma(*reinterpret_cast<const Pair*>(base[a] - 1), w[a * 3 + 1], acc);
+                acc = pair_fma(c0[a], w[a * 3 + 2], acc);
             }
             v[0] = relu_half2(acc);
         }
@@ -165,9 +143,9 @@ subsample_first_fused_kernel(const float* __restrict__ in, const __half* __restr
                 // columns 2*m1 + 1 and 2*m1 + 2: 16-byte aligned, because an even column sits at an odd index
                 const ulonglong2 nx = *reinterpret_cast<const ulonglong2*>(base[a] + 2 * m + 2);
                 // (column -1 is outside)
-                acc = fma_pair(c0[a], m == 0 && part == 0 ? 0ull : w[a * 3 + 0], acc);
-                acc = fma_pair(c1[a], w[a * 3 + 1], acc);
-                acc = fma_pair(nx.x, w[a * 3 + 2], acc);
+                acc = pair_fma(c0[a], m == 0 && part == 0 ? 0ull : w[a * 3 + 0], acc);
+                acc = pair_fma(c1[a], w[a * 3 + 1], acc);
+                acc = pair_fma(nx.x, w[a * 3 + 2], acc);
                 c0[a] = nx.x;
                 c1[a] = nx.y;
             }
@@ -176,13 +154,13 @@ subsample_first_fused_kernel(const float* __restrict__ in, const __half* __restr
     };
     // output m2 takes features 2*m2 - 1, 2*m2, 2*m2 + 1 as taps 0, 1, 2
     auto scatter = [&](Pair (&sums)[kFirstOuts], const Pair (&w)[9], int kf, const __half2 (&v)[2 * kFirstOuts + 1]) {
-        Pair left = half2_pair(v[0]);
+        Pair left = pair_of(v[0]);
 #pragma unroll
         for (int m = 0; m < kFirstOuts; ++m) {
-            if (m > 0 || part > 0) sums[m] = fma_pair(left, w[kf * 3 + 0], sums[m]);
-            sums[m] = fma_pair(half2_pair(v[2 * m + 1]), w[kf * 3 + 1], sums[m]);
-            left = half2_pair(v[2 * m + 2]);
-            sums[m] = fma_pair(left, w[kf * 3 + 2], sums[m]);
+            if (m > 0 || part > 0) sums[m] = pair_fma(left, w[kf * 3 + 0], sums[m]);
+            sums[m] = pair_fma(pair_of(v[2 * m + 1]), w[kf * 3 + 1], sums[m]);
+            left = pair_of(v[2 * m + 2]);
+            sums[m] = pair_fma(left, w[kf * 3 + 2], sums[m]);
         }
     };
 
@@ -222,7 +200,7 @@ subsample_first_fused_kernel(const float* __restrict__ in, const __half* __restr
             __half2 h[kFirstOuts];
 #pragma unroll
             for (int m = 0; m < kFirstOuts; ++m) {
-                const float2 f = split_pair(cur[m]);
+                const float2 f = halves_of(cur[m]);
                 h[m] = __floats2half2_rn(f.x, f.y);
                 const float2 r = __half22float2(__habs2(h[m]));
                 // non-negative floats order like their bits
@@ -251,7 +229,7 @@ subsample_first_fused_kernel(const float* __restrict__ in, const __half* __restr
             __half* dst = static_cast<__half*>(out) + row0 * kChannels + ch;
 #pragma unroll
             for (int m = 0; m < kFirstOuts; ++m) {
-                const float2 f = split_pair(cur[m]);
+                const float2 f = halves_of(cur[m]);
                 *reinterpret_cast<__half2*>(dst + static_cast<size_t>(m) * kChannels) = __floats2half2_rn(f.x, f.y);
             }
         }
@@ -302,7 +280,7 @@ subsample_depthwise_kernel(const __half* __restrict__ in, const __half* __restri
 #pragma unroll
     for (int g = 0; g < kDepthwiseRun; ++g)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) sums[g][c] = half2_pair(reinterpret_cast<const __half2*>(bias)[c]);
+        for (int c = 0; c < 4; ++c) sums[g][c] = pair_of(reinterpret_cast<const __half2*>(bias)[c]);
     const __half* src = in + static_cast<size_t>(utt) * in_cap * in_feats * kChannels + ch;
     constexpr int kCols = 2 * kDepthwiseRun + 1;
 #pragma unroll
@@ -322,7 +300,7 @@ subsample_depthwise_kernel(const __half* __restrict__ in, const __half* __restri
         for (int kt = 0; kt < 3; ++kt)
 #pragma unroll
             for (int c = 0; c < 4; ++c)
-                tap[kt][c] = make_pair(__half2float(taps[(2 * c) * 9 + kf * 3 + kt]), __half2float(taps[(2 * c + 1) * 9 + kf * 3 + kt]));
+                tap[kt][c] = pair_of(__half2float(taps[(2 * c) * 9 + kf * 3 + kt]), __half2float(taps[(2 * c + 1) * 9 + kf * 3 + kt]));
 #pragma unroll
         for (int j = 0; j < kCols; ++j) {
             const __half2* h = reinterpret_cast<const __half2*>(&col[j]);
@@ -330,11 +308,11 @@ subsample_depthwise_kernel(const __half* __restrict__ in, const __half* __restri
             if (t < 0 || t >= in_feats) continue;
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-                const Pair v = half2_pair(h[c]);
+                const Pair v = pair_of(h[c]);
                 // column j is tap j - 2 g of output g
 #pragma unroll
                 for (int g = 0; g < kDepthwiseRun; ++g)
-                    if (j - 2 * g >= 0 && j - 2 * g < 3) sums[g][c] = fma_pair(v, tap[j - 2 * g][c], sums[g][c]);
+                    if (j - 2 * g >= 0 && j - 2 * g < 3) sums[g][c] = pair_fma(v, tap[j - 2 * g][c], sums[g][c]);
             }
         }
     }
@@ -346,7 +324,7 @@ subsample_depthwise_kernel(const __half* __restrict__ in, const __half* __restri
         __half2* h = reinterpret_cast<__half2*>(&raw);
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            const float2 f = split_pair(sums[g][c]);
+            const float2 f = halves_of(sums[g][c]);
             h[c] = __floats2half2_rn(f.x, f.y);
         }
         *reinterpret_cast<uint4*>(dst + static_cast<size_t>(g) * kChannels) = raw;
