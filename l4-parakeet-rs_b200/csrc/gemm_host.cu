@@ -349,8 +349,9 @@ int pk100_gemm_chained(void* stream_v, const pk100_gemm_args* a, bool b_settled)
     // 64-column tiles where they still fit one wave: such a launch is bound by the round trips of its operand
     // ring (1.7 us each, the weights come from DRAM), and eight 24 KB stages hold a K of 1024 bytes whole where
     // the 128-column tile has five stages, for twice the CTAs and half the epilogue.  Encoder of a 4 s request
-    // (128 rows, 24 layers, GLU rule below included) 340 us shorter, of a 60 s one (768 rows) 210 us; FF contract
-    // with a 30 % live K at 128 .. 1024 rows 14.0 -> 12.6 us per call.
+    // (128 rows, 24 layers, GLU rule below included) 340 us shorter, of a 60 s one (768 rows) 210 us; back to back,
+    // 128-column tiles against these: FF contract with a 30 % live K 13.8 / 12.2 us at 128 rows, 12.9 / 11.0 at 512,
+    // 13.6 / 12.1 at 1024; K = 1024 INT8 6.4 / 5.8, 6.6 / 5.9, 6.8 / 6.1.
     const bool tiny = a->n % 64 == 0 && static_cast<long long>(m_tiles) * (a->n / 64) <= cta_budget(*a);
     bool narrow = a->n % 256 != 0;
     if (!narrow) {

@@ -334,8 +334,9 @@ class PipelineEngine:
         tokens only when its buffers are needed again or the newest batch has been queued.  Steady
         state per batch: the larger of the (slowed) encode and the decoder-cluster time of a batch
         divided by the clusters in flight, instead of encode + longest chain.  Measured for batches of
-        8 x 60 s: one lockstep cluster per batch and four batches in flight (the defaults) give 11.5 ms
-        per batch; four clusters per batch and two batches in flight 19.9 ms; a batch on its own 34.4 ms."""
+        8 x 60 s: one lockstep cluster per batch and four batches in flight (the defaults) give 10.8 ms per
+        batch, two clusters and three batches 12.8 ms, four clusters and two batches 16.4 ms; the same
+        batch on its own takes 30.7 ms."""
         depth = max(2, int(depth))
         if not hasattr(self, "_extra_slots"):
             self._extra_slots, self._collect_streams, self._slot_status = [], [], []
@@ -360,8 +361,8 @@ class PipelineEngine:
             return [b.tokens_host[u, :int(counts[u])].numpy().copy() for u in range(utterances)]
 
         # The last batch of a sequence of known length has nothing behind it to leave SMs for: it is decoded on
-        # all clusters that the batches in flight do not hold (6 batches of 8 x 60 s: 1.20 -> 1.34 times the rate
-        # of the code before the persistent attention kernel, measured beside it).
+        # all clusters that the batches in flight do not hold (6 batches of 8 x 60 s as a list 82.5 ms, as an
+        # iterator, which has no last batch, 91.5 ms).
         try:
             last = len(batches) - 1
         except (TypeError, NotImplementedError):          # (no length, or an iterable that does not know it)
