@@ -1415,18 +1415,27 @@ namespace {
 
 // Can this device run a 16-CTA cluster of the cluster decoder?  Asked once per device and
 // kernel variant (one or two LSTM layers).
-// Calls f with the kernel for (layers, numerics, utterances of the call) its threads and its shared-memory bytes.
+// Calls f with the kernel for (layers, numerics, utterances of the call) and its threads and its shared-memory bytes.
 template <typename F>
 auto with_cluster_kernel(int layers, bool cache, int utterances, F&& f) {
 #define PK_PICK(L, C, N) return f(tdt_cluster_kernel<L, C, N>, cl_threads(N), static_cast<int>(sizeof(CSmem<L, C, N>)))
+// (two utterances: the form for up to two with two layers, the one for up to four with one: us per round 6.7 against 6.9
+// and 7.1 against 7.1 for the two-layer numerics, 5.7 against 5.4 and 3.7 against 3.5 for the one-layer ones)
+#define PK_SIZES(L, C)                                           \
+    do {                                                         \
+        if (utterances <= 1) PK_PICK(L, C, 1);                   \
+        if constexpr (L == 2)                                    \
+            if (utterances <= 2) PK_PICK(L, C, 2);               \
+        if (utterances <= 4) PK_PICK(L, C, 4);                   \
+        PK_PICK(L, C, 8);                                        \
+    } while (0)
     if (layers == 1) {
-        if (cache) { if (utterances <= 4) PK_PICK(1, true, 4); PK_PICK(1, true, 8); }
-        if (utterances <= 4) PK_PICK(1, false, 4);
-        PK_PICK(1, false, 8);
+        if (cache) PK_SIZES(1, true);
+        PK_SIZES(1, false);
     }
-    if (cache) { if (utterances <= 4) PK_PICK(2, true, 4); PK_PICK(2, true, 8); }
-    if (utterances <= 4) PK_PICK(2, false, 4);
-    PK_PICK(2, false, 8);
+    if (cache) PK_SIZES(2, true);
+    PK_SIZES(2, false);
+#undef PK_SIZES
 #undef PK_PICK
 }
 
@@ -1447,10 +1456,10 @@ cudaLaunchConfig_t cluster_config(cudaLaunchAttribute& attr, int threads, int sm
 
 // Can the current device host this variant?  Sets the kernel's attributes on the first call per device.
 bool cluster_decoder_available_for(int layers, bool cache, int utterances = 1, int* capacity = nullptr) {
-    static std::atomic<int> known[64][8];      // 0 = unknown, else 1 + clusters the device holds at once
+    static std::atomic<int> known[64][16];     // 0 = unknown, else 1 + clusters the device holds at once
     int dev = 0;
     if (layers < 1 || layers > 2 || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
-    std::atomic<int>& slot = known[dev][(layers - 1) * 4 + (cache ? 2 : 0) + (utterances > 4 ? 1 : 0)];
+    std::atomic<int>& slot = known[dev][(layers - 1) * 8 + (cache ? 4 : 0) + (utterances > 1) + (utterances > 2) + (utterances > 4)];
     if (slot.load() == 0) {
         const int clusters = with_cluster_kernel(layers, cache, utterances, [&](auto kernel, int threads, int smem) {
             int max_smem = 0, n = 0;
