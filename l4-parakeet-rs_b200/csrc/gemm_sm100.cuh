@@ -57,6 +57,9 @@ struct GemmParams {
     // Bytes of one output row in a warp's 32-row slice when the slices leave through shared
     // memory and a TMA store (64 or 128); 0 = each thread stores its row piece directly.
     int store_row_bytes;
+    // Order of the work items: the column tiles of a row tile follow each other (A is read from HBM once, B stays
+    // in L2), or the row tiles of a column tile (B is fetched piece by piece).
+    int n_inner;
     // B was complete before the chain of dependent launches began: the first stages of the weights are
     // requested before the wait for the kernel in front.
     int b_settled;
@@ -357,8 +360,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         }
         const int tile = worker + i * workers;
         if (tile >= num_tiles) return false;
-        mg = tile % m_groups;
-        nt = tile / m_groups;
+        const int inner = p.n_inner != 0 ? n_tiles : m_groups;
+        const int outer_i = tile / inner, inner_i = tile - outer_i * inner;
+        mg = p.n_inner != 0 ? outer_i : inner_i;
+        nt = p.n_inner != 0 ? inner_i : outer_i;
         return true;
     };
 
