@@ -121,6 +121,12 @@ static int make_out_map(CUtensorMap* map, const GemmParams& p) {
     return row_bytes;
 }
 
+// Tensor map of the residual with the boxes of the output slices (fp16 output leaving by TMA stores).
+static int make_residual_map(CUtensorMap* map, const GemmParams& p) {
+    if (p.residual == nullptr || p.store_row_bytes == 0 || p.out_type != OUT_F16) return 0;
+    return make_map(map, p.residual, 2, p.m, p.n, p.ld_res, 32, p.store_row_bytes) == PK100_OK ? 1 : 0;
+}
+
 static int sm_count() {
     static int count = 0;
     if (count == 0) {
@@ -174,6 +180,8 @@ static int launch_pair(const pk100_gemm_args& a, const GemmParams& p_in, cudaStr
     if (rc != PK100_OK) return rc;
     CUtensorMap map_out = map_a;
     p.store_row_bytes = make_out_map<Epi>(&map_out, p);
+    CUtensorMap map_res = map_a;
+    p.res_tma = make_residual_map(&map_res, p);
     const int m_groups = (a.m + 2 * kBlockM - 1) / (2 * kBlockM);
     const int n_tiles = (p.n + BlockN - 1) / BlockN;
     int pairs = cta_budget(a) / 2;
@@ -191,7 +199,7 @@ static int launch_pair(const pk100_gemm_args& a, const GemmParams& p_in, cudaStr
     attr.val.clusterDim.z = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, map_a, map_b, map_out, p);
+    const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, map_a, map_b, map_out, map_res, p);
     if (err != cudaSuccess) {
         cudaGetLastError();
         return static_cast<int>(err);
@@ -223,11 +231,13 @@ static int launch(const pk100_gemm_args& a, const GemmParams& p_in, cudaStream_t
     if (rc != PK100_OK) return rc;
     CUtensorMap map_out = map_a;
     if constexpr (gemm_store_bytes<Epi, BSRC_TMA, BlockN>() > 0) p.store_row_bytes = make_out_map<Epi, BlockN>(&map_out, p);
+    CUtensorMap map_res = map_a;
+    p.res_tma = make_residual_map(&map_res, p);
     const int m_tiles = (a.m + kBlockM - 1) / kBlockM;
     const int n_tiles = (p.n + BlockN - 1) / BlockN;
     int ctas = cta_budget(a);
     if (ctas > m_tiles * n_tiles) ctas = m_tiles * n_tiles;
-    pk100_launch_chained(kernel, dim3(ctas), dim3(GemmWarps<BSRC_TMA>::kThreads), Smem::kTotal, stream, map_a, map_b, map_out, p);
+    pk100_launch_chained(kernel, dim3(ctas), dim3(GemmWarps<BSRC_TMA>::kThreads), Smem::kTotal, stream, map_a, map_b, map_out, map_res, p);
     return pk100_launch_status();
 }
 
@@ -252,7 +262,7 @@ static int launch_w4(const pk100_gemm_args& a, const GemmParams& p, cudaStream_t
     int ctas = cta_budget(a);
     if (ctas > m_items * n_tiles) ctas = m_items * n_tiles;
     // neither B nor the output has a tensor map
-    pk100_launch_chained(kernel, dim3(ctas), dim3(GemmWarps<BSRC_W4G128>::kThreads), Smem::kTotal, stream, map_a, map_a, map_a, p);
+    pk100_launch_chained(kernel, dim3(ctas), dim3(GemmWarps<BSRC_W4G128>::kThreads), Smem::kTotal, stream, map_a, map_a, map_a, map_a, p);
     return pk100_launch_status();
 }
 

@@ -16,6 +16,8 @@
 
 #include <cuda_fp8.h>
 
+#include <type_traits>
+
 #include "ptx_sm100.cuh"
 
 namespace pk100 {
@@ -60,6 +62,9 @@ struct GemmParams {
     // Order of the work items: the column tiles of a row tile follow each other (A is read from HBM once, B stays
     // in L2), or the row tiles of a column tile (B is fetched piece by piece).
     int n_inner;
+    // The residual has a tensor map with the boxes of the output slices: it arrives by TMA in the slice that the
+    // output then leaves from (needs store_row_bytes and fp16 output).
+    int res_tma;
     // B was complete before the chain of dependent launches began: the first stages of the weights are
     // requested before the wait for the kernel in front.
     int b_settled;
@@ -81,8 +86,7 @@ struct GemmWarps {
 };
 
 // Shared memory the epilogue warps stage their output slices in for the TMA store: 32 rows of
-// up to 128 bytes per warp (64 bytes for the INT8 sparse-out tiles).  Only the 256-column TMA
-// kernels use it.
+// up to 128 bytes per warp (64 bytes for the INT8 sparse-out tiles).  The 64-column and the INT4 kernels have none.
 template <int Epi, int BSrc, int BlockN>
 constexpr int gemm_store_bytes() {
     if (BSrc != BSRC_TMA) return 0;
@@ -282,7 +286,7 @@ __device__ __forceinline__ int live_k_blocks(uint64_t mask) {
 template <int Kind, int BlockN, int SwizzleBytes, int Epi, int BSrc, int CtaGroup = 1>
 __global__ void __launch_bounds__(GemmWarps<BSrc>::kThreads, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-            const __grid_constant__ CUtensorMap map_out,
+            const __grid_constant__ CUtensorMap map_out, const __grid_constant__ CUtensorMap map_res,
             const GemmParams p) {
     static_assert(CtaGroup == 1 || (CtaGroup == 2 && BlockN == 256 && BSrc == BSRC_TMA), "pairs: 256 columns, TMA");
     constexpr int kBRows = BlockN / CtaGroup;               // B rows staged by this CTA
@@ -315,6 +319,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     uint64_t* empty_bar = full_bar + kStages;
     uint64_t* tmem_full_bar = empty_bar + kStages;
     uint64_t* tmem_empty_bar = tmem_full_bar + 2;
+    uint64_t* res_bar = tmem_empty_bar + 2;                   // one per epilogue warp
+    static_assert(2 * kStages + 4 + GemmWarps<BSrc>::kEpilogue <= 64, "barriers fit their area");
     uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(tail + 64 * 8);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tail + 64 * 8 + 8);
     float* s_cols = reinterpret_cast<float*>(tail + 64 * 8 + 16);   // per-warp scale / bias slices
@@ -379,6 +385,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
             mbar_init(tmem_full_bar + b, 1);
             mbar_init(tmem_empty_bar + b, kEpiWarps * CtaGroup);
         }
+        for (int i = 0; i < GemmWarps<BSrc>::kEpilogue; ++i) mbar_init(res_bar + i, 1);
         fence_barrier_init();
         prefetch_tensormap(&map_a);
         if constexpr (BSrc == BSRC_TMA) prefetch_tensormap(&map_b);
@@ -689,6 +696,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         if (work_item(0, mg, nt)) prefetch_cols(nt);
         int local = 0;
         bool ok = true;
+        // Output slice of this warp (32 rows x kColsPerWarp columns): staged in shared memory and written by one TMA
+        // store when the host set that up, else stored per thread.  The residual comes the same way, requested before
+        // the wait for the accumulator (per thread it would be one 16-byte request per lane, 2 KB apart: us at 6144
+        // rows so / by TMA: FF contract 25.0 / 23.1, fp16 output projection 21.8 / 20.1, pointwise-2 16.9 / 14.6).
+        const bool staged = Smem::kStoreBytes > 0 && p.store_row_bytes != 0;
+        const bool res_tma = Epi == EPI_LINEAR && staged && p.res_tma != 0;
         for (; ok && work_item(local, mg, nt); ++local) {
             const int mt = (mg * CtaGroup + static_cast<int>(rank)) * kMTiles + sub;   // this warp's 128-row tile
             const int buf = local & 1;
@@ -733,9 +746,31 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
             constexpr int kAhead = kPieces < 2 ? kPieces : 2;
             [[maybe_unused]] uint4 res_pre[kAhead][2];
             const bool has_residual = Epi == EPI_LINEAR && p.residual != nullptr;
+            uint8_t* const stage = store_smem + ew * (Smem::kStoreBytes / kEpiWarps);
+            // first column and row of the warp's slice; false: outside the matrix
+            auto slice_at = [&](int& col0, int& row0) {
+                col0 = n0 + part * kColsPerWarp;
+                row0 = mt * kBlockM + quad * 32;
+                return row0 < p.m && col0 < (Epi == EPI_GLU ? p.n / 2 : p.n);
+            };
+            if (staged) {
+                if (lane == 0) {
+                    bulk_wait_read_all();          // the previous tile's store has read the slice
+                    if (res_tma) {
+                        int col0, row0;
+                        if (slice_at(col0, row0)) {
+                            mbar_arrive_expect_tx(res_bar + ew, 32 * p.store_row_bytes);
+                            tma_load_2d(stage, &map_res, res_bar + ew, col0, row0);
+                        } else {
+                            mbar_arrive(res_bar + ew);
+                        }
+                    }
+                }
+                __syncwarp();
+            }
             auto fetch_residual = [&](uint4 (&dst)[2], int c) {
                 const int col = n0 + part * kColsPerWarp + c * 16;
-                if (has_residual && row < p.m && col < p.n) {
+                if (has_residual && !res_tma && row < p.m && col < p.n) {
                     const uint4* rp = reinterpret_cast<const uint4*>(
                         p.residual + static_cast<size_t>(row) * p.ld_res + col);
                     dst[0] = rp[0];
@@ -759,17 +794,19 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
             const size_t obytes = out_elem_bytes(p.out_type);
 
             const bool zero_row = row >= p.valid_rows;
-            // Output slice of this warp (32 rows x kColsPerWarp columns): staged in shared memory
-            // and written by one TMA store when the host set that up, else stored per thread.
-            const bool staged = Smem::kStoreBytes > 0 && p.store_row_bytes != 0;
-            uint8_t* stage = store_smem + ew * (Smem::kStoreBytes / kEpiWarps);
-            uint8_t* stage_row = stage + lane * p.store_row_bytes;
+            uint8_t* const stage_row = stage + lane * p.store_row_bytes;
             const int swz = p.store_row_bytes == 128 ? (lane & 7) : ((lane >> 1) & 3);
-            if (staged) {
-                if (lane == 0) bulk_wait_read_all();   // the previous tile's store has read the slice
-                __syncwarp();
+            if (res_tma) {
+                const bool here = mbar_wait_bounded(res_bar + ew, local & 1, abort_flag);
+                if (!__all_sync(0xffffffffu, here)) {
+                    ok = false;
+                    break;
+                }
             }
             if constexpr (Epi == EPI_LINEAR) {
+                // from_slice: the residual comes from the staging slice
+                auto walk = [&](auto from_slice) {
+                constexpr bool kFromSlice = decltype(from_slice)::value;
 #pragma unroll 1
                 for (int cg = 0; cg < kPieces; cg += kAhead) {
 #pragma unroll
@@ -785,8 +822,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                         // piece, outside the element loops: left inside, every element pays for the
                         // predicated-off SiLU and residual code (22 instructions per element measured).
                         float v[16];
-                        const uint4 res_raw[2] = {res_pre[ci][0], res_pre[ci][1]};
-                        if (c + kAhead < kPieces) fetch_residual(res_pre[ci], c + kAhead);
+                        uint4 res_raw[2];
+                        if constexpr (kFromSlice) {
+                            res_raw[0] = *reinterpret_cast<const uint4*>(stage_row + (((2 * c) ^ swz) << 4));
+                            res_raw[1] = *reinterpret_cast<const uint4*>(stage_row + (((2 * c + 1) ^ swz) << 4));
+                        } else {
+                            res_raw[0] = res_pre[ci][0];
+                            res_raw[1] = res_pre[ci][1];
+                            if (c + kAhead < kPieces) fetch_residual(res_pre[ci], c + kAhead);
+                        }
                         const float rs_live = live ? rs : 0.0f;
                         if (!live) {              // accumulator never written: any bit pattern
 #pragma unroll
@@ -808,7 +852,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
 #pragma unroll
                             for (int j = 0; j < 16; ++j) v[j] = fmaxf(v[j], 0.0f);
                         }
-                        if (has_residual) {
+                        if (kFromSlice || has_residual) {
                             const __half2* res_h = reinterpret_cast<const __half2*>(res_raw);
 #pragma unroll
                             for (int j = 0; j < 16; j += 2) {
@@ -824,7 +868,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
 #pragma unroll
                             for (int j = 0; j < 16; ++j) v[j] = 0.0f;
                         }
-                        if (staged) {
+                        if (kFromSlice || staged) {
                             stage_piece(stage_row, c, swz, p.out_type, p.out_scale, v);
                         } else {
                             uint8_t* out_row = reinterpret_cast<uint8_t*>(p.out) +
@@ -834,6 +878,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                     }
                 }
                 }
+                };
+                if (Smem::kStoreBytes > 0 && res_tma) walk(std::true_type{});
+                else walk(std::false_type{});
             } else if constexpr (Epi == EPI_GLU) {
                 // accumulator columns [0, BlockN/2) hold values, [BlockN/2, BlockN) their gates
 #pragma unroll 1
@@ -946,9 +993,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                 // generic-proxy writes of the slice -> visible to the TMA engine
                 fence_proxy_async_smem();
                 __syncwarp();
-                const int col0 = n0 + part * kColsPerWarp;
-                const int row0 = mt * kBlockM + quad * 32;
-                if (lane == 0 && row0 < p.m && col0 < (Epi == EPI_GLU ? p.n / 2 : p.n)) {
+                int col0, row0;
+                if (lane == 0 && slice_at(col0, row0)) {
                     tma_store_2d(&map_out, stage, col0, row0);
                     bulk_commit_group();
                 }

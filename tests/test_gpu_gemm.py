@@ -433,3 +433,41 @@ def test_one_wave_tiles_give_the_bits_of_wide_tiles(pk, cuda, kind, m, n, k):
             pk.ops.gemm(a, b, out=out, status=st, max_ctas=ctas, **form, **kw)
         assert int(st.item()) == 0
         assert torch.equal(outs[0].view(torch.uint8), outs[1].view(torch.uint8)), form
+
+
+@pytest.mark.parametrize("kind", ["f16", "e4m3", "s8", "w4"])
+@pytest.mark.parametrize("m,n,k,ld_res,in_place", [(1, 32, 128, 40, False), (127, 96, 256, 96, True), (129, 160, 128, 168, False),
+                                                   (300, 1024, 1024, 1024, True), (6272, 1024, 256, 1032, False), (20000, 256, 128, 256, True)])
+def test_residual_slices_give_the_bits_of_a_separate_sum(pk, cuda, kind, m, n, k, ld_res, in_place):
+    """fp16 output with a residual: the residual's slices come by TMA where the output leaves that way.  The same
+    product as fp32 without it gives v; f16(fma(alpha, v, r)) has to be the result bit for bit (alpha is a power of
+    two, so the fp64 sum below is rounded to fp32 once, like the fused one).  Ragged rows and columns, distances
+    of the residual's rows beyond its width, in place and not."""
+    L = pk.lib
+    g = torch.Generator().manual_seed(m + n)
+    w = (torch.randn((n, k), generator=g) * 0.05).half().to(cuda)
+    x = torch.randn((m, k), generator=g).half().to(cuda)
+    kw = {}
+    if kind == "f16":
+        a, b, kid = x, w, L.KIND_F16
+    elif kind == "w4":
+        b, kw["b_group_scales"] = pk.ops.pack_weight_rows(w, L.PACK_S4_G128)
+        a, kid = x, L.KIND_F16_W4G128
+    else:
+        code = L.PACK_S8 if kind == "s8" else L.PACK_E4M3
+        b, kw["col_scales"] = pk.ops.pack_weight_rows(w, code)
+        a, kw["row_scales"] = pk.ops.pack_weight_rows(x, code)
+        kid = L.KIND_S8 if kind == "s8" else L.KIND_E4M3
+    st = _status(cuda)
+    v = torch.empty((m, n), dtype=torch.float32, device=cuda)
+    pk.ops.gemm(a, b, kind=kid, out=v, out_type=L.OUT_F32, status=st, n=n, **kw)
+    res = torch.randn((m, ld_res), generator=g).half().to(cuda)
+    before = res.clone()
+    out = res if in_place else torch.full((m + 1, n), 7.0, dtype=torch.float16, device=cuda)
+    pk.ops.gemm(a, b, kind=kid, out=out[:m, :n], residual=res[:, :n], alpha=0.5, status=st, n=n, **kw)
+    torch.cuda.synchronize()
+    assert int(st.item()) == 0
+    want = (0.5 * v.double() + before[:, :n].double()).float().half()
+    assert torch.equal(out[:m, :n], want)
+    if not in_place:
+        assert bool((out[m] == 7.0).all())
