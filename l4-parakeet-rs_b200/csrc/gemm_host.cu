@@ -412,7 +412,14 @@ int pk100_gemm_chained(void* stream_v, const pk100_gemm_args* a, bool b_settled)
         return PK100_ERR_UNSUPPORTED;
     }
     case PK100_EPI_SPARSE_OUT:
-        if (a->kind == PK100_KIND_E4M3) return launch<KIND_F8, 256, 128, EPI_SPARSE_OUT>(*a, p, stream);
+        if (a->kind == PK100_KIND_E4M3) {
+            // narrower tiles where they still fit one wave, as above: 8.1 -> 6.4 us at 128 and 256 rows (64 columns
+            // each), 8.2 -> 7.3 at 512 (128)
+            if (static_cast<long long>(m_tiles) * (a->n / 64) <= cta_budget(*a)) return launch<KIND_F8, 64, 128, EPI_SPARSE_OUT>(*a, p, stream);
+            if (a->n % 128 == 0 && static_cast<long long>(m_tiles) * (a->n / 128) <= cta_budget(*a))
+                return launch<KIND_F8, 128, 128, EPI_SPARSE_OUT>(*a, p, stream);
+            return launch<KIND_F8, 256, 128, EPI_SPARSE_OUT>(*a, p, stream);
+        }
         if (a->kind == PK100_KIND_F16) return launch<KIND_F16, 256, 128, EPI_SPARSE_OUT>(*a, p, stream);
         return PK100_ERR_UNSUPPORTED;
     default:

@@ -912,13 +912,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                 }
             } else {
                 // EPI_SPARSE_OUT: SiLU, per-(128 x 64) tile max|a| against tau, INT8 store.
-                // Each epilogue warp owns one 64-column sparsity tile of its 32 rows.  Kept lean
+                // Each epilogue warp owns one 64-column sparsity tile of its 32 rows, or the half or quarter of one
+                // (128- and 64-column tiles).  Kept lean
                 // (about 8 instructions per element) because with K = 1024 the MMAs of a tile take
                 // only ~4k cycles: SiLU(x) = x/2 * (1 + tanh(x/2)) costs one MUFU (tanh.approx),
                 // the x32 of the INT8 encoding is folded into the same FMA, the codes are produced
                 // in the first pass and held packed (16 registers).
-                static_assert(Epi != EPI_SPARSE_OUT || (BlockN == 256 && kColsPerWarp == 64),
-                              "sparse-out: 256-column tiles, one 64-column tile per warp");
+                static_assert(Epi != EPI_SPARSE_OUT || (kColsPerWarp <= 64 && 64 % kColsPerWarp == 0), "sparse-out: whole parts of one tile");
+                constexpr int kTileParts = 64 / kColsPerWarp;   // column slices that share a sparsity tile
+                const int group = part / kTileParts;
                 uint32_t q[kPieces][4];                       // INT8 codes, 4 per register
                 float tile_max = 0.0f;                        // max |a * out_scale|
                 // a * out_scale = s * (1 + tanh(h)) with s = x/2 * out_scale and h = x/2; rows that
@@ -957,20 +959,20 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                 // (double-buffered by tile parity: a warp can be a whole tile ahead of its peers)
                 float* red = s_reduce + (local & 1) * kEpiWarps;
                 if (lane == 0) red[ew] = tile_max;
-                // the four warps (one per lane quadrant) that share this 64-column tile
-                asm volatile("bar.sync %0, 128;" ::"r"(2 + part) : "memory");
+                // the warps (four lane quadrants of each slice) that share this 64-column tile
+                asm volatile("bar.sync %0, %1;" ::"r"(2 + group), "n"(128 * kTileParts) : "memory");
                 const int n_tiles64 = p.n / 64;
                 float mx = 0.0f;
 #pragma unroll
-                for (int qd = 0; qd < 4; ++qd) mx = fmaxf(mx, red[part * 4 + qd]);
+                for (int i = 0; i < 4 * kTileParts; ++i) mx = fmaxf(mx, red[group * 4 * kTileParts + i]);
                 mx *= 1.0f / p.out_scale;                       // statistic in activation units
                 const bool keep = mx >= p.tau;
                 // a kept tile whose largest |a * out_scale| exceeds 127 lost information to the clamp:
                 // reported as status bit 3 (value 8), nothing else changes
-                if (keep && mx * p.out_scale > 127.0f && quad == 0 && lane == 0 && p.status != nullptr)
-                    atomicOr(p.status, 8);
-                const int tile64 = n0 / 64 + part;
-                if (quad == 0 && lane == 0 && tile64 < n_tiles64 && mt < m_tiles) {
+                const bool reports = quad == 0 && lane == 0 && part % kTileParts == 0;
+                if (keep && mx * p.out_scale > 127.0f && reports && p.status != nullptr) atomicOr(p.status, 8);
+                const int tile64 = n0 / 64 + group;
+                if (reports && tile64 < n_tiles64 && mt < m_tiles) {
                     p.keep_out[static_cast<size_t>(mt) * n_tiles64 + tile64] = keep ? 1 : 0;
                     if (p.stats_out != nullptr)
                         p.stats_out[static_cast<size_t>(mt) * n_tiles64 + tile64] = mx;

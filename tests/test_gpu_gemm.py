@@ -471,3 +471,27 @@ def test_residual_slices_give_the_bits_of_a_separate_sum(pk, cuda, kind, m, n, k
     assert torch.equal(out[:m, :n], want)
     if not in_place:
         assert bool((out[m] == 7.0).all())
+
+
+@pytest.mark.parametrize("rows", [1, 128, 130, 256, 257, 300, 512])
+def test_sparse_out_narrow_tiles_give_the_bits_of_wide_tiles(pk, cuda, rows):
+    """Sparse-out launches that fit one wave take 64- or 128-column tiles: codes, flags, statistics and the clamp
+    report are those of 256-column tiles (which a cap on the CTAs forces)."""
+    L = pk.lib
+    g = torch.Generator().manual_seed(rows)
+    q8 = torch.randint(0, 120, (rows, 1024), generator=g, dtype=torch.uint8).to(cuda)
+    b, scales = pk.ops.pack_weight_rows((torch.randn((4096, 1024), generator=g) * 0.02).half().to(cuda), L.PACK_E4M3)
+    tiles = (rows + 127) // 128
+    results = []
+    for ctas in (0, 4):
+        out = torch.full((rows, 4096), 55, dtype=torch.int8, device=cuda)
+        keep = torch.full((tiles, 64), 9, dtype=torch.uint8, device=cuda)
+        stats = torch.full((tiles, 64), -1.0, device=cuda)
+        st = _status(cuda)
+        pk.ops.gemm(q8, b, kind=L.KIND_E4M3, epilogue=L.EPI_SPARSE_OUT, row_scale=0.02, col_scales=scales, out=out,
+                    out_type=L.OUT_S8, out_scale=32.0, tau=2.0, keep_out=keep, stats_out=stats, status=st, max_ctas=ctas)
+        torch.cuda.synchronize()
+        results.append((out, keep, stats, int(st.item())))
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+    assert torch.equal(results[0][2], results[1][2]) and results[0][3] == results[1][3]
+    assert 0 < int(results[0][1].sum()) <= tiles * 64
