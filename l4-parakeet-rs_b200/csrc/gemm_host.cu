@@ -105,16 +105,16 @@ static int encode_map(CUtensorMap* map, const void* base, int elem_bytes, uint64
 }
 
 // Tensor map of the output for the staged TMA store (256-column kernels, 128-column linear kernels): every epilogue
-// warp owns 32 rows x (tile columns / 4).  Only slices with 64- or 128-byte rows leave that way
+// warp owns 32 rows x (tile columns / 4); INT4 weights: 32 rows x 64 columns at a time.  Only slices with 64- or 128-byte rows leave that way
 // (their swizzle modes); anything else keeps per-thread stores.  Returns the row bytes or 0.
-template <int Epi, int BlockN = 256>
+template <int Epi, int BlockN = 256, int BSrc = BSRC_TMA>
 static int make_out_map(CUtensorMap* map, const GemmParams& p) {
     const int out_cols = Epi == EPI_GLU ? p.n / 2 : p.n;
-    const int cols_per_warp = (Epi == EPI_GLU ? BlockN / 2 : BlockN) / (GemmWarps<BSRC_TMA>::kEpilogue / 4);
+    const int cols_per_warp = BSrc == BSRC_W4G128 ? 64 : (Epi == EPI_GLU ? BlockN / 2 : BlockN) / (GemmWarps<BSRC_TMA>::kEpilogue / 4);
     const int obytes = p.out_type == OUT_F16 ? 2 : (p.out_type == OUT_F32 ? 4 : 1);
     const int row_bytes = cols_per_warp * obytes;
     if (row_bytes != 64 && row_bytes != 128) return 0;
-    if (BlockN == 128 && row_bytes != 64) return 0;      // its staging holds 64-byte rows only
+    if (BSrc == BSRC_TMA && BlockN == 128 && row_bytes != 64) return 0;      // its staging holds 64-byte rows only
     if ((reinterpret_cast<uintptr_t>(p.out) & 15u) != 0) return 0;
     if ((static_cast<size_t>(p.ld_out) * obytes) % 16 != 0) return 0;
     if (make_map(map, p.out, obytes, p.m, out_cols, p.ld_out, 32, row_bytes) != PK100_OK) return 0;
@@ -242,10 +242,12 @@ static int launch(const pk100_gemm_args& a, const GemmParams& p_in, cudaStream_t
 }
 
 // fp16 activations x INT4 group-128 weights, dequantised in shared memory by producer warps.
-static int launch_w4(const pk100_gemm_args& a, const GemmParams& p, cudaStream_t stream) {
+static int launch_w4(const pk100_gemm_args& a, const GemmParams& p_in, cudaStream_t stream) {
     constexpr int BlockN = 128;
     constexpr int kMTiles = GemmWarps<BSRC_W4G128>::kMTiles;
-    using Smem = GemmSmem<BlockN, 128, BlockN * kMTiles, 0, kBlockM * kMTiles>;
+    using Smem = GemmSmem<BlockN, 128, BlockN * kMTiles, gemm_store_bytes<EPI_LINEAR, BSRC_W4G128, BlockN>(), kBlockM * kMTiles,
+                          gemm_code_bytes<BSRC_W4G128>()>;
+    GemmParams p = p_in;
     auto kernel = gemm_kernel<KIND_F16, BlockN, 128, EPI_LINEAR, BSRC_W4G128>;
     static bool configured = false;
     if (!configured) {
@@ -254,15 +256,19 @@ static int launch_w4(const pk100_gemm_args& a, const GemmParams& p, cudaStream_t
         if (err != cudaSuccess) return static_cast<int>(err);
         configured = true;
     }
-    CUtensorMap map_a;
-    const int rc = make_map(&map_a, a.a, 2, a.m, a.k, a.lda, kBlockM, 128);
+    CUtensorMap map_a, map_b;
+    int rc = make_map(&map_a, a.a, 2, a.m, a.k, a.lda, kBlockM, 128);
     if (rc != PK100_OK) return rc;
+    rc = make_map(&map_b, a.b, 1, a.n, a.k / 2, a.k / 2, BlockN, 128);        // the codes
+    if (rc != PK100_OK) return rc;
+    CUtensorMap map_out = map_a, map_res = map_a;
+    p.store_row_bytes = make_out_map<EPI_LINEAR, BlockN, BSRC_W4G128>(&map_out, p);
+    p.res_tma = make_residual_map(&map_res, p);
     const int m_items = (a.m + kBlockM * kMTiles - 1) / (kBlockM * kMTiles);   // 256-row work items
     const int n_tiles = (p.n + BlockN - 1) / BlockN;
     int ctas = cta_budget(a);
     if (ctas > m_items * n_tiles) ctas = m_items * n_tiles;
-    // neither B nor the output has a tensor map
-    pk100_launch_chained(kernel, dim3(ctas), dim3(GemmWarps<BSRC_W4G128>::kThreads), Smem::kTotal, stream, map_a, map_a, map_a, map_a, p);
+    pk100_launch_chained(kernel, dim3(ctas), dim3(GemmWarps<BSRC_W4G128>::kThreads), Smem::kTotal, stream, map_a, map_b, map_out, map_res, p);
     return pk100_launch_status();
 }
 
@@ -345,7 +351,6 @@ int pk100_gemm_chained(void* stream_v, const pk100_gemm_args* a, bool b_settled)
     p.keep_out = a->keep_out;
     p.stats_out = a->stats_out;
     p.keep_in = a->keep_in;
-    p.w4_codes = w4 ? static_cast<const uint8_t*>(a->b) : nullptr;
     p.w4_scales = w4 ? static_cast<const __half*>(a->b_group_scales) : nullptr;
     p.status = a->status;
     p.b_settled = b_settled ? 1 : 0;

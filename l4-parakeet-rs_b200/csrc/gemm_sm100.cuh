@@ -9,7 +9,8 @@
 //               accumulator, apply scales / bias / activation / residual / quantisation, store
 //               through shared memory and a TMA store (or per thread)
 // INT4 group-128 weights: 8 epilogue warps + 8 warps that dequantise the B stage into shared
-// memory; a work item is 256 x 128 (two 128-row accumulators share every dequantised B stage).
+// memory from codes that TMA brings there; a work item is 256 x 128 (two 128-row accumulators share every
+// dequantised B stage).
 // Accumulators are double-buffered in TMEM so the MMAs of tile i+1 overlap the epilogue of
 // tile i.  All waits are bounded (ptx_sm100.cuh).
 #pragma once
@@ -53,8 +54,7 @@ struct GemmParams {
     // tile sparsity, consumer side
     const uint8_t* keep_in;      // [ceil(m/128), k/64] or nullptr
     // INT4 group-128 weights (BSRC_W4G128)
-    const uint8_t* w4_codes;     // [n, k/2], low nibble = even k
-    const __half* w4_scales;     // [k/128, n]
+    const __half* w4_scales;     // [k/128, n] (the codes [n, k/2], low nibble = even k, are B's tensor map)
     int* status;                 // set non-zero when a bounded wait gave up
     // Bytes of one output row in a warp's 32-row slice when the slices leave through shared
     // memory and a TMA store (64 or 128); 0 = each thread stores its row piece directly.
@@ -86,19 +86,24 @@ struct GemmWarps {
 };
 
 // Shared memory the epilogue warps stage their output slices in for the TMA store: 32 rows of
-// up to 128 bytes per warp (64 bytes for the INT8 sparse-out tiles).  The 64-column and the INT4 kernels have none.
+// up to 128 bytes per warp (64 bytes for the INT8 sparse-out tiles).  The 64-column kernels have none; INT4
+// weights: a slice is half of a warp's columns, the two halves follow each other through it.
 template <int Epi, int BSrc, int BlockN>
 constexpr int gemm_store_bytes() {
-    if (BSrc != BSRC_TMA) return 0;
+    if (BSrc != BSRC_TMA) return GemmWarps<BSrc>::kEpilogue * 32 * 128;
     // 128-column linear tiles: 32 columns per warp, 64-byte rows for fp16 output
     if (BlockN == 128 && Epi == EPI_LINEAR) return GemmWarps<BSrc>::kEpilogue * 32 * 64;
     if (BlockN != 256) return 0;
     return GemmWarps<BSrc>::kEpilogue * 32 * (Epi == EPI_SPARSE_OUT ? 64 : 128);
 }
 
+// INT4 codes on their way to the dequantisation warps: two buffers of 128 rows x 128 bytes (256 K values)
+template <int BSrc>
+constexpr int gemm_code_bytes() { return BSrc == BSRC_W4G128 ? 2 * 128 * 128 : 0; }
+
 // BRows = B rows staged per CTA per stage, EpiCols = accumulator columns of the tile,
 // StoreBytes = output staging for the TMA store.
-template <int BRows, int SwizzleBytes, int EpiCols = BRows, int StoreBytes = 0, int ARows = kBlockM>
+template <int BRows, int SwizzleBytes, int EpiCols = BRows, int StoreBytes = 0, int ARows = kBlockM, int CodeBytes = 0>
 struct GemmSmem {
     static constexpr int kStageA = ARows * SwizzleBytes;
     static constexpr int kStageB = BRows * SwizzleBytes;
@@ -109,15 +114,15 @@ struct GemmSmem {
     static constexpr int kSchedTiles = 512;
     static constexpr int kSchedOffset = 64 * 8 + 16 + 32 * EpiCols + 64 * 4;
     static constexpr int kTailBytes = kSchedOffset + kSchedTiles * (8 + 2);
-    static constexpr int kStoreBytes = StoreBytes;
+    static constexpr int kStoreBytes = StoreBytes, kCodeBytes = CodeBytes;
     // 227 KB per CTA, less the tail, the output staging and 1 KB of alignment slack; the
     // pipeline is not depth-sensitive (2 and 4 stages measured alike), so staging comes first
-    static constexpr int kBudget = 227 * 1024 - 1024 - kTailBytes - kStoreBytes;
+    static constexpr int kBudget = 227 * 1024 - 1024 - kTailBytes - kStoreBytes - kCodeBytes;
     static constexpr int kStagesRaw = kBudget / kStageBytes;
     static constexpr int kStages = kStagesRaw > 8 ? 8 : kStagesRaw;
     static_assert(kStages >= 2, "at least a double-buffered operand pipeline");
     static constexpr int kTileBytes = kStages * kStageBytes;
-    static constexpr int kTotal = kTileBytes + kStoreBytes + kTailBytes + 1024;
+    static constexpr int kTotal = kTileBytes + kStoreBytes + kCodeBytes + kTailBytes + 1024;
 };
 
 __device__ __forceinline__ float silu_f(float v) { return __fdividef(v, 1.0f + __expf(-v)); }
@@ -292,7 +297,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     constexpr int kBRows = BlockN / CtaGroup;               // B rows staged by this CTA
     constexpr int kMTiles = GemmWarps<BSrc>::kMTiles;       // 128-row accumulators per work item
     using Smem = GemmSmem<kBRows, SwizzleBytes, BlockN * kMTiles, gemm_store_bytes<Epi, BSrc, BlockN>(),
-                          kBlockM * kMTiles>;
+                          kBlockM * kMTiles, gemm_code_bytes<BSrc>()>;
     constexpr int kStages = Smem::kStages;
     constexpr int kElemBytes = Kind == KIND_F16 ? 2 : 1;
     constexpr int kBlockK = SwizzleBytes / kElemBytes;       // elements per K block
@@ -314,13 +319,16 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     uint8_t* smem = reinterpret_cast<uint8_t*>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     uint8_t* store_smem = smem + Smem::kTileBytes;            // 1 KB aligned: stage sizes are
-    uint8_t* tail = store_smem + Smem::kStoreBytes;
+    [[maybe_unused]] uint8_t* code_smem = store_smem + Smem::kStoreBytes;
+    uint8_t* tail = code_smem + Smem::kCodeBytes;
     uint64_t* full_bar = reinterpret_cast<uint64_t*>(tail);
     uint64_t* empty_bar = full_bar + kStages;
     uint64_t* tmem_full_bar = empty_bar + kStages;
     uint64_t* tmem_empty_bar = tmem_full_bar + 2;
     uint64_t* res_bar = tmem_empty_bar + 2;                   // one per epilogue warp
-    static_assert(2 * kStages + 4 + GemmWarps<BSrc>::kEpilogue <= 64, "barriers fit their area");
+    uint64_t* code_full_bar = res_bar + GemmWarps<BSrc>::kEpilogue;       // INT4 codes: two buffers
+    uint64_t* code_empty_bar = code_full_bar + 2;
+    static_assert(2 * kStages + 4 + GemmWarps<BSrc>::kEpilogue + 4 <= 64, "barriers fit their area");
     uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(tail + 64 * 8);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tail + 64 * 8 + 8);
     float* s_cols = reinterpret_cast<float*>(tail + 64 * 8 + 16);   // per-warp scale / bias slices
@@ -386,9 +394,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
             mbar_init(tmem_empty_bar + b, kEpiWarps * CtaGroup);
         }
         for (int i = 0; i < GemmWarps<BSrc>::kEpilogue; ++i) mbar_init(res_bar + i, 1);
+        if constexpr (BSrc == BSRC_W4G128) {
+            for (int b = 0; b < 2; ++b) {
+                mbar_init(code_full_bar + b, 1);
+                mbar_init(code_empty_bar + b, GemmWarps<BSrc>::kDequant);
+            }
+        }
         fence_barrier_init();
         prefetch_tensormap(&map_a);
-        if constexpr (BSrc == BSRC_TMA) prefetch_tensormap(&map_b);
+        prefetch_tensormap(&map_b);
     }
     if (warp == 1) {
         if constexpr (CtaGroup == 2) {
@@ -582,52 +596,65 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         // W = f16(code * scale) is written straight into the 128-byte-swizzled layout the MMA
         // descriptor expects (16-byte chunk c of row r lives at chunk c ^ (r & 7)), made visible to
         // the async proxy, then the warp arrives on `full`.
+        // Codes arrive by TMA in groups of 4 K blocks (128 bytes of every row), one group ahead; thread 0 requests
+        // them.  (Fetched by the threads that use them, 16 bytes per row, they were one request per lane and the
+        // warps waited for them: 34.5 -> 28.7 us at 6144 x 1024 and 81 -> 72 us at 6144 x 4096 with the staged output.)
         const int dq = static_cast<int>(threadIdx.x) - 32 * (2 + kEpiWarps);
         const int brow = dq & 127;
         const int half = dq >> 7;                 // warp-uniform
+        const int groups = (k_blocks + 3) / 4;
         int stage = 0;
         uint32_t phase = 0;
         bool ok = true;
         int mg, nt;
+        int next_it = 0, next_group = 0, requested = 0;       // thread 0: the group to request next
+        auto request_codes = [&]() {
+            int mg_, nt_;
+            if (!work_item(next_it, mg_, nt_)) return;
+            const int b = requested & 1;
+            mbar_arrive_expect_tx(code_full_bar + b, Smem::kCodeBytes / 2);
+            tma_load_2d(code_smem + b * (Smem::kCodeBytes / 2), &map_b, code_full_bar + b, next_group * 128, nt_ * BlockN);
+            requested += 1;
+            if (++next_group == groups) {
+                next_group = 0;
+                next_it += 1;
+            }
+        };
+        if (dq == 0) {
+            request_codes();
+            request_codes();
+        }
+        int used = 0;                             // groups converted so far
         for (int it = 0; ok && work_item(it, mg, nt); ++it) {
             const int n = nt * BlockN + brow;
             const bool row_ok = n < p.n;
-            const uint8_t* codes = p.w4_codes + static_cast<size_t>(row_ok ? n : 0) * (p.k / 2) + half * 16;
-            // Software pipeline over groups of 4 K blocks (= one 128-byte line of this row's codes, two
-            // scale groups): the next group's codes and scales are in flight while this group is
-            // converted, so neither the L2 nor the DRAM latency of the weight stream is exposed.
-            uint4 next_raw[4];
+            // the scales of the next group are in flight while this one is converted
             float next_scale[2];
-            auto fetch_group = [&](int kg) {
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    next_raw[j] = (row_ok && kg + j < k_blocks)
-                        ? __ldg(reinterpret_cast<const uint4*>(codes + (kg + j) * 32)) : make_uint4(0, 0, 0, 0);
+            auto fetch_scales = [&](int kg) {
 #pragma unroll
                 for (int i = 0; i < 2; ++i)
                     next_scale[i] = (row_ok && kg + 2 * i < k_blocks)
                         ? __half2float(p.w4_scales[static_cast<size_t>(kg / 2 + i) * p.n + n]) : 0.0f;
             };
-            fetch_group(0);
+            fetch_scales(0);
             const __half2 bias2 = __halves2half2(__ushort_as_half(0x6408), __ushort_as_half(0x6408));
-            for (int kg = 0; kg < k_blocks && ok; kg += 4) {
-                uint4 cur[4];
-                float cur_scale[2];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) cur[j] = next_raw[j];
-                cur_scale[0] = next_scale[0];
-                cur_scale[1] = next_scale[1];
-                if (kg + 4 < k_blocks) fetch_group(kg + 4);
+            for (int kg = 0; kg < k_blocks && ok; kg += 4, ++used) {
+                const float cur_scale[2] = {next_scale[0], next_scale[1]};
+                const uint8_t* code_row = code_smem + (used & 1) * (Smem::kCodeBytes / 2) + brow * 128;
+                ok = __all_sync(0xffffffffu, mbar_wait_bounded(code_full_bar + (used & 1), (used >> 1) & 1, abort_flag));
+                if (!ok) break;
+                if (kg + 4 < k_blocks) fetch_scales(kg + 4);
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     if (kg + j >= k_blocks) break;
+                    const uint4 codes = *reinterpret_cast<const uint4*>(code_row + (((2 * j + half) ^ (brow & 7)) << 4));
                     const bool got = mbar_wait_bounded(empty_bar + stage, phase ^ 1u, abort_flag);
                     if (!__all_sync(0xffffffffu, got)) {
                         ok = false;
                         break;
                     }
                     uint8_t* row_base = smem + stage * Smem::kStageBytes + Smem::kStageA + brow * 128;
-                    const uint32_t words[4] = {cur[j].x, cur[j].y, cur[j].z, cur[j].w};
+                    const uint32_t words[4] = {codes.x, codes.y, codes.z, codes.w};
                     const __half2 scale2 = __float2half2_rn(cur_scale[j / 2]);
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {          // chunk c = K values 8c .. 8c+7 = one code word
@@ -660,6 +687,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                         phase ^= 1u;
                     }
                 }
+                if (!ok) break;
+                // this warp is done with the buffer; the group after next goes there once all warps are
+                __syncwarp();
+                if (lane == 0) mbar_arrive(code_empty_bar + (used & 1));
+                if (dq == 0) {
+                    if (mbar_wait_bounded(code_empty_bar + (used & 1), (used >> 1) & 1, abort_flag)) request_codes();
+                }
+                __syncwarp();
             }
         }
     } else {
@@ -700,6 +735,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         // store when the host set that up, else stored per thread.  The residual comes the same way, requested before
         // the wait for the accumulator (per thread it would be one 16-byte request per lane, 2 KB apart: us at 6144
         // rows so / by TMA: FF contract 25.0 / 23.1, fp16 output projection 21.8 / 20.1, pointwise-2 16.9 / 14.6).
+        constexpr int kSlices = BSrc == BSRC_W4G128 ? 2 : 1, kSliceCols = kColsPerWarp / kSlices;
         const bool staged = Smem::kStoreBytes > 0 && p.store_row_bytes != 0;
         const bool res_tma = Epi == EPI_LINEAR && staged && p.res_tma != 0;
         for (; ok && work_item(local, mg, nt); ++local) {
@@ -747,18 +783,18 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
             [[maybe_unused]] uint4 res_pre[kAhead][2];
             const bool has_residual = Epi == EPI_LINEAR && p.residual != nullptr;
             uint8_t* const stage = store_smem + ew * (Smem::kStoreBytes / kEpiWarps);
-            // first column and row of the warp's slice; false: outside the matrix
-            auto slice_at = [&](int& col0, int& row0) {
-                col0 = n0 + part * kColsPerWarp;
+            // first column and row of the warp's slice number sl; false: outside the matrix
+            auto slice_at = [&](int sl, int& col0, int& row0) {
+                col0 = n0 + part * kColsPerWarp + sl * kSliceCols;
                 row0 = mt * kBlockM + quad * 32;
                 return row0 < p.m && col0 < (Epi == EPI_GLU ? p.n / 2 : p.n);
             };
-            if (staged) {
+            auto open_slice = [&](int sl) {
                 if (lane == 0) {
-                    bulk_wait_read_all();          // the previous tile's store has read the slice
+                    bulk_wait_read_all();          // the store before has read the slice
                     if (res_tma) {
                         int col0, row0;
-                        if (slice_at(col0, row0)) {
+                        if (slice_at(sl, col0, row0)) {
                             mbar_arrive_expect_tx(res_bar + ew, 32 * p.store_row_bytes);
                             tma_load_2d(stage, &map_res, res_bar + ew, col0, row0);
                         } else {
@@ -767,7 +803,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                     }
                 }
                 __syncwarp();
-            }
+            };
+            if (staged) open_slice(0);
             auto fetch_residual = [&](uint4 (&dst)[2], int c) {
                 const int col = n0 + part * kColsPerWarp + c * 16;
                 if (has_residual && !res_tma && row < p.m && col < p.n) {
@@ -796,8 +833,21 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
             const bool zero_row = row >= p.valid_rows;
             uint8_t* const stage_row = stage + lane * p.store_row_bytes;
             const int swz = p.store_row_bytes == 128 ? (lane & 7) : ((lane >> 1) & 3);
+            auto close_slice = [&](int sl) {
+                // generic-proxy writes of the slice -> visible to the TMA engine
+                fence_proxy_async_smem();
+                __syncwarp();
+                int col0, row0;
+                if (lane == 0 && slice_at(sl, col0, row0)) {
+                    tma_store_2d(&map_out, stage, col0, row0);
+                    bulk_commit_group();
+                }
+            };
+#pragma unroll 1
+            for (int sl = 0; sl < kSlices; ++sl) {
+            if (kSlices > 1 && sl > 0 && staged) open_slice(sl);
             if (res_tma) {
-                const bool here = mbar_wait_bounded(res_bar + ew, local & 1, abort_flag);
+                const bool here = mbar_wait_bounded(res_bar + ew, (local * kSlices + sl) & 1, abort_flag);
                 if (!__all_sync(0xffffffffu, here)) {
                     ok = false;
                     break;
@@ -808,10 +858,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                 auto walk = [&](auto from_slice) {
                 constexpr bool kFromSlice = decltype(from_slice)::value;
 #pragma unroll 1
-                for (int cg = 0; cg < kPieces; cg += kAhead) {
+                for (int cg = sl * (kPieces / kSlices); cg < (sl + 1) * (kPieces / kSlices); cg += kAhead) {
 #pragma unroll
                 for (int ci = 0; ci < kAhead; ++ci) {
-                    const int c = cg + ci;
+                    const int c = cg + ci, in_slice = c - sl * (kPieces / kSlices);
                     const int col_local = part * kColsPerWarp + c * 16;
                     uint32_t r[16];
                     tmem_ld_32x16(taddr_base + col_local, r);
@@ -824,8 +874,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                         float v[16];
                         uint4 res_raw[2];
                         if constexpr (kFromSlice) {
-                            res_raw[0] = *reinterpret_cast<const uint4*>(stage_row + (((2 * c) ^ swz) << 4));
-                            res_raw[1] = *reinterpret_cast<const uint4*>(stage_row + (((2 * c + 1) ^ swz) << 4));
+                            res_raw[0] = *reinterpret_cast<const uint4*>(stage_row + (((2 * in_slice) ^ swz) << 4));
+                            res_raw[1] = *reinterpret_cast<const uint4*>(stage_row + (((2 * in_slice + 1) ^ swz) << 4));
                         } else {
                             res_raw[0] = res_pre[ci][0];
                             res_raw[1] = res_pre[ci][1];
@@ -869,7 +919,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                             for (int j = 0; j < 16; ++j) v[j] = 0.0f;
                         }
                         if (kFromSlice || staged) {
-                            stage_piece(stage_row, c, swz, p.out_type, p.out_scale, v);
+                            stage_piece(stage_row, in_slice, swz, p.out_type, p.out_scale, v);
                         } else {
                             uint8_t* out_row = reinterpret_cast<uint8_t*>(p.out) +
                                 (static_cast<size_t>(row) * p.ld_out + col) * obytes;
@@ -991,16 +1041,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                         dst[c] = keep ? make_uint4(q[c][0], q[c][1], q[c][2], q[c][3]) : make_uint4(0, 0, 0, 0);
                 }
             }
-            if (staged) {
-                // generic-proxy writes of the slice -> visible to the TMA engine
-                fence_proxy_async_smem();
-                __syncwarp();
-                int col0, row0;
-                if (lane == 0 && slice_at(col0, row0)) {
-                    tma_store_2d(&map_out, stage, col0, row0);
-                    bulk_commit_group();
-                }
+            if (staged) close_slice(sl);
             }
+            if (!ok) break;
             // release the accumulator buffer
             tc_fence_before_sync();
             __syncwarp();
