@@ -227,7 +227,8 @@ static int launch(const pk100_gemm_args& a, const GemmParams& p_in, cudaStream_t
     CUtensorMap map_a, map_b;
     int rc = make_map(&map_a, a.a, elem, a.m, a.k, a.lda, kBlockM, SwizzleBytes);
     if (rc != PK100_OK) return rc;
-    rc = make_map(&map_b, a.b, elem, a.n, a.k, a.ldb, BlockN / 2, SwizzleBytes);
+    // GLU: one box of values, one of gates
+    rc = make_map(&map_b, a.b, elem, a.n, a.k, a.ldb, Epi == EPI_GLU ? BlockN / 2 : BlockN, SwizzleBytes);
     if (rc != PK100_OK) return rc;
     CUtensorMap map_out = map_a;
     if constexpr (gemm_store_bytes<Epi, BSRC_TMA, BlockN>() > 0) p.store_row_bytes = make_out_map<Epi, BlockN>(&map_out, p);

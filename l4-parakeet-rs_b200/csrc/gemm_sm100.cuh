@@ -3,7 +3,8 @@
 //   D[M,N] = epilogue( A[M,K] . B[N,K]^T )      A, B row-major ("K-major")
 //
 // One CTA per SM loops over 128 x BLOCK_N output tiles.
-//   warp 0      TMA producer: global -> swizzled shared-memory stage ring
+//   warp 0      TMA producer of A: global -> swizzled shared-memory stage ring
+//   last warp   TMA producer of B (of the INT4 codes)
 //   warp 1      tcgen05.mma issuer (one elected lane); owns the TMEM allocation
 //   warps 2..17 epilogue (16 warps, four per TMEM lane quadrant): tcgen05.ld the fp32/s32
 //               accumulator, apply scales / bias / activation / residual / quantisation, store
@@ -82,7 +83,8 @@ struct GemmWarps {
     static constexpr int kMTiles = BSrc == BSRC_W4G128 ? 2 : 1;
     static constexpr int kEpilogue = BSrc == BSRC_W4G128 ? 8 : 16;
     static constexpr int kDequant = BSrc == BSRC_W4G128 ? 8 : 0;
-    static constexpr int kThreads = 32 * (2 + kEpilogue + kDequant);
+    static constexpr int kProducerB = 2 + kEpilogue + kDequant;      // index of the last warp
+    static constexpr int kThreads = 32 * (kProducerB + 1);
 };
 
 // Shared memory the epilogue warps stage their output slices in for the TMA store: 32 rows of
@@ -336,7 +338,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     uint64_t* s_live = reinterpret_cast<uint64_t*>(tail + Smem::kSchedOffset);   // live mask per 128-row tile
     uint16_t* s_order = reinterpret_cast<uint16_t*>(s_live + Smem::kSchedTiles);  // tiles, most live K blocks first
 
-    const int warp = static_cast<int>(threadIdx.x) / 32;
+    const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x) / 32, 0);    // (known to be the same in all lanes)
     const int lane = static_cast<int>(threadIdx.x) % 32;
 
     const uint32_t rank = CtaGroup == 2 ? cluster_ctarank() : 0u;   // 0 = leader of the pair
@@ -385,15 +387,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     if (threadIdx.x == 0) {
         *abort_flag = 0;
         for (int s = 0; s < kStages; ++s) {
-            // full: one arrive.expect_tx from the TMA lane (+ the dequantisation warps)
-            mbar_init(full_bar + s, 1 + GemmWarps<BSrc>::kDequant);
+            // full: one arrive.expect_tx from each TMA lane (pairs: one) or the dequantisation warps of the block's parity
+            mbar_init(full_bar + s, CtaGroup == 2 ? 1 : BSrc == BSRC_TMA ? 2 : 1 + GemmWarps<BSrc>::kDequant / 2);
             mbar_init(empty_bar + s, 1);
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(tmem_full_bar + b, 1);
             mbar_init(tmem_empty_bar + b, kEpiWarps * CtaGroup);
         }
-        for (int i = 0; i < GemmWarps<BSrc>::kEpilogue; ++i) mbar_init(res_bar + i, 1);
         if constexpr (BSrc == BSRC_W4G128) {
             for (int b = 0; b < 2; ++b) {
                 mbar_init(code_full_bar + b, 1);
@@ -403,6 +404,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         fence_barrier_init();
         prefetch_tensormap(&map_a);
         prefetch_tensormap(&map_b);
+    }
+    if (warp == 2) {                              // (side by side: one thread would spend 16 stores on them)
+        if (lane < GemmWarps<BSrc>::kEpilogue) mbar_init(res_bar + lane, 1);
+        fence_barrier_init();
     }
     if (warp == 1) {
         if constexpr (CtaGroup == 2) {
@@ -419,33 +424,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     if constexpr (CtaGroup == 2) cluster_sync_all();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_ptr_smem;
-    // Weights of the first work item's first stages: requested while the previous kernel drains, so that the
-    // DRAM latency of a layer's weights (read once per pass) is not on the chain of small launches.
-    int b_ahead = 0;
-    if constexpr (CtaGroup == 1 && BSrc == BSRC_TMA) {
-        if (p.b_settled != 0 && p.keep_in == nullptr) b_ahead = k_blocks < kStages ? k_blocks : kStages;
-    }
-    auto load_b = [&](int stage, int nt_, int kb) {
-        uint8_t* sb = smem + stage * Smem::kStageBytes + Smem::kStageA;
-        const int n_first = Epi == EPI_GLU ? nt_ * kBHalf : nt_ * BlockN;
-        const int n_second = Epi == EPI_GLU ? p.n / 2 + nt_ * kBHalf : n_first + kBHalf;
-        tma_load_2d(sb, &map_b, full_bar + stage, kb * kBlockK, n_first);
-        tma_load_2d(sb + kBHalf * SwizzleBytes, &map_b, full_bar + stage, kb * kBlockK, n_second);
-    };
-    if constexpr (CtaGroup == 1 && BSrc == BSRC_TMA) {
-        if (b_ahead > 0 && threadIdx.x == 0) {
-            int mg, nt;
-            if (work_item(0, mg, nt)) {
-                for (int s = 0; s < b_ahead; ++s) {
-                    mbar_arrive_expect_tx(full_bar + s, Smem::kStageBytes);
-                    load_b(s, nt, s);
-                }
-            }
-        }
-    }
-    // everything above touched only shared / tensor memory, kernel parameters and settled weights: under a
-    // programmatic dependent launch it overlapped the previous kernel's tail
-    grid_dependency_wait();
+    // everything above touched only shared / tensor memory and kernel parameters: under a programmatic dependent
+    // launch it overlapped the previous kernel's tail.  Settled weights are requested meanwhile, as far as the ring
+    // takes them, so that their DRAM latency (they are read once per pass) is not on the chain of small launches.
+    if (!(warp == GemmWarps<BSrc>::kProducerB && p.b_settled != 0 && p.keep_in == nullptr)) grid_dependency_wait();
     if (balanced) {
         for (int t = static_cast<int>(threadIdx.x); t < m_tiles; t += static_cast<int>(blockDim.x)) {
             LiveMaskRow row;
@@ -465,22 +447,32 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         __syncthreads();
     }
 
+    // The roles that issue TMA and MMA instructions run their loops with the whole warp and elect a lane for the
+    // instructions alone: their operands live in uniform registers, which the compiler has to fill one by one
+    // behind a lane test.  Cycles a K block of four MMAs cost its issuer (the tensor core takes 128 to 512) behind a
+    // lane test / so: 532 / 400 with 64-column tiles, 844 / 661 with 256-column tiles of K = 1024; the TMA issuers
+    // 330 / 210.  us, before / after: FF expand 30.6 / 28.5 at 6144 rows, 194 / 178 at 45 056; FF contract 12.4 / 10.7
+    // at 768, 23.2 / 21.9 at 6144; output projection 9.1 / 8.3 at 768; INT4 28.8 / 25.6 at 6144 x 1024, 72 / 64 at
+    // 6144 x 4096.
+    auto warp_wait = [&](uint64_t* bar, uint32_t parity) {
+        return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, abort_flag)) != 0;
+    };
     if (warp == 0) {
         // ------------------------------------------------------ TMA producer
-        if (lane == 0) {
-            int stage = 0;
-            uint32_t phase = 0;
-            bool ok = true;
-            int mg, nt;
-            for (int it = 0; ok && work_item(it, mg, nt); ++it) {
-                const int m0 = (mg * CtaGroup + static_cast<int>(rank)) * kBlockM * kMTiles;
-                const uint64_t live_mask = group_live_mask(mg);
-                for (int kb = 0; kb < k_blocks; ++kb) {
-                    if (p.keep_in != nullptr && !k_block_live<SwizzleBytes>(live_mask, kb)) continue;
-                    if (!mbar_wait_bounded(empty_bar + stage, phase ^ 1u, abort_flag)) {
-                        ok = false;
-                        break;
-                    }
+        int stage = 0;
+        uint32_t phase = 0;
+        bool ok = true;
+        int mg, nt;
+        for (int it = 0; ok && work_item(it, mg, nt); ++it) {
+            const int m0 = (mg * CtaGroup + static_cast<int>(rank)) * kBlockM * kMTiles;
+            const uint64_t live_mask = group_live_mask(mg);
+            for (int kb = 0; kb < k_blocks; ++kb) {
+                if (p.keep_in != nullptr && !k_block_live<SwizzleBytes>(live_mask, kb)) continue;
+                if (!warp_wait(empty_bar + stage, phase ^ 1u)) {
+                    ok = false;
+                    break;
+                }
+                if (elect_one()) {
                     uint8_t* sa = smem + stage * Smem::kStageBytes;
                     [[maybe_unused]] uint8_t* sb = sa + Smem::kStageA;
                     if constexpr (CtaGroup == 2) {
@@ -496,10 +488,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                         tma_load_2d_pair(sa, &map_a, bar, kb * kBlockK, m0);
                         tma_load_2d_pair(sb, &map_b, bar, kb * kBlockK, n_rows);
                     } else if constexpr (BSrc == BSRC_TMA) {
-                        const bool ahead = it == 0 && kb < b_ahead;      // (stage kb: its B is on the way)
-                        if (!ahead) mbar_arrive_expect_tx(full_bar + stage, Smem::kStageBytes);
+                        mbar_arrive_expect_tx(full_bar + stage, Smem::kStageA);
                         tma_load_2d(sa, &map_a, full_bar + stage, kb * kBlockK, m0);
-                        if (!ahead) load_b(stage, nt, kb);
                     } else {
                         // 128-row boxes of A, one per accumulator that has rows
                         const bool second = m0 + kBlockM < p.m;
@@ -508,16 +498,67 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                         if (second)
                             tma_load_2d(sa + Smem::kStageA / 2, &map_a, full_bar + stage, kb * kBlockK, m0 + kBlockM);
                     }
-                    if (++stage == kStages) {
-                        stage = 0;
-                        phase ^= 1u;
+                }
+                __syncwarp();
+                if (++stage == kStages) {
+                    stage = 0;
+                    phase ^= 1u;
+                }
+            }
+        }
+    } else if (warp == GemmWarps<BSrc>::kProducerB) {
+        // -------------------------------------------------- B (or code) producer
+        if (CtaGroup == 1) {
+            int stage = 0;
+            uint32_t phase = 0;
+            bool ok = true;
+            int mg, nt;
+            for (int it = 0; ok && work_item(it, mg, nt); ++it) {
+                if constexpr (BSrc == BSRC_TMA) {
+                    const uint64_t live_mask = group_live_mask(mg);
+                    for (int kb = 0; kb < k_blocks; ++kb) {
+                        if (p.keep_in != nullptr && !k_block_live<SwizzleBytes>(live_mask, kb)) continue;
+                        if (!warp_wait(empty_bar + stage, phase ^ 1u)) {
+                            ok = false;
+                            break;
+                        }
+                        if (elect_one()) {
+                            uint8_t* sb = smem + stage * Smem::kStageBytes + Smem::kStageA;
+                            mbar_arrive_expect_tx(full_bar + stage, Smem::kStageB);
+                            if constexpr (Epi == EPI_GLU) {                // boxes of values and of their gates
+                                tma_load_2d(sb, &map_b, full_bar + stage, kb * kBlockK, nt * kBHalf);
+                                tma_load_2d(sb + kBHalf * SwizzleBytes, &map_b, full_bar + stage, kb * kBlockK, p.n / 2 + nt * kBHalf);
+                            } else {
+                                tma_load_2d(sb, &map_b, full_bar + stage, kb * kBlockK, nt * BlockN);
+                            }
+                        }
+                        __syncwarp();
+                        if (++stage == kStages) {
+                            stage = 0;
+                            phase ^= 1u;
+                        }
+                    }
+                } else {
+                    // codes in groups of 4 K blocks (128 bytes of every row) through two buffers
+                    for (int kb = 0; kb < k_blocks; kb += 4) {
+                        if (!warp_wait(code_empty_bar + stage, phase ^ 1u)) {
+                            ok = false;
+                            break;
+                        }
+                        if (elect_one()) {
+                            mbar_arrive_expect_tx(code_full_bar + stage, Smem::kCodeBytes / 2);
+                            tma_load_2d(code_smem + stage * (Smem::kCodeBytes / 2), &map_b, code_full_bar + stage, kb * 32, nt * BlockN);
+                        }
+                        __syncwarp();
+                        stage ^= 1;
+                        phase ^= stage == 0 ? 1u : 0u;
                     }
                 }
             }
         }
     } else if (warp == 1) {
         // -------------------------------------------------------- MMA issuer
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
             constexpr uint32_t idesc = make_instr_desc<Kind>(kBlockM * CtaGroup, BlockN);
             int stage = 0;
             uint32_t phase = 0;
@@ -528,7 +569,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                 const int buf = local & 1;
                 const uint32_t acc_phase = (local >> 1) & 1;
                 const uint64_t live_mask = group_live_mask(mg);
-                if (!mbar_wait_bounded(tmem_empty_bar + buf, acc_phase ^ 1u, abort_flag)) {
+                if (!warp_wait(tmem_empty_bar + buf, acc_phase ^ 1u)) {
                     ok = false;
                     break;
                 }
@@ -538,92 +579,83 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                 uint32_t accumulate = 0;
                 for (int kb = 0; kb < k_blocks; ++kb) {
                     if (p.keep_in != nullptr && !k_block_live<SwizzleBytes>(live_mask, kb)) continue;
-                    if (!mbar_wait_bounded(full_bar + stage, phase, abort_flag)) {
+                    if (!warp_wait(full_bar + stage, phase)) {
                         ok = false;
                         break;
                     }
                     tc_fence_after_sync();
-                    const uint32_t sa = smem_u32(smem + stage * Smem::kStageBytes);
-                    const uint32_t sb = sa + Smem::kStageA;
-                    const uint64_t desc_a = make_smem_desc<SwizzleBytes>(sa);
-                    const uint64_t desc_b = make_smem_desc<SwizzleBytes>(sb);
+                    if (elect_one()) {
+                        const uint32_t sa = smem_u32(smem + stage * Smem::kStageBytes);
+                        const uint32_t sb = sa + Smem::kStageA;
+                        const uint64_t desc_a = make_smem_desc<SwizzleBytes>(sa);
+                        const uint64_t desc_b = make_smem_desc<SwizzleBytes>(sb);
+                        bool first = accumulate == 0;
 #pragma unroll
-                    for (int j = 0; j < kMmasPerBlock; ++j) {
-                        // advance 32 bytes along K inside the swizzle atom: +2 in 16-byte units
-                        if constexpr (CtaGroup == 2)
-                            tc_mma_pair<Kind>(tmem_d, desc_a + 2u * j, desc_b + 2u * j, idesc, accumulate);
-                        else
-                            tc_mma<Kind>(tmem_d, desc_a + 2u * j, desc_b + 2u * j, idesc, accumulate);
-                        if constexpr (kMTiles == 2) {
-                            // the second 128 rows of A (16 KB on: 1024 descriptor units) against the same B
-                            if (second)
-                                tc_mma<Kind>(tmem_d + BlockN, desc_a + 1024u + 2u * j, desc_b + 2u * j, idesc, accumulate);
+                        for (int j = 0; j < kMmasPerBlock; ++j) {
+                            // advance 32 bytes along K inside the swizzle atom: +2 in 16-byte units
+                            if constexpr (CtaGroup == 2)
+                                tc_mma_pair<Kind>(tmem_d, desc_a + 2u * j, desc_b + 2u * j, idesc, first ? 0u : 1u);
+                            else
+                                tc_mma<Kind>(tmem_d, desc_a + 2u * j, desc_b + 2u * j, idesc, first ? 0u : 1u);
+                            if constexpr (kMTiles == 2) {
+                                // the second 128 rows of A (16 KB on: 1024 descriptor units) against the same B
+                                if (second)
+                                    tc_mma<Kind>(tmem_d + BlockN, desc_a + 1024u + 2u * j, desc_b + 2u * j, idesc, first ? 0u : 1u);
+                            }
+                            first = false;
                         }
-                        accumulate = 1;
+                        // free the stage (in both CTAs of a pair) once the MMAs retire
+                        if constexpr (CtaGroup == 2) {
+                            tc_commit_pair(map_to_cta(smem_u32(empty_bar + stage), 0));
+                            tc_commit_pair(map_to_cta(smem_u32(empty_bar + stage), 1));
+                        } else {
+                            tc_commit(empty_bar + stage);
+                        }
                     }
-                    // free the stage (in both CTAs of a pair) once the MMAs retire
-                    if constexpr (CtaGroup == 2) {
-                        tc_commit_pair(map_to_cta(smem_u32(empty_bar + stage), 0));
-                        tc_commit_pair(map_to_cta(smem_u32(empty_bar + stage), 1));
-                    } else {
-                        tc_commit(empty_bar + stage);
-                    }
+                    accumulate = 1;
+                    __syncwarp();
                     if (++stage == kStages) {
                         stage = 0;
                         phase ^= 1u;
                     }
                 }
                 if (!ok) break;
-                if constexpr (CtaGroup == 2) {
-                    if (accumulate != 0) {
-                        tc_commit_pair(map_to_cta(smem_u32(tmem_full_bar + buf), 0));
-                        tc_commit_pair(map_to_cta(smem_u32(tmem_full_bar + buf), 1));
+                if (elect_one()) {
+                    if constexpr (CtaGroup == 2) {
+                        if (accumulate != 0) {
+                            tc_commit_pair(map_to_cta(smem_u32(tmem_full_bar + buf), 0));
+                            tc_commit_pair(map_to_cta(smem_u32(tmem_full_bar + buf), 1));
+                        } else {
+                            mbar_arrive_cluster(map_to_cta(smem_u32(tmem_full_bar + buf), 0));
+                            mbar_arrive_cluster(map_to_cta(smem_u32(tmem_full_bar + buf), 1));
+                        }
+                    } else if (accumulate != 0) {
+                        tc_commit(tmem_full_bar + buf);
                     } else {
-                        mbar_arrive_cluster(map_to_cta(smem_u32(tmem_full_bar + buf), 0));
-                        mbar_arrive_cluster(map_to_cta(smem_u32(tmem_full_bar + buf), 1));
+                        mbar_arrive(tmem_full_bar + buf);  // no live K block: accumulator unused
                     }
-                } else if (accumulate != 0) {
-                    tc_commit(tmem_full_bar + buf);
-                } else {
-                    mbar_arrive(tmem_full_bar + buf);  // no live K block: accumulator unused
                 }
+                __syncwarp();
             }
         }
-    } else if (BSrc == BSRC_W4G128 && warp >= 2 + kEpiWarps) {
+    } else if (BSrc == BSRC_W4G128 && warp >= 2 + kEpiWarps) {      // (and not the last warp: above)
         // ------------------------------------- INT4 -> fp16 B-operand producer
-        // 256 threads: thread dq converts half h = dq / 128 (32 K values = 16 bytes of codes) of
-        // row dq % 128 of the 128-row B stage per K block, one fp16 scale per 128 K.
+        // Two teams of 4 warps, one for the even and one for the odd K blocks: what a block costs a warp is the
+        // latency of its chain (codes -> halves -> shared memory -> proxy fence -> arrival, about 700 cycles for one
+        // half of a row and 900 for a whole one), so two blocks are converted side by side.  A thread converts a
+        // whole row of a block (64 K values = 32 bytes of codes), one fp16 scale per 128 K.
         // W = f16(code * scale) is written straight into the 128-byte-swizzled layout the MMA
         // descriptor expects (16-byte chunk c of row r lives at chunk c ^ (r & 7)), made visible to
         // the async proxy, then the warp arrives on `full`.
-        // Codes arrive by TMA in groups of 4 K blocks (128 bytes of every row), one group ahead; thread 0 requests
-        // them.  (Fetched by the threads that use them, 16 bytes per row, they were one request per lane and the
-        // warps waited for them: 34.5 -> 28.7 us at 6144 x 1024 and 81 -> 72 us at 6144 x 4096 with the staged output.)
+        // Codes arrive by TMA in groups of 4 K blocks (fetched by the threads that use them, 16 bytes per row, they
+        // were one request per lane).
         const int dq = static_cast<int>(threadIdx.x) - 32 * (2 + kEpiWarps);
-        const int brow = dq & 127;
-        const int half = dq >> 7;                 // warp-uniform
-        const int groups = (k_blocks + 3) / 4;
-        int stage = 0;
+        const int team = (dq / 32) & 1, brow = (dq / 64) * 32 + lane;
+        static_assert(BSrc == BSRC_TMA || kStages >= 3, "a stage for each team and one for the MMAs");
+        int stage = team;
         uint32_t phase = 0;
         bool ok = true;
         int mg, nt;
-        int next_it = 0, next_group = 0, requested = 0;       // thread 0: the group to request next
-        auto request_codes = [&]() {
-            int mg_, nt_;
-            if (!work_item(next_it, mg_, nt_)) return;
-            const int b = requested & 1;
-            mbar_arrive_expect_tx(code_full_bar + b, Smem::kCodeBytes / 2);
-            tma_load_2d(code_smem + b * (Smem::kCodeBytes / 2), &map_b, code_full_bar + b, next_group * 128, nt_ * BlockN);
-            requested += 1;
-            if (++next_group == groups) {
-                next_group = 0;
-                next_it += 1;
-            }
-        };
-        if (dq == 0) {
-            request_codes();
-            request_codes();
-        }
         int used = 0;                             // groups converted so far
         for (int it = 0; ok && work_item(it, mg, nt); ++it) {
             const int n = nt * BlockN + brow;
@@ -645,24 +677,28 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                 if (!ok) break;
                 if (kg + 4 < k_blocks) fetch_scales(kg + 4);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
+                for (int jj = 0; jj < 2; ++jj) {
+                    const int j = 2 * jj + team;
                     if (kg + j >= k_blocks) break;
-                    const uint4 codes = *reinterpret_cast<const uint4*>(code_row + (((2 * j + half) ^ (brow & 7)) << 4));
+                    uint32_t words[8];
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const uint4 codes = *reinterpret_cast<const uint4*>(code_row + (((2 * j + h) ^ (brow & 7)) << 4));
+                        words[4 * h] = codes.x; words[4 * h + 1] = codes.y; words[4 * h + 2] = codes.z; words[4 * h + 3] = codes.w;
+                    }
                     const bool got = mbar_wait_bounded(empty_bar + stage, phase ^ 1u, abort_flag);
                     if (!__all_sync(0xffffffffu, got)) {
                         ok = false;
                         break;
                     }
                     uint8_t* row_base = smem + stage * Smem::kStageBytes + Smem::kStageA + brow * 128;
-                    const uint32_t words[4] = {codes.x, codes.y, codes.z, codes.w};
-                    const __half2 scale2 = __float2half2_rn(cur_scale[j / 2]);
+                    const __half2 scale2 = __float2half2_rn(cur_scale[jj]);
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {          // chunk c = K values 8c .. 8c+7 = one code word
-                        const int c = 4 * half + i;
+                    for (int c = 0; c < 8; ++c) {          // chunk c = K values 8c .. 8c+7 = one code word
                         // nibble n -> fp16 (1024 + (n ^ 8)) by OR-ing the biased nibble into the
                         // mantissa of 1024.0, minus 1032.0 = the signed code, exactly; HMUL2 by the
                         // fp16 group scale then rounds once, i.e. f16(code * scale).
-                        const uint32_t wbits = words[i] ^ 0x88888888u;   // two's complement -> offset binary
+                        const uint32_t wbits = words[c] ^ 0x88888888u;   // two's complement -> offset binary
                         // nibbles (e, e + 4) of the word land in the two halves of one register with
                         // one shift and one AND-OR; the byte permutes below put K back in order
                         __half2 v[4];
@@ -682,19 +718,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                     fence_proxy_async_smem();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(full_bar + stage);
-                    if (++stage == kStages) {
-                        stage = 0;
+                    stage += 2;
+                    if (stage >= kStages) {
+                        stage -= kStages;
                         phase ^= 1u;
                     }
                 }
                 if (!ok) break;
-                // this warp is done with the buffer; the group after next goes there once all warps are
                 __syncwarp();
-                if (lane == 0) mbar_arrive(code_empty_bar + (used & 1));
-                if (dq == 0) {
-                    if (mbar_wait_bounded(code_empty_bar + (used & 1), (used >> 1) & 1, abort_flag)) request_codes();
-                }
-                __syncwarp();
+                if (lane == 0) mbar_arrive(code_empty_bar + (used & 1));       // this warp is done with the buffer
             }
         }
     } else {
