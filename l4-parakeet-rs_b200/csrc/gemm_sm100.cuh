@@ -821,22 +821,26 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                 row0 = mt * kBlockM + quad * 32;
                 return row0 < p.m && col0 < (Epi == EPI_GLU ? p.n / 2 : p.n);
             };
-            auto open_slice = [&](int sl) {
+            // the store before has read the slice: waited for where the slice is filled, by the residual or by the output
+            // (at the head of the tile the wait was exposed: QKV 22.5 -> 21.6 us at 6144 rows)
+            auto slice_free = [&]() {
+                if (lane == 0) bulk_wait_read_all();
+                __syncwarp();
+            };
+            auto fetch_slice = [&](int sl) {
+                slice_free();
                 if (lane == 0) {
-                    bulk_wait_read_all();          // the store before has read the slice
-                    if (res_tma) {
-                        int col0, row0;
-                        if (slice_at(sl, col0, row0)) {
-                            mbar_arrive_expect_tx(res_bar + ew, 32 * p.store_row_bytes);
-                            tma_load_2d(stage, &map_res, res_bar + ew, col0, row0);
-                        } else {
-                            mbar_arrive(res_bar + ew);
-                        }
+                    int col0, row0;
+                    if (slice_at(sl, col0, row0)) {
+                        mbar_arrive_expect_tx(res_bar + ew, 32 * p.store_row_bytes);
+                        tma_load_2d(stage, &map_res, res_bar + ew, col0, row0);
+                    } else {
+                        mbar_arrive(res_bar + ew);
                     }
                 }
                 __syncwarp();
             };
-            if (staged) open_slice(0);
+            if (res_tma) fetch_slice(0);
             auto fetch_residual = [&](uint4 (&dst)[2], int c) {
                 const int col = n0 + part * kColsPerWarp + c * 16;
                 if (has_residual && !res_tma && row < p.m && col < p.n) {
@@ -877,7 +881,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
             };
 #pragma unroll 1
             for (int sl = 0; sl < kSlices; ++sl) {
-            if (kSlices > 1 && sl > 0 && staged) open_slice(sl);
+            if (kSlices > 1 && sl > 0 && res_tma) fetch_slice(sl);
             if (res_tma) {
                 const bool here = mbar_wait_bounded(res_bar + ew, (local * kSlices + sl) & 1, abort_flag);
                 if (!__all_sync(0xffffffffu, here)) {
@@ -898,6 +902,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                     uint32_t r[16];
                     tmem_ld_32x16(taddr_base + col_local, r);
                     tmem_ld_wait();
+                    if (!kFromSlice && staged && in_slice == 0) slice_free();
                     const int col = n0 + col_local;
                     if (row < p.m && col < p.n) {
                         // The run-time switches (activation, residual, dead rows) are taken once per
@@ -914,7 +919,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                             if (c + kAhead < kPieces) fetch_residual(res_pre[ci], c + kAhead);
                         }
                         const float rs_live = live ? rs : 0.0f;
-                        if (!live) {              // accumulator never written: any bit pattern
+                        if (p.keep_in != nullptr && !live) {      // accumulator never written: any bit pattern
 #pragma unroll
                             for (int j = 0; j < 16; ++j) r[j] = 0u;
                         }
@@ -946,9 +951,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
 #pragma unroll
                             for (int j = 0; j < 16; ++j) v[j] *= p.alpha;
                         }
-                        if (zero_row) {
+                        if (p.valid_rows < p.m) {
+                            if (zero_row) {
 #pragma unroll
-                            for (int j = 0; j < 16; ++j) v[j] = 0.0f;
+                                for (int j = 0; j < 16; ++j) v[j] = 0.0f;
+                            }
                         }
                         if (kFromSlice || staged) {
                             stage_piece(stage_row, in_slice, swz, p.out_type, p.out_scale, v);
@@ -972,6 +979,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                     tmem_ld_32x16(taddr_base + col_local, rv);
                     tmem_ld_32x16(taddr_base + kBHalf + col_local, rg);
                     tmem_ld_wait();
+                    if (staged && c == 0) slice_free();
                     const int col = n0 + col_local;
                     if (row < p.m && col < p.n / 2) {
                         float v[16];
@@ -1061,6 +1069,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                 }
                 const int col = n0 + part * kColsPerWarp;
                 if (staged) {
+                    slice_free();
 #pragma unroll
                     for (int c = 0; c < kPieces; ++c)
                         *reinterpret_cast<uint4*>(stage_row + ((c ^ swz) << 4)) =
