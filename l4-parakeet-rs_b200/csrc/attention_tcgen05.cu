@@ -30,10 +30,10 @@
 // memory and shared memory are full), so what counts is the length of the chain and what the next tile can
 // start meanwhile.  Q, P and the first key block of the next tile are loaded, and its QP product is issued,
 // while the softmax warps finish this one.
-// Measured back to back (the kernel with one CTA per tile and two full passes over scores and position scores
-// in parentheses): 203 us at 45 056 rows (456), 36.5 us at 6144 (66), 22 us at 768 (23).  A tile takes 17 k
-// cycles in a CTA's steady state, from 43 k: 8.1 k instructions per scheduler at 40 % issue, tensor pipe 18 %,
-// shared memory 45 %; the first tile of a CTA takes 30 k, which is what the 48 tiles of 768 rows show.
+// Measured back to back: 179 us at 45 056 rows, 33 us at 6144, 15 us at 768, 10.4 us at 128 (with the issuing roles
+// behind a lane test 201, 36, 15.2, 10.7; one CTA per tile and two full passes over scores and position scores: 456
+// and 66 us for the first two).  The softmax warps' issue slots, the tensor pipe and shared memory are each far from
+// full; the first tile of a CTA takes about twice a later one, which is what the 48 tiles of 768 rows show.
 // Every wait is a bounded mbarrier wait; when one expires the kernel raises the status word and all
 // roles leave through the common teardown (tensor memory freed).
 #include <cuda.h>
@@ -174,6 +174,9 @@ __device__ __forceinline__ bool att_wait(uint64_t* bar, uint32_t parity, volatil
 }
 #define ATT_WAIT(index, parity)                                                         \
     if (!(ok = att_wait(&sm.bar[index], (parity), abort_flag))) break
+// a whole warp waits
+#define ATT_WARP_WAIT(index, parity)                                                    \
+    if (!(ok = __all_sync(0xffffffffu, att_wait(&sm.bar[index], (parity), abort_flag)) != 0)) break
 
 __global__ void __launch_bounds__(kThreads, 1)
 local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
@@ -181,7 +184,7 @@ local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const 
                                const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_out, const Params p) {
     extern __shared__ uint8_t att5_raw[];
     Smem& sm = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(att5_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-    const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid / 32, 0), lane = tid % 32;     // (warp: known to be the same in all lanes)
     // (head, tile) items of this CTA, heads outermost: a range meets two heads at most a few times
     const long long items = static_cast<long long>(kHeads) * p.tiles;
     const int first_item = static_cast<int>(items * blockIdx.x / gridDim.x);
@@ -227,98 +230,97 @@ local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const 
     // (the middle key block is in every tile), bits 0 and 2 those of the first and last key block.
     uint32_t ph = 0;
 
+    // The two issuing roles run as whole warps and elect a lane for the TMA and MMA instructions alone: their operands
+    // live in uniform registers, which the compiler has to fill one by one behind a lane test (about 130 cycles an
+    // MMA, of which a tile has 72).
     if (warp == kSoftmaxWarps) {
         // ------------------------------------------------------------ TMA producer
-        if (lane == 0) {
-            uint32_t before = 0, ph_before = 0;        // key blocks and parities of the tile before (0: none)
-            if (!p.early) grid_dependency_wait();
-            int head = first_head, tile = first_tile - 1;
-            for (int item = first_item; ok && item < last_item; ++item) {
-                if (++tile == p.tiles) { tile = 0; ++head; }
-                const TilePlace at(p.rows, tile);
-                if (at.padding()) continue;
-                const uint32_t blocks = at.blocks(), par = (ph >> 1) & 1u;
-                const int key_row = at.base + at.q0 - kReach;
-                auto load_block = [&](int slot, const CUtensorMap* map, int bar, int b) {
-                    mbar_arrive_expect_tx(&sm.bar[bar], kSlotBytes);
-#pragma unroll 1
-                    for (int a = 0; a < 2; ++a)
-                        tma_load_2d(sm.slot[slot] + a * kAtomBytes, map, &sm.bar[bar], head * kDim + a * 64, key_row + b * 128);
-                };
-                auto load_queries = [&] {
-                    mbar_arrive_expect_tx(&sm.bar[B_Q_IN], kSlotBytes);
-                    for (int a = 0; a < 2; ++a)
-                        tma_load_2d(sm.q + a * kAtomBytes, &map_q, &sm.bar[B_Q_IN], head * kDim + a * 64, at.base + at.q0);
-                };
-                if (before != 0) load_queries();       // the score products of the tile before have retired
-                // position rows: slot 0 held V0 (or K1), slot 1 held V1 of the tile before
-                mbar_arrive_expect_tx(&sm.bar[B_P_IN], 2 * kSlotBytes + kTailBytes);
-                for (int a = 0; a < 2; ++a)
-                    tma_load_2d(sm.tail + a * (kTailBytes / 2), &map_p16, &sm.bar[B_P_IN], a * 64, head * kPosRows + 256);
-                if (before & 1u) ATT_WAIT(B_PV_DONE + 0, ph_before & 1u);
-                if (before != 0 && !(before & 1u)) ATT_WAIT(B_PV_DONE + 1, (ph_before >> 1) & 1u);
-                for (int a = 0; a < 2; ++a)
-                    tma_load_2d(sm.slot[0] + a * kAtomBytes, &map_p, &sm.bar[B_P_IN], a * 64, head * kPosRows);
-                if (before != 0) ATT_WAIT(B_PV_DONE + 1, (ph_before >> 1) & 1u);
-                for (int a = 0; a < 2; ++a)
-                    tma_load_2d(sm.slot[1] + a * kAtomBytes, &map_p, &sm.bar[B_P_IN], a * 64, head * kPosRows + 128);
-                if (before & 4u) ATT_WAIT(B_PV_DONE + 2, (ph_before >> 2) & 1u);
-                if (before == 0) {
-                    if (p.early) grid_dependency_wait();
-                    load_queries();
+        uint32_t before = 0, ph_before = 0;            // key blocks and parities of the tile before (0: none)
+        if (!p.early) grid_dependency_wait();
+        int head = first_head, tile = first_tile - 1;
+        for (int item = first_item; ok && item < last_item; ++item) {
+            if (++tile == p.tiles) { tile = 0; ++head; }
+            const TilePlace at(p.rows, tile);
+            if (at.padding()) continue;
+            const uint32_t blocks = at.blocks(), par = (ph >> 1) & 1u;
+            const int key_row = at.base + at.q0 - kReach;
+            // one 128-row operand block: its two 64-feature atoms
+            auto load_pair = [&](uint8_t* dst, int atom_bytes, const CUtensorMap* map, int bar, int x, int row, int arm_bytes) {
+                if (elect_one()) {
+                    if (arm_bytes > 0) mbar_arrive_expect_tx(&sm.bar[bar], arm_bytes);
+                    tma_load_2d(dst, map, &sm.bar[bar], x, row);
+                    tma_load_2d(dst + atom_bytes, map, &sm.bar[bar], x + 64, row);
                 }
-                if (blocks & 1u) load_block(slot_of_key(0), &map_k, B_K_IN + 0, 0);
-                // the other key blocks: once the position rows have been multiplied
-                ATT_WAIT(B_QP_DONE, par);
-                ATT_WAIT(B_VP_DONE, par);
-                load_block(slot_of_key(1), &map_k, B_K_IN + 1, 1);
-                if (blocks & 4u) load_block(slot_of_key(2), &map_k, B_K_IN + 2, 2);
-                // values: V0 after K1, V1 after K2 (or the position rows), V2 after K0
-                ATT_WAIT(B_S_DONE + 1, par);
-                ATT_WAIT(B_UK_DONE + 1, par);
-                if (blocks & 1u) load_block(0, &map_v, B_V_IN + 0, 0);
-                if (blocks & 4u) {
-                    ATT_WAIT(B_S_DONE + 2, (ph >> 2) & 1u);
-                    ATT_WAIT(B_UK_DONE + 2, (ph >> 2) & 1u);
-                }
-                load_block(1, &map_v, B_V_IN + 1, 1);
-                if (blocks & 4u) {
-                    if (blocks & 1u) {
-                        ATT_WAIT(B_S_DONE + 0, ph & 1u);
-                        ATT_WAIT(B_UK_DONE + 0, ph & 1u);
-                    }
-                    load_block(2, &map_v, B_V_IN + 2, 2);
-                }
-                before = blocks;
-                ph_before = ph;
-                ph ^= blocks;
+                __syncwarp();
+            };
+            auto load_block = [&](int slot, const CUtensorMap* map, int bar, int b) {
+                load_pair(sm.slot[slot], kAtomBytes, map, bar, head * kDim, key_row + b * 128, kSlotBytes);
+            };
+            auto load_queries = [&] { load_pair(sm.q, kAtomBytes, &map_q, B_Q_IN, head * kDim, at.base + at.q0, kSlotBytes); };
+            if (before != 0) load_queries();           // the score products of the tile before have retired
+            // position rows: slot 0 held V0 (or K1), slot 1 held V1 of the tile before
+            load_pair(sm.tail, kTailBytes / 2, &map_p16, B_P_IN, 0, head * kPosRows + 256, 2 * kSlotBytes + kTailBytes);
+            if (before & 1u) ATT_WARP_WAIT(B_PV_DONE + 0, ph_before & 1u);
+            if (before != 0 && !(before & 1u)) ATT_WARP_WAIT(B_PV_DONE + 1, (ph_before >> 1) & 1u);
+            load_pair(sm.slot[0], kAtomBytes, &map_p, B_P_IN, 0, head * kPosRows, 0);
+            if (before != 0) ATT_WARP_WAIT(B_PV_DONE + 1, (ph_before >> 1) & 1u);
+            load_pair(sm.slot[1], kAtomBytes, &map_p, B_P_IN, 0, head * kPosRows + 128, 0);
+            if (before & 4u) ATT_WARP_WAIT(B_PV_DONE + 2, (ph_before >> 2) & 1u);
+            if (before == 0) {
+                if (p.early) grid_dependency_wait();
+                load_queries();
             }
+            if (blocks & 1u) load_block(slot_of_key(0), &map_k, B_K_IN + 0, 0);
+            // the other key blocks: once the position rows have been multiplied
+            ATT_WARP_WAIT(B_QP_DONE, par);
+            ATT_WARP_WAIT(B_VP_DONE, par);
+            load_block(slot_of_key(1), &map_k, B_K_IN + 1, 1);
+            if (blocks & 4u) load_block(slot_of_key(2), &map_k, B_K_IN + 2, 2);
+            // values: V0 after K1, V1 after K2 (or the position rows), V2 after K0
+            ATT_WARP_WAIT(B_S_DONE + 1, par);
+            ATT_WARP_WAIT(B_UK_DONE + 1, par);
+            if (blocks & 1u) load_block(0, &map_v, B_V_IN + 0, 0);
+            if (blocks & 4u) {
+                ATT_WARP_WAIT(B_S_DONE + 2, (ph >> 2) & 1u);
+                ATT_WARP_WAIT(B_UK_DONE + 2, (ph >> 2) & 1u);
+            }
+            load_block(1, &map_v, B_V_IN + 1, 1);
+            if (blocks & 4u) {
+                if (blocks & 1u) {
+                    ATT_WARP_WAIT(B_S_DONE + 0, ph & 1u);
+                    ATT_WARP_WAIT(B_UK_DONE + 0, ph & 1u);
+                }
+                load_block(2, &map_v, B_V_IN + 2, 2);
+            }
+            before = blocks;
+            ph_before = ph;
+            ph ^= blocks;
         }
     } else if (warp == kSoftmaxWarps + 1) {
         // ------------------------------------------------------------- MMA issuer
-        if (lane == 0) {
-            constexpr uint32_t idesc128 = make_instr_desc<KIND_F16>(128, 128);
-            constexpr uint32_t idesc16 = make_instr_desc<KIND_F16>(128, 16);
-            // B = V[keys, features] as it lies in memory: MN-major (features contiguous),
-            // 8-key groups 1024 bytes apart, the second 64 features 16 KB on; 16 keys = 2048 bytes
-            constexpr uint32_t idesc_v = idesc128 | (1u << 16);
-            const uint64_t desc_q = make_smem_desc<128>(smem_u32(sm.q)), desc_tail = make_smem_desc<128>(smem_u32(sm.tail));
-            const uint64_t desc_slot[2] = {make_smem_desc<128>(smem_u32(sm.slot[0])), make_smem_desc<128>(smem_u32(sm.slot[1]))};
-            // K step of 16 halves inside a K-major operand block, in descriptor units of 16 bytes
-            auto k_offset = [](int ks) { return static_cast<uint32_t>((ks / 4) * (kAtomBytes / 16) + 2 * (ks % 4)); };
-            bool any = false;
-            int tile = first_tile - 1;
-            if (!p.early) grid_dependency_wait();              // (the geometry)
-            for (int item = first_item; ok && item < last_item; ++item) {
-                if (++tile == p.tiles) tile = 0;
-                const TilePlace at(p.rows, tile);
-                if (at.padding()) continue;
-                const uint32_t blocks = at.blocks(), par = (ph >> 1) & 1u;
-                ATT_WAIT(B_Q_IN, par);
-                ATT_WAIT(B_P_IN, par);
-                tc_fence_after_sync();
-                // (columns [0, 272) are free: P_READY of the tile before came after their last read)
-#pragma unroll 1
+        constexpr uint32_t idesc128 = make_instr_desc<KIND_F16>(128, 128);
+        constexpr uint32_t idesc16 = make_instr_desc<KIND_F16>(128, 16);
+        // B = V[keys, features] as it lies in memory: MN-major (features contiguous),
+        // 8-key groups 1024 bytes apart, the second 64 features 16 KB on; 16 keys = 2048 bytes
+        constexpr uint32_t idesc_v = idesc128 | (1u << 16);
+        const uint64_t desc_q = make_smem_desc<128>(smem_u32(sm.q)), desc_tail = make_smem_desc<128>(smem_u32(sm.tail));
+        const uint64_t desc_slot[2] = {make_smem_desc<128>(smem_u32(sm.slot[0])), make_smem_desc<128>(smem_u32(sm.slot[1]))};
+        // K step of 16 halves inside a K-major operand block, in descriptor units of 16 bytes
+        auto k_offset = [](int ks) { return static_cast<uint32_t>((ks / 4) * (kAtomBytes / 16) + 2 * (ks % 4)); };
+        bool any = false;
+        int tile = first_tile - 1;
+        if (!p.early) grid_dependency_wait();          // (the geometry)
+        for (int item = first_item; ok && item < last_item; ++item) {
+            if (++tile == p.tiles) tile = 0;
+            const TilePlace at(p.rows, tile);
+            if (at.padding()) continue;
+            const uint32_t blocks = at.blocks(), par = (ph >> 1) & 1u;
+            ATT_WARP_WAIT(B_Q_IN, par);
+            ATT_WARP_WAIT(B_P_IN, par);
+            tc_fence_after_sync();
+            // (columns [0, 272) are free: P_READY of the tile before came after their last read)
+            if (elect_one()) {
+#pragma unroll
                 for (int ks = 0; ks < 8; ++ks) {           // 16 features per MMA
                     const uint32_t off = k_offset(ks);
                     tc_mma<KIND_F16>(tmem, desc_q + off, desc_slot[0] + off, idesc128, ks > 0);
@@ -326,42 +328,48 @@ local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const 
                     tc_mma<KIND_F16>(tmem + 256u, desc_q + off, desc_tail + (ks / 4) * (kTailBytes / 32) + 2u * (ks % 4), idesc16, ks > 0);
                 }
                 tc_commit(&sm.bar[B_QP_DONE]);
-                // S_0 and the context share their columns
-                if (any) ATT_WAIT(B_CTX_READ, par ^ 1u);
-                any = true;
+            }
+            __syncwarp();
+            // S_0 and the context share their columns
+            if (any) ATT_WARP_WAIT(B_CTX_READ, par ^ 1u);
+            any = true;
 #pragma unroll 1
-                for (int b = 0; b < 3; ++b) {
-                    if (!((blocks >> b) & 1u)) continue;
-                    if (b == 1) ATT_WAIT(B_QP_DRAINED, par);   // columns [0, 272) are free
-                    ATT_WAIT(B_K_IN + b, (ph >> b) & 1u);
-                    tc_fence_after_sync();
-                    const uint64_t desc_k = desc_slot[0] + static_cast<uint32_t>(slot_of_key(b) * (kSlotBytes / 16));
-#pragma unroll 1
+            for (int b = 0; b < 3; ++b) {
+                if (!((blocks >> b) & 1u)) continue;
+                if (b == 1) ATT_WARP_WAIT(B_QP_DRAINED, par);   // columns [0, 272) are free
+                ATT_WARP_WAIT(B_K_IN + b, (ph >> b) & 1u);
+                tc_fence_after_sync();
+                const uint64_t desc_k = desc_slot[0] + static_cast<uint32_t>(slot_of_key(b) * (kSlotBytes / 16));
+                if (elect_one()) {
+#pragma unroll
                     for (int ks = 0; ks < 8; ++ks)
                         tc_mma<KIND_F16>(tmem + score_col(b), desc_q + k_offset(ks), desc_k + k_offset(ks), idesc128, ks > 0);
                     tc_commit(&sm.bar[B_S_DONE + b]);
                 }
-                if (!ok) break;
-                uint32_t accumulate = 0;
+                __syncwarp();
+            }
+            if (!ok) break;
+            uint32_t accumulate = 0;
 #pragma unroll 1
-                for (int b = 0; b < 3; ++b) {
-                    if (!((blocks >> b) & 1u)) continue;
-                    ATT_WAIT(B_V_IN + b, (ph >> b) & 1u);
-                    ATT_WAIT(B_P_READY + b, (ph >> b) & 1u);
-                    tc_fence_after_sync();
-                    const uint64_t desc_v = static_cast<uint64_t>((smem_u32(sm.slot[b]) & 0x3FFFFu) >> 4) |
-                                            (static_cast<uint64_t>(kAtomBytes >> 4) << 16) | (64ull << 32) |
-                                            (1ull << 46) | (2ull << 61);
-                    const uint64_t desc_p = make_smem_desc<128>(smem_u32(sm.pr[b & 1]));
-#pragma unroll 1
-                    for (int ks = 0; ks < 8; ++ks) {       // 16 keys per MMA
-                        tc_mma<KIND_F16>(tmem + kCtxCol, desc_p + k_offset(ks), desc_v + ks * 128u, idesc_v, accumulate);
-                        accumulate = 1;
-                    }
+            for (int b = 0; b < 3; ++b) {
+                if (!((blocks >> b) & 1u)) continue;
+                ATT_WARP_WAIT(B_V_IN + b, (ph >> b) & 1u);
+                ATT_WARP_WAIT(B_P_READY + b, (ph >> b) & 1u);
+                tc_fence_after_sync();
+                const uint64_t desc_v = static_cast<uint64_t>((smem_u32(sm.slot[b]) & 0x3FFFFu) >> 4) |
+                                        (static_cast<uint64_t>(kAtomBytes >> 4) << 16) | (64ull << 32) |
+                                        (1ull << 46) | (2ull << 61);
+                const uint64_t desc_p = make_smem_desc<128>(smem_u32(sm.pr[b & 1]));
+                if (elect_one()) {
+#pragma unroll
+                    for (int ks = 0; ks < 8; ++ks)         // 16 keys per MMA
+                        tc_mma<KIND_F16>(tmem + kCtxCol, desc_p + k_offset(ks), desc_v + ks * 128u, idesc_v, ks > 0 ? 1u : accumulate);
                     tc_commit(&sm.bar[B_PV_DONE + b]);
                 }
-                ph ^= blocks;
+                __syncwarp();
+                accumulate = 1;
             }
+            ph ^= blocks;
         }
     } else {
         // ------------------------------------------ bias terms, QP drain, softmax, output
