@@ -104,3 +104,30 @@ def test_packed_rows_are_the_rows_of_the_uniform_layout(pk, cuda, precision, fra
         assert torch.equal(out[base[u]:base[u] + rows[u]], want[u * seg:u * seg + rows[u]])
     uniform = sub.run_rows(mel, frames, seg, mf, torch.empty_like(want))
     assert torch.equal(uniform, want) and bool(want.any())
+
+
+@pytest.mark.parametrize("frames", [1, 2, 3, 5, 8, 129, 1030])
+def test_first_stage_on_tensor_cores_at_the_edges(pk, cuda, frames):
+    """The E4M3 variant's first convolution (tensor cores, up to 32 output frames per CTA) against the oracle at the
+    shortest utterances and around the ends of a CTA's range; infinite mel values and taps end where they ended on
+    the fp32 pipes: a tap outside the utterance is not multiplied."""
+    w = pk.synth.subsampling_weights(3)
+    mel = pk.synth.mel_input(90 + frames, frames) * 3.0
+    sub = pk.subsampling.Subsampling(w, cuda, precision="fp8")
+    rows = pk.subsampling.output_frames(frames)
+    stride = pk.pipeline.seg_stride_for(rows)
+    got = host(sub.run(dev(mel[None]), stride))[:rows]
+    assert int(sub.status.item()) == 0
+    want = O.subsampling(mel, w, fp8=True)
+    assert nrmse(got, want) <= 1e-2                  # as in test_subsampling_matches_oracle
+    # a tap of -inf on the first frame row (never inside a one-frame utterance) and on the left column
+    odd = {k: v.copy() for k, v in w.items()}
+    odd["conv0_w"][5, 0] = -np.inf                   # frame tap 0, feature tap 0: outside at frame 0 and at feature 0
+    odd["conv0_w"][5, 1] = -np.inf if frames == 1 else odd["conv0_w"][5, 1]
+    sub = pk.subsampling.Subsampling(odd, cuda, precision="fp8")
+    got = host(sub.run(dev(np.abs(mel)[None] + 1.0), stride))[:rows]
+    if frames == 1:                                  # the taps never meet a value: the result of finite ones
+        odd["conv0_w"][5, 0] = odd["conv0_w"][5, 1] = 0.0
+        want = O.subsampling(np.abs(mel) + 1.0, odd, fp8=True)
+        assert nrmse(got, want) <= 1e-2
+    assert np.isfinite(got).all()                    # -inf sums end at the ReLU
