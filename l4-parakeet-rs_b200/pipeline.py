@@ -420,12 +420,14 @@ class PipelineEngine:
             # subsampling output with room for the dropped rows in front of a 128-aligned block
             self._chunk_rows = torch.zeros((self.seg_stride + 128, 1024), dtype=torch.float16, device=self.device)
             self._chunk_valid = torch.zeros(1, dtype=torch.int32, device=self.device)
-        self.sub.run(self.mel_dev[:1], self.seg_stride + 128, mel_frames=self.mel_frames_dev[:1], out=self._chunk_rows)
-        x = self._chunk_rows[lead_rows:lead_rows + self.seg_stride]
+        # rows laid out for this chunk, not for the engine's capacity (the bits do not depend on the padding)
+        seg = max(seg_stride_for(rows), 128)
+        self.sub.run_rows(self.mel_dev[:1], max(frames, 1), seg_stride_for(sub_mod.output_frames(frames)) + 128,
+                          self.mel_frames_dev[:1], self._chunk_rows)
         self._chunk_valid.fill_(rows)
-        encoded = self.enc.run(x, self.state_b[:self.seg_stride], self.ws, 1, self.seg_stride, rows,
+        encoded = self.enc.run(self._chunk_rows[lead_rows:lead_rows + seg], self.state_b[:seg], self.ws, 1, seg, rows,
                                seg_valid=self._chunk_valid)
-        self.dec.project(encoded, out=self.enc_proj[:self.seg_stride])
+        self.dec.project(encoded, out=self.enc_proj[:seg])
         return self.enc_proj[:rows]
 
     # ---- optional stage in front: PCM -> log-mel (src/cuda/pipeline.rs:437-470 runs it first)

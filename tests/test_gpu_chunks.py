@@ -108,3 +108,19 @@ def test_long_utterance_from_mel_in_two_chunks(pk, cuda):
     tokens, _, counts = eng.dec.decode(rows_dev, 1, 1536, fr, 15000, lstm_cache="int8")
     torch.cuda.synchronize()
     assert np.array_equal(host(tokens)[0][:int(host(counts)[0])], whole_tokens) and len(whole_tokens) > 100
+
+
+@pytest.mark.parametrize("rows,lead", [(1, 0), (128, 0), (129, 1), (700, 1), (1500, 0)])
+def test_chunk_rows_do_not_depend_on_the_engine(pk, cuda, rows, lead):
+    """`encode_chunk` lays its rows out for the chunk: an engine of twice the chunk's size, after a longer chunk, gives
+    the rows of an engine that just fits it."""
+    frames = 8 * (rows + lead)
+    mel = torch.from_numpy(pk.synth.mel_input(78, frames))
+    out = []
+    for cap in (frames, 2 * frames + 1000):
+        eng = pk.pipeline.PipelineEngine(cuda, layers=LAYERS, decoder_layers=1, seed=6, max_utterances=1, mel_frames=cap)
+        if cap > frames:
+            eng.encode_chunk(torch.from_numpy(pk.synth.mel_input(79, cap)), 0, cap // 8)
+        out.append(host(eng.encode_chunk(mel, lead, rows)).copy())
+        assert out[-1].shape == (rows, 640) and eng.status() == 0
+    assert np.array_equal(out[0], out[1]) and np.abs(out[0]).max() > 0
