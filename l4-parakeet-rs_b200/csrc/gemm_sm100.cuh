@@ -447,18 +447,19 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         __syncthreads();
     }
 
-    // The roles that issue TMA and MMA instructions run their loops with the whole warp and elect a lane for the
-    // instructions alone: their operands live in uniform registers, which the compiler has to fill one by one
-    // behind a lane test.  Cycles a K block of four MMAs cost its issuer (the tensor core takes 128 to 512) behind a
-    // lane test / so: 532 / 400 with 64-column tiles, 844 / 661 with 256-column tiles of K = 1024; the TMA issuers
-    // 330 / 210.  us, before / after: FF expand 30.6 / 28.5 at 6144 rows, 194 / 178 at 45 056; FF contract 12.4 / 10.7
-    // at 768, 23.2 / 21.9 at 6144; output projection 9.1 / 8.3 at 768; INT4 28.8 / 25.6 at 6144 x 1024, 72 / 64 at
-    // 6144 x 4096.
+    // The roles that issue TMA and MMA instructions run their loops with the whole warp and predicate the
+    // instructions alone on an elected lane: their operands live in uniform registers, which the compiler has to fill
+    // one by one behind a lane test, and a branch around them costs its reconvergence.  Cycles a K block of four MMAs
+    // cost its issuer (the tensor core takes 128 to 512) behind a lane test / behind a branch on the elected lane: 532 /
+    // 400 with 64-column tiles, 844 / 661 with 256-column tiles of K = 1024; the TMA issuers 330 / 210.  us, lane test /
+    // branch / predicates: FF expand 30.6 / 27.0 / 25.5 at 6144 rows; FF contract 12.4 / 10.9 / 9.8 at 768, 23.2 / 21.9 /
+    // 21.2 at 6144; output projection 9.1 / 8.0 / 7.3 at 768; INT4 28.8 / 24.8 / 23.8 at 6144 x 1024.
     auto warp_wait = [&](uint64_t* bar, uint32_t parity) {
         return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, abort_flag)) != 0;
     };
     if (warp == 0) {
         // ------------------------------------------------------ TMA producer
+        const bool leader = elect_one();
         int stage = 0;
         uint32_t phase = 0;
         bool ok = true;
@@ -472,11 +473,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                     ok = false;
                     break;
                 }
-                if (elect_one()) {
-                    uint8_t* sa = smem + stage * Smem::kStageBytes;
-                    [[maybe_unused]] uint8_t* sb = sa + Smem::kStageA;
-                    if constexpr (CtaGroup == 2) {
-                        // the leader's barrier counts the bytes of both CTAs
+                uint8_t* sa = smem + stage * Smem::kStageBytes;
+                if constexpr (CtaGroup == 2) {
+                    if (leader) {
+                        uint8_t* sb = sa + Smem::kStageA;
+                        // the leading CTA's barrier counts the bytes of both
                         if (rank == 0) mbar_arrive_expect_tx(full_bar + stage, 2 * Smem::kStageBytes);
                         const uint32_t bar = map_to_cta(smem_u32(full_bar + stage), 0);
                         int n_rows;
@@ -487,19 +488,18 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                         }
                         tma_load_2d_pair(sa, &map_a, bar, kb * kBlockK, m0);
                         tma_load_2d_pair(sb, &map_b, bar, kb * kBlockK, n_rows);
-                    } else if constexpr (BSrc == BSRC_TMA) {
-                        mbar_arrive_expect_tx(full_bar + stage, Smem::kStageA);
-                        tma_load_2d(sa, &map_a, full_bar + stage, kb * kBlockK, m0);
-                    } else {
-                        // 128-row boxes of A, one per accumulator that has rows
-                        const bool second = m0 + kBlockM < p.m;
-                        mbar_arrive_expect_tx(full_bar + stage, second ? Smem::kStageA : Smem::kStageA / 2);
-                        tma_load_2d(sa, &map_a, full_bar + stage, kb * kBlockK, m0);
-                        if (second)
-                            tma_load_2d(sa + Smem::kStageA / 2, &map_a, full_bar + stage, kb * kBlockK, m0 + kBlockM);
                     }
+                    __syncwarp();
+                } else if constexpr (BSrc == BSRC_TMA) {
+                    mbar_arrive_expect_tx_if(leader, full_bar + stage, Smem::kStageA);
+                    tma_load_2d_if(leader, sa, &map_a, full_bar + stage, kb * kBlockK, m0);
+                } else {
+                    // 128-row boxes of A, one per accumulator that has rows
+                    const bool second = m0 + kBlockM < p.m;
+                    mbar_arrive_expect_tx_if(leader, full_bar + stage, second ? Smem::kStageA : Smem::kStageA / 2);
+                    tma_load_2d_if(leader, sa, &map_a, full_bar + stage, kb * kBlockK, m0);
+                    tma_load_2d_if(leader && second, sa + Smem::kStageA / 2, &map_a, full_bar + stage, kb * kBlockK, m0 + kBlockM);
                 }
-                __syncwarp();
                 if (++stage == kStages) {
                     stage = 0;
                     phase ^= 1u;
@@ -509,6 +509,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     } else if (warp == GemmWarps<BSrc>::kProducerB) {
         // -------------------------------------------------- B (or code) producer
         if (CtaGroup == 1) {
+            const bool leader = elect_one();
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -522,17 +523,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                             ok = false;
                             break;
                         }
-                        if (elect_one()) {
-                            uint8_t* sb = smem + stage * Smem::kStageBytes + Smem::kStageA;
-                            mbar_arrive_expect_tx(full_bar + stage, Smem::kStageB);
-                            if constexpr (Epi == EPI_GLU) {                // boxes of values and of their gates
-                                tma_load_2d(sb, &map_b, full_bar + stage, kb * kBlockK, nt * kBHalf);
-                                tma_load_2d(sb + kBHalf * SwizzleBytes, &map_b, full_bar + stage, kb * kBlockK, p.n / 2 + nt * kBHalf);
-                            } else {
-                                tma_load_2d(sb, &map_b, full_bar + stage, kb * kBlockK, nt * BlockN);
-                            }
+                        uint8_t* sb = smem + stage * Smem::kStageBytes + Smem::kStageA;
+                        mbar_arrive_expect_tx_if(leader, full_bar + stage, Smem::kStageB);
+                        if constexpr (Epi == EPI_GLU) {                // boxes of values and of their gates
+                            tma_load_2d_if(leader, sb, &map_b, full_bar + stage, kb * kBlockK, nt * kBHalf);
+                            tma_load_2d_if(leader, sb + kBHalf * SwizzleBytes, &map_b, full_bar + stage, kb * kBlockK, p.n / 2 + nt * kBHalf);
+                        } else {
+                            tma_load_2d_if(leader, sb, &map_b, full_bar + stage, kb * kBlockK, nt * BlockN);
                         }
-                        __syncwarp();
                         if (++stage == kStages) {
                             stage = 0;
                             phase ^= 1u;
@@ -545,11 +543,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                             ok = false;
                             break;
                         }
-                        if (elect_one()) {
-                            mbar_arrive_expect_tx(code_full_bar + stage, Smem::kCodeBytes / 2);
-                            tma_load_2d(code_smem + stage * (Smem::kCodeBytes / 2), &map_b, code_full_bar + stage, kb * 32, nt * BlockN);
-                        }
-                        __syncwarp();
+                        mbar_arrive_expect_tx_if(leader, code_full_bar + stage, Smem::kCodeBytes / 2);
+                        tma_load_2d_if(leader, code_smem + stage * (Smem::kCodeBytes / 2), &map_b, code_full_bar + stage, kb * 32, nt * BlockN);
                         stage ^= 1;
                         phase ^= stage == 0 ? 1u : 0u;
                     }
@@ -559,6 +554,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     } else if (warp == 1) {
         // -------------------------------------------------------- MMA issuer
         if (rank == 0) {
+            const bool leader = elect_one();
             constexpr uint32_t idesc = make_instr_desc<Kind>(kBlockM * CtaGroup, BlockN);
             int stage = 0;
             uint32_t phase = 0;
@@ -584,36 +580,30 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                         break;
                     }
                     tc_fence_after_sync();
-                    if (elect_one()) {
-                        const uint32_t sa = smem_u32(smem + stage * Smem::kStageBytes);
-                        const uint32_t sb = sa + Smem::kStageA;
-                        const uint64_t desc_a = make_smem_desc<SwizzleBytes>(sa);
-                        const uint64_t desc_b = make_smem_desc<SwizzleBytes>(sb);
-                        bool first = accumulate == 0;
+                    const uint32_t sa = smem_u32(smem + stage * Smem::kStageBytes);
+                    const uint32_t sb = sa + Smem::kStageA;
+                    const uint64_t desc_a = make_smem_desc<SwizzleBytes>(sa);
+                    const uint64_t desc_b = make_smem_desc<SwizzleBytes>(sb);
+                    if constexpr (CtaGroup == 2) {
+                        if (leader) {
+#pragma unroll
+                            for (int j = 0; j < kMmasPerBlock; ++j)
+                                tc_mma_pair<Kind>(tmem_d, desc_a + 2u * j, desc_b + 2u * j, idesc, j > 0 ? 1u : accumulate);
+                            // free the stage in both CTAs of the pair once the MMAs retire
+                            tc_commit_pair(map_to_cta(smem_u32(empty_bar + stage), 0));
+                            tc_commit_pair(map_to_cta(smem_u32(empty_bar + stage), 1));
+                        }
+                    } else {
 #pragma unroll
                         for (int j = 0; j < kMmasPerBlock; ++j) {
                             // advance 32 bytes along K inside the swizzle atom: +2 in 16-byte units
-                            if constexpr (CtaGroup == 2)
-                                tc_mma_pair<Kind>(tmem_d, desc_a + 2u * j, desc_b + 2u * j, idesc, first ? 0u : 1u);
-                            else
-                                tc_mma<Kind>(tmem_d, desc_a + 2u * j, desc_b + 2u * j, idesc, first ? 0u : 1u);
-                            if constexpr (kMTiles == 2) {
-                                // the second 128 rows of A (16 KB on: 1024 descriptor units) against the same B
-                                if (second)
-                                    tc_mma<Kind>(tmem_d + BlockN, desc_a + 1024u + 2u * j, desc_b + 2u * j, idesc, first ? 0u : 1u);
-                            }
-                            first = false;
+                            tc_mma_if<Kind>(leader, tmem_d, desc_a + 2u * j, desc_b + 2u * j, idesc, j > 0 ? 1u : accumulate);
+                            // the second 128 rows of A (16 KB on: 1024 descriptor units) against the same B
+                            if constexpr (kMTiles == 2) tc_mma_if<Kind>(leader && second, tmem_d + BlockN, desc_a + 1024u + 2u * j, desc_b + 2u * j, idesc, j > 0 ? 1u : accumulate);
                         }
-                        // free the stage (in both CTAs of a pair) once the MMAs retire
-                        if constexpr (CtaGroup == 2) {
-                            tc_commit_pair(map_to_cta(smem_u32(empty_bar + stage), 0));
-                            tc_commit_pair(map_to_cta(smem_u32(empty_bar + stage), 1));
-                        } else {
-                            tc_commit(empty_bar + stage);
-                        }
+                        tc_commit_if(leader, empty_bar + stage);       // free the stage once the MMAs retire
                     }
                     accumulate = 1;
-                    __syncwarp();
                     if (++stage == kStages) {
                         stage = 0;
                         phase ^= 1u;

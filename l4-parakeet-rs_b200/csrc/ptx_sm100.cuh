@@ -280,6 +280,35 @@ __device__ __forceinline__ void tmem_ld_wait() {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// The same, issued where `leader` is set: a predicate on the instruction instead of a branch around it.
+template <int Kind>
+__device__ __forceinline__ void tc_mma_if(bool leader, uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+    if constexpr (Kind == KIND_F16)
+        asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
+            ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(static_cast<uint32_t>(leader)) : "memory");
+    else if constexpr (Kind == KIND_F8)
+        asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t@q tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}\n"
+            ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(static_cast<uint32_t>(leader)) : "memory");
+    else
+        asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t@q tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}\n"
+            ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(static_cast<uint32_t>(leader)) : "memory");
+}
+__device__ __forceinline__ void tc_commit_if(bool leader, uint64_t* bar) {
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n"
+                 ::"r"(smem_u32(bar)), "r"(static_cast<uint32_t>(leader)) : "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive_expect_tx_if(bool leader, uint64_t* bar, uint32_t bytes) {
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}\n"
+                 ::"r"(smem_u32(bar)), "r"(bytes), "r"(static_cast<uint32_t>(leader)) : "memory");
+}
+__device__ __forceinline__ void tma_load_2d_if(bool leader, void* smem_dst, const CUtensorMap* map, uint64_t* bar, int32_t c0, int32_t c1) {
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+                 "@q cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t}\n"
+                 ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1),
+                   "r"(static_cast<uint32_t>(leader)) : "memory");
+}
+
 // ------------------------------------------------- CTA pairs (cta_group::2)
 // Two CTAs of a cluster share one 256-row MMA tile: each stages its own 128 rows of A and
 // half of the B rows, the even ("leader") CTA issues the MMAs for both, each CTA keeps the
