@@ -5,7 +5,7 @@ inside libpk100.so.  Tensors must be CUDA and contiguous where stated.
 """
 from __future__ import annotations
 
-import ctypes as C
+import struct
 
 import torch
 
@@ -14,12 +14,21 @@ from . import lib as L
 EPS = 1e-5
 
 
+# The arguments of a GEMM as bytes (native sizes and alignment): filling the structure field by field took half of
+# the host time of a launch.
+_GEMM_ARGS = struct.Struct("@" + "".join({L.i32: "i", L.f32: "f", L.vp: "P"}[t] for _, t in L.GemmArgs._fields_) + "0P")
+assert _GEMM_ARGS.size == L.C.sizeof(L.GemmArgs)
+_gemm = L.lib["pk100_gemm"]                      # (a function object of its own, with bytes as its argument)
+_gemm.argtypes, _gemm.restype = [L.vp, L.C.c_char_p], L.i32
+
+
 def _ptr(t):
-    return None if t is None else C.c_void_p(t.data_ptr())
+    return 0 if t is None else t.data_ptr()
 
 
 def _stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    # torch.cuda.current_stream().cuda_stream without the Stream object around it
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _need(t, dtype=None):
@@ -37,22 +46,19 @@ def gemm(a, b, *, kind, out, epilogue=L.EPI_LINEAR, row_scales=None, row_scale=1
     """D = epilogue(A . B^T); see `pk100_gemm` in include/pk100.h."""
     _need(a), _need(b), _need(out)
     m, k = a.shape
-    nn = b.shape[0] if n is None else n
-    args = L.GemmArgs(
-        kind=kind, epilogue=epilogue, m=m, n=nn, k=k,
-        a=a.data_ptr(), lda=a.stride(0), b=b.data_ptr(), ldb=b.stride(0),
-        row_scales=None if row_scales is None else row_scales.data_ptr(), row_scale=row_scale,
-        col_scales=None if col_scales is None else col_scales.data_ptr(),
-        bias=None if bias is None else bias.data_ptr(), act=act,
-        residual=None if residual is None else residual.data_ptr(),
-        ld_res=0 if residual is None else residual.stride(0), alpha=alpha, valid_rows=valid_rows,
-        out=out.data_ptr(), ld_out=out.stride(0), out_type=out_type, out_scale=out_scale, tau=tau,
-        keep_out=None if keep_out is None else keep_out.data_ptr(),
-        stats_out=None if stats_out is None else stats_out.data_ptr(),
-        keep_in=None if keep_in is None else keep_in.data_ptr(),
-        status=None if status is None else status.data_ptr(), max_ctas=max_ctas,
-        b_group_scales=None if b_group_scales is None else b_group_scales.data_ptr())
-    L.check(L.lib.pk100_gemm(_stream(), C.byref(args)), "pk100_gemm")
+    fields = (                                   # in the order of GemmArgs
+        kind, epilogue, m, b.shape[0] if n is None else n, k,
+        a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0),
+        _ptr(row_scales), row_scale, _ptr(col_scales), _ptr(bias),
+        act, _ptr(residual), 0 if residual is None else residual.stride(0), alpha, valid_rows,
+        out.data_ptr(), out.stride(0), out_type, out_scale,
+        tau, _ptr(keep_out), _ptr(stats_out), _ptr(keep_in),
+        _ptr(status), max_ctas, _ptr(b_group_scales))
+    try:
+        args = _GEMM_ARGS.pack(*fields)
+    except (struct.error, OverflowError):        # what only the structure's own conversions take
+        args = bytes(L.GemmArgs(*fields))
+    L.check(_gemm(_stream(), args), "pk100_gemm")
     return out
 
 
