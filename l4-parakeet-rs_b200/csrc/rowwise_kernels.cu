@@ -523,10 +523,14 @@ __global__ void glu_masked_kernel(const __half* __restrict__ in, __half* __restr
 // One CTA = 256 threads x 4 channels = all 1024 channels of a strip of kStrip rows; the 8 halo rows come
 // from L2.  Two neighbouring channels share every packed fp32 instruction (fma.rn.f32x2 and friends,
 // each half rounds like the scalar one).  A window of 9 rows slides down the strip in registers;
-// the row's E4M3 scale takes one warp reduction and one exchange through shared memory.  Long strips read
+// the row's E4M3 scale takes one warp reduction and one exchange through shared memory; scale and divisor of eight
+// rows are formed once per warp, a row per lane, and handed round by shuffles (every thread
+// formed them for every row before).  Long strips read
 // fewer halo rows, short ones keep every SM busy: 16 rows where that gives the device two CTAs per SM,
-// else 8.  Bound by issue slots (convolution, BatchNorm, SiLU and E4M3 rounding of every element).  45 056
-// rows: 155 us with scalar instructions and full divisions, 91 us now; 768 rows: 10.6 -> 6.2 us.
+// else 8 (strips of 32 rows: 77 -> 75 us at 45 056 rows, 42.7 -> 44.7 at 24 576).  Bound by issue slots
+// (convolution, BatchNorm, SiLU and E4M3 rounding of every element).  us, divisors per thread / per lane: 94.4 / 77.2
+// at 45 056 rows, 16.6 / 13.7 at 6144, 5.8 / 5.0 at 768, 4.7 / 4.0 at 128 (155 at 45 056 with scalar instructions and
+// full divisions).
 template <bool Quantize, int kStrip>
 __global__ void __launch_bounds__(256, 2)
 depthwise_bn_silu_kernel(const __half* __restrict__ in, const __half* __restrict__ wdw,
@@ -627,18 +631,23 @@ depthwise_bn_silu_kernel(const __half* __restrict__ in, const __half* __restrict
                 if (lane == 0) s_max[blk][i][warp] = __uint_as_float(mx);
             }
         }
-        if constexpr (Quantize) __syncthreads();
+        RowDivisor mine(1.0f, 1.0f);                   // lane j: that of row j mod 8 of the block
+        if constexpr (Quantize) {
+            __syncthreads();
+            const int row = lane % 8;
+            const float4 a = *reinterpret_cast<const float4*>(&s_max[blk][row][0]), b = *reinterpret_cast<const float4*>(&s_max[blk][row][4]);
+            const float mx = fmaxf(fmaxf(fmaxf(a.x, a.y), fmaxf(a.z, a.w)), fmaxf(fmaxf(b.x, b.y), fmaxf(b.z, b.w)));
+            const float scale = mx > 0.0f ? __fdiv_rn(mx, 448.0f) : 1.0f;
+            mine = RowDivisor(scale);
+            if (tid < 8 && r0 + blk * 8 + tid < stride) row_scales[base + r0 + blk * 8 + tid] = scale;
+        }
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const int r = r0 + blk * 8 + i;
-            if (r >= stride) continue;
+            if (r >= stride) continue;                 // the same for the whole CTA
             const size_t grow = base + r;
             if constexpr (Quantize) {
-                const float4 a = *reinterpret_cast<const float4*>(&s_max[blk][i][0]), b = *reinterpret_cast<const float4*>(&s_max[blk][i][4]);
-                const float mx = fmaxf(fmaxf(fmaxf(a.x, a.y), fmaxf(a.z, a.w)), fmaxf(fmaxf(b.x, b.y), fmaxf(b.z, b.w)));
-                const float scale = mx > 0.0f ? __fdiv_rn(mx, 448.0f) : 1.0f;
-                const RowDivisor div(scale);
-                if (tid == 0) row_scales[grow] = scale;
+                const RowDivisor div(__shfl_sync(0xffffffffu, mine.s, i), __shfl_sync(0xffffffffu, mine.y, i));
                 const float2 p = __half22float2(y[i][0]), q = __half22float2(y[i][1]);
                 const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(div(p.x), div(p.y)), __NV_SATFINITE, __NV_E4M3);
                 const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(div(q.x), div(q.y)), __NV_SATFINITE, __NV_E4M3);
