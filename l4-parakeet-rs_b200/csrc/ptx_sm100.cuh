@@ -202,7 +202,7 @@ __device__ __forceinline__ void tc_commit(uint64_t* bar) {
                  ::"r"(smem_u32(bar)) : "memory");
 }
 
-enum : int { KIND_F16 = 0, KIND_F8 = 1, KIND_I8 = 2, KIND_TF32 = 3 };
+enum : int { KIND_F16 = 0, KIND_F8 = 1, KIND_I8 = 2 };
 
 // D[tmem] (+)= A[smem] * B[smem]^T, M x N x (32 bytes of K) per instruction.
 template <int Kind>
@@ -217,11 +217,6 @@ __device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint64_t desc_a, uint64_
         asm volatile(
             "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
             "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}\n"
-            ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
-    } else if constexpr (Kind == KIND_TF32) {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}\n"
             ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
     } else {
         asm volatile(
@@ -270,10 +265,6 @@ __device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r
 }
 __device__ __forceinline__ void tmem_st_wait() {
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-}
-
-__device__ __forceinline__ void tmem_ld_32x1(uint32_t taddr, uint32_t& r) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(r) : "r"(taddr) : "memory");
 }
 
 __device__ __forceinline__ void tmem_ld_wait() {
@@ -401,11 +392,11 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr) {
 
 // Instruction descriptor: dense, K-major A and B, M x N tile.
 //   c_format [4,6): 1 = F32, 2 = S32;  a_format [7,10), b_format [10,13):
-//   kind::f16: 0 = F16;  kind::f8f6f4: 0 = E4M3;  kind::i8: 1 = signed;  kind::tf32: 2 = TF32.
+//   kind::f16: 0 = F16;  kind::f8f6f4: 0 = E4M3;  kind::i8: 1 = signed.
 template <int Kind>
 __host__ __device__ constexpr uint32_t make_instr_desc(int m, int n) {
     const uint32_t c_format = Kind == KIND_I8 ? 2u : 1u;
-    const uint32_t ab_format = Kind == KIND_I8 ? 1u : (Kind == KIND_TF32 ? 2u : 0u);
+    const uint32_t ab_format = Kind == KIND_I8 ? 1u : 0u;
     return (c_format << 4) | (ab_format << 7) | (ab_format << 10) |
            (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
 }

@@ -25,12 +25,9 @@ __device__ __forceinline__ int frames_of(const int* per_utt, int utt, int unifor
 
 // both halves rounded to fp16 and through ReLU; a NaN becomes 0 (max.f16x2 returns the operand that is a number,
 // the .relu form of the conversion would keep it)
-__device__ __forceinline__ __half2 relu_half2(float x, float y) {
-    return __hmax2(__floats2half2_rn(x, y), __half2half2(__ushort_as_half(0)));
-}
 __device__ __forceinline__ __half2 relu_half2(Pair v) {
     const float2 f = halves_of(v);
-    return relu_half2(f.x, f.y);
+    return __hmax2(__floats2half2_rn(f.x, f.y), __half2half2(__ushort_as_half(0)));
 }
 
 // E4M3 codes of one row, absmax / 448 per row: the arithmetic of pk100_pack_weight_rows
@@ -49,7 +46,10 @@ __device__ __forceinline__ float e4m3_row_scale(float absmax) { return absmax > 
 // is the reference's (kernels/sm89/subsampling.cu:11-179); the out-of-range taps it skips are zero
 // taps on zero values here.
 // Bound by its fp32 multiply-adds (about 6000 packed warp instructions per output frame).  8 x 60 s: 405 us
-// with one frame per CTA, one channel per thread and three rows per frame, 330 us now.
+// with one frame per CTA, one channel per thread and three rows per frame, 330 us now (E4M3 372 us, where
+// a quantising pass of 270 us followed before).
+// Fp8: the result leaves as E4M3 with one scale per (frame, feature) row of 256 channels; each row
+// is first rounded to fp16, as when a separate kernel quantises the fp16 tensor.
 // in [utt][in_stride frames][128] fp32 -> out [utt][out_cap][32][256]
 constexpr int kFirstOuts = 8;                              // output features per thread
 constexpr int kFirstMaxFrames = 8;
@@ -57,14 +57,18 @@ constexpr int first_rows(int frames) { return 4 * frames + 3; }   // mel rows 4*
 constexpr int kFirstThreads = 256;                         // 128 channel pairs x 2 parts
 constexpr int kFirstPitch = kMelBins + 2;                  // column t at index t + 1, one zero column on each side
 
+template <bool Fp8>
 __global__ void __launch_bounds__(kFirstThreads, 2)
 subsample_first_fused_kernel(const float* __restrict__ in, const __half* __restrict__ w0,
                              const __half* __restrict__ b0, const __half* __restrict__ w1,
-                             const __half* __restrict__ b1, __half* __restrict__ out,
+                             const __half* __restrict__ b1, void* __restrict__ out, float* __restrict__ out_scales,
                              int in_stride, int in_frames_uniform, const int* __restrict__ in_frames_per_utt,
                              int out_cap, int run) {
     extern __shared__ __align__(16) uint8_t first_smem[];
     auto mel = reinterpret_cast<float2 (*)[kFirstPitch]>(first_smem);      // [first_rows(run)]
+    constexpr int kRows = 2 * kFirstOuts;                  // output features of this CTA
+    __shared__ float row_max[2][4][kRows];                 // [frame parity][warp of a part][feature]
+    __shared__ float2 row_div[2][kRows];                   // [frame parity][feature]: divisor and reciprocal
     __shared__ Pair taps[2][9][kChannels / 2];             // both convolutions' taps as channel pairs
     const int tid = threadIdx.x;
     const int ch = (tid % 128) * 2;                        // channels ch, ch + 1
@@ -191,308 +195,46 @@ subsample_first_fused_kernel(const float* __restrict__ in, const __half* __restr
             }
         }
         const size_t row0 = (static_cast<size_t>(utt) * out_cap + f2) * 32 + part * kFirstOuts;
-        __half* dst = out + row0 * kChannels + ch;
+        if constexpr (Fp8) {
+            const int warp = tid / 32, lane = tid % 32, local = (tid / 128) * kFirstOuts, par = i & 1;
+            __half2 h[kFirstOuts];
 #pragma unroll
-        for (int m = 0; m < kFirstOuts; ++m) {
-            const float2 f = halves_of(cur[m]);
-            *reinterpret_cast<__half2*>(dst + static_cast<size_t>(m) * kChannels) = __floats2half2_rn(f.x, f.y);
+            for (int m = 0; m < kFirstOuts; ++m) {
+                const float2 f = halves_of(cur[m]);
+                h[m] = __floats2half2_rn(f.x, f.y);
+                const float2 r = __half22float2(__habs2(h[m]));
+                // non-negative floats order like their bits
+                const unsigned top = __reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(r.x, r.y)));
+                if (lane == 0) row_max[par][warp % 4][local + m] = __uint_as_float(top);
+            }
+            __syncthreads();
+            if (tid < kRows) {                             // one division and one reciprocal per row
+                const float scale = e4m3_row_scale(fmaxf(fmaxf(row_max[par][0][tid], row_max[par][1][tid]),
+                                                         fmaxf(row_max[par][2][tid], row_max[par][3][tid])));
+                const RowDivisor div(scale);
+                row_div[par][tid] = make_float2(div.s, div.y);
+                out_scales[(static_cast<size_t>(utt) * out_cap + f2) * 32 + blockIdx.z * kRows + tid] = scale;
+            }
+            __syncthreads();
+            uint8_t* dst = static_cast<uint8_t*>(out) + row0 * kChannels + ch;
+#pragma unroll
+            for (int m = 0; m < kFirstOuts; ++m) {
+                const float2 d = row_div[par][local + m];
+                const RowDivisor div(d.x, d.y);
+                const float2 f = __half22float2(h[m]);
+                *reinterpret_cast<uint16_t*>(dst + static_cast<size_t>(m) * kChannels) =
+                    static_cast<uint16_t>(__nv_cvt_float2_to_fp8x2(make_float2(div(f.x), div(f.y)), __NV_SATFINITE, __NV_E4M3));
+            }
+        } else {
+            __half* dst = static_cast<__half*>(out) + row0 * kChannels + ch;
+#pragma unroll
+            for (int m = 0; m < kFirstOuts; ++m) {
+                const float2 f = halves_of(cur[m]);
+                *reinterpret_cast<__half2*>(dst + static_cast<size_t>(m) * kChannels) = __floats2half2_rn(f.x, f.y);
+            }
         }
 #pragma unroll
         for (int m = 0; m < kFirstOuts; ++m) cur[m] = next[m];
-    }
-}
-
-// The same two convolutions for the E4M3 variant with the first one on the tensor cores: its inputs are a
-// contraction of 9 taps per (frame, feature), done as tcgen05.mma kind::tf32 with D[channel][feature] =
-// taps[channel][K = 32] . columns[feature][K = 32].  A mel value enters as three tf32 parts that add up to it
-// exactly (11 + 11 + 2 bits of its 24) against the same fp16 tap, which tf32 holds exactly: K = 9 taps x 3 parts,
-// then 1 x bias, so every product is exact and the sum is an fp32 one, as before (its order is the tensor core's).
-// The fp16 variant keeps the fp32 pipes: its rounding to fp16 is that of the reference's sequence of sums.
-// The result leaves as E4M3 with one scale per (frame, feature) row of 256 channels; each row is first rounded to
-// fp16, as when a separate kernel quantises the fp16 tensor.
-// An accumulator row is a channel and lies in one thread's TMEM lane, so the thread walks the features of its
-// channel like the kernel above: ReLU, fp16 rounding, depthwise sums of 16 output features in registers.
-//   warps 0-15   channel = 128 * half + TMEM lane, half of the 64 features each
-//   warps 16-17  one thread per feature builds the columns of the next intermediate row and one issues its MMAs;
-//                columns and accumulators are double-buffered.
-// Bound by the step of a row: build, MMAs, read and depthwise sums, with two rows in flight (issue slots 54 %, tensor
-// pipe 9 %).  The whole E4M3 stage at 8 x 60 s: 568 us with the first convolution on the fp32 pipes, 457 us; one
-// utterance of 60 s 116 -> 97 us.  Error of the stage's result against 64 bits: 5.1208e-2, 5.0595e-2, 5.0411e-2 at
-// 100, 1201 and 6000 frames in both forms.
-constexpr int kConvMaxFrames = 32;                         // output frames of a CTA
-constexpr int kConvFeats = kMelBins / 2;                   // 64 features of an intermediate row
-constexpr int kConvOuts = 16;                              // output features per thread
-constexpr int kConvWarps = 16, kConvThreads = 32 * (kConvWarps + 2);
-constexpr uint32_t kConvTmemCols = 2 * 2 * kConvFeats;     // two buffers x two channel halves
-
-struct ConvSmem {
-    alignas(1024) uint8_t taps[2][128 * 128];              // [channel half]: 128 rows of 32 tf32, 128-byte swizzle
-    alignas(1024) uint8_t columns[2][kConvFeats * 128];    // [buffer]: 64 rows of 32 tf32
-    float row_max[2][8][32];                               // [frame parity][32 channels][output feature]
-    alignas(16) float2 row_div[2][32];                     // [frame parity][output feature]: divisor and reciprocal
-    uint64_t full[2], empty[2];
-    uint32_t tmem_base;
-    int abort;
-    float mel[first_rows(kConvMaxFrames)][kFirstPitch];    // column t at index t + 1
-};
-
-__global__ void __launch_bounds__(kConvThreads, 1)
-subsample_first_tcgen05_kernel(const float* __restrict__ in, const __half* __restrict__ w0, const __half* __restrict__ b0,
-                               const __half* __restrict__ w1, const __half* __restrict__ b1, uint8_t* __restrict__ out,
-                               float* __restrict__ out_scales, int in_stride, int in_frames_uniform,
-                               const int* __restrict__ in_frames_per_utt, int out_cap, int run, int* status) {
-    extern __shared__ uint8_t conv_raw[];
-    ConvSmem& sm = *reinterpret_cast<ConvSmem*>((reinterpret_cast<uintptr_t>(conv_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid / 32, 0), lane = tid % 32;
-    const int first = blockIdx.x * run, utt = blockIdx.y;
-    const int in_frames = frames_of(in_frames_per_utt, utt, in_frames_uniform);
-    const int f1_frames = (in_frames + 1) / 2, f2_frames = (f1_frames + 1) / 2;
-    if (first >= f2_frames) return;
-    const int frames = min(run, f2_frames - first);
-    // intermediate row k is row 2 * first - 1 + k; row 0 only where it exists, the last one likewise
-    const int k_first = first > 0 ? 0 : 1, k_last = 2 * frames - 1 + (2 * (first + frames - 1) + 1 < f1_frames ? 1 : 0);
-    volatile int* abort_flag = &sm.abort;
-
-    // ---- set-up: mel rows, taps as the A operand, barriers, tensor memory
-    const float* src = in + static_cast<size_t>(utt) * in_stride * kMelBins;
-    for (int i = tid; i < first_rows(frames) * kFirstPitch; i += kConvThreads) {
-        const int row = i / kFirstPitch, t = i % kFirstPitch - 1;
-        const int f = 4 * first - 3 + row;
-        (&sm.mel[0][0])[i] = (f >= 0 && f < in_frames && t >= 0 && t < kMelBins) ? src[static_cast<size_t>(f) * kMelBins + t] : 0.0f;
-    }
-    for (int i = tid; i < kChannels * 8; i += kConvThreads) {
-        const int c = i / 8, chunk = i % 8;
-        float v[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int k = chunk * 4 + e;
-            v[e] = k < 27 ? __half2float(w0[c * 9 + k / 3]) : k == 27 ? __half2float(b0[c]) : 0.0f;
-        }
-        *reinterpret_cast<float4*>(sm.taps[c / 128] + (c % 128) * 128 + ((chunk ^ (c & 7)) << 4)) = make_float4(v[0], v[1], v[2], v[3]);
-    }
-    fence_proxy_async_smem();
-    if (tid == 0) {
-        sm.abort = 0;
-        for (int i = 0; i < 2; ++i) {
-            mbar_init(&sm.full[i], 1);
-            mbar_init(&sm.empty[i], kConvWarps);
-        }
-        fence_barrier_init();
-    }
-    if (warp == kConvWarps) {
-        tmem_alloc(&sm.tmem_base, kConvTmemCols);
-        tmem_relinquish();
-    }
-    tc_fence_before_sync();
-    __syncthreads();
-    tc_fence_after_sync();
-    const uint32_t tmem = sm.tmem_base;
-
-    if (warp >= kConvWarps) {
-        // ---------------------------------------------- columns of the next row, MMAs
-        const int m = tid - 32 * kConvWarps;               // feature
-        constexpr uint32_t idesc = make_instr_desc<KIND_TF32>(128, kConvFeats);
-        // barrier of the two warps; they leave together when a wait of either gave up
-        auto both_warps = [](bool mine) {
-            uint32_t all;
-            asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbarrier.cta.red.and.pred p, 2, 64, q;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
-                         : "=r"(all) : "r"(static_cast<uint32_t>(mine)) : "memory");
-            return all != 0;
-        };
-        for (int k = k_first; k <= k_last; ++k) {
-            const int n = k - k_first, buf = n & 1;
-            const bool got = mbar_wait_bounded(&sm.empty[buf], ((n >> 1) & 1) ^ 1u, abort_flag);
-            float v[32];
-#pragma unroll
-            for (int a = 0; a < 3; ++a)
-#pragma unroll
-                for (int t = 0; t < 3; ++t) {
-                    const float x = sm.mel[2 * k + a][2 * m + t];
-                    const float hi = __uint_as_float(__float_as_uint(x) & 0xFFFFE000u);
-                    const float rest = isinf(x) ? 0.0f : x - hi;
-                    const float mid = __uint_as_float(__float_as_uint(rest) & 0xFFFFE000u);
-                    v[(a * 3 + t) * 3] = hi;
-                    v[(a * 3 + t) * 3 + 1] = mid;
-                    v[(a * 3 + t) * 3 + 2] = rest - mid;
-                }
-            v[27] = 1.0f;
-            v[28] = v[29] = v[30] = v[31] = 0.0f;
-            uint8_t* row = sm.columns[buf] + m * 128;
-#pragma unroll
-            for (int c = 0; c < 8; ++c)
-                *reinterpret_cast<float4*>(row + ((c ^ (m & 7)) << 4)) = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
-            fence_proxy_async_smem();
-            if (!both_warps(got)) break;
-            if (warp == kConvWarps) {                      // (the whole warp, so that the operands are uniform)
-                tc_fence_after_sync();
-                const uint64_t desc_b = make_smem_desc<128>(smem_u32(sm.columns[buf]));
-                if (elect_one()) {
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const uint64_t desc_a = make_smem_desc<128>(smem_u32(sm.taps[h]));
-#pragma unroll
-                        for (int ks = 0; ks < 4; ++ks)
-                            tc_mma<KIND_TF32>(tmem + buf * 2 * kConvFeats + h * kConvFeats, desc_a + 2u * ks, desc_b + 2u * ks, idesc, ks > 0);
-                    }
-                    tc_commit(&sm.full[buf]);
-                }
-                __syncwarp();
-            }
-        }
-    } else {
-        // ---------------------------------------------- ReLU, fp16, depthwise convolution, E4M3 rows
-        const int quad = warp % 4, half = (warp / 4) % 2, part = warp / 8;
-        const int ch = half * 128 + quad * 32 + lane;
-        const uint32_t lane_addr = tmem + (static_cast<uint32_t>(quad * 32) << 16) + half * kConvFeats + part * 2 * kConvOuts;
-        float taps[9];
-#pragma unroll
-        for (int i = 0; i < 9; ++i) taps[i] = __half2float(w1[ch * 9 + i]);
-        const float bias1 = __half2float(b1[ch]);
-        // A tap outside the utterance is not multiplied: that shows where the tap is not finite (0 x inf), so such
-        // a channel is summed here
-        bool odd = false;
-#pragma unroll
-        for (int i = 0; i < 9; ++i) odd |= (__half_as_ushort(w0[ch * 9 + i]) & 0x7C00) == 0x7C00;
-        const bool any_odd = __any_sync(0xffffffffu, odd);
-        auto plain_sum = [&](int k, int feat) {
-            float acc = __half2float(b0[ch]);
-            const int f1 = 2 * first - 1 + k;
-            for (int a = 0; a < 3; ++a)
-                for (int t = 0; t < 3; ++t) {
-                    const int f = 2 * f1 - 1 + a;
-                    if (f >= 0 && f < in_frames && 2 * feat + t > 0) acc = fmaf(sm.mel[2 * k + a][2 * feat + t], __half2float(w0[ch * 9 + a * 3 + t]), acc);
-                }
-            return __float_as_uint(acc);
-        };
-        float cur[kConvOuts], next[kConvOuts];
-#pragma unroll
-        for (int j = 0; j < kConvOuts; ++j) cur[j] = bias1;
-        bool ok = true;
-        // row k as frame taps `kf` of `sums` (and taps 0 of `next` where `both`)
-        auto walk_row = [&](int k, auto kf_c, auto both_c, float (&sums)[kConvOuts]) {
-            constexpr int kf = decltype(kf_c)::value;
-            constexpr bool both = decltype(both_c)::value;
-            const int n = k - k_first, buf = n & 1;
-            ok = __all_sync(0xffffffffu, mbar_wait_bounded(&sm.full[buf], (n >> 1) & 1, abort_flag)) && ok;
-            tc_fence_after_sync();
-            const uint32_t at = lane_addr + buf * 2 * kConvFeats;
-            float left = 0.0f;
-            if (part > 0) {                                // the odd feature left of the first output
-                uint32_t r;
-                tmem_ld_32x1(at - 1u, r);
-                tmem_ld_wait();
-                if (odd) r = plain_sum(k, part * 2 * kConvOuts - 1);
-                left = __half2float(__float2half_rn(fmaxf(__uint_as_float(r), 0.0f)));
-            }
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                uint32_t r[16];
-                __syncwarp();
-                tmem_ld_32x16(at + 16 * i, r);
-                tmem_ld_wait();
-                if (i == 1) {                              // everything of this row has been read
-                    tc_fence_before_sync();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&sm.empty[buf]);
-                }
-                if (any_odd && odd) {
-#pragma unroll 1
-                    for (int j = 0; j < 16; ++j) {
-                        const uint32_t v = plain_sum(k, part * 2 * kConvOuts + 16 * i + j);
-#pragma unroll
-                        for (int e = 0; e < 16; ++e) r[e] = e == j ? v : r[e];
-                    }
-                }
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const int m = 8 * i + j;               // output feature kConvOuts * part + m
-                    const float2 f = __half22float2(relu_half2(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1])));
-                    if (m > 0 || part > 0) {
-                        sums[m] = fmaf(left, taps[kf * 3], sums[m]);
-                        if constexpr (both) next[m] = fmaf(left, taps[0], next[m]);
-                    }
-                    sums[m] = fmaf(f.y, taps[kf * 3 + 2], fmaf(f.x, taps[kf * 3 + 1], sums[m]));
-                    if constexpr (both) next[m] = fmaf(f.y, taps[2], fmaf(f.x, taps[1], next[m]));
-                    left = f.y;
-                }
-            }
-        };
-        using std::integral_constant;
-        if (first > 0) walk_row(0, integral_constant<int, 0>{}, std::false_type{}, cur);
-#pragma unroll 1
-        for (int i = 0; i < frames; ++i) {
-            const int f2 = first + i, par = i & 1;
-#pragma unroll
-            for (int j = 0; j < kConvOuts; ++j) next[j] = bias1;
-            walk_row(2 * i + 1, integral_constant<int, 1>{}, std::false_type{}, cur);
-            if (2 * i + 2 <= k_last) walk_row(2 * i + 2, integral_constant<int, 2>{}, std::true_type{}, cur);
-            // largest |value| of each output feature over the warp's channels: the pairs of features are dealt over
-            // the lanes while they are reduced (9 shuffles for 16 maxima; a NaN is no maximum)
-            __half2 h[kConvOuts / 2];
-            uint32_t top[kConvOuts / 2];
-            __syncwarp();
-#pragma unroll
-            for (int j = 0; j < kConvOuts / 2; ++j) {
-                h[j] = __floats2half2_rn(cur[2 * j], cur[2 * j + 1]);
-                cur[2 * j] = next[2 * j];
-                cur[2 * j + 1] = next[2 * j + 1];
-                const __half2 a = __hmax2(__habs2(h[j]), __half2half2(__ushort_as_half(0)));
-                top[j] = *reinterpret_cast<const uint32_t*>(&a);
-            }
-            auto max2 = [](uint32_t x, uint32_t y) {
-                const __half2 m = __hmax2(*reinterpret_cast<const __half2*>(&x), *reinterpret_cast<const __half2*>(&y));
-                return *reinterpret_cast<const uint32_t*>(&m);
-            };
-#pragma unroll
-            for (int n = kConvOuts / 4; n >= 1; n /= 2) {   // n pairs stay, those of the upper lanes are the upper ones
-                const bool upper = (lane & (4 * n)) != 0;
-#pragma unroll
-                for (int j = 0; j < n; ++j) {
-                    const uint32_t mine = upper ? top[j + n] : top[j], theirs = upper ? top[j] : top[j + n];
-                    top[j] = max2(mine, __shfl_xor_sync(0xffffffffu, theirs, 4 * n));
-                }
-            }
-            top[0] = max2(top[0], __shfl_xor_sync(0xffffffffu, top[0], 2));
-            top[0] = max2(top[0], __shfl_xor_sync(0xffffffffu, top[0], 1));
-            if (lane % 4 == 0)
-                *reinterpret_cast<float2*>(&sm.row_max[par][half * 4 + quad][part * kConvOuts + 2 * (lane / 4)]) =
-                    __half22float2(*reinterpret_cast<const __half2*>(&top[0]));
-            asm volatile("bar.sync 1, 512;" ::: "memory");
-            const size_t row0 = (static_cast<size_t>(utt) * out_cap + f2) * 32;
-            if (tid < 32) {                                // one division and one reciprocal per row
-                float top = sm.row_max[par][0][tid];
-#pragma unroll
-                for (int g = 1; g < 8; ++g) top = fmaxf(top, sm.row_max[par][g][tid]);
-                const float scale = e4m3_row_scale(top);
-                const RowDivisor div(scale);
-                sm.row_div[par][tid] = make_float2(div.s, div.y);
-                out_scales[row0 + tid] = scale;
-            }
-            asm volatile("bar.sync 1, 512;" ::: "memory");
-            uint8_t* dst = out + (row0 + part * kConvOuts) * kChannels + ch;
-#pragma unroll
-            for (int j = 0; j < kConvOuts / 2; ++j) {
-                const float4 d = *reinterpret_cast<const float4*>(&sm.row_div[par][part * kConvOuts + 2 * j]);
-                const RowDivisor div0(d.x, d.y), div1(d.z, d.w);
-                const float2 f = __half22float2(h[j]);
-                const unsigned codes = __nv_cvt_float2_to_fp8x2(make_float2(div0(f.x), div1(f.y)), __NV_SATFINITE, __NV_E4M3);
-                dst[static_cast<size_t>(2 * j) * kChannels] = static_cast<uint8_t>(codes);
-                dst[static_cast<size_t>(2 * j + 1) * kChannels] = static_cast<uint8_t>(codes >> 8);
-            }
-        }
-        if (!ok && lane == 0 && status != nullptr) atomicExch(status, 1);
-    }
-    if (*abort_flag != 0) {
-        // MMAs still in flight land before shared and tensor memory are released
-        const uint64_t start = global_timer_ns();
-        while (global_timer_ns() - start < 200000ull) __nanosleep(1000);
-        if (tid == 0 && status != nullptr) atomicExch(status, 1);
-    }
-    tc_fence_before_sync();
-    __syncthreads();
-    if (warp == kConvWarps) {
-        tc_fence_after_sync();
-        tmem_dealloc(tmem, kConvTmemCols);
     }
 }
 
@@ -747,29 +489,18 @@ static int run_subsampling(void* stream_v, const pk100_subsampling_weights* w, c
 
     const auto *w0 = static_cast<const __half*>(w->conv0_w), *b0 = static_cast<const __half*>(w->conv0_b);
     const auto *w1 = static_cast<const __half*>(w->dw1_w), *b1 = static_cast<const __half*>(w->dw1_b);
-    // frames per CTA: whole waves over the device, each CTA with at most `most` frames
-    const long long sms = pk100_cta_budget(), total = u * c.f2;
-    auto frames_per_cta = [&](int most) {
-        const long long waves = (total + sms * most - 1) / (sms * most);
-        return static_cast<int>((total + sms * waves - 1) / (sms * waves));
-    };
-    if (q != nullptr) {
-        constexpr int bytes = static_cast<int>(sizeof(ConvSmem)) + 1024;
-        const cudaError_t err = cudaFuncSetAttribute(subsample_first_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        if (err != cudaSuccess) return static_cast<int>(err);
-        const int run = frames_per_cta(kConvMaxFrames);
-        subsample_first_tcgen05_kernel<<<dim3((c.f2 + run - 1) / run, utterances), kConvThreads, bytes, stream>>>(
-            mel, w0, b0, w1, b1, q2, q2_scales, mel_stride, frames, mel_frames, c.f2, run, status);
-    } else {
-        // (a frame range takes two CTAs, one per half of the features, on the 2 that an SM holds)
-        const cudaError_t err = cudaFuncSetAttribute(subsample_first_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     sizeof(float2) * kFirstPitch * first_rows(kFirstMaxFrames));
-        if (err != cudaSuccess) return static_cast<int>(err);
-        const int run = frames_per_cta(kFirstMaxFrames);
-        subsample_first_fused_kernel<<<dim3((c.f2 + run - 1) / run, utterances, 32 / (2 * kFirstOuts)), kFirstThreads,
-                                       sizeof(float2) * kFirstPitch * first_rows(run), stream>>>(
-            mel, w0, b0, w1, b1, s2, mel_stride, frames, mel_frames, c.f2, run);
-    }
+    // frames per CTA: whole waves over the 2 resident CTAs of every SM (a frame range takes two CTAs, one per
+    // half of the features), each CTA with at most kFirstMaxFrames frames
+    const long long sms = pk100_cta_budget(), total = u * c.f2, waves = (total + sms * kFirstMaxFrames - 1) / (sms * kFirstMaxFrames);
+    const int run = static_cast<int>((total + sms * waves - 1) / (sms * waves));
+    const dim3 first_grid((c.f2 + run - 1) / run, utterances, 32 / (2 * kFirstOuts));
+    const size_t first_bytes = sizeof(float2) * kFirstPitch * first_rows(run);
+    auto first_kernel = q != nullptr ? subsample_first_fused_kernel<true> : subsample_first_fused_kernel<false>;
+    const cudaError_t err = cudaFuncSetAttribute(first_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 sizeof(float2) * kFirstPitch * first_rows(kFirstMaxFrames));
+    if (err != cudaSuccess) return static_cast<int>(err);
+    first_kernel<<<first_grid, kFirstThreads, first_bytes, stream>>>(mel, w0, b0, w1, b1, q != nullptr ? static_cast<void*>(q2) : s2,
+                                                                     q2_scales, mel_stride, frames, mel_frames, c.f2, run);
     int rc = pk100_launch_status();
     if (rc != PK100_OK) return rc;
 

@@ -469,12 +469,17 @@ def _conv_s2(x, w, b):
     reference's tap order (kernels/sm89/subsampling.cu:37-58, :100-124)."""
     f_in, t_in, _ = x.shape
     f_out, t_out = (f_in + 1) // 2, (t_in + 1) // 2
-    xp = np.zeros((2 * f_out + 2, 2 * t_out + 2, x.shape[2]), dtype=F32)
-    xp[1:1 + f_in, 1:1 + t_in] = x
     acc = np.broadcast_to(np.asarray(b, dtype=F32), (f_out, t_out, 256)).copy()
+
+    def inside(tap, n_in, n_out):
+        """Outputs whose input 2 * output - 1 + tap exists, and those inputs: taps outside are not multiplied."""
+        lo, hi = int(tap == 0), min(n_out, (n_in - tap) // 2 + 1)
+        return slice(lo, hi), slice(2 * lo - 1 + tap, max(2 * hi - 2 + tap, 0), 2)
+
     for kf in range(3):
         for kt in range(3):
-            acc += xp[kf:kf + 2 * f_out:2, kt:kt + 2 * t_out:2] * np.asarray(w, dtype=F32)[:, kf, kt]
+            (fo, fi), (to, ti) = inside(kf, f_in, f_out), inside(kt, t_in, t_out)
+            acc[fo, to] += np.asarray(x[fi, ti], dtype=F32) * np.asarray(w, dtype=F32)[:, kf, kt]
     return acc
 
 

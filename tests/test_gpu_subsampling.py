@@ -106,28 +106,58 @@ def test_packed_rows_are_the_rows_of_the_uniform_layout(pk, cuda, precision, fra
     assert torch.equal(uniform, want) and bool(want.any())
 
 
+def _first_stage(sub, frames, stride):
+    """What the first kernel left in the workspace after a run of one utterance: fp16 rows, or E4M3 codes and scales."""
+    def up256(n):
+        return (n + 255) // 256 * 256
+
+    f2 = ((frames + 1) // 2 + 1) // 2
+    f3 = (f2 + 1) // 2
+    rows = f2 * 32
+    if sub.q is None:
+        return sub._ws[:rows * 512].view(torch.float16).view(rows, 256).clone()
+    at = 2 * up256(rows * 512) + 2 * up256(f3 * 16 * 512) + up256(stride * 8192) + 256
+    codes = sub._ws[at:at + rows * 256].view(rows, 256).clone()
+    at += up256(rows * 256)
+    return codes, sub._ws[at:at + rows * 4].view(torch.float32).clone()
+
+
+@pytest.mark.parametrize("frames", [1, 2, 3, 5, 8, 129, 1030, 4001])
+def test_e4m3_variant_codes_the_rows_of_the_fp16_variant(pk, cuda, frames):
+    """Both variants take the same fp32 sums in the same order and round them to fp16; the E4M3 variant then codes the
+    rows: codes and scales are those of the quantiser on the fp16 variant's rows, bit for bit."""
+    w = pk.synth.subsampling_weights(3)
+    mel = dev(pk.synth.mel_input(90 + frames, frames)[None] * 3.0)
+    stride = pk.pipeline.seg_stride_for(pk.subsampling.output_frames(frames))
+    stages = []
+    for precision in ("fp16", "fp8"):
+        sub = pk.subsampling.Subsampling(w, cuda, precision=precision)
+        sub.run(mel, stride)
+        torch.cuda.synchronize()
+        assert int(sub.status.item()) == 0
+        stages.append(_first_stage(sub, frames, stride))
+    codes, scales = pk.ops.pack_weight_rows(stages[0], pk.lib.PACK_E4M3)
+    assert bool(stages[0].any()) and bool(torch.isfinite(stages[0]).all())
+    assert torch.equal(stages[1][0], codes.view(torch.uint8)) and torch.equal(stages[1][1], scales)
+
+
 @pytest.mark.parametrize("frames", [1, 2, 3, 5, 8, 129, 1030])
-def test_first_stage_on_tensor_cores_at_the_edges(pk, cuda, frames):
-    """The E4M3 variant's first convolution (tensor cores, up to 32 output frames per CTA) against the oracle at the
-    shortest utterances and around the ends of a CTA's range; infinite mel values and taps end where they ended on
-    the fp32 pipes: a tap outside the utterance is not multiplied."""
+def test_e4m3_variant_at_the_edges(pk, cuda, frames):
+    """The E4M3 variant against the oracle at the shortest utterances and around the ends of a CTA's range, with finite
+    taps and with taps of -inf: where such a tap lies inside, the sum ends at the ReLU; outside it is not
+    multiplied and the sum is that of the other taps."""
     w = pk.synth.subsampling_weights(3)
     mel = pk.synth.mel_input(90 + frames, frames) * 3.0
-    sub = pk.subsampling.Subsampling(w, cuda, precision="fp8")
     rows = pk.subsampling.output_frames(frames)
     stride = pk.pipeline.seg_stride_for(rows)
-    got = host(sub.run(dev(mel[None]), stride))[:rows]
-    assert int(sub.status.item()) == 0
-    want = O.subsampling(mel, w, fp8=True)
-    assert nrmse(got, want) <= 1e-2                  # as in test_subsampling_matches_oracle
-    # a tap of -inf on the first frame row (never inside a one-frame utterance) and on the left column
     odd = {k: v.copy() for k, v in w.items()}
     odd["conv0_w"][5, 0] = -np.inf                   # frame tap 0, feature tap 0: outside at frame 0 and at feature 0
-    odd["conv0_w"][5, 1] = -np.inf if frames == 1 else odd["conv0_w"][5, 1]
-    sub = pk.subsampling.Subsampling(odd, cuda, precision="fp8")
-    got = host(sub.run(dev(np.abs(mel)[None] + 1.0), stride))[:rows]
-    if frames == 1:                                  # the taps never meet a value: the result of finite ones
-        odd["conv0_w"][5, 0] = odd["conv0_w"][5, 1] = 0.0
-        want = O.subsampling(np.abs(mel) + 1.0, odd, fp8=True)
-        assert nrmse(got, want) <= 1e-2
-    assert np.isfinite(got).all()                    # -inf sums end at the ReLU
+    odd["conv0_w"][9, 7] = -np.inf                   # frame tap 2: outside at an odd utterance's last frame
+    odd["dw1_w"][[5, 9]] = 4.0                       # their features weigh in every row
+    for weights, x in ((w, mel), (odd, np.abs(mel) + 1.0)):
+        sub = pk.subsampling.Subsampling(weights, cuda, precision="fp8")
+        got = host(sub.run(dev(x[None]), stride))[:rows]
+        assert int(sub.status.item()) == 0
+        want = O.subsampling(x, weights, fp8=True)
+        assert np.isfinite(got).all() and np.isfinite(want).all()
+        assert nrmse(got, want) <= 1e-2              # as in test_subsampling_matches_oracle
