@@ -106,12 +106,14 @@ static int encode_map(CUtensorMap* map, const void* base, int elem_bytes, uint64
 
 // Tensor map of the output for the staged TMA store (256-column kernels, 128-column linear kernels): every epilogue
 // warp owns 32 rows x (tile columns / 4); INT4 weights: 32 rows x 64 columns at a time.  Only slices with 64- or 128-byte rows leave that way
-// (their swizzle modes); anything else keeps per-thread stores.  Returns the row bytes or 0.
+// (their swizzle modes); anything else keeps per-thread stores, and so does fp32 output, which the staging does not encode.
+// Returns the row bytes or 0.
 template <int Epi, int BlockN = 256, int BSrc = BSRC_TMA>
 static int make_out_map(CUtensorMap* map, const GemmParams& p) {
     const int out_cols = Epi == EPI_GLU ? p.n / 2 : p.n;
     const int cols_per_warp = BSrc == BSRC_W4G128 ? 64 : (Epi == EPI_GLU ? BlockN / 2 : BlockN) / (GemmWarps<BSRC_TMA>::kEpilogue / 4);
-    const int obytes = p.out_type == OUT_F16 ? 2 : (p.out_type == OUT_F32 ? 4 : 1);
+    if (p.out_type == OUT_F32) return 0;
+    const int obytes = p.out_type == OUT_F16 ? 2 : 1;
     const int row_bytes = cols_per_warp * obytes;
     if (row_bytes != 64 && row_bytes != 128) return 0;
     if (BSrc == BSRC_TMA && BlockN == 128 && row_bytes != 64) return 0;      // its staging holds 64-byte rows only

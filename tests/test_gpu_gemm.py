@@ -495,3 +495,32 @@ def test_sparse_out_narrow_tiles_give_the_bits_of_wide_tiles(pk, cuda, rows):
     assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
     assert torch.equal(results[0][2], results[1][2]) and results[0][3] == results[1][3]
     assert 0 < int(results[0][1].sum()) <= tiles * 64
+
+
+@pytest.mark.parametrize("kind", ["f16", "e4m3"])
+@pytest.mark.parametrize("m,n,k", [(1, 256, 128), (129, 512, 256), (300, 2048, 1024)])
+def test_glu_float_output_does_not_depend_on_the_tile_width(pk, cuda, kind, m, n, k):
+    """fp32 output of the GLU epilogue: 256-column tiles (which a cap on the CTAs forces) give the bits of 128-column
+    ones, and rounded to fp16 those of the fp16 output; ragged rows, an output wider than the matrix."""
+    L = pk.lib
+    g = torch.Generator().manual_seed(m + n)
+    w = (torch.randn((n, k), generator=g) * 0.05).half().to(cuda)
+    x = torch.randn((m, k), generator=g).half().to(cuda)
+    kw = {}
+    a, b, kid = x, w, L.KIND_F16
+    if kind == "e4m3":
+        b, kw["col_scales"] = pk.ops.pack_weight_rows(w, L.PACK_E4M3)
+        a, kw["row_scales"] = pk.ops.pack_weight_rows(x, L.PACK_E4M3)
+        kid = L.KIND_E4M3
+    st = _status(cuda)
+    outs = []
+    for ctas in (0, 1):
+        for dtype, code in ((torch.float32, L.OUT_F32), (torch.float16, L.OUT_F16)):
+            out = torch.full((m + 1, n // 2 + 8), 7.0, dtype=dtype, device=cuda)
+            pk.ops.gemm(a, b, kind=kid, epilogue=L.EPI_GLU, out=out[:m], out_type=code, status=st, max_ctas=ctas, **kw)
+            torch.cuda.synchronize()
+            assert bool((out[m] == 7.0).all()) and bool((out[:, n // 2:] == 7.0).all())
+            outs.append(out[:m, :n // 2])
+    assert int(st.item()) == 0
+    assert torch.equal(outs[0], outs[2]) and torch.equal(outs[1], outs[3])
+    assert torch.equal(outs[0].half(), outs[1]) and bool(outs[0].any())
