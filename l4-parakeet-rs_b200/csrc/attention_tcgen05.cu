@@ -309,7 +309,7 @@ local_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const 
         auto k_offset = [](int ks) { return static_cast<uint32_t>((ks / 4) * (kAtomBytes / 16) + 2 * (ks % 4)); };
         bool any = false;
         int tile = first_tile - 1;
-        if (!p.early) grid_dependency_wait();          // (the geometry)
+        grid_dependency_wait();          // geometry, Q: the bounded waits begin behind the kernel in front
         for (int item = first_item; ok && item < last_item; ++item) {
             if (++tile == p.tiles) tile = 0;
             const TilePlace at(p.rows, tile);

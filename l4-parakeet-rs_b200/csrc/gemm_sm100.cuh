@@ -425,9 +425,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_ptr_smem;
     // everything above touched only shared / tensor memory and kernel parameters: under a programmatic dependent
-    // launch it overlapped the previous kernel's tail.  Settled weights are requested meanwhile, as far as the ring
-    // takes them, so that their DRAM latency (they are read once per pass) is not on the chain of small launches.
-    if (!(warp == GemmWarps<BSrc>::kProducerB && p.b_settled != 0 && p.keep_in == nullptr)) grid_dependency_wait();
+    // launch it overlapped the previous kernel's tail.  Settled weights are requested meanwhile, as far as the empty
+    // ring takes them, so that their DRAM latency (they are read once per pass) is not on the chain of small
+    // launches; their producer waits for the previous kernel where it would wait for a stage to be freed, because
+    // that wait is bounded and the previous kernel is not.
+    const bool b_early = warp == GemmWarps<BSrc>::kProducerB && p.b_settled != 0 && p.keep_in == nullptr;
+    if (!b_early) grid_dependency_wait();
     if (balanced) {
         for (int t = static_cast<int>(threadIdx.x); t < m_tiles; t += static_cast<int>(blockDim.x)) {
             LiveMaskRow row;
@@ -510,6 +513,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         // -------------------------------------------------- B (or code) producer
         if (CtaGroup == 1) {
             const bool leader = elect_one();
+            int early = b_early ? (BSrc == BSRC_TMA ? kStages : 2) : -1;    // requests that the empty ring still takes
+            auto before_request = [&] {
+                if (early == 0) grid_dependency_wait();
+                if (early >= 0) --early;
+            };
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -519,6 +527,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                     const uint64_t live_mask = group_live_mask(mg);
                     for (int kb = 0; kb < k_blocks; ++kb) {
                         if (p.keep_in != nullptr && !k_block_live<SwizzleBytes>(live_mask, kb)) continue;
+                        before_request();
                         if (!warp_wait(empty_bar + stage, phase ^ 1u)) {
                             ok = false;
                             break;
@@ -539,6 +548,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                 } else {
                     // codes in groups of 4 K blocks (128 bytes of every row) through two buffers
                     for (int kb = 0; kb < k_blocks; kb += 4) {
+                        before_request();
                         if (!warp_wait(code_empty_bar + stage, phase ^ 1u)) {
                             ok = false;
                             break;
