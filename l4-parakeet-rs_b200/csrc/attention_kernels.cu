@@ -504,14 +504,8 @@ extern "C" int pk100_local_relpos_attention(
                               ldo, segments, seg_stride);
     if (rc != PK100_OK) return rc;
     if (segments == 0) return PK100_OK;
-    static bool configured = false;
-    if (!configured) {
-        const cudaError_t err = cudaFuncSetAttribute(local_attention_mma_kernel,
-                                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     static_cast<int>(sizeof(AttnSmem)));
-        if (err != cudaSuccess) return static_cast<int>(err);
-        configured = true;
-    }
+    const cudaError_t granted = pk100_grant_smem<local_attention_mma_kernel>(static_cast<int>(sizeof(AttnSmem)));
+    if (granted != cudaSuccess) return static_cast<int>(granted);
     AttnParams p{static_cast<const __half*>(query), ldq, static_cast<const __half*>(key), ldk,
                  static_cast<const __half*>(value), ldv, static_cast<const __half*>(position),
                  static_cast<const __half*>(bias_u), static_cast<const __half*>(bias_v),

@@ -688,13 +688,8 @@ int pk100_local_attention_rows(void* stream_v, const void* query, int ldq, const
     if (rc != PK100_OK) return rc;
 
     constexpr int smem_bytes = static_cast<int>(sizeof(Smem)) + 1024;
-    static bool configured = false;
-    if (!configured) {
-        const cudaError_t err = cudaFuncSetAttribute(local_attention_tcgen05_kernel,
-                                                     cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
-        if (err != cudaSuccess) return static_cast<int>(err);
-        configured = true;
-    }
+    const cudaError_t granted = pk100_grant_smem<local_attention_tcgen05_kernel>(smem_bytes);
+    if (granted != cudaSuccess) return static_cast<int>(granted);
     const int tiles = total_rows / kTile;
     Params p{static_cast<const __half*>(bias_u), static_cast<const __half*>(bias_v), static_cast<__half*>(output), ldo,
              tiles, geometry, constants_settled ? 1 : 0, status};

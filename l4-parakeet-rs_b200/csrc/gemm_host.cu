@@ -129,17 +129,6 @@ static int make_residual_map(CUtensorMap* map, const GemmParams& p) {
     return make_map(map, p.residual, 2, p.m, p.n, p.ld_res, 32, p.store_row_bytes) == PK100_OK ? 1 : 0;
 }
 
-static int sm_count() {
-    static int count = 0;
-    if (count == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev);
-        if (count <= 0) count = 148;
-    }
-    return count;
-}
-
 // CTA pairs (cta_group::2) for the 256-column kernels.  Off by default: on B200 the pair
 // path measured 5-15 % slower than one CTA per tile (the peer's B half arrives over the same
 // SM ingress as the TMA traffic it saves), so it is kept as a validated alternative.
@@ -152,7 +141,7 @@ static std::atomic<int> g_cta_cap{0};
 extern "C" void pk100_set_gemm_cta_cap(int ctas) { g_cta_cap.store(ctas > 0 ? ctas : 0); }
 static int shared_budget() {
     const int cap = g_cta_cap.load(std::memory_order_relaxed);
-    return cap > 0 && cap < sm_count() ? cap : sm_count();
+    return cap > 0 && cap < pk100_sm_count() ? cap : pk100_sm_count();
 }
 static int cta_budget(const pk100_gemm_args& a) { return a.max_ctas > 0 ? a.max_ctas : shared_budget(); }
 extern "C" void pk100_set_dependent_launch(int enable) { g_dependent_launch.store(enable != 0); }
@@ -166,14 +155,9 @@ static int launch_pair(const pk100_gemm_args& a, const GemmParams& p_in, cudaStr
     constexpr int BlockN = 256;
     using Smem = GemmSmem<BlockN / 2, SwizzleBytes, BlockN, gemm_store_bytes<Epi, BSRC_TMA, BlockN>()>;
     GemmParams p = p_in;
-    auto kernel = gemm_kernel<Kind, BlockN, SwizzleBytes, Epi, BSRC_TMA, 2>;
-    static bool configured = false;
-    if (!configured) {
-        const cudaError_t err = cudaFuncSetAttribute(
-            kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem::kTotal);
-        if (err != cudaSuccess) return static_cast<int>(err);
-        configured = true;
-    }
+    constexpr auto kernel = gemm_kernel<Kind, BlockN, SwizzleBytes, Epi, BSRC_TMA, 2>;
+    const cudaError_t granted = pk100_grant_smem<kernel>(Smem::kTotal);
+    if (granted != cudaSuccess) return static_cast<int>(granted);
     constexpr int elem = Kind == KIND_F16 ? 2 : 1;
     CUtensorMap map_a, map_b;
     int rc = make_map(&map_a, a.a, elem, a.m, a.k, a.lda, kBlockM, SwizzleBytes);
@@ -217,14 +201,9 @@ static int launch(const pk100_gemm_args& a, const GemmParams& p_in, cudaStream_t
     }
     using Smem = GemmSmem<BlockN, SwizzleBytes, BlockN, gemm_store_bytes<Epi, BSRC_TMA, BlockN>()>;
     GemmParams p = p_in;
-    auto kernel = gemm_kernel<Kind, BlockN, SwizzleBytes, Epi, BSRC_TMA>;
-    static bool configured = false;
-    if (!configured) {
-        const cudaError_t err = cudaFuncSetAttribute(
-            kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem::kTotal);
-        if (err != cudaSuccess) return static_cast<int>(err);
-        configured = true;
-    }
+    constexpr auto kernel = gemm_kernel<Kind, BlockN, SwizzleBytes, Epi, BSRC_TMA>;
+    const cudaError_t granted = pk100_grant_smem<kernel>(Smem::kTotal);
+    if (granted != cudaSuccess) return static_cast<int>(granted);
     constexpr int elem = Kind == KIND_F16 ? 2 : 1;
     CUtensorMap map_a, map_b;
     int rc = make_map(&map_a, a.a, elem, a.m, a.k, a.lda, kBlockM, SwizzleBytes);
@@ -251,14 +230,9 @@ static int launch_w4(const pk100_gemm_args& a, const GemmParams& p_in, cudaStrea
     using Smem = GemmSmem<BlockN, 128, BlockN * kMTiles, gemm_store_bytes<EPI_LINEAR, BSRC_W4G128, BlockN>(), kBlockM * kMTiles,
                           gemm_code_bytes<BSRC_W4G128>()>;
     GemmParams p = p_in;
-    auto kernel = gemm_kernel<KIND_F16, BlockN, 128, EPI_LINEAR, BSRC_W4G128>;
-    static bool configured = false;
-    if (!configured) {
-        const cudaError_t err = cudaFuncSetAttribute(
-            kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem::kTotal);
-        if (err != cudaSuccess) return static_cast<int>(err);
-        configured = true;
-    }
+    constexpr auto kernel = gemm_kernel<KIND_F16, BlockN, 128, EPI_LINEAR, BSRC_W4G128>;
+    const cudaError_t granted = pk100_grant_smem<kernel>(Smem::kTotal);
+    if (granted != cudaSuccess) return static_cast<int>(granted);
     CUtensorMap map_a, map_b;
     int rc = make_map(&map_a, a.a, 2, a.m, a.k, a.lda, kBlockM, 128);
     if (rc != PK100_OK) return rc;

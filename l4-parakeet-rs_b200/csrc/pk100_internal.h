@@ -4,6 +4,8 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
+
 #include "../../include/pk100.h"
 
 // Maps the sticky-free launch error of the last kernel launch to the ABI's
@@ -20,6 +22,34 @@ static inline int pk100_launch_status() {
     }
     cudaGetLastError();   // clear the non-sticky launch error so later calls are not poisoned
     return static_cast<int>(err);
+}
+
+// What belongs to one device is remembered per device (a process may drive several, from several threads); devices
+// behind the table are asked each time.
+constexpr int kPk100Devices = 64;
+
+// Lets `Kernel` use `bytes` of dynamic shared memory on the current device.
+template <auto Kernel>
+static inline cudaError_t pk100_grant_smem(int bytes) {
+    static std::atomic<bool> granted[kPk100Devices];
+    int dev = 0;
+    cudaError_t err = cudaGetDevice(&dev);
+    if (err != cudaSuccess) return err;
+    if (dev < kPk100Devices && granted[dev].load(std::memory_order_relaxed)) return cudaSuccess;
+    err = cudaFuncSetAttribute(reinterpret_cast<const void*>(Kernel), cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (err == cudaSuccess && dev < kPk100Devices) granted[dev].store(true, std::memory_order_relaxed);
+    return err;
+}
+
+// SMs of the current device (148 where it cannot be asked).
+inline int pk100_sm_count() {
+    static std::atomic<int> counts[kPk100Devices];
+    int dev = 0, count = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 148;
+    if (dev < kPk100Devices && (count = counts[dev].load(std::memory_order_relaxed)) > 0) return count;
+    if (cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || count <= 0) return 148;
+    if (dev < kPk100Devices) counts[dev].store(count, std::memory_order_relaxed);
+    return count;
 }
 
 // Programmatic dependent launch for the kernels of the per-block chain (LayerNorm, GEMMs,
