@@ -5,6 +5,7 @@
 
 #include <atomic>
 #include <mutex>
+#include <type_traits>
 
 #include "gemm_sm100.cuh"
 #include "pk100_internal.h"
@@ -123,10 +124,17 @@ static int make_out_map(CUtensorMap* map, const GemmParams& p) {
     return row_bytes;
 }
 
-// Tensor map of the residual with the boxes of the output slices (fp16 output leaving by TMA stores).
-static int make_residual_map(CUtensorMap* map, const GemmParams& p) {
-    if (p.residual == nullptr || p.store_row_bytes == 0 || p.out_type != OUT_F16) return 0;
-    return make_map(map, p.residual, 2, p.m, p.n, p.ld_res, 32, p.store_row_bytes) == PK100_OK ? 1 : 0;
+// Calls f(true or false type: the residual arrives by TMA, its tensor map).  It does where fp16 output leaves by TMA
+// stores: the map has the boxes of the output slices.
+template <int Epi, int BSrc, int BlockN, typename F>
+static int with_residual(const GemmParams& p, const CUtensorMap& any, F&& f) {
+    if constexpr (Epi == EPI_LINEAR && gemm_store_bytes<Epi, BSrc, BlockN>() > 0) {
+        CUtensorMap map;
+        if (p.residual != nullptr && p.store_row_bytes != 0 && p.out_type == OUT_F16 &&
+            make_map(&map, p.residual, 2, p.m, p.n, p.ld_res, 32, p.store_row_bytes) == PK100_OK)
+            return f(std::true_type{}, map);
+    }
+    return f(std::false_type{}, any);
 }
 
 // CTA pairs (cta_group::2) for the 256-column kernels.  Off by default: on B200 the pair
@@ -155,9 +163,6 @@ static int launch_pair(const pk100_gemm_args& a, const GemmParams& p_in, cudaStr
     constexpr int BlockN = 256;
     using Smem = GemmSmem<BlockN / 2, SwizzleBytes, BlockN, gemm_store_bytes<Epi, BSRC_TMA, BlockN>()>;
     GemmParams p = p_in;
-    constexpr auto kernel = gemm_kernel<Kind, BlockN, SwizzleBytes, Epi, BSRC_TMA, 2>;
-    const cudaError_t granted = pk100_grant_smem<kernel>(Smem::kTotal);
-    if (granted != cudaSuccess) return static_cast<int>(granted);
     constexpr int elem = Kind == KIND_F16 ? 2 : 1;
     CUtensorMap map_a, map_b;
     int rc = make_map(&map_a, a.a, elem, a.m, a.k, a.lda, kBlockM, SwizzleBytes);
@@ -166,8 +171,6 @@ static int launch_pair(const pk100_gemm_args& a, const GemmParams& p_in, cudaStr
     if (rc != PK100_OK) return rc;
     CUtensorMap map_out = map_a;
     p.store_row_bytes = make_out_map<Epi>(&map_out, p);
-    CUtensorMap map_res = map_a;
-    p.res_tma = make_residual_map(&map_res, p);
     const int m_groups = (a.m + 2 * kBlockM - 1) / (2 * kBlockM);
     const int n_tiles = (p.n + BlockN - 1) / BlockN;
     int pairs = cta_budget(a) / 2;
@@ -185,13 +188,18 @@ static int launch_pair(const pk100_gemm_args& a, const GemmParams& p_in, cudaStr
     attr.val.clusterDim.z = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, map_a, map_b, map_out, map_res, p);
-    if (err != cudaSuccess) {
-        cudaGetLastError();
-        return static_cast<int>(err);
-    }
-    pk100_count_launch();
-    return PK100_OK;
+    return with_residual<Epi, BSRC_TMA, BlockN>(p, map_a, [&](auto res_tma, const CUtensorMap& map_res) -> int {
+        constexpr auto kernel = gemm_kernel<Kind, BlockN, SwizzleBytes, Epi, BSRC_TMA, 2, decltype(res_tma)::value>;
+        cudaError_t err = pk100_grant_smem<kernel>(Smem::kTotal);
+        if (err != cudaSuccess) return static_cast<int>(err);
+        err = cudaLaunchKernelEx(&cfg, kernel, map_a, map_b, map_out, map_res, p);
+        if (err != cudaSuccess) {
+            cudaGetLastError();
+            return static_cast<int>(err);
+        }
+        pk100_count_launch();
+        return PK100_OK;
+    });
 }
 
 template <int Kind, int BlockN, int SwizzleBytes, int Epi>
@@ -201,9 +209,6 @@ static int launch(const pk100_gemm_args& a, const GemmParams& p_in, cudaStream_t
     }
     using Smem = GemmSmem<BlockN, SwizzleBytes, BlockN, gemm_store_bytes<Epi, BSRC_TMA, BlockN>()>;
     GemmParams p = p_in;
-    constexpr auto kernel = gemm_kernel<Kind, BlockN, SwizzleBytes, Epi, BSRC_TMA>;
-    const cudaError_t granted = pk100_grant_smem<kernel>(Smem::kTotal);
-    if (granted != cudaSuccess) return static_cast<int>(granted);
     constexpr int elem = Kind == KIND_F16 ? 2 : 1;
     CUtensorMap map_a, map_b;
     int rc = make_map(&map_a, a.a, elem, a.m, a.k, a.lda, kBlockM, SwizzleBytes);
@@ -213,14 +218,17 @@ static int launch(const pk100_gemm_args& a, const GemmParams& p_in, cudaStream_t
     if (rc != PK100_OK) return rc;
     CUtensorMap map_out = map_a;
     if constexpr (gemm_store_bytes<Epi, BSRC_TMA, BlockN>() > 0) p.store_row_bytes = make_out_map<Epi, BlockN>(&map_out, p);
-    CUtensorMap map_res = map_a;
-    p.res_tma = make_residual_map(&map_res, p);
     const int m_tiles = (a.m + kBlockM - 1) / kBlockM;
     const int n_tiles = (p.n + BlockN - 1) / BlockN;
     int ctas = cta_budget(a);
     if (ctas > m_tiles * n_tiles) ctas = m_tiles * n_tiles;
-    pk100_launch_chained(kernel, dim3(ctas), dim3(GemmWarps<BSRC_TMA>::kThreads), Smem::kTotal, stream, map_a, map_b, map_out, map_res, p);
-    return pk100_launch_status();
+    return with_residual<Epi, BSRC_TMA, BlockN>(p, map_a, [&](auto res_tma, const CUtensorMap& map_res) -> int {
+        constexpr auto kernel = gemm_kernel<Kind, BlockN, SwizzleBytes, Epi, BSRC_TMA, 1, decltype(res_tma)::value>;
+        const cudaError_t granted = pk100_grant_smem<kernel>(Smem::kTotal);
+        if (granted != cudaSuccess) return static_cast<int>(granted);
+        pk100_launch_chained(kernel, dim3(ctas), dim3(GemmWarps<BSRC_TMA>::kThreads), Smem::kTotal, stream, map_a, map_b, map_out, map_res, p);
+        return pk100_launch_status();
+    });
 }
 
 // fp16 activations x INT4 group-128 weights, dequantised in shared memory by producer warps.
@@ -230,23 +238,24 @@ static int launch_w4(const pk100_gemm_args& a, const GemmParams& p_in, cudaStrea
     using Smem = GemmSmem<BlockN, 128, BlockN * kMTiles, gemm_store_bytes<EPI_LINEAR, BSRC_W4G128, BlockN>(), kBlockM * kMTiles,
                           gemm_code_bytes<BSRC_W4G128>()>;
     GemmParams p = p_in;
-    constexpr auto kernel = gemm_kernel<KIND_F16, BlockN, 128, EPI_LINEAR, BSRC_W4G128>;
-    const cudaError_t granted = pk100_grant_smem<kernel>(Smem::kTotal);
-    if (granted != cudaSuccess) return static_cast<int>(granted);
     CUtensorMap map_a, map_b;
     int rc = make_map(&map_a, a.a, 2, a.m, a.k, a.lda, kBlockM, 128);
     if (rc != PK100_OK) return rc;
     rc = make_map(&map_b, a.b, 1, a.n, a.k / 2, a.k / 2, BlockN, 128);        // the codes
     if (rc != PK100_OK) return rc;
-    CUtensorMap map_out = map_a, map_res = map_a;
+    CUtensorMap map_out = map_a;
     p.store_row_bytes = make_out_map<EPI_LINEAR, BlockN, BSRC_W4G128>(&map_out, p);
-    p.res_tma = make_residual_map(&map_res, p);
     const int m_items = (a.m + kBlockM * kMTiles - 1) / (kBlockM * kMTiles);   // 256-row work items
     const int n_tiles = (p.n + BlockN - 1) / BlockN;
     int ctas = cta_budget(a);
     if (ctas > m_items * n_tiles) ctas = m_items * n_tiles;
-    pk100_launch_chained(kernel, dim3(ctas), dim3(GemmWarps<BSRC_W4G128>::kThreads), Smem::kTotal, stream, map_a, map_b, map_out, map_res, p);
-    return pk100_launch_status();
+    return with_residual<EPI_LINEAR, BSRC_W4G128, BlockN>(p, map_a, [&](auto res_tma, const CUtensorMap& map_res) -> int {
+        constexpr auto kernel = gemm_kernel<KIND_F16, BlockN, 128, EPI_LINEAR, BSRC_W4G128, 1, decltype(res_tma)::value>;
+        const cudaError_t granted = pk100_grant_smem<kernel>(Smem::kTotal);
+        if (granted != cudaSuccess) return static_cast<int>(granted);
+        pk100_launch_chained(kernel, dim3(ctas), dim3(GemmWarps<BSRC_W4G128>::kThreads), Smem::kTotal, stream, map_a, map_b, map_out, map_res, p);
+        return pk100_launch_status();
+    });
 }
 
 static bool aligned16(const void* ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 15u) == 0; }

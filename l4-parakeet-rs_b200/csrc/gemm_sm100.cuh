@@ -18,8 +18,6 @@
 
 #include <cuda_fp8.h>
 
-#include <type_traits>
-
 #include "ptx_sm100.cuh"
 
 namespace pk100 {
@@ -63,9 +61,6 @@ struct GemmParams {
     // Order of the work items: the column tiles of a row tile follow each other (A is read from HBM once, B stays
     // in L2), or the row tiles of a column tile (B is fetched piece by piece).
     int n_inner;
-    // The residual has a tensor map with the boxes of the output slices: it arrives by TMA in the slice that the
-    // output then leaves from (needs store_row_bytes and fp16 output).
-    int res_tma;
     // B was complete before the chain of dependent launches began: the first stages of the weights are
     // requested before the wait for the kernel in front.
     int b_settled;
@@ -290,11 +285,16 @@ __device__ __forceinline__ int live_k_blocks(uint64_t mask) {
 // Each CTA stages its own 128 rows of A and BlockN/2 rows of B, so a tile costs 2/3 of the
 // operand traffic of two independent 128 x BlockN tiles; the even CTA issues the MMAs, each CTA
 // runs the epilogue of its own 128 accumulator rows.
-template <int Kind, int BlockN, int SwizzleBytes, int Epi, int BSrc, int CtaGroup = 1>
+// ResTma: the residual has a tensor map with the boxes of the output slices and arrives by TMA in the slice that the
+// output then leaves from (needs store_row_bytes and fp16 output).  A kernel of its own: with both forms in one the
+// 256-column linear kernels spilled 36 bytes a thread, which tiles of a short K, bound by their epilogue, showed.  us at
+// N = K = 256 without a residual, one kernel / two: E4M3 at 384 000 rows 84.7 / 81.1, fp16 84.2 / 81.2.
+template <int Kind, int BlockN, int SwizzleBytes, int Epi, int BSrc, int CtaGroup = 1, bool ResTma = false>
 __global__ void __launch_bounds__(GemmWarps<BSrc>::kThreads, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
             const __grid_constant__ CUtensorMap map_out, const __grid_constant__ CUtensorMap map_res,
             const GemmParams p) {
+    static_assert(!ResTma || (Epi == EPI_LINEAR && gemm_store_bytes<Epi, BSrc, BlockN>() > 0), "residual slices: staged linear output");
     static_assert(CtaGroup == 1 || (CtaGroup == 2 && BlockN == 256 && BSrc == BSRC_TMA), "pairs: 256 columns, TMA");
     constexpr int kBRows = BlockN / CtaGroup;               // B rows staged by this CTA
     constexpr int kMTiles = GemmWarps<BSrc>::kMTiles;       // 128-row accumulators per work item
@@ -769,7 +769,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         // rows so / by TMA: FF contract 25.0 / 23.1, fp16 output projection 21.8 / 20.1, pointwise-2 16.9 / 14.6).
         constexpr int kSlices = BSrc == BSRC_W4G128 ? 2 : 1, kSliceCols = kColsPerWarp / kSlices;
         const bool staged = Smem::kStoreBytes > 0 && p.store_row_bytes != 0;
-        const bool res_tma = Epi == EPI_LINEAR && staged && p.res_tma != 0;
         for (; ok && work_item(local, mg, nt); ++local) {
             const int mt = (mg * CtaGroup + static_cast<int>(rank)) * kMTiles + sub;   // this warp's 128-row tile
             const int buf = local & 1;
@@ -813,7 +812,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
             constexpr int kPieces = kColsPerWarp / 16;
             constexpr int kAhead = kPieces < 2 ? kPieces : 2;
             [[maybe_unused]] uint4 res_pre[kAhead][2];
-            const bool has_residual = Epi == EPI_LINEAR && p.residual != nullptr;
+            const bool has_residual = Epi == EPI_LINEAR && !ResTma && p.residual != nullptr;      // read per thread
             uint8_t* const stage = store_smem + ew * (Smem::kStoreBytes / kEpiWarps);
             // first column and row of the warp's slice number sl; false: outside the matrix
             auto slice_at = [&](int sl, int& col0, int& row0) {
@@ -822,7 +821,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                 return row0 < p.m && col0 < (Epi == EPI_GLU ? p.n / 2 : p.n);
             };
             // the store before has read the slice: waited for where the slice is filled, by the residual or by the output
-            // (at the head of the tile the wait was exposed: QKV 22.5 -> 21.6 us at 6144 rows)
+            // (at the head of the tile the wait was exposed: QKV 22.5 -> 21.6 us at 6144 rows; inside the loop over the
+            // linear epilogue's pieces it cost 81.1 / 76.7 and 81.2 / 79.0 us for the products named above)
             auto slice_free = [&]() {
                 if (lane == 0) bulk_wait_read_all();
                 __syncwarp();
@@ -840,10 +840,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                 }
                 __syncwarp();
             };
-            if (res_tma) fetch_slice(0);
+            if constexpr (ResTma) fetch_slice(0);
             auto fetch_residual = [&](uint4 (&dst)[2], int c) {
                 const int col = n0 + part * kColsPerWarp + c * 16;
-                if (has_residual && !res_tma && row < p.m && col < p.n) {
+                if (has_residual && row < p.m && col < p.n) {
                     const uint4* rp = reinterpret_cast<const uint4*>(
                         p.residual + static_cast<size_t>(row) * p.ld_res + col);
                     dst[0] = rp[0];
@@ -881,8 +881,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
             };
 #pragma unroll 1
             for (int sl = 0; sl < kSlices; ++sl) {
-            if (kSlices > 1 && sl > 0 && res_tma) fetch_slice(sl);
-            if (res_tma) {
+            if (Epi == EPI_LINEAR && !ResTma && staged) slice_free();
+            if constexpr (ResTma) {
+                if (kSlices > 1 && sl > 0) fetch_slice(sl);
                 const bool here = mbar_wait_bounded(res_bar + ew, (local * kSlices + sl) & 1, abort_flag);
                 if (!__all_sync(0xffffffffu, here)) {
                     ok = false;
@@ -890,9 +891,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                 }
             }
             if constexpr (Epi == EPI_LINEAR) {
-                // from_slice: the residual comes from the staging slice
-                auto walk = [&](auto from_slice) {
-                constexpr bool kFromSlice = decltype(from_slice)::value;
 #pragma unroll 1
                 for (int cg = sl * (kPieces / kSlices); cg < (sl + 1) * (kPieces / kSlices); cg += kAhead) {
 #pragma unroll
@@ -902,7 +900,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                     uint32_t r[16];
                     tmem_ld_32x16(taddr_base + col_local, r);
                     tmem_ld_wait();
-                    if (!kFromSlice && staged && in_slice == 0) slice_free();
                     const int col = n0 + col_local;
                     if (row < p.m && col < p.n) {
                         // The run-time switches (activation, residual, dead rows) are taken once per
@@ -910,7 +907,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                         // predicated-off SiLU and residual code (22 instructions per element measured).
                         float v[16];
                         uint4 res_raw[2];
-                        if constexpr (kFromSlice) {
+                        if constexpr (ResTma) {
                             res_raw[0] = *reinterpret_cast<const uint4*>(stage_row + (((2 * in_slice) ^ swz) << 4));
                             res_raw[1] = *reinterpret_cast<const uint4*>(stage_row + (((2 * in_slice + 1) ^ swz) << 4));
                         } else {
@@ -939,7 +936,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
 #pragma unroll
                             for (int j = 0; j < 16; ++j) v[j] = fmaxf(v[j], 0.0f);
                         }
-                        if (kFromSlice || has_residual) {
+                        if (ResTma || has_residual) {
                             const __half2* res_h = reinterpret_cast<const __half2*>(res_raw);
 #pragma unroll
                             for (int j = 0; j < 16; j += 2) {
@@ -957,7 +954,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                                 for (int j = 0; j < 16; ++j) v[j] = 0.0f;
                             }
                         }
-                        if (kFromSlice || staged) {
+                        if (ResTma || staged) {
                             stage_piece(stage_row, in_slice, swz, p.out_type, p.out_scale, v);
                         } else {
                             uint8_t* out_row = reinterpret_cast<uint8_t*>(p.out) +
@@ -967,9 +964,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                     }
                 }
                 }
-                };
-                if (Smem::kStoreBytes > 0 && res_tma) walk(std::true_type{});
-                else walk(std::false_type{});
             } else if constexpr (Epi == EPI_GLU) {
                 // accumulator columns [0, BlockN/2) hold values, [BlockN/2, BlockN) their gates
 #pragma unroll 1

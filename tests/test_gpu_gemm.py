@@ -524,3 +524,35 @@ def test_glu_float_output_does_not_depend_on_the_tile_width(pk, cuda, kind, m, n
     assert int(st.item()) == 0
     assert torch.equal(outs[0], outs[2]) and torch.equal(outs[1], outs[3])
     assert torch.equal(outs[0].half(), outs[1]) and bool(outs[0].any())
+
+
+@pytest.mark.parametrize("kind", ["f16", "e4m3", "w4"])
+@pytest.mark.parametrize("m,n,k,ctas", [(1, 64, 128, 0), (129, 128, 128, 1), (300, 256, 256, 1), (300, 1024, 1024, 0)])
+def test_residual_with_outputs_that_are_no_fp16(pk, cuda, kind, m, n, k, ctas):
+    """Only fp16 output takes its residual by TMA.  fp32 output rounds to the fp16 output, 8-bit outputs are the codes of
+    the fp16 output times out_scale; 64-, 128- and 256-column tiles (one CTA forces the wide ones)."""
+    L = pk.lib
+    g = torch.Generator().manual_seed(m + n)
+    w = (torch.randn((n, k), generator=g) * 0.05).half().to(cuda)
+    x = torch.randn((m, k), generator=g).half().to(cuda)
+    kw = dict(residual=torch.randn((m, n + 8), generator=g).half().to(cuda)[:, :n], alpha=0.5, out_scale=16.0, max_ctas=ctas, n=n)
+    a, b, kid = x, w, L.KIND_F16
+    if kind == "w4":
+        b, kw["b_group_scales"] = pk.ops.pack_weight_rows(w, L.PACK_S4_G128)
+        kid = L.KIND_F16_W4G128
+    elif kind == "e4m3":
+        b, kw["col_scales"] = pk.ops.pack_weight_rows(w, L.PACK_E4M3)
+        a, kw["row_scales"] = pk.ops.pack_weight_rows(x, L.PACK_E4M3)
+        kid = L.KIND_E4M3
+    st = _status(cuda)
+    outs = {}
+    for code, dtype in ((L.OUT_F16, torch.float16), (L.OUT_F32, torch.float32), (L.OUT_E4M3, torch.uint8), (L.OUT_S8, torch.int8)):
+        outs[code] = torch.zeros((m, n), dtype=dtype, device=cuda)
+        pk.ops.gemm(a, b, kind=kid, out=outs[code], out_type=code, status=st, **kw)
+    torch.cuda.synchronize()
+    assert int(st.item()) == 0
+    half = outs[L.OUT_F16]
+    scaled = half.float() * 16.0
+    assert torch.equal(outs[L.OUT_F32].half(), half) and bool(half.any())
+    assert torch.equal(outs[L.OUT_E4M3], scaled.to(torch.float8_e4m3fn).view(torch.uint8))
+    assert torch.equal(outs[L.OUT_S8], scaled.round().clamp(-127, 127).to(torch.int8))
