@@ -26,9 +26,14 @@ def _ptr(t):
     return 0 if t is None else t.data_ptr()
 
 
+# torch.cuda.current_stream().cuda_stream without the Stream object around it, where torch has it (a private name)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream():
-    # torch.cuda.current_stream().cuda_stream without the Stream object around it
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    if _raw_stream is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(torch.cuda.current_device())
 
 
 def _need(t, dtype=None):

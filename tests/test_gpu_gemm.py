@@ -556,3 +556,18 @@ def test_residual_with_outputs_that_are_no_fp16(pk, cuda, kind, m, n, k, ctas):
     assert torch.equal(outs[L.OUT_F32].half(), half) and bool(half.any())
     assert torch.equal(outs[L.OUT_E4M3], scaled.to(torch.float8_e4m3fn).view(torch.uint8))
     assert torch.equal(outs[L.OUT_S8], scaled.round().clamp(-127, 127).to(torch.int8))
+
+
+def test_stream_without_the_private_call(pk, cuda, monkeypatch):
+    """The current stream's handle comes from torch's public call where the private one is missing."""
+    x, w = torch.randn((8, 128), device=cuda).half(), torch.randn((32, 128), device=cuda).half()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    outs = []
+    with torch.cuda.stream(side):
+        for raw in (pk.ops._raw_stream, None):
+            monkeypatch.setattr(pk.ops, "_raw_stream", raw)
+            assert pk.ops._stream() == side.cuda_stream
+            outs.append(pk.ops.gemm(x, w, out=torch.zeros((8, 32), dtype=torch.float16, device=cuda), kind=pk.lib.KIND_F16))
+    side.synchronize()
+    assert torch.equal(outs[0], outs[1]) and bool(outs[0].any())
