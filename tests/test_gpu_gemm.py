@@ -571,3 +571,37 @@ def test_stream_without_the_private_call(pk, cuda, monkeypatch):
             outs.append(pk.ops.gemm(x, w, out=torch.zeros((8, 32), dtype=torch.float16, device=cuda), kind=pk.lib.KIND_F16))
     side.synchronize()
     assert torch.equal(outs[0], outs[1]) and bool(outs[0].any())
+
+
+@pytest.mark.parametrize("row_scale,tau,report", [(0.01, 0.8, 0), (0.05, 4.0, 8)])
+@pytest.mark.parametrize("rows", [1, 129, 300])
+@pytest.mark.parametrize("n", [64, 192, 320, 640])
+def test_sparse_out_tile_widths_agree_at_ragged_columns(pk, cuda, n, rows, row_scale, tau, report):
+    """Columns that leave the last 256-column tile ragged: 64-, 128- (where they divide n) and 256-column tiles give the
+    same codes, flags and statistics, nothing behind them, and the same clamp report (status 8) whichever column slices
+    share the sparsity tile."""
+    L = pk.lib
+    g = torch.Generator().manual_seed(rows + n)
+    q8 = torch.randint(0, 120, (rows, 1024), generator=g, dtype=torch.uint8).to(cuda)
+    b, scales = pk.ops.pack_weight_rows((torch.randn((n, 1024), generator=g) * 0.02).half().to(cuda), L.PACK_E4M3)
+    tiles = (rows + 127) // 128
+    results = []
+    for ctas in [0, 1] + ([tiles * (n // 128)] if n % 128 == 0 else []):
+        out = torch.full((rows + 1, n + 16), 55, dtype=torch.int8, device=cuda)
+        keep = torch.full((tiles + 1, n // 64), 9, dtype=torch.uint8, device=cuda)
+        stats = torch.full((tiles + 1, n // 64), -1.0, device=cuda)
+        st = _status(cuda)
+        pk.ops.gemm(q8, b, kind=L.KIND_E4M3, epilogue=L.EPI_SPARSE_OUT, row_scale=row_scale, col_scales=scales, out=out[:rows],
+                    out_type=L.OUT_S8, out_scale=32.0, tau=tau, keep_out=keep, stats_out=stats, status=st, max_ctas=ctas)
+        torch.cuda.synchronize()
+        assert bool((out[rows] == 55).all()) and bool((out[:, n:] == 55).all())
+        assert bool((keep[tiles] == 9).all()) and bool((stats[tiles] == -1.0).all()) and bool((stats[:tiles] >= 0.0).all())
+        results.append((out, keep, stats))
+        live = keep[:tiles].bool()
+        assert torch.equal(live, stats[:tiles] >= tau)
+        clipped = bool((stats[:tiles][live] * 32.0 > 127.0).any())
+        assert int(st.item()) == (8 if clipped else 0) and (report == 8 or not clipped)
+    for other in results[1:]:
+        for a, b_ in zip(results[0], other):
+            assert torch.equal(a, b_)
+    assert report == 0 or rows == 1 or clipped
