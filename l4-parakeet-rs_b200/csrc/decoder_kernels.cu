@@ -1413,14 +1413,12 @@ extern "C" int pk100_tdt_decode_exchange(void* stream_v, const pk100_decoder_wei
 
 namespace {
 
-// Can this device run a 16-CTA cluster of the cluster decoder?  Asked once per device and
-// kernel variant (one or two LSTM layers).
 // Calls f with the kernel for (layers, numerics, utterances of the call) and its threads and its shared-memory bytes.
 template <typename F>
 auto with_cluster_kernel(int layers, bool cache, int utterances, F&& f) {
 #define PK_PICK(L, C, N) return f(tdt_cluster_kernel<L, C, N>, cl_threads(N), static_cast<int>(sizeof(CSmem<L, C, N>)))
-// (two utterances: the form for up to two with two layers, the one for up to four with one: us per round 6.7 against 6.9
-// and 7.1 against 7.1 for the two-layer numerics, 5.7 against 5.4 and 3.7 against 3.5 for the one-layer ones)
+// Two utterances: the form for up to two with two layers, the one for up to four with one.  us per round, form for two /
+// for four: two layers 7.07 / 7.20 with INT8 codes, 7.08 / 7.12 in fp16 (750 frames each); one layer 5.7 / 5.4 and 3.7 / 3.5.
 #define PK_SIZES(L, C)                                           \
     do {                                                         \
         if (utterances <= 1) PK_PICK(L, C, 1);                   \

@@ -112,8 +112,9 @@ struct GemmSmem {
     static constexpr int kSchedOffset = 64 * 8 + 16 + 32 * EpiCols + 64 * 4;
     static constexpr int kTailBytes = kSchedOffset + kSchedTiles * (8 + 2);
     static constexpr int kStoreBytes = StoreBytes, kCodeBytes = CodeBytes;
-    // 227 KB per CTA, less the tail, the output staging and 1 KB of alignment slack; the
-    // pipeline is not depth-sensitive (2 and 4 stages measured alike), so staging comes first
+    // 227 KB per CTA, less the tail, the output staging and 1 KB of alignment slack.  Staging comes first: 256-column
+    // tiles of many rows measured alike with 2 and 4 stages.  (Launches of one wave are bound by the round trips of this
+    // ring instead, so the host gives them narrower tiles and with them more stages.)
     static constexpr int kBudget = 227 * 1024 - 1024 - kTailBytes - kStoreBytes - kCodeBytes;
     static constexpr int kStagesRaw = kBudget / kStageBytes;
     static constexpr int kStages = kStagesRaw > 8 ? 8 : kStagesRaw;

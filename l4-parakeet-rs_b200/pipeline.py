@@ -334,9 +334,9 @@ class PipelineEngine:
         tokens only when its buffers are needed again or the newest batch has been queued.  Steady
         state per batch: the larger of the (slowed) encode and the decoder-cluster time of a batch
         divided by the clusters in flight, instead of encode + longest chain.  Measured for batches of
-        8 x 60 s: one lockstep cluster per batch and four batches in flight (the defaults) give 10.8 ms per
-        batch, two clusters and three batches 12.8 ms, four clusters and two batches 16.4 ms; the same
-        batch on its own takes 30.7 ms."""
+        8 x 60 s: one lockstep cluster per batch and four batches in flight (the defaults) give 8.7 ms per
+        batch, the same batch on its own takes 18.8 ms.  (With earlier kernels 10.8 and 30.7 ms, and two clusters
+        with three batches 12.8 ms, four clusters with two 16.4 ms.)"""
         depth = max(2, int(depth))
         if not hasattr(self, "_extra_slots"):
             self._extra_slots, self._collect_streams, self._slot_status = [], [], []

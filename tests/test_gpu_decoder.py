@@ -306,9 +306,9 @@ def test_rounds_whose_scores_are_all_nan_decode_as_blank(pk, cuda, kernel):
 @pytest.mark.parametrize("cache", ["fp16", "int8"])
 @pytest.mark.parametrize("layers", [1, 2])
 def test_team_sizes_give_the_tokens_of_single_utterances(pk, cuda, layers, cache):
-    """The cluster kernel serves an utterance with 4, 2 or 1 control warps and has variants for up to 4
-    and up to 8 utterances: every batch size decodes like its utterances alone (ragged lengths, one of
-    them empty), with random blanks in between."""
+    """The cluster kernel serves one or two utterances with five control warps in common and more with a warp each, in
+    variants for up to 1, 2 (two layers), 4 and 8 utterances: every batch size decodes like its utterances
+    alone (ragged lengths, one of them empty), with random blanks in between."""
     w = pk.synth.decoder_weights(21, layers)
     w["b_joint"] = w["b_joint"].copy()
     w["b_joint"][1024] += 0.8                        # blanks often enough to cover rounds without an LSTM step
